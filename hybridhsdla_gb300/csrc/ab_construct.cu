@@ -234,6 +234,25 @@ __global__ void __launch_bounds__(kThreads) construct_ab_kernel(DevSystem sys, c
                 col[idx] = out;
             }
             // phase-free per-type rows M_t = [A_t; B_t] / e^{i 2pi K.tau} (shared by every atom of type t)
+            if (ent.R) {
+                double *rcol = ent.R + ldm * gi;
+                const int nrm = twoL * nt;
+                for (int idx = threadIdx.x; idx < nrm; idx += blockDim.x) {
+                    const int t = idx / twoL;
+                    const int r = idx - t * twoL;
+                    const bool isB = r >= L;
+                    const int lm = isB ? r - L : r;
+                    const int l = l_of[lm];
+                    double out = 0.0;
+                    if (l <= sys.type_lmax[t]) {
+                        const int tl = t * nl + l, l0 = l * (l + 1);
+                        const double c = sys.vol_prefac * sys.inv_w[tl];
+                        const double y = lm >= l0 ? ylm[lm].x : -ylm[2 * l0 - lm].y;
+                        out = (y * c) * (isB ? bu[tl] : au[tl]);
+                    }
+                    rcol[idx] = out;
+                }
+            }
             if (M) {
                 double2 *mcol = M + ldm * gi;
                 const int nrm = twoL * nt;
@@ -375,6 +394,26 @@ __global__ void __launch_bounds__(kThreads) construct_rows_kernel(DevSystem sys,
             for (int c = 0; c < ncols; ++c) {
                 const int64_t gc = col0 + c;
                 const KEntry &ent = tab.e[entry_of(tab, gc)];
+                if (ent.R) {
+                    // the real form: Re of the rows m >= 0, Im of the rows m > 0 in place of -m
+                    double *rcol = ent.R + ldm * (gc - ent.col_begin);
+                    for (int idx = threadIdx.x; idx < twoL * nt; idx += blockDim.x) {
+                        const int t = idx / twoL;
+                        if (sys.num_rots > 0 && sys.type_rot[t] != rho) continue;
+                        const int r = idx - t * twoL;
+                        const bool isB = r >= L;
+                        const int lm = isB ? r - L : r;
+                        const int l = l_of[lm];
+                        double out = 0.0;
+                        if (l <= sys.type_lmax[t]) {
+                            const int tl = t * nl + l, l0 = l * (l + 1);
+                            const double y = lm >= l0 ? ylm[c * L + lm].x : -ylm[c * L + 2 * l0 - lm].y;
+                            out = (y * cf[tl]) * (isB ? bu[c * tnl + tl] : au[c * tnl + tl]);
+                        }
+                        rcol[idx] = out;
+                    }
+                    continue;
+                }
                 if (!ent.M) continue;
                 double2 *mcol = ent.M + ldm * (gc - ent.col_begin);
                 for (int idx = threadIdx.x; idx < twoL * nt; idx += blockDim.x) {
@@ -499,6 +538,53 @@ __global__ void __launch_bounds__(kTfThreads) tfull_kernel(const double2 *__rest
     }
 }
 
+// T' = V^H T V of every type: rows and columns (l, m > 0) and (l, -m) of T, whose matching rows
+// are p + i q and (-1)^m (p - i q), become those of the real rows p and q; four entries of T per
+// entry of T', added in an order that keeps T' Hermitian.
+__global__ void __launch_bounds__(kTfThreads) treal_kernel(const double2 *__restrict__ tf, int L, double *__restrict__ tr) {
+    const int n = 2 * L, t = blockIdx.y;
+    const double2 *T = tf + (int64_t)t * n * n;
+    double *out = tr + (int64_t)t * 2 * n * n;
+    // the indices of rows (l, |m|) and (l, -|m|), m's sign and parity of row x of a type
+    auto split = [&](int x, int &p, int &q, int &m) {
+        const int h = x >= L ? L : 0, lm = x - h;
+        int l = (int)sqrt((double)lm);
+        while (l * l > lm) --l;
+        while ((l + 1) * (l + 1) <= lm) ++l;
+        m = lm - l * (l + 1);
+        const int a = m < 0 ? -m : m;
+        p = h + l * (l + 1) + a;
+        q = h + l * (l + 1) - a;
+    };
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < (int64_t)n * n; e += (int64_t)gridDim.x * blockDim.x) {
+        const int k = (int)(e % n), r = (int)(e / n);
+        int rp, rq, rm, cp, cq, cm;
+        split(r, rp, rq, rm);
+        split(k, cp, cq, cm);
+        const double sr = (rm & 1) ? -1.0 : 1.0, sc = (cm & 1) ? -1.0 : 1.0;
+        auto at = [&](int a, int b, double s) {
+            const double2 v = T[a + (int64_t)n * b];
+            return make_double2(s * v.x, s * v.y);
+        };
+        const double2 z = make_double2(0.0, 0.0);
+        const double2 t1 = at(rp, cp, 1.0);
+        const double2 t2 = rm && cm ? at(rq, cq, sr * sc) : z;
+        const double2 t3 = cm ? at(rp, cq, sc) : z, t4 = rm ? at(rq, cp, sr) : z;
+        auto add = [](double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); };
+        auto neg = [](double2 a) { return make_double2(-a.x, -a.y); };
+        const bool qr = rm < 0, qc = cm < 0;
+        double2 v;
+        if (!qr && !qc) v = add(add(t1, t2), add(t3, t4));
+        else if (qr && qc) v = add(add(t1, t2), neg(add(t3, t4)));
+        else {
+            const double2 d = add(add(t1, neg(t2)), qc ? add(t4, neg(t3)) : add(t3, neg(t4)));
+            v = qc ? make_double2(-d.y, d.x) : make_double2(d.y, -d.x);     // i d, -i d
+        }
+        out[k + (int64_t)n * r] = v.x;
+        out[k + (int64_t)n * (n + r)] = v.y;
+    }
+}
+
 __global__ void sf_phase_kernel(const double *pos, int na, int h0, int h1, int h2, int e0, int e1, int e2,
                                 double2 *ph) {
     const int64_t n0 = (int64_t)na * e0, n1 = (int64_t)na * e1, total = n0 + n1 + (int64_t)na * e2;
@@ -531,6 +617,14 @@ cudaError_t launch_tfull(const double2 *aa, const double2 *ab, const double2 *bb
     return cudaGetLastError();
 }
 
+cudaError_t launch_treal(const double2 *tf, int nt, int L, double *tr, cudaStream_t st) {
+    if (nt <= 0 || L <= 0) return cudaSuccess;
+    const int64_t nn = 4 * (int64_t)L * L;
+    const dim3 grid((unsigned)std::min<int64_t>((nn + kTfThreads - 1) / kTfThreads, 128), (unsigned)nt);
+    treal_kernel<<<grid, kTfThreads, 0, st>>>(tf, L, tr);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_sf_phases(const double *pos, int na, const int *half, const int *ext, double2 *ph, cudaStream_t st) {
     const int64_t total = (int64_t)na * (ext[0] + ext[1] + ext[2]);
     if (total <= 0) return cudaSuccess;
@@ -551,7 +645,7 @@ cudaError_t launch_apply_phase(const DevSystem &sys, const DevKpoint &kp, const 
                                double2 *X, int64_t ldx, cudaStream_t st) {
     KTable tab;
     tab.nk = 1; tab.ldc = ldx; tab.ldm = ldz; tab.total_cols = kp.n_g;
-    tab.e[0] = KEntry{kp, nullptr, nullptr, Z, X, 0};
+    tab.e[0] = KEntry{kp, nullptr, nullptr, Z, X, 0, nullptr};
     return launch_apply_phase_multi(sys, tab, st);
 }
 
@@ -559,14 +653,14 @@ cudaError_t launch_construct_ab(const DevSystem &sys, const DevKpoint &kp, doubl
                                 cudaStream_t st, double2 *M, int64_t ldm) {
     KTable tab;
     tab.nk = 1; tab.ldc = ldc; tab.ldm = ldm; tab.total_cols = kp.n_g;
-    tab.e[0] = KEntry{kp, C, M, nullptr, nullptr, 0};
+    tab.e[0] = KEntry{kp, C, M, nullptr, nullptr, 0, nullptr};
     return launch_construct_ab_multi(sys, tab, st);
 }
 
 cudaError_t launch_construct_ab_multi(const DevSystem &sys, const KTable &tab, cudaStream_t st) {
     if (tab.total_cols <= 0) return cudaSuccess;
     bool anyM = false, anyC = false;
-    for (int k = 0; k < tab.nk; ++k) { anyM = anyM || tab.e[k].M; anyC = anyC || tab.e[k].C; }
+    for (int k = 0; k < tab.nk; ++k) { anyM = anyM || tab.e[k].M || tab.e[k].R; anyC = anyC || tab.e[k].C; }
     const bool rot = sys.atom_rotmat != nullptr;
     const size_t smem_rows = rows_kernel_smem(sys.L, sys.max_lmax, sys.num_types);
     // (the column-per-CTA kernel below for many types at a high lmax, whose tables do not fit;

@@ -67,6 +67,8 @@ struct KEntry {
     const double2 *Z;           // per-type product, ld KTable::ldm (phase expansion input)
     double2 *X;                 // per-atom output, ld KTable::ldc (phase expansion output)
     int64_t col_begin;          // first global column of this k-point
+    double *R;                  // real per-type rows (2 L nt) x n_g, ld KTable::ldm, or nullptr: row
+                                // (l, m >= 0) of M's real part, row (l, -m) of row (l, m)'s imaginary part
 };
 struct KTable {
     int nk = 0;
@@ -94,6 +96,9 @@ cudaError_t launch_construct_ab(const DevSystem &sys, const DevKpoint &kp, doubl
 // for T_BB (doubles as bit patterns).
 cudaError_t launch_tfull(const double2 *aa, const double2 *ab, const double2 *bb, int nt, int L, double2 *tf,
                          unsigned long long *stats, cudaStream_t st);
+// The real form of the T blocks (see real_products.cu): tr holds per type 4L columns of 2L values,
+// column r the row r of Re T', column 2L + r the row r of Im T', T' = V^H T V with T from launch_tfull.
+cudaError_t launch_treal(const double2 *tf, int nt, int L, double *tr, cudaStream_t st);
 // Per-atom structure phases along each axis, ph[o] = e^{i 2pi (i - half_c) pos[3 j + c]} with o
 // running over c, then atom j, then i in [0, ext_c).
 cudaError_t launch_sf_phases(const double *pos, int na, const int *half, const int *ext, double2 *ph, cudaStream_t st);
@@ -121,6 +126,10 @@ cudaError_t launch_fp64_jobs(const Fp64Job *d_jobs, int num_jobs, int64_t total_
 // S, H (ld ldo); g the k-point's G-vectors [n][3] on the device.
 struct SfEntry {
     const double2 *PS = nullptr, *PH = nullptr;   // per-type products, type slot b at + b pstride
+    // or (PS and PH NULL) as fixed-point numbers: S, and the real and imaginary parts of H, element
+    // (r, c) times 2^(el[r] + er[c] - 8 - frac) with er = ers for S and erh for H
+    const long long *RS = nullptr, *RHr = nullptr, *RHi = nullptr;
+    const int32_t *el = nullptr, *ers = nullptr, *erh = nullptr;
     double2 *S = nullptr, *H = nullptr;
     // what a combine that is not the first adds to (NULL: S and H themselves, ldo)
     const double2 *Si = nullptr, *Hi = nullptr;
@@ -135,6 +144,7 @@ struct SfTab {
     int nk = 0, type = 0, ntypes = 1;             // the batch: types [type, type + ntypes) in slots
     int slot0 = 0;                                // slot0, slot0 + 1, ...
     int64_t col0 = 0, col1 = INT64_MAX;           // the columns combined (of every entry)
+    int frac = 0;                                 // fixed-point products: their fraction bits
     int64_t xrow1 = 0;                            // rows below it go to the entries' Sx, Hx when set
 
     int dx = 0, dy = 0, dz = 0, ny = 0, nz = 0;   // box offsets (half widths) and extents

@@ -134,6 +134,9 @@ struct hsdla_plan {
     const unsigned long long *tcheck_host = nullptr;
     std::vector<int32_t> tcheck_class_type;
     double *wt = nullptr;
+    double *wt_real = nullptr;       // the same for the real rows (2 wt where m != 0)
+    double *TR = nullptr;            // real T blocks [nt][4L][2L] (Ozaki)
+    bool real = false;               // the structure-factor form runs on real rows (real_products.cu)
     double2 *sf_tab = nullptr;
     SfTab sf_dims{};                 // box extents and offsets (entries filled per group)
     int tbatch = 1;                  // types whose products are combined into S and H in one pass
@@ -804,12 +807,14 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     // grouped by type and the table itself over the box of G-vector differences g_col - g_row
     const char *sf_env = getenv("HSDLA_SF");
     pl->sf = pl->hoist && !(sf_env && strtol(sf_env, nullptr, 10) == 0);
+    pl->real = pl->sf && pl->opts.precision == HSDLA_PREC_OZAKI_FP8;
     int half[3] = {0, 0, 0}, ext[3] = {1, 1, 1};
     if (pl->sf) {
         for (int i = 0; i < nk; ++i)
             for (int64_t q = 0; q < kpts[i].n_g; ++q)
                 for (int c = 0; c < 3; ++c) half[c] = std::max(half[c], 2 * std::abs(kpts[i].g[3 * q + c]));
         for (int c = 0; c < 3; ++c) ext[c] = 2 * half[c] + 1;
+        add(sizeof(double) * 2 * L * nt);
         add(sizeof(double) * 2 * L * nt);
         add(sizeof(int32_t) * (na + nt + 1));
     }
@@ -822,6 +827,7 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
         add(sizeof(double2) * (int64_t)na * (ext[0] + ext[1] + ext[2]));
         add(sizeof(double2) * (int64_t)nt * ext[0] * ext[1] * ext[2]);
     }
+    if (pl->real) add(sizeof(double) * 2 * tf_elems);
     const double p_tables = pms();
     rc = ctx_malloc(ctx, &pl->tables, bytes);
     if (rc) { delete pl; return rc; }
@@ -901,6 +907,13 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
                     wt[(size_t)2 * L * t + L + lm] = (l <= s->type_lmax[t]) ? s->type_dE_u_norm[t * nl + l] : 0.0;
                 }
         pl->wt = (double *)put(wt.data(), sizeof(double) * wt.size());
+        // the rows (l, m) and (l, -m) of a real pair carry both complex rows' weight
+        for (int t = 0; t < nt; ++t)
+            for (int h = 0; h < 2; ++h)
+                for (int l = 0; l < nl; ++l)
+                    for (int lm = l * l; lm < (l + 1) * (l + 1); ++lm)
+                        if (lm != l * (l + 1)) wt[(size_t)2 * L * t + (size_t)h * L + lm] *= 2.0;
+        pl->wt_real = (double *)put(wt.data(), sizeof(double) * wt.size());
         std::vector<int32_t> ord;
         std::vector<int32_t> tb(nt + 1, 0);
         for (int t = 0; t < nt; ++t) {
@@ -928,6 +941,7 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
         d_ex = (double2 *)dev_only(sizeof(double2) * (int64_t)na * (ext[0] + ext[1] + ext[2]));
         pl->sf_tab = (double2 *)dev_only(sizeof(double2) * (int64_t)nt * ext[0] * ext[1] * ext[2]);
     }
+    if (pl->real) pl->TR = (double *)dev_only(sizeof(double) * 2 * tf_elems);
     std::vector<unsigned long long> tstats((size_t)5 * nt, 0);
     {
         // the pending copies as one byte range split evenly over up to four threads (one copying
@@ -962,6 +976,7 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     cudaError_t e = cudaMemcpyAsync(pl->tables, stage, upload_bytes, cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(d_stats, 0, sizeof(unsigned long long) * 5 * nt, ctx->stream);
     if (e == cudaSuccess) e = launch_tfull(d_taa, d_tab, d_tbb, nt, L, pl->Tfull, d_stats, ctx->stream);
+    if (e == cudaSuccess && pl->real) e = launch_treal(pl->Tfull, nt, L, pl->TR, ctx->stream);
     if (e == cudaSuccess && pl->sf) e = launch_sf_phases(D.atom_pos, na, half, ext, d_ex, ctx->stream);
     if (e == cudaSuccess && pl->sf)
         e = launch_sf_table(d_ex, d_ex + (size_t)na * ext[0], d_ex + (size_t)na * (ext[0] + ext[1]), d_order,
@@ -1011,6 +1026,9 @@ int64_t kpoint_fp64_bytes(const hsdla_plan *pl, int64_t G) {
     const int64_t K = pl->twoLa, ldm = 2 * (int64_t)pl->L * pl->nt;
     auto r = [](int64_t x) { return (x + 1023) / 1024 * 1024; };        // each buffer is 1 KB aligned
     // structure-factor form: M, Z and the two products of each type of a combine batch (no C, no X)
+    if (pl->real)       // the same on real rows: R, Z' (two parts) and three products
+        return r(ldm * G * (int64_t)sizeof(double)) + r(2 * ldm * G * (int64_t)sizeof(double)) +
+               3 * r(pl->tbatch * G * G * (int64_t)sizeof(double));
     if (pl->sf) return 2 * r(ldm * G * (int64_t)sizeof(double2)) + 2 * r(pl->tbatch * G * G * (int64_t)sizeof(double2));
     const int64_t nCX = pl->opts.precision == HSDLA_PREC_FP64 ? 2 : 1;   // FP64 keeps C and X apart
     int64_t b = nCX * r(K * G * (int64_t)sizeof(double2));
@@ -1032,8 +1050,7 @@ int64_t group_persist_bytes(const hsdla_plan *pl, const std::vector<int> &kidx) 
     std::vector<int64_t> G;
     for (int i : kidx) G.push_back(pl->kps[i].n_g);
     if (pl->opts.precision == HSDLA_PREC_OZAKI_FP8)
-        return ozaki_group_persist_bytes(pl->oz.num_slices, 2 * (int64_t)pl->L, pl->na, pl->nt, G,
-                                         pl->sf ? std::max(pl->panels, pl->nt) : pl->panels);
+        return ozaki_group_persist_bytes(pl->oz.num_slices, 2 * (int64_t)pl->L, pl->na, pl->nt, G, pl->panels, pl->sf);
     // the FP64 group keeps two job tables, each rounded up to 1 KiB: the T applications (one per
     // type when hoisted, else one per atom, per k-point) and the S/H products (two per type in
     // the structure-factor form, else two, per k-point)
@@ -1152,7 +1169,9 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
         g.persist_bytes = group_persist_bytes(pl, g.kidx);
         int rcp = ctx_malloc(ctx, &g.persist, g.persist_bytes);
         if (rcp) return rcp;
-        g.ev_dom.assign(pl->sf ? 2 * pl->nt : 2, nullptr);
+        // one pair per S/H product launch: FP64 runs one per type, Ozaki one per combine batch
+        // (streamed host output adds pairs for its column blocks)
+        g.ev_dom.assign(pl->real ? 2 * std::max(2, (pl->nt + pl->tbatch - 1) / pl->tbatch) : pl->sf ? 2 * pl->nt : 2, nullptr);
         for (auto &e : g.ev_dom) CUDA_TRY(ctx, cudaEventCreate(&e));
         char *pp = reinterpret_cast<char *>(g.persist);
         auto keep = [&](int64_t bytes) { char *r = pp; pp += (bytes + 1023) / 1024 * 1024; return r; };
@@ -1177,6 +1196,27 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
                           ? reinterpret_cast<double2 *>(take(K * G * (int64_t)sizeof(double2)))
                           : e.C;   // Ozaki: X reuses C once C is sliced
             }
+            OzKBufs b;
+            b.G = G;
+            if (pl->real) {
+                b.R = reinterpret_cast<double *>(take(ldm * G * (int64_t)sizeof(double)));
+                b.ZR = reinterpret_cast<long long *>(take(2 * ldm * G * (int64_t)sizeof(long long)));
+                b.pstride = G * G;
+                const int64_t pb = pl->tbatch * G * G * (int64_t)sizeof(double);
+                b.RS = reinterpret_cast<long long *>(take(pb));
+                b.RHr = reinterpret_cast<long long *>(take(pb));
+                b.RHi = reinterpret_cast<long long *>(take(pb));
+                e.R = b.R;
+                e.M = nullptr;
+                e.Z = nullptr;
+                SfEntry &f = g.sft.e[q];
+                f = SfEntry();
+                f.RS = b.RS; f.RHr = b.RHr; f.RHi = b.RHi;
+                f.ldp = G; f.n = G; f.pstride = b.pstride; f.g = pk.dk.g;
+                kb.push_back(b);
+                continue;
+            }
+            e.R = nullptr;
             e.M = pl->hoist ? reinterpret_cast<double2 *>(take(ldm * G * (int64_t)sizeof(double2))) : nullptr;
             double2 *Z = pl->hoist ? reinterpret_cast<double2 *>(take(ldm * G * (int64_t)sizeof(double2))) : nullptr;
             e.Z = Z;
@@ -1187,13 +1227,7 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
                 f.PH = reinterpret_cast<double2 *>(take(pl->tbatch * G * G * (int64_t)sizeof(double2)));
                 f.ldp = G; f.n = G; f.pstride = G * G; f.g = pk.dk.g;
             }
-            OzKBufs b;
-            b.CX = e.C; b.M = e.M; b.Z = Z; b.G = G;
-            if (pl->sf) {
-                b.PS = const_cast<double2 *>(g.sft.e[q].PS);
-                b.PH = const_cast<double2 *>(g.sft.e[q].PH);
-                b.pstride = g.sft.e[q].pstride;
-            }
+            b.CX = e.C; b.M = e.M; b.Z = Z;
             kb.push_back(b);
         }
         kt.total_cols = col;
@@ -1208,17 +1242,11 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
             d.twoL = twoL; d.na = pl->na; d.nt = pl->nt; d.hoist = pl->hoist;
             d.w = pl->w; d.Tfull = pl->Tfull; d.atom_type = pl->atom_type.data();
             d.panels = pl->panels;
-            d.sf = pl->sf; d.wt = pl->wt; d.sf_tab = pl->sf_tab; d.tbatch = pl->tbatch;
+            d.sf = pl->sf; d.wt = pl->wt_real; d.TR = pl->TR; d.sf_tab = pl->sf_tab; d.tbatch = pl->tbatch;
             char *oz_ws = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(p) + 1023) & ~uintptr_t(1023));
             int rc = ozaki_group_prepare(pl->oz, d, kb, oz_ws, g.persist, st, &g.oz);
             if (rc) return set_err(ctx, rc, "group set-up failed: %s", ozaki_last_error());
-            // streamed host output runs the S/H products as one launch per column block: an event
-            // pair for each, where there are more blocks than types
-            const size_t nev = 2 * (size_t)ozaki_group_output_blocks(g.oz);
-            while (pl->sf && g.ev_dom.size() < nev) {
-                g.ev_dom.push_back(nullptr);
-                CUDA_TRY(ctx, cudaEventCreate(&g.ev_dom.back()));
-            }
+            if (pl->real) ozaki_group_sf_exponents(g.oz, g.sft);
             g.ev_t.assign(2 * ozaki_group_tapply_events(g.oz), nullptr);
             for (auto &e : g.ev_t) CUDA_TRY(ctx, cudaEventCreate(&e));
         } else {
@@ -1362,7 +1390,8 @@ void run_groups_flop_one(const hsdla_plan *pl, const hsdla_plan::Group &g, doubl
     for (int q = 0; q < g.ktab.nk; ++q) {
         const double G = (double)g.ktab.e[q].kp.n_g;
         const double lower = 4.0 * G * (G + 1.0) * Klen;
-        *dom_flop += 2.0 * lower * (g.oz ? sl * (sl + 1) / 2 : 1.0);
+        // (the real form: three real products where the complex form has eight)
+        *dom_flop += 2.0 * lower * (g.oz ? sl * (sl + 1) / 2 : 1.0) * (pl->real ? 0.375 : 1.0);
     }
 }
 
@@ -1473,6 +1502,12 @@ int run_groups(hsdla_plan *pl, cudaStream_t st, bool timed, float *ms_ab, float 
             const bool streamed = defer && pl->dl->direct && ozaki_group_streamable(g.oz);
             SfTab host_tab{};
             if (streamed) host_tab = host_output_tab(pl, g);
+            // streamed host output runs the products as one launch per column block: an event pair
+            // for each
+            while (streamed && g.ev_dom.size() < 2 * (size_t)ozaki_group_output_blocks(g.oz)) {
+                g.ev_dom.push_back(nullptr);
+                CUDA_TRY(ctx, cudaEventCreate(&g.ev_dom.back()));
+            }
             const int rc = ozaki_group_run(g.oz, pl->dsys, g.ktab, st, g.ev_dom.data(), (int)g.ev_dom.size(), &nl,
                                            defer, timed ? g.ev_t.data() : nullptr, timed ? (int)g.ev_t.size() : 0,
                                            streamed ? &host_tab : nullptr);

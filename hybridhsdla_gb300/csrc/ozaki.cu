@@ -42,6 +42,8 @@
 #include <vector>
 
 #include "ozaki.cuh"
+#include "ptx.cuh"
+#include "real_products.cuh"
 
 namespace hsdla {
 
@@ -60,7 +62,6 @@ constexpr int kStages = 3;
 constexpr int kStageBytes = 4 * kTileM * kKBlock;   // Ar, Ai, Br, Bi boxes
 constexpr int kThreads = 320;        // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue
 constexpr int kEpiWarps = 8;         // two per TMEM lane quadrant, each drains half the columns
-constexpr long long kWaitCycles = 2000000000LL;    // ~1 s at 2 GHz
 constexpr int kExactTerms = 1 << 24;                // FP32 exact-integer bound
 constexpr int kSyncEvery = 64;                      // stages per lockstep epoch (cooperative launches)
 constexpr int kRetired = 0x7F7F7F7F;                // progress value of a CTA that has no work left
@@ -71,8 +72,6 @@ struct OzJob {
     int32_t lmap, rmap;        // tensor-map index (0..3) of the left / right digit operand
     int32_t lower;             // 1: only tiles and elements with row >= col
     int32_t accum;             // 1: the first unit of a tile adds to the output instead of storing
-    int32_t ksteps_last;       // pair tiles: K steps of 32 bytes the last k-block holds (1-4; 0: 4)
-    int32_t reserved0;
     int64_t lplane, rplane;    // rows per digit plane in each map
     int64_t lrow0, rrow0;      // first operand row (output row / col 0) inside a plane
     int64_t lk0, rk0;          // first contraction byte (multiple of 128)
@@ -86,113 +85,11 @@ struct OzJob {
     const int32_t *er;         // exponent of each output col (job-relative)
 };
 
-// ------------------------------------------------------------- PTX wrappers
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Bounded wait.  Returns false (and raises the CTA abort flag) when the budget expires
-// or another role already aborted.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *err,
-                                          int where, long long budget = kWaitCycles) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    while (!mbar_try_wait(bar, parity)) {
-        if (*abort_flag) return false;
-        if (clock64() - t0 > budget) {
-            *abort_flag = 1;
-            atomicCAS(err, 0, kDevTimeout * 16 + where);
-            return false;
-        }
-    }
-    return true;
-}
-// Wait that ignores the abort flag (used only while draining in-flight work), still bounded.
-__device__ __forceinline__ void mbar_drain_wait(uint64_t *bar, uint32_t parity) {
-    const long long t0 = clock64();
-    while (!mbar_try_wait(bar, parity))
-        if (clock64() - t0 > kWaitCycles) return;
-}
-
-__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, uint64_t *bar, int x, int y) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n" ::"r"(
-            smem_u32(dst)),
-        "l"((uint64_t)map), "r"(smem_u32(bar)), "r"(x), "r"(y)
-        : "memory");
-}
-
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr & 0x3FFFF) >> 4);          // start address
-    d |= (uint64_t)1 << 16;                          // leading byte offset (unused for SW128 K-major)
-    d |= (uint64_t)(1024 >> 4) << 32;                // stride byte offset: 8 rows x 128 B
-    d |= (uint64_t)1 << 46;                          // descriptor version (sm_100 family)
-    d |= (uint64_t)2 << 61;                          // SWIZZLE_128B
-    return d;
-}
-
 // kind::f8f6f4, A = B = e4m3, D = f32, both K-major, M = 128, N = 128
 __host__ __device__ constexpr uint32_t idesc_f8(bool negA) {
     return (1u << 4) | (0u << 7) | (0u << 10) | ((negA ? 1u : 0u) << 13) | (0u << 14) | (0u << 15) | (0u << 16) |
            ((uint32_t)(kTileN >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
 }
-
-__device__ __forceinline__ void mma_f8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                       uint32_t accumulate) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n}\n" ::"r"(
-            d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void mma_commit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar))
-                 : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
-        "%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-}
-template <int kN>
-__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[kN]) {
-    if constexpr (kN == 32) tmem_ld32(taddr, r);
-    else tmem_ld16(taddr, r);
-}
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
 
 // ------------------------------------------------------- work decomposition
 __device__ __forceinline__ int job_of(const OzJob *jobs, int num_jobs, int64_t tile) {
@@ -561,8 +458,6 @@ constexpr int kLdCols = kLdColsPair();
 #define HSDLA_DRAIN_BUFS 1
 #endif
 constexpr int kPairStages = HSDLA_PAIR_STAGES;
-constexpr int kPairStagesHalf = 4;          // 48 KB stages of the half-width tiles
-constexpr int kPairStagesMax = kPairStages > kPairStagesHalf ? kPairStages : kPairStagesHalf;
 constexpr int kDrainBufs = HSDLA_DRAIN_BUFS;
 constexpr int kStageCols = HSDLA_PAIR_STAGING_KB * 1024 / kPairEpiWarps / kDrainBufs / 512;   // columns per buffer
 constexpr int kStageWarpBytes = kDrainBufs * kStageCols * 32 * 16;   // buffers x columns x 32 rows x 16 B
@@ -599,130 +494,31 @@ template <int N>
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;\n" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;\n" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ uint32_t cluster_size() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;\n" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ uint32_t mapa_rank(uint32_t saddr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"(saddr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-}
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_addr) : "memory");
-}
-__device__ __forceinline__ void tma_load_2d_pair(void *dst, const CUtensorMap *map, uint32_t bar_cluster, int x,
-                                                 int y) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], "
-        "[%2];\n" ::"r"(smem_u32(dst)),
-        "l"((uint64_t)map), "r"(bar_cluster), "r"(x), "r"(y)
-        : "memory");
-}
+#ifndef HSDLA_COLLECTOR_A
+#define HSDLA_COLLECTOR_A 1
+#endif
+struct __align__(8) PairBarriers {
+    uint64_t full[kPairStages];   // leader: both CTAs' bytes of a stage landed
+    uint64_t empty[kPairStages];  // each CTA: the stage's MMAs completed (multicast commit)
+    uint64_t tfull;              // each CTA: the accumulator is complete (multicast commit)
+    uint64_t tempty;             // leader: the epilogue warps of both CTAs drained it
+};
+
+constexpr size_t kPairSmem = (size_t)kPairStages * kStageBytes + kPairStageBytes + 1024;
+static_assert(kPairSmem <= 227 * 1024, "pair kernel shared memory");
 __host__ __device__ constexpr uint32_t idesc_f8_pair(bool negA) {
     return (1u << 4) | ((negA ? 1u : 0u) << 13) | ((uint32_t)(kPairTile >> 3) << 17) |
            ((uint32_t)(kPairTile >> 4) << 24);
 }
-__device__ __forceinline__ void mma_f8_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                            uint32_t accumulate) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n}\n" ::"r"(
-            d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// The same MMA with the left operand's collector buffer: kFill reads A from shared memory and
-// keeps it for the next MMA, which (kFill = false: lastuse) takes A from the buffer and frees it.
-template <bool kFill>
-__device__ __forceinline__ void mma_f8_pair_ca(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                               uint32_t accumulate) {
-    if constexpr (kFill)
-        asm volatile(
-            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-            " tcgen05.mma.cta_group::2.kind::f8f6f4.collector::a::fill [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-            "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-            : "memory");
-    else
-        asm volatile(
-            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-            " tcgen05.mma.cta_group::2.kind::f8f6f4.collector::a::lastuse [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-            "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-            : "memory");
-}
-#ifndef HSDLA_COLLECTOR_A
-#define HSDLA_COLLECTOR_A 1
-#endif
-__device__ __forceinline__ void mma_commit_pair(uint64_t *bar) {
-    const uint16_t both = 3;
-    asm volatile(
-        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n" ::"r"(
-            smem_u32(bar)),
-        "h"(both)
-        : "memory");
-}
 
-struct __align__(8) PairBarriers {
-    uint64_t full[kPairStagesMax];   // leader: both CTAs' bytes of a stage landed
-    uint64_t empty[kPairStagesMax];  // each CTA: the stage's MMAs completed (multicast commit)
-    uint64_t tfull[2];           // each CTA: a TMEM buffer's accumulator is complete (multicast commit)
-    uint64_t tempty[2];          // leader: the epilogue warps of both CTAs drained the buffer
-};
-
-// Accumulation units of a pair launch, in drain order.  Unit u sums, per K-chunk, the digit pairs
-// (i, t - i) of diagonal t = t[u] into the FP32 accumulator and drains it with weight 2^(2-5t).
-// A merged unit also sums the pairs (i, t + 1 - i) of the next diagonal, with the left digits
-// scaled by 2^-5 (planes 2s .. 4s-1 of the left operand): the two diagonals share one drain.
-constexpr int kMaxUnits = kOzMaxSlices + 1;
-constexpr uint8_t kUnitMerged = 1;
-struct PairUnits {
-    int32_t n;
-    int8_t t[kMaxUnits];
-    uint8_t flags[kMaxUnits];
-};
-
-// Tile shape of a pair launch.  kHalves = 1: one 256 x 256 accumulator (re + im, all 512 TMEM
-// columns), so a unit's MMAs wait while the previous unit drains.  kHalves = 2: every unit runs
-// as two halves of 128 output columns (MMA N = 128) into alternating TMEM buffers, so one half
-// drains while the other computes; the left operand is staged once per half (1.5x the operand
-// traffic of kHalves = 1) and the right operand's stage holds 64 rows per CTA (its own tensor map).
-template <int kHalves>
-struct PairShape {
-    static constexpr int kN = kPairTile / kHalves;             // output columns of a unit half
-    static constexpr int kBRows = kN / 2;                      // right-operand rows a CTA stages
-    static constexpr int kStageBytes = 2 * kTileM * kKBlock + 2 * kBRows * kKBlock;
-    static constexpr int kStages = kHalves == 1 ? kPairStages : kPairStagesHalf;
-    static constexpr int kBufCols = 2 * kN;                    // TMEM columns of a buffer (re + im)
-    static constexpr int kColsPerWarp = 4 * kN / kPairEpiWarps;   // per quadrant: 4 warps share kN
-    static constexpr int kChunks = kColsPerWarp / 32;
-    static constexpr size_t kSmem = (size_t)kStages * kStageBytes + kPairStageBytes + 1024;
-    static_assert(kChunks >= 1 && kColsPerWarp % 32 == 0, "epilogue column split");
-    static_assert(kStages <= kPairStagesMax, "stage barriers");
-    static_assert(kSmem <= 227 * 1024, "pair kernel shared memory");
-};
-__host__ __device__ constexpr uint32_t idesc_f8_pair_n(bool negA, int n) {
-    return (1u << 4) | ((negA ? 1u : 0u) << 13) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kPairTile >> 4) << 24);
-}
-
-template <int kHalves>
 __global__ void __launch_bounds__(kPairThreads, 1)
     oz_pair_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap map1,
                    const __grid_constant__ CUtensorMap map2, const __grid_constant__ CUtensorMap map3,
                    const OzJob *__restrict__ jobs, int num_jobs, int64_t total_tiles, int s, int *err,
-                   const int4 *__restrict__ tile_list, int *progress, int sync_every, int slack,
-                   const __grid_constant__ PairUnits units) {
-    using Shape = PairShape<kHalves>;
-    constexpr int kStages = Shape::kStages;
-    constexpr int kStageB = Shape::kStageBytes;
-    constexpr int kN = Shape::kN;
+                   const int4 *__restrict__ tile_list, int *progress, int sync_every, int slack) {
+    constexpr int kStages = kPairStages;
+    constexpr int kStageB = kStageBytes;
+    constexpr int kN = kPairTile;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -754,7 +550,8 @@ __global__ void __launch_bounds__(kPairThreads, 1)
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < kStages; ++i) { mbar_init(&bars.full[i], 1); mbar_init(&bars.empty[i], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&bars.tfull[b], 1); mbar_init(&bars.tempty[b], 2 * kPairEpiWarps); }
+        mbar_init(&bars.tfull, 1);
+        mbar_init(&bars.tempty, 2 * kPairEpiWarps);
         abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         for (int i = 0; i < 4; ++i) asm volatile("prefetch.tensormap [%0];\n" ::"l"((uint64_t)map_of(i)) : "memory");
@@ -771,9 +568,8 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_sh;
     const uint32_t full0_leader = mapa_rank(smem_u32(&bars.full[0]), 0);
-    const uint32_t tempty0_leader = mapa_rank(smem_u32(&bars.tempty[0]), 0);
-    const int64_t half = (int64_t)rank * (kPairTile / 2);     // this CTA's rows of a tile
-    const int64_t bhalf = (int64_t)rank * Shape::kBRows;        // this CTA's right-operand rows of a half
+    const uint32_t tempty_leader = mapa_rank(smem_u32(&bars.tempty), 0);
+    const int64_t half = (int64_t)rank * (kPairTile / 2);     // this CTA's rows of a tile, and of the right operand
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producers (both CTAs)
@@ -786,37 +582,29 @@ __global__ void __launch_bounds__(kPairThreads, 1)
                 int64_t tm, tn;
                 const OzJob &j = resolve_tile(jobs, num_jobs, tile_list, tile, tm, tn);
                 const CUtensorMap *lm = map_of(j.lmap), *rm = map_of(j.rmap);
-                for (int u = 0; ok && u < units.n; ++u) {
-                    const int t = units.t[u], merged = (units.flags[u] & kUnitMerged) ? 1 : 0;
-                    const int64_t ck = merged ? j.nkb : chunk_kblocks(min(s, t - 1) - max(1, t - s) + 1);
+                for (int t = 2; ok && t <= s + 1; ++t) {
+                    const int ilo = max(1, t - s), ihi = min(s, t - 1);
+                    const int64_t ck = chunk_kblocks(ihi - ilo + 1);
                     for (int64_t cb = 0; ok && cb < j.nkb; cb += ck) {
                         const int64_t ce = min(j.nkb, cb + ck);
-                        for (int h = 0; ok && h < kHalves; ++h) {
-                            for (int64_t kb = cb; ok && kb < ce; ++kb) {
-                                for (int part = 0; ok && part <= merged; ++part) {
-                                    const int tt = t + part, ilo = max(1, tt - s), ihi = min(s, tt - 1);
-                                    for (int i = ilo; i <= ihi; ++i) {
-                                        const int jj = tt - i;
-                                        const int lp = (part ? 2 * s : 0) + 2 * (i - 1);   // scaled planes of a merged part
-                                        if (leader && progress && issued > 0 && issued % sync_every == 0 &&
-                                            !grid_lockstep(progress, (int)npairs, (int)(issued / sync_every),
-                                                           &abort_flag, err, (int)pair, slack)) { ok = false; break; }
-                                        if (!pwait(&bars.empty[stage], phase ^ 1, 1, stage, (int)issued)) { ok = false; break; }
-                                        unsigned char *st = smem + stage * kStageB;
-                                        if (leader) mbar_expect_tx(&bars.full[stage], 2 * kStageB);
-                                        const uint32_t fb = full0_leader + stage * 8;
-                                        const int xl = (int)(j.lk0 + kb * kKBlock), xr = (int)(j.rk0 + kb * kKBlock);
-                                        const int64_t yl = j.lrow0 + tm * kPairTile + half;
-                                        const int64_t yr = j.rrow0 + tn * kPairTile + h * kN + bhalf;
-                                        tma_load_2d_pair(st, lm, fb, xl, (int)(lp * j.lplane + yl));
-                                        tma_load_2d_pair(st + 16384, lm, fb, xl, (int)((lp + 1) * j.lplane + yl));
-                                        tma_load_2d_pair(st + 32768, rm, fb, xr, (int)((2 * (jj - 1)) * j.rplane + yr));
-                                        tma_load_2d_pair(st + 32768 + Shape::kBRows * kKBlock, rm, fb, xr,
-                                                         (int)((2 * (jj - 1) + 1) * j.rplane + yr));
-                                        ++issued;
-                                        if (++stage == kStages) { stage = 0; phase ^= 1; }
-                                    }
-                                }
+                        for (int64_t kb = cb; ok && kb < ce; ++kb) {
+                            for (int i = ilo; i <= ihi; ++i) {
+                                const int jj = t - i;
+                                if (leader && progress && issued > 0 && issued % sync_every == 0 &&
+                                    !grid_lockstep(progress, (int)npairs, (int)(issued / sync_every), &abort_flag, err,
+                                                   (int)pair, slack)) { ok = false; break; }
+                                if (!pwait(&bars.empty[stage], phase ^ 1, 1, stage, (int)issued)) { ok = false; break; }
+                                unsigned char *st = smem + stage * kStageB;
+                                if (leader) mbar_expect_tx(&bars.full[stage], 2 * kStageB);
+                                const uint32_t fb = full0_leader + stage * 8;
+                                const int xl = (int)(j.lk0 + kb * kKBlock), xr = (int)(j.rk0 + kb * kKBlock);
+                                const int64_t yl = j.lrow0 + tm * kPairTile + half, yr = j.rrow0 + tn * kPairTile + half;
+                                tma_load_2d_pair(st, lm, fb, xl, (int)((2 * (i - 1)) * j.lplane + yl));
+                                tma_load_2d_pair(st + 16384, lm, fb, xl, (int)((2 * (i - 1) + 1) * j.lplane + yl));
+                                tma_load_2d_pair(st + 32768, rm, fb, xr, (int)((2 * (jj - 1)) * j.rplane + yr));
+                                tma_load_2d_pair(st + 49152, rm, fb, xr, (int)((2 * (jj - 1) + 1) * j.rplane + yr));
+                                ++issued;
+                                if (++stage == kStages) { stage = 0; phase ^= 1; }
                             }
                         }
                     }
@@ -837,100 +625,76 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         if (lane == 0 && leader) {
             int stage = 0;
             uint32_t phase = 0;
-            int64_t unit = 0;            // unit chunks issued (each uses every buffer once)
-            int hb = 0;                  // buffer of a partially issued half
+            int64_t unit = 0;            // units issued
             bool ok = true;
-            const uint32_t id_pos = idesc_f8_pair_n(false, kN), id_neg = idesc_f8_pair_n(true, kN);
+            const uint32_t id_pos = idesc_f8_pair(false), id_neg = idesc_f8_pair(true);
             const uint32_t sbase = smem_u32(smem);
+            const uint32_t d_re = tmem_base, d_im = d_re + kN;
             for (int64_t tile = pair; ok && tile < total_tiles; tile += npairs) {
                 int64_t tm_, tn_;
                 const OzJob &j = resolve_tile(jobs, num_jobs, tile_list, tile, tm_, tn_);
                 // the job's fields in registers: the asm statements below clobber memory, and the
                 // issuer must not reload them between MMAs
                 const int64_t jnkb = j.nkb;
-                const int jksl = j.ksteps_last > 0 ? j.ksteps_last : kKBlock / 32;
-                for (int u = 0; ok && u < units.n; ++u) {
-                    const int t = units.t[u], merged = (units.flags[u] & kUnitMerged) ? 1 : 0;
-                    const int64_t ck = merged ? jnkb : chunk_kblocks(min(s, t - 1) - max(1, t - s) + 1);
+                for (int t = 2; ok && t <= s + 1; ++t) {
+                    const int ilo = max(1, t - s), ihi = min(s, t - 1);
+                    const int64_t ck = chunk_kblocks(ihi - ilo + 1);
                     for (int64_t cb = 0; ok && cb < jnkb; cb += ck) {
                         const int64_t ce = min(jnkb, cb + ck);
-                        for (int h = 0; ok && h < kHalves; ++h) {
-                            hb = h;
-                            const uint32_t d_re = tmem_base + h * Shape::kBufCols, d_im = d_re + kN;
-                            if (!pwait(&bars.tempty[h], (uint32_t)((unit & 1) ^ 1), 2, stage, (int)unit)) { ok = false; break; }
-                            tc_fence_after();
-                            bool first = true;
-                            for (int64_t kb = cb; ok && kb < ce; ++kb) {
-                                for (int part = 0; ok && part <= merged; ++part) {
-                                    const int tt = t + part, ilo = max(1, tt - s), ihi = min(s, tt - 1);
-                                    for (int i = ilo; i <= ihi; ++i) {
-                                        if (!pwait(&bars.full[stage], phase, 3, stage, (int)unit)) { ok = false; break; }
-                                        tc_fence_after();
-                                        const uint32_t a_re = sbase + stage * kStageB, a_im = a_re + 16384;
-                                        const uint32_t b_re = a_re + 32768, b_im = b_re + Shape::kBRows * kKBlock;
-                                        // The stage's four descriptors once; a 32-byte step along K adds 2
-                                        // to the start-address field (16-byte units; shared-memory
-                                        // addresses stay below 2^18, so the field never carries).  The
-                                        // single issuing thread has ~64 cycles per N = 128 MMA.
-                                        const uint64_t dar = sw128_desc(a_re), dai = sw128_desc(a_im);
-                                        const uint64_t dbr = sw128_desc(b_re), dbi = sw128_desc(b_im);
-                                        auto step = [&](uint32_t kk) {
-                                            const uint64_t o = 2u * kk;
-                                            const uint32_t acc = first ? 0u : 1u;
-#if HSDLA_COLLECTOR_A
-                                            // the two MMAs of the real left plane back to back, the
-                                            // second taking A from the collector buffer.  (Not for
-                                            // the imaginary plane: an MMA that reads A from the
-                                            // collector does not apply the negate-A bit, measured:
-                                            // the -A_im B_re term came out as +A_im B_re.)
-                                            mma_f8_pair_ca<true>(d_re, dar + o, dbr + o, id_pos, acc);
-                                            mma_f8_pair_ca<false>(d_im, dar + o, dbi + o, id_pos, acc);
-                                            mma_f8_pair(d_re, dai + o, dbi + o, id_pos, 1u);
-                                            mma_f8_pair(d_im, dai + o, dbr + o, id_neg, 1u);
-#else
-                                            mma_f8_pair(d_re, dar + o, dbr + o, id_pos, acc);
-                                            mma_f8_pair(d_re, dai + o, dbi + o, id_pos, 1u);
-                                            mma_f8_pair(d_im, dar + o, dbi + o, id_pos, acc);
-                                            mma_f8_pair(d_im, dai + o, dbr + o, id_neg, 1u);
-#endif
-                                            first = false;
-                                        };
-                                        // whole blocks as straight-line code (a bound in this loop slowed the
-                                        // launches by 2-10%).  With 256 x 256 accumulators the job's last
-                                        // k-block stops early, where the K steps past the contraction length
-                                        // hold zero digits (lmax 8: 2L = 162 of 256; c1 -10%); the half-width
-                                        // tiles keep whole blocks, as the check alone cost them 3-6% (c2, c3)
-                                        if (kHalves == 2 || kb + 1 < jnkb || jksl == kKBlock / 32) {
+                        if (!pwait(&bars.tempty, (uint32_t)((unit & 1) ^ 1), 2, stage, (int)unit)) { ok = false; break; }
+                        tc_fence_after();
+                        bool first = true;
+                        for (int64_t kb = cb; ok && kb < ce; ++kb) {
+                            for (int i = ilo; i <= ihi; ++i) {
+                                if (!pwait(&bars.full[stage], phase, 3, stage, (int)unit)) { ok = false; break; }
+                                tc_fence_after();
+                                const uint32_t a_re = sbase + stage * kStageB, a_im = a_re + 16384;
+                                const uint32_t b_re = a_re + 32768, b_im = a_re + 49152;
+                                // The stage's four descriptors once; a 32-byte step along K adds 2
+                                // to the start-address field (16-byte units; shared-memory
+                                // addresses stay below 2^18, so the field never carries).
+                                const uint64_t dar = sw128_desc(a_re), dai = sw128_desc(a_im);
+                                const uint64_t dbr = sw128_desc(b_re), dbi = sw128_desc(b_im);
 #pragma unroll
-                                            for (int kk = 0; kk < kKBlock / 32; ++kk) step(kk);
-                                        } else {
-                                            step(0);
-                                            if (jksl > 1) step(1);
-                                            if (jksl > 2) step(2);
-                                        }
-                                        mma_commit_pair(&bars.empty[stage]);
-                                        if (++stage == kStages) { stage = 0; phase ^= 1; }
-                                    }
+                                for (int kk = 0; kk < kKBlock / 32; ++kk) {
+                                    const uint64_t o = 2u * kk;
+                                    const uint32_t acc = first ? 0u : 1u;
+#if HSDLA_COLLECTOR_A
+                                    // the two MMAs of the real left plane back to back, the
+                                    // second taking A from the collector buffer.  (Not for
+                                    // the imaginary plane: an MMA that reads A from the
+                                    // collector does not apply the negate-A bit, measured:
+                                    // the -A_im B_re term came out as +A_im B_re.)
+                                    mma_f8_pair_ca<true>(d_re, dar + o, dbr + o, id_pos, acc);
+                                    mma_f8_pair_ca<false>(d_im, dar + o, dbi + o, id_pos, acc);
+                                    mma_f8_pair(d_re, dai + o, dbi + o, id_pos, 1u);
+                                    mma_f8_pair(d_im, dai + o, dbr + o, id_neg, 1u);
+#else
+                                    mma_f8_pair(d_re, dar + o, dbr + o, id_pos, acc);
+                                    mma_f8_pair(d_re, dai + o, dbi + o, id_pos, 1u);
+                                    mma_f8_pair(d_im, dar + o, dbi + o, id_pos, acc);
+                                    mma_f8_pair(d_im, dai + o, dbr + o, id_neg, 1u);
+#endif
+                                    first = false;
                                 }
+                                mma_commit_pair(&bars.empty[stage]);
+                                if (++stage == kStages) { stage = 0; phase ^= 1; }
                             }
-                            if (!ok) break;
-                            mma_commit_pair(&bars.tfull[h]);
                         }
                         if (!ok) break;
+                        mma_commit_pair(&bars.tfull);
                         ++unit;
                     }
                 }
             }
             if (!ok) {
-                // a partially issued half may still be running: commit it and wait (bounded)
-                mma_commit_pair(&bars.tfull[hb]);
-                mbar_drain_wait(&bars.tfull[hb], (uint32_t)(unit & 1));
+                // a partially issued unit may still be running: commit it and wait (bounded)
+                mma_commit_pair(&bars.tfull);
+                mbar_drain_wait(&bars.tfull, (uint32_t)(unit & 1));
             } else if (unit > 0) {
                 // the last unit's MMAs and both CTAs' drains of it
-                for (int h = 0; h < kHalves; ++h) {
-                    mbar_drain_wait(&bars.tfull[h], (uint32_t)((unit - 1) & 1));
-                    mbar_drain_wait(&bars.tempty[h], (uint32_t)((unit - 1) & 1));
-                }
+                mbar_drain_wait(&bars.tfull, (uint32_t)((unit - 1) & 1));
+                mbar_drain_wait(&bars.tempty, (uint32_t)((unit - 1) & 1));
             }
         }
     } else {
@@ -941,7 +705,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         // successive updates of an element come from one thread and stay in program order; the
         // SM never waits on the output.  Only stored elements (row < m, col < n, lower: row >=
         // col) are written.
-        constexpr int kCols = Shape::kColsPerWarp, kCh = Shape::kChunks;
+        constexpr int kCols = kColsPerWarp, kCh = kChunksPerWarp;
         const int q = warp & 3;                      // TMEM lane quadrant of this warp
         const int cbeg = ((warp - 2) >> 2) * kCols;  // its share of a buffer's columns
         unsigned char *stg = smem + kStages * kStageB + (warp - 2) * kStageWarpBytes;
@@ -959,42 +723,38 @@ __global__ void __launch_bounds__(kPairThreads, 1)
             const int erow = row < m ? j.el[row] : 0;
             double2 *out = j.out;
             // The tile's column exponents, loaded once for all its units: lane l holds column
-            // tn*256 + h*kN + cbeg + 32c + l of half h, chunk c in ex[h kCh + c], with each chunk's
+            // tn*256 + cbeg + 32c + l of chunk c in ex[c], with each chunk's
             // range for the fast-path test.  The registers rotate after each chunk, so the current
             // chunk's are always in ex[0] (after a unit's chunks they are back in order).
             const int32_t *er = j.er;
-            int ex[kHalves * kCh], exlo[kHalves * kCh], exhi[kHalves * kCh];
+            int ex[kCh], exlo[kCh], exhi[kCh];
 #pragma unroll
-            for (int x = 0; x < kHalves * kCh; ++x) {
-                const int64_t col = tn * kPairTile + (x / kCh) * kN + cbeg + 32 * (x % kCh) + lane;
+            for (int x = 0; x < kCh; ++x) {
+                const int64_t col = tn * kPairTile + cbeg + 32 * x + lane;
                 ex[x] = col < n ? __ldg(er + col) : 0;
             }
 #pragma unroll
-            for (int x = 0; x < kHalves * kCh; ++x) {
+            for (int x = 0; x < kCh; ++x) {
                 exlo[x] = __reduce_min_sync(0xffffffffu, ex[x]);
                 exhi[x] = __reduce_max_sync(0xffffffffu, ex[x]);
             }
-            for (int u = 0; ok && u < units.n; ++u) {
-                const int t = units.t[u];
-                const uint8_t fl = units.flags[u];
-                const int64_t ck =
-                    (fl & kUnitMerged) ? nkb : chunk_kblocks(min(s, t - 1) - max(1, t - s) + 1);
+            for (int t = 2; ok && t <= s + 1; ++t) {
+                const int64_t ck = chunk_kblocks(min(s, t - 1) - max(1, t - s) + 1);
                 const int kb = 2 - 5 * t + erow;
                 // 2^(kb + e_col) as an FP64 exponent bias: the row's part plus e_col << 20
                 const uint32_t rbias = pow2_ebias(kb);
                 for (int64_t cb = 0; ok && cb < nkb; cb += ck) {
-                    const bool first = (u == 0 && cb == 0) && !accum;
-                    const uint64_t pol = (u == units.n - 1 && cb + ck >= nkb) ? pol_first : pol_last;
-#pragma unroll 1
-                    for (int h = 0; h < kHalves; ++h) {
-                        if (!pwait(&bars.tfull[h], (uint32_t)(unit & 1), 4, warp, (int)unit)) { ok = false; break; }
+                    const bool first = (t == 2 && cb == 0) && !accum;
+                    const uint64_t pol = (t == s + 1 && cb + ck >= nkb) ? pol_first : pol_last;
+                    {
+                        if (!pwait(&bars.tfull, (uint32_t)(unit & 1), 4, warp, (int)unit)) { ok = false; break; }
                         tc_fence_after();
-                        // the previous half's copies are complete: successive updates stay in order
+                        // the previous unit's copies are complete: successive updates stay in order
                         if (lane < kStageCols) bulk_wait_all();
-                        const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + h * Shape::kBufCols;
+                        const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16);
 #pragma unroll 1
                         for (int c = 0; c < kCh; ++c) {
-                            const int64_t colb = tn * kPairTile + h * kN + cbeg + 32 * c;
+                            const int64_t colb = tn * kPairTile + cbeg + 32 * c;
                             const bool fast = __all_sync(0xffffffffu, pow2_ok(kb + exlo[0]) && pow2_ok(kb + exhi[0]));
 #pragma unroll
                             for (int hh = 0; hh < 32; hh += kLdCols) {
@@ -1005,7 +765,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
                                 if (c == kCh - 1 && hh + kLdCols >= 32) {
                                     tc_fence_before();
                                     __syncwarp();
-                                    if (lane == 0) mbar_arrive_remote(tempty0_leader + h * 8);
+                                    if (lane == 0) mbar_arrive_remote(tempty_leader);
                                 }
 #pragma unroll
                                 for (int g4 = 0; g4 < kLdCols; g4 += kStageCols, ++rd) {
@@ -1046,17 +806,16 @@ __global__ void __launch_bounds__(kPairThreads, 1)
                             // the next chunk's exponents into ex[0]
                             const int xe = ex[0], xl = exlo[0], xh = exhi[0];
 #pragma unroll
-                            for (int x = 0; x + 1 < kHalves * kCh; ++x) {
+                            for (int x = 0; x + 1 < kCh; ++x) {
                                 ex[x] = ex[x + 1];
                                 exlo[x] = exlo[x + 1];
                                 exhi[x] = exhi[x + 1];
                             }
-                            ex[kHalves * kCh - 1] = xe;
-                            exlo[kHalves * kCh - 1] = xl;
-                            exhi[kHalves * kCh - 1] = xh;
+                            ex[kCh - 1] = xe;
+                            exlo[kCh - 1] = xl;
+                            exhi[kCh - 1] = xh;
                         }
                     }
-                    if (!ok) break;
                     ++unit;
                 }
             }
@@ -1108,29 +867,17 @@ struct SliceTab {
     const double *v2 = nullptr;
     uint8_t *digits2 = nullptr;
     int32_t *expo2 = nullptr;
-    // 1: the (first) operand's digits also go, scaled by 2^-5, to planes 2s .. 4s-1 (the left
-    // operand of merged accumulation units)
-    int scaled = 0;
     SliceEntry e[kMaxGroup];
 };
 
 // e4m3 byte of the digit idx - 16 (idx in [0, 32]), per CTA of the slicing kernel: a digit is
 // one shared-memory load instead of an integer-to-float conversion and half a packing conversion
 __shared__ uint8_t g_e4m3_lut[33];
-// Four e4m3 digits (|d| <= 16) times 2^-5: every nonzero digit is normal with exponent field >= 7
-// (|d| >= 1), so subtracting 5 from the field (0x28 from the byte, no borrow) scales it exactly
-// (d / 32 >= 2^-5 stays normal); zeros keep their bytes.
-__device__ __forceinline__ uint32_t scale4_e4m3_2m5(uint32_t w) {
-    return w - (0x28282828u & __vcmpne4(w & 0x7f7f7f7fu, 0u));
-}
-
 // The planes of U = X + B from the least significant: plane i (0 = most significant) holds
 // ((U >> 5 (s-1-i)) & 31) - 16 for i >= 1, and the top plane the rest, U >> 5 (s-1) in
 // [-16, 16].  A running arithmetic shift by 5 leaves each field in the low bits in turn (the low
 // bits are the same for arithmetic and logical shifts).
-// kScaled: each digit also goes, times 2^-5 (exact in e4m3 for |d| <= 16: d / 32 >= 2^-5 is
-// normal), to plane 2s + 2i + part.
-template <int kVec, bool kScaled>
+template <int kVec>
 __device__ __forceinline__ void write_part(const long long (&x)[kVec], int part, int s, uint8_t *row, int64_t plane) {
     long long u[kVec];
 #pragma unroll
@@ -1151,19 +898,14 @@ __device__ __forceinline__ void write_part(const long long (&x)[kVec], int part,
         uint8_t *dst = row + (int64_t)(2 * i + part) * plane;
         if (kVec == 8) *reinterpret_cast<uint2 *>(dst) = make_uint2(w0, w1);
         else *reinterpret_cast<uint32_t *>(dst) = w0;
-        if (kScaled) {
-            uint8_t *dsc = row + (int64_t)(2 * s + 2 * i + part) * plane;
-            if (kVec == 8) *reinterpret_cast<uint2 *>(dsc) = make_uint2(scale4_e4m3_2m5(w0), scale4_e4m3_2m5(w1));
-            else *reinterpret_cast<uint32_t *>(dsc) = scale4_e4m3_2m5(w0);
-        }
     }
 }
 
-template <int kVec, bool kScaled = false>
+template <int kVec>
 __device__ __forceinline__ void write_planes(const long long (&ur)[kVec], const long long (&ui)[kVec], int s,
                                              uint8_t *row, int64_t plane) {
-    write_part<kVec, kScaled>(ur, 0, s, row, plane);
-    write_part<kVec, kScaled>(ui, 1, s, row, plane);
+    write_part<kVec>(ur, 0, s, row, plane);
+    write_part<kVec>(ui, 1, s, row, plane);
 }
 
 // Maximum over the block of non-negative doubles given as bit patterns (which order like the
@@ -1237,7 +979,7 @@ __device__ __noinline__ void weighted_chunk(const double2 *zc, const double *vv,
 #ifndef HSDLA_SLICE_CTAS
 #define HSDLA_SLICE_CTAS 2
 #endif
-template <bool kDual, bool kScaled>
+template <bool kDual>
 __global__ void __launch_bounds__(kSliceThreads, HSDLA_SLICE_CTAS) oz_slice_kernel(const __grid_constant__ SliceTab tab) {
     // values per thread and step of the digit pass (the dual pass keeps two operands' state)
     constexpr int kV = kDual ? 4 : kSliceVec;
@@ -1320,7 +1062,7 @@ __global__ void __launch_bounds__(kSliceThreads, HSDLA_SLICE_CTAS) oz_slice_kern
                     xi[u] = B + rint_pow2(z.y, kx);
                 }
             }
-            write_planes<kV, kScaled>(xr, xi, s, tab.digits + r * pitch + kp0, plane);
+            write_planes<kV>(xr, xi, s, tab.digits + r * pitch + kp0, plane);
             if (kDual)      // the chunk again (an L1 hit) for the weighted operand
                 weighted_chunk<kV>(zc, v2 + b * rpb + rr0, nv, kw, B, s, tab.digits2 + r * pitch + kp0, plane);
         }
@@ -1355,7 +1097,7 @@ struct DigitOperand {
     int32_t *expo = nullptr;
     int64_t plane_rows = 0, Kpad = 0, pitch = 0;
     CUtensorMap map;
-    CUtensorMap map64;         // 64-row boxes: the right operand of half-width pair tiles
+    CUtensorMap map64;         // 64-row boxes: a right operand of the real products
 };
 
 int64_t env_int(const char *name, int64_t dflt) {
@@ -1376,8 +1118,9 @@ int64_t pitch_pad() {
     return p;
 }
 
-// box_rows: rows of a TMA box (kTileM; 64 for the right operand of half-width pair tiles)
-int make_map(DigitOperand &d, int s, int box_rows = kTileM, CUtensorMap *dst = nullptr) {
+// box_rows: rows of a TMA box (kTileM; 64 for the right operand of the real products)
+// and contraction bytes of one: 128 with the 128-byte swizzle, 64 with the 64-byte one
+int make_map(DigitOperand &d, int planes, int box_rows = kTileM, CUtensorMap *dst = nullptr, int box_bytes = kKBlock) {
     PFN_encodeTiled enc = get_encode();
     if (!enc) { g_oz_err = "cuTensorMapEncodeTiled unavailable"; return HSDLA_ERR_CUDA; }
     if (d.Kpad % 128 != 0 || d.pitch % 16 != 0 || d.pitch < d.Kpad ||
@@ -1385,14 +1128,15 @@ int make_map(DigitOperand &d, int s, int box_rows = kTileM, CUtensorMap *dst = n
         g_oz_err = "digit operand misaligned";
         return HSDLA_ERR_ARG;
     }
-    const int64_t rows = d.plane_rows * 2 * s;
+    const int64_t rows = d.plane_rows * planes;
     if (rows > INT32_MAX || d.Kpad > INT32_MAX) { g_oz_err = "digit operand too large for TMA"; return HSDLA_ERR_UNSUPPORTED; }
     cuuint64_t dims[2] = {(cuuint64_t)d.Kpad, (cuuint64_t)rows};
     cuuint64_t strides[1] = {(cuuint64_t)d.pitch};
-    cuuint32_t box[2] = {(cuuint32_t)kKBlock, (cuuint32_t)box_rows};
+    cuuint32_t box[2] = {(cuuint32_t)box_bytes, (cuuint32_t)box_rows};
     cuuint32_t es[2] = {1, 1};
     CUresult r = enc(dst ? dst : &d.map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, d.digits, dims, strides, box, es,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     box_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) { g_oz_err = "cuTensorMapEncodeTiled failed"; return HSDLA_ERR_CUDA; }
     return HSDLA_OK;
@@ -1412,7 +1156,7 @@ struct Arena {
     }
 };
 
-// planes: digit planes (2s; 4s with the 2^-5-scaled copies of a merged-unit left operand)
+// planes: digit planes (0: 2s)
 int64_t operand_bytes(int s, int64_t rows, int64_t Kpad, int planes = 0) {
     const int64_t pr = round_up(rows, kTileM) + kTileM;
     return round_up((planes ? planes : 2 * s) * pr * (Kpad + pitch_pad()), 1024) + round_up(4 * pr, 1024);
@@ -1436,10 +1180,8 @@ SliceTab slice_table(const double2 *Z, int64_t ldz, const double *v, int64_t Kin
 }
 
 cudaError_t slice_launch(const SliceTab &t, cudaStream_t st) {
-    if (t.digits2 && t.scaled) oz_slice_kernel<true, true><<<(unsigned)t.plane_rows, kSliceThreads, 0, st>>>(t);
-    else if (t.digits2) oz_slice_kernel<true, false><<<(unsigned)t.plane_rows, kSliceThreads, 0, st>>>(t);
-    else if (t.scaled) oz_slice_kernel<false, true><<<(unsigned)t.plane_rows, kSliceThreads, 0, st>>>(t);
-    else oz_slice_kernel<false, false><<<(unsigned)t.plane_rows, kSliceThreads, 0, st>>>(t);
+    if (t.digits2) oz_slice_kernel<true><<<(unsigned)t.plane_rows, kSliceThreads, 0, st>>>(t);
+    else oz_slice_kernel<false><<<(unsigned)t.plane_rows, kSliceThreads, 0, st>>>(t);
     return cudaGetLastError();
 }
 
@@ -1458,37 +1200,6 @@ bool use_pair() {
     static const bool b = env_int("HSDLA_PAIR", 1) != 0;
     return b;
 }
-
-// Accumulation units of a pair launch (see PairUnits).  Diagonals t and t + 1 share a unit when
-// the left operand carries the 2^-5-scaled planes, each fits one K-chunk, and either the sum
-// stays exact -- every partial sum a multiple of 2^-5 below 2^19, with |sum| <= K x 2 (re/im) x
-// 256 (|product|) x (n_t + n_{t+1} / 32), K the contraction bytes that can hold nonzero digits
-// (kvalid, at most nkb 128: the slicer writes zero digits past 2L in each type's k-blocks, so the
-// per-type products of lmax 8 (2L = 162) count 162, not 256) -- or t >= kLooseT, where even an FP32
-// rounding (2^-24 of the sum) stays far below the result's FP64 precision.  The low-order
-// diagonals are not small everywhere: in a Gram element (S_gg) the products d_p(M_k) d_p(W_k) of
-// rows with w_k = 1 add up with one sign, so diagonal 2p carries ~K 2^8 2^(2-10p) whatever the
-// size of S_gg -- from t = 9 on below 2^-26 of S_gg, and exact here anyway (|sum| ~ 2^14).
-constexpr int kLooseT = 9;
-PairUnits pair_units(int s, int64_t nkb, bool merge, int64_t kvalid = 0) {
-    PairUnits p;
-    memset(&p, 0, sizeof(p));
-    auto pairs = [&](int t) { return std::min(s, t - 1) - std::max(1, t - s) + 1; };
-    const int64_t K = kvalid > 0 ? std::min(kvalid, nkb * kKBlock) : nkb * kKBlock;
-    for (int t = 2; t <= s + 1;) {
-        bool m = false;
-        if (merge && t + 1 <= s + 1 && chunk_kblocks(pairs(t)) >= nkb && chunk_kblocks(pairs(t + 1)) >= nkb) {
-            const int64_t bound = K * 2 * 256;
-            m = t >= kLooseT || bound * (32 * pairs(t) + pairs(t + 1)) <= ((int64_t)1 << 24);
-        }
-        p.t[p.n] = (int8_t)t;
-        p.flags[p.n] = m ? kUnitMerged : 0;
-        ++p.n;
-        t += m ? 2 : 1;
-    }
-    return p;
-}
-PairUnits pair_units_plain(int s) { return pair_units(s, 0, false); }
 
 // Host-built tile schedule.  Persistent CTAs take tiles g, g + grid, ... so tiles that are
 // close in the list run at the same time and share their operand panels in L2.  Lower-
@@ -1535,7 +1246,7 @@ void build_schedule(const std::vector<OzJob> &jobs, std::vector<int4> &list, int
 
 constexpr int kProgressCap = 1024;   // progress slots (>= SM count, multiple of 4)
 // Streamed host output: the S/H launches of all types are cut into at most kMaxOutBlocks launches
-// of whole waves of pair tiles; the tiles are ordered by kOutColumnBlocks column blocks (of about
+// of whole waves of tiles; the tiles are ordered by kOutColumnBlocks column blocks (of about
 // equal tile counts), so that the columns a launch completes are combined and sent to the host
 // while the next launch runs.  Only the part completed by the last launch stays exposed.
 constexpr int kMaxOutBlocks = 8;
@@ -1739,12 +1450,12 @@ struct OzGroup {
     int *d_progress = nullptr;
     int *d_err = nullptr;
     bool pair = false;          // S/H on CTA-pair tiles
-    PairUnits units{};          // their accumulation units
-    PairUnits units_t{};        // the T application's (structure-factor form on pair tiles)
-    int halves = 1;             // 2: structure-factor S/H launches on half-width pair tiles
-    int halves_t = 1;           // the same for the T application
-    bool merged = true;         // S/H units merge adjacent digit diagonals where exact
-    bool sf = false;            // structure-factor form
+    bool sf = false;            // structure-factor form, on real rows:
+    RealSliceTab rM, rX;        // the slicing of R (and R diag(w)) and of Z'
+    RealJob *d_rjobs_t = nullptr, *d_rjobs_sh = nullptr;   // T application; 3 nk products per type
+    RealBands bands{}, bands_t{};   // digit-pair order of the products and of the T application
+    int halves = 2;             // the products' configuration (see set_sh_tiles)
+    bool merged = true;
     int tbatch = 1;             // its types per combine batch
     // with one batch: the first side_types types are combined on a side stream while the S/H
     // launches of the others run (the combine is FP64-bound, the products tensor-bound)
@@ -1795,12 +1506,11 @@ int upload_schedule(std::vector<OzJob> &jobs, OzJob *d_jobs, int4 *d_list, int64
 
 // Launch of a prepared pair-tile job table: clusters of two CTAs, one per SM, as many pairs as
 // can be resident (at most one per tile); cooperative when the lockstep slots are given.
-template <int kHalves>
-cudaError_t launch_pair_t(const CUtensorMap *maps, int s, int *d_err, const OzJob *d_jobs, int n_jobs, int64_t total,
-                          const int4 *d_list, int *d_progress, cudaStream_t st, const PairUnits &units) {
+cudaError_t launch_pair(const CUtensorMap *maps, int s, int *d_err, const OzJob *d_jobs, int n_jobs, int64_t total,
+                        const int4 *d_list, int *d_progress, cudaStream_t st) {
     if (total <= 0) return cudaSuccess;
-    const size_t smem = PairShape<kHalves>::kSmem;
-    cudaError_t e = cudaFuncSetAttribute(oz_pair_kernel<kHalves>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const size_t smem = kPairSmem;
+    cudaError_t e = cudaFuncSetAttribute(oz_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[2];
@@ -1817,7 +1527,7 @@ cudaError_t launch_pair_t(const CUtensorMap *maps, int s, int *d_err, const OzJo
     if (max_pairs == 0) {
         cfg.gridDim = dim3(2);
         int nc = 0;
-        e = cudaOccupancyMaxActiveClusters(&nc, (const void *)oz_pair_kernel<kHalves>, &cfg);
+        e = cudaOccupancyMaxActiveClusters(&nc, (const void *)oz_pair_kernel, &cfg);
         if (e != cudaSuccess) return e;
         if (nc < 1) return cudaErrorInvalidConfiguration;
         max_pairs = nc;
@@ -1843,16 +1553,8 @@ cudaError_t launch_pair_t(const CUtensorMap *maps, int s, int *d_err, const OzJo
     // lockstep epoch (stages) and how many epochs a pair may lead the slowest one
     static const int sync_every = (int)std::max<int64_t>(8, env_int("HSDLA_SYNC_EVERY", kSyncEvery));
     static const int slack = (int)std::max<int64_t>(1, env_int("HSDLA_SYNC_SLACK", 1));
-    return cudaLaunchKernelEx(&cfg, oz_pair_kernel<kHalves>, maps[0], maps[1], maps[2], maps[3], d_jobs, n_jobs, total,
-                              s, d_err, d_list, lockstep ? d_progress : (int *)nullptr, sync_every, slack, units);
-}
-
-// halves = 2: the half-width tiles, whose right-operand maps (maps[j.rmap] of every job) must have
-// 64-row boxes (make_map(.., kPairTile / 4)); 1: 128-row boxes.
-cudaError_t launch_pair(const CUtensorMap *maps, int s, int *d_err, const OzJob *d_jobs, int n_jobs, int64_t total,
-                        const int4 *d_list, int *d_progress, cudaStream_t st, const PairUnits &units, int halves = 1) {
-    return halves == 2 ? launch_pair_t<2>(maps, s, d_err, d_jobs, n_jobs, total, d_list, d_progress, st, units)
-                       : launch_pair_t<1>(maps, s, d_err, d_jobs, n_jobs, total, d_list, d_progress, st, units);
+    return cudaLaunchKernelEx(&cfg, oz_pair_kernel, maps[0], maps[1], maps[2], maps[3], d_jobs, n_jobs, total,
+                              s, d_err, d_list, lockstep ? d_progress : (int *)nullptr, sync_every, slack);
 }
 
 // Launch of a prepared job table (no host synchronisation; capturable).
@@ -1906,8 +1608,8 @@ int ozaki_herkx(OzakiPlan &oz, const double2 *P, int64_t ldp, const double2 *Q, 
     cudaError_t e = slice(P, ldp, nullptr, K, n, Kpad, Kpad, s, dp, st);
     if (e == cudaSuccess) e = slice(Q, ldq, w, K, n, Kpad, Kpad, s, dq, st);
     if (e != cudaSuccess) { g_oz_err = cudaGetErrorString(e); return HSDLA_ERR_CUDA; }
-    int rc = make_map(dp, s);
-    if (!rc) rc = make_map(dq, s);
+    int rc = make_map(dp, 2 * s);
+    if (!rc) rc = make_map(dq, 2 * s);
     if (rc) return rc;
     CUtensorMap maps[4] = {dp.map, dq.map, dp.map, dp.map};
     std::vector<OzJob> jobs(1);
@@ -1918,14 +1620,12 @@ int ozaki_herkx(OzakiPlan &oz, const double2 *P, int64_t ldp, const double2 *Q, 
     j.nkb = Kpad / kKBlock; j.m = n; j.n = n;
     j.out = out; j.ldo = ldo; j.el = dp.expo; j.er = dq.expo;
     if (use_pair()) {
-        // CTA-pair 256 x 256 tiles with 256 x 256 accumulators, one exact unit per diagonal and
-        // K chunk (no merged units: the left operand has no scaled planes), pairs in lockstep
+        // CTA-pair 256 x 256 tiles, one exact unit per diagonal and K chunk, pairs in lockstep
         int *d_progress = ar.take<int>(kProgressCap);
         int64_t tiles = 0;
         rc = upload_schedule(jobs, d_jobs, d_list, tiles, kPairTile);
         if (rc) return rc;
-        const cudaError_t el = launch_pair(maps, s, oz.d_error, d_jobs, 1, tiles, d_list, d_progress, st,
-                                           pair_units(s, j.nkb, false), 1);
+        const cudaError_t el = launch_pair(maps, s, oz.d_error, d_jobs, 1, tiles, d_list, d_progress, st);
         if (el != cudaSuccess) { g_oz_err = cudaGetErrorString(el); return HSDLA_ERR_CUDA; }
     } else {
         rc = launch_gemm(jobs, maps, s, oz.d_error, d_jobs, st, nullptr, nullptr, d_list);
@@ -1946,13 +1646,13 @@ static int64_t atom_stride(int64_t twoL) { return round_up(twoL, 16); }
 int64_t ozaki_group_bytes(int s, int64_t twoL, int64_t na, int64_t nt, const std::vector<int64_t> &G, int panels,
                           bool hoist, bool sf) {
     const int64_t bpad = atom_stride(twoL), rows = group_rows(G);
-    if (sf) {      // M (with its scaled copy on pair tiles), M diag(w_t) and Z digits: each
-                   // type's rows on whole k-blocks
-        const int64_t KT = round_up(twoL, kKBlock) * nt;
+    if (sf) {      // digits of the real rows R, of R diag(w_t) and of Z' (two parts): each type's
+                   // rows on whole k-blocks
+        const int64_t KT = round_up(round_up(twoL, kRealKBlock) * nt, kKBlock);
         auto dig = [&](int64_t planes) {
             return round_up(planes * rows * (KT + pitch_pad()), 1024) + round_up(4 * rows, 1024);
         };
-        return dig((use_pair() ? 4 : 2) * s) + 2 * dig(2 * s) + 4096;
+        return 2 * dig(s) + dig(2 * s) + 4096;
     }
     const int64_t Kp = round_up(bpad * panel_atoms(na, panels), kKBlock);
     const int64_t Kx = hoist ? std::max(Kp, round_up(bpad * nt, kKBlock)) : Kp;
@@ -1961,34 +1661,40 @@ int64_t ozaki_group_bytes(int s, int64_t twoL, int64_t na, int64_t nt, const std
 }
 
 int64_t ozaki_group_persist_bytes(int s, int64_t twoL, int64_t na, int64_t nt, const std::vector<int64_t> &G,
-                                  int panels) {
+                                  int panels, bool sf) {
     const int64_t bpad = round_up(atom_stride(twoL), kKBlock);    // T operand: one atom's rows per plane row
     const int64_t nk = (int64_t)G.size();
-    int64_t tiles_t = 0, tiles_sh = 0, tiles_blk = 0;
+    if (sf) {
+        int64_t tiles_t = 0, tiles_sh = 0;
+        for (int64_t g : G) {
+            const int64_t tn = (g + kRealTileN - 1) / kRealTileN, tm = (g + kRealTileM - 1) / kRealTileM;
+            tiles_t += nt * ((2 * twoL + kRealTileM - 1) / kRealTileM) * tn;
+            tiles_sh += 3 * nt * tm * tn;                // (more than the lower triangle's)
+        }
+        return operand_bytes(s, 2 * nt * twoL, bpad, s) + round_up(sizeof(RealJob) * nk * nt, 1024) +
+               round_up(sizeof(RealJob) * 3 * nk * nt, 1024) + round_up(sizeof(int4) * (tiles_t + 1), 1024) +
+               2 * round_up(sizeof(int4) * (tiles_sh + 1), 1024) + 8192;
+    }
+    int64_t tiles_t = 0, tiles_sh = 0;
     for (int64_t g : G) {
-        const int64_t T = (g + kTileN - 1) / kTileN, Tp = (g + kPairTile - 1) / kPairTile;
+        const int64_t T = (g + kTileN - 1) / kTileN;
         tiles_t += std::max(na, nt) * ((twoL + kTileM - 1) / kTileM) * T;
         tiles_sh += T * (T + 1);
-        tiles_blk += Tp * (Tp + 1);
     }
-    return operand_bytes(s, nt * twoL, bpad, use_pair() ? 4 * s : 2 * s) +
-           round_up(sizeof(OzJob) * nk * (std::max(na, nt) + 2), 1024) +
+    return operand_bytes(s, nt * twoL, bpad, 2 * s) + round_up(sizeof(OzJob) * nk * (std::max(na, nt) + 2), 1024) +
            round_up(sizeof(OzJob) * 2 * nk * panels, 1024) + round_up(sizeof(int4) * (tiles_t + panels), 1024) +
-           round_up(sizeof(int4) * (tiles_sh + 1), 1024) + round_up(sizeof(int) * kProgressCap, 1024) +
-           round_up(sizeof(int4) * (nt * tiles_blk + 1), 1024) + 8192;
+           round_up(sizeof(int4) * (tiles_sh + 1), 1024) + round_up(sizeof(int) * kProgressCap, 1024) + 8192;
 }
 
-// The streamed host output's launches (pair tiles).  The tile columns are split into
-// kOutColumnBlocks ranges of about equal lower-triangle tile counts; the tile list runs through
-// them in order, and within a range type by type, each type in the per-type schedule's order (so
-// that the pairs working at a time share few types' operands in L2).  The list is then cut into
-// launches of whole waves (one tile per cluster pair of the GPU); launch b leaves columns
-// [blk_col[b], blk_col[b+1]) complete (possibly none).  jobs0: the first type's S/H jobs.
-static int build_output_blocks(OzGroup *g, const std::vector<OzJob> &jobs0, int64_t tile) {
-    std::vector<int4> l0;
-    build_schedule(jobs0, l0, tile);
+// The streamed host output's launches.  The output columns are split into kOutColumnBlocks ranges
+// (whole tile columns) of about equal lower-triangle areas; the tile list runs through them in
+// order, and within a range type by type, each type in the per-type schedule's order (so that the
+// pairs working at a time share few types' operands in L2).  The list is then cut into launches of
+// whole waves (one tile per cluster pair of the GPU); launch b leaves columns
+// [blk_col[b], blk_col[b+1]) complete (possibly none).  l0: the first type's tiles.
+static int build_output_blocks(OzGroup *g, const std::vector<int4> &l0) {
     int64_t T = 0;
-    for (const auto &j : jobs0) T = std::max<int64_t>(T, (j.n + tile - 1) / tile);
+    for (const int4 &e : l0) T = std::max<int64_t>(T, e.z + 1);
     g->nblk = 0;
     if (T < 2) return HSDLA_OK;
     const int C = (int)std::min<int64_t>(kOutColumnBlocks, T);
@@ -2022,19 +1728,25 @@ static int build_output_blocks(OzGroup *g, const std::vector<OzJob> &jobs0, int6
     for (int64_t i0 = 0; i0 < N && g->nblk < kMaxOutBlocks; ++g->nblk) {
         const int64_t i1 = g->nblk + 1 == kMaxOutBlocks ? N : std::min(N, i0 + per);
         g->blk_begin[g->nblk + 1] = i1;
-        g->blk_col[g->nblk + 1] = std::max(g->blk_col[g->nblk], open[i1] * tile);
+        g->blk_col[g->nblk + 1] = std::max(g->blk_col[g->nblk], open[i1] * kRealTileN);
         i0 = i1;
     }
-    g->blk_col[g->nblk] = T * tile;
+    g->blk_col[g->nblk] = T * kRealTileN;
     const cudaError_t e = cudaMemcpy(g->d_list_blk, lb.data(), sizeof(int4) * N, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) { g_oz_err = cudaGetErrorString(e); return HSDLA_ERR_CUDA; }
     return HSDLA_OK;
 }
 
-// Structure-factor form of a group: digit planes of M, M diag(w_t) and Z (2L rows per type, each
-// type's rows starting on a k-block so that the per-type products never mix types), the T
-// application Z_t = T_t M_t, and per type one S/H launch into the products PS, PH followed by the
-// combine into S and H.
+static void set_sh_tiles(OzGroup *g, int halves, bool merged) {
+    g->halves = halves;
+    g->merged = merged;
+    g->bands = real_bands(g->s, merged ? 2 : 1, halves, g->twoL);
+}
+
+// Structure-factor form of a group, on the real rows (real_products.cu): digit planes of R, R
+// diag(w_t) and Z' (2L rows per type, each type's rows starting on a k-block so that the per-type
+// products never mix types), the T application Z'_t = T'_t R_t, and the products S, Re H, Im H of
+// every type of a combine batch in one launch, followed by the combine into S and H.
 static int group_prepare_sf(OzakiPlan &oz, const OzGroupDesc &d, const std::vector<OzKBufs> &kb, void *ws,
                             void *persist, cudaStream_t st, OzGroup **out) {
     auto *g = new OzGroup();
@@ -2043,20 +1755,18 @@ static int group_prepare_sf(OzakiPlan &oz, const OzGroupDesc &d, const std::vect
     g->nk = (int)kb.size();
     g->hoist = true;
     g->twoL = d.twoL; g->na = d.na; g->nt = d.nt;
-    // type stride along the contraction: whole 128-byte k-blocks (TMA boxes aligned to them; a
-    // 32-byte stride for lmax 8 put every other type's boxes across 128-byte lines: c3 10.3 -> 12.4 ms)
-    g->pair = use_pair();
-    g->bpad = round_up(d.twoL, kKBlock);
-    const int64_t tkb = g->bpad / kKBlock, KT = g->bpad * d.nt;
-    // K steps of 32 bytes in a type's last k-block (the contraction length is 2L per type)
-    const int ksl = (int)((d.twoL - (tkb - 1) * kKBlock + 31) / 32);
+    // type stride along the contraction: whole 64-byte chunks
+    g->bpad = round_up(d.twoL, kRealKBlock);
+    const int64_t tkb = g->bpad / kRealKBlock, KT = round_up(g->bpad * d.nt, kKBlock);
+    // K steps of 32 bytes in a type's last chunk (the contraction length is 2L per type)
+    const int ksl = (int)((d.twoL - (tkb - 1) * kRealKBlock + 31) / 32);
     g->kb = kb;
     g->d_err = oz.d_error;
     g->sf_tab = d.sf_tab;
     g->tbatch = std::max(1, d.tbatch);
-    // HSDLA_COMBINE_OVERLAP=1: the first half of the combine on a side stream, next to the S/H
-    // launches of the other types.  Off by default: on the 8000-column workload the co-running
-    // combine slowed the S/H launches by more than it saved (31.7 against 31.4 ms per k-point).
+    // HSDLA_COMBINE_OVERLAP=1: the first half of the combine on a side stream, next to the products
+    // of the other types.  Off by default: on the 8000-column workload the co-running combine slowed
+    // the products by more than it saved.
     if (g->tbatch >= d.nt && d.nt >= 2 && env_int("HSDLA_COMBINE_OVERLAP", 0) != 0) {
         g->side_types = (int)(d.nt / 2);
         if (cudaStreamCreateWithFlags(&g->side, cudaStreamNonBlocking) != cudaSuccess ||
@@ -2082,138 +1792,101 @@ static int group_prepare_sf(OzakiPlan &oz, const OzGroupDesc &d, const std::vect
         o.digits = ar.take<uint8_t>(planes * o.plane_rows * o.pitch);
         o.expo = ar.take<int32_t>(o.plane_rows);
     };
-    // M: the S/H products' left operand; on pair tiles with its digits scaled by 2^-5 as well
-    // (planes 2s .. 4s-1), the merged accumulation units' left digits
-    carve_rows(g->dM, g->pair ? 4 * s : 2 * s);
-    carve_rows(g->dW, 2 * s);    // M diag(w_t)
-    carve_rows(g->dX, 2 * s);    // Z
-    // T: the left operand of the T application, with its scaled copy on pair tiles
-    carve_operand(keep, g->dT, s, d.nt * d.twoL, tkb * kKBlock, g->pair ? 4 * s : 2 * s);
+    carve_rows(g->dM, s);        // R
+    carve_rows(g->dW, s);        // R diag(w_t)
+    carve_rows(g->dX, 2 * s);    // Z'
+    carve_operand(keep, g->dT, s, 2 * d.nt * d.twoL, round_up(g->bpad, kKBlock), s);
     const int64_t nk = g->nk;
-    int64_t tiles_t = 0, tiles_sh = 0;
-    for (int64_t x : G) {
-        const int64_t T = (x + kTileN - 1) / kTileN;
-        tiles_t += d.nt * ((d.twoL + kTileM - 1) / kTileM) * T;
-        tiles_sh += T * (T + 1);
-    }
-    g->d_jobs_t = keep.take<OzJob>(nk * (d.nt + 2));
-    g->d_jobs_sh = keep.take<OzJob>(2 * nk * d.nt);
-    g->d_list_t = keep.take<int4>(tiles_t + 1);
-    g->d_list_sh = keep.take<int4>(tiles_sh + 1);
-    g->d_progress = keep.take<int>(kProgressCap);
-    int64_t tiles_blk = 0;
-    for (int64_t x : G) {
-        const int64_t Tp = (x + kPairTile - 1) / kPairTile;
-        tiles_blk += Tp * (Tp + 1);
-    }
-    g->d_list_blk = keep.take<int4>(d.nt * tiles_blk + 1);
     auto fail = [&](int code) { ozaki_group_destroy(g); return code; };
-    auto table = [&](const DigitOperand &o, int which) {
-        SliceTab t;
-        t.nk = g->nk; t.s = s; t.ldz = d.twoL * d.nt; t.Kin = d.twoL * d.nt; t.rpb = d.twoL; t.bpad = g->bpad;
-        t.digits = o.digits; t.Kpad = KT; t.plane_rows = o.plane_rows; t.pitch = o.pitch; t.expo = o.expo;
-        for (int k = 0; k < g->nk; ++k) t.e[k] = SliceEntry{which == 0 ? kb[k].M : kb[k].Z, kb[k].G, g->row0[k]};
+    auto table = [&](const DigitOperand &o, int parts) {
+        RealSliceTab t;
+        t.nk = g->nk; t.s = s; t.parts = parts;
+        t.ldz = parts * d.twoL * d.nt; t.blocks = d.nt; t.rpb = d.twoL; t.bstride = parts * d.twoL;
+        t.pstride = d.twoL; t.bpad = g->bpad;
+        t.digits = o.digits; t.plane_rows = o.plane_rows; t.pitch = o.pitch; t.expo = o.expo;
+        for (int k = 0; k < g->nk; ++k)
+            t.e[k] = RealSliceEntry{parts == 1 ? (const void *)kb[k].R : (const void *)kb[k].ZR, kb[k].G, g->row0[k]};
         return t;
     };
-    g->tM = table(g->dM, 0);              // dual: M and M diag(w_t)
-    g->tM.scaled = g->pair ? 1 : 0;
-    g->tM.v2 = d.wt;
-    g->tM.digits2 = g->dW.digits;
-    g->tM.expo2 = g->dW.expo;
-    OzPanel p;                            // one "panel" carries the Z slicing table
-    p.a0 = 0; p.a1 = d.na;
-    p.tX = table(g->dX, 1);
-    g->pan.push_back(p);
+    g->rM = table(g->dM, 1);              // dual: R and R diag(w_t)
+    g->rM.v2 = d.wt;
+    g->rM.digits2 = g->dW.digits;
+    g->rM.expo2 = g->dW.expo;
+    g->bands_t = real_bands(s, 2, 2, d.twoL);
+    g->rX = table(g->dX, 2);
+    g->rX.frac = g->bands_t.frac;         // Z' in fixed point, with T's row and R's column exponents
+    g->rX.el = g->dT.expo;
+    g->rX.er = g->dM.expo;
     g->panels = 1;
-    SliceTab tT = slice_table(d.Tfull, d.twoL, nullptr, d.twoL, d.nt * d.twoL, d.twoL, g->bpad, s, g->dT);
-    tT.scaled = g->pair ? 1 : 0;
-    cudaError_t e = slice_launch(tT, st);    // stream-ordered before every use of the T digits
+    RealSliceTab tT;
+    tT.nk = 1; tT.s = s; tT.ldz = d.twoL; tT.blocks = 1; tT.rpb = d.twoL; tT.bstride = d.twoL; tT.bpad = g->bpad;
+    tT.digits = g->dT.digits; tT.plane_rows = g->dT.plane_rows; tT.pitch = g->dT.pitch; tT.expo = g->dT.expo;
+    tT.e[0] = RealSliceEntry{d.TR, 2 * d.nt * d.twoL, 0};
+    cudaError_t e = launch_real_slice(tT, st);    // stream-ordered before every use of the T digits
     if (e != cudaSuccess) { g_oz_err = cudaGetErrorString(e); return fail(HSDLA_ERR_CUDA); }
-    int rc = make_map(g->dM, g->pair ? 2 * s : s);
-    if (!rc) rc = make_map(g->dW, s);
-    if (!rc) rc = make_map(g->dX, s);
-    if (!rc) rc = make_map(g->dT, g->pair ? 2 * s : s);
-    // half-width pair tiles (HSDLA_PAIR_HALVES=1: full width; the tile tuner may switch the S/H
-    // launches): the right operands' 64-row maps, made for both shapes
-    g->halves = g->pair && env_int("HSDLA_PAIR_HALVES", 2) == 2 ? 2 : 1;
-    g->halves_t = g->halves;
-    if (!rc && g->pair) rc = make_map(g->dM, 2 * s, kPairTile / 4, &g->dM.map64);
-    if (!rc && g->pair) rc = make_map(g->dW, s, kPairTile / 4, &g->dW.map64);
-    if (!rc && g->pair) rc = make_map(g->dX, s, kPairTile / 4, &g->dX.map64);
+    // left operands in boxes of a CTA's 128 rows, right operands of its 64 rows
+    int rc = make_map(g->dM, s, kRealTileM / 2, &g->dM.map, kRealKBlock);
+    if (!rc) rc = make_map(g->dT, s, kRealTileM / 2, &g->dT.map, kRealKBlock);
+    if (!rc) rc = make_map(g->dM, s, kRealBRows, &g->dM.map64, kRealKBlock);
+    if (!rc) rc = make_map(g->dW, s, kRealBRows, &g->dW.map64, kRealKBlock);
+    if (!rc) rc = make_map(g->dX, 2 * s, kRealBRows, &g->dX.map64, kRealKBlock);
     if (rc) return fail(rc);
-    // T application per type: Z_t = T_t M_t
-    std::vector<OzJob> jt;
+    // T application per type: the real and imaginary rows of Z'_t = T'_t R_t as one product
+    std::vector<RealJob> jt, jsh;
     for (int k = 0; k < g->nk; ++k)
         for (int64_t t = 0; t < d.nt; ++t) {
-            OzJob j;
+            RealJob j;
             memset(&j, 0, sizeof(j));
-            j.lmap = 3; j.rmap = 0;
-            j.lplane = g->dT.plane_rows; j.rplane = g->dM.plane_rows;
-            j.lrow0 = t * d.twoL; j.rrow0 = g->row0[k];
+            j.rmap = 0; j.rstep = 1;
+            j.lplane = g->dT.plane_rows; j.rplane = g->rows;
+            j.lrow0 = 2 * t * d.twoL; j.rrow0 = g->row0[k];
             j.rk0 = t * g->bpad;
-            j.nkb = tkb;
-            j.ksteps_last = ksl;
-            j.m = d.twoL; j.n = kb[k].G;
-            j.out = kb[k].Z + d.twoL * t; j.ldo = d.twoL * d.nt;
-            j.el = g->dT.expo + t * d.twoL; j.er = g->dM.expo + g->row0[k];
+            j.nkb = tkb; j.ksteps_last = ksl;
+            j.m = 2 * d.twoL; j.n = kb[k].G;
+            j.out = kb[k].ZR + 2 * d.twoL * t; j.ldo = 2 * d.twoL * d.nt;
             jt.push_back(j);
         }
-    g->n_jobs_t = (int)jt.size();
-    // on pair tiles (256 x 256: one tile row per type) in merged accumulation units
-    rc = upload_schedule(jt, g->d_jobs_t, g->d_list_t, g->tiles_t, g->pair ? kPairTile : kTileN);
-    g->units_t = g->pair ? pair_units(s, tkb, env_int("HSDLA_MERGE", 1) != 0, d.twoL) : pair_units_plain(s);
-    if (rc) return fail(rc);
-    g->maps_t[0] = g->halves_t == 2 ? g->dM.map64 : g->dM.map;  // right operand
-    g->maps_t[1] = g->dM.map; g->maps_t[2] = g->dM.map; g->maps_t[3] = g->dT.map;
-    // per type: S_t = M_t^H diag(w_t) M_t and H_t = M_t^H Z_t into the products; on pair tiles
-    // with merged accumulation units (HSDLA_MERGE=0: one per diagonal)
-    g->merged = env_int("HSDLA_MERGE", 1) != 0;
-    g->units = g->pair ? pair_units(s, tkb, g->merged, d.twoL) : pair_units_plain(s);
-    const int64_t tile = g->pair ? kPairTile : kTileN;
-    g->n_jobs_sh = 2 * g->nk;
-    std::vector<OzJob> all;
-    for (int64_t t = 0; t < d.nt; ++t) {
-        std::vector<OzJob> jsh;
+    for (int64_t t = 0; t < d.nt; ++t)
         for (int k = 0; k < g->nk; ++k)
-            for (int which = 0; which < 2; ++which) {
-                OzJob j;
+            for (int which = 0; which < 3; ++which) {     // S, Re H, Im H
+                RealJob j;
                 memset(&j, 0, sizeof(j));
-                j.lmap = 0; j.rmap = which == 0 ? 1 : 2; j.lower = 1;
+                j.rmap = which == 0 ? 0 : 1; j.lower = 1;
+                j.rstep = which == 0 ? 1 : 2; j.rpart = which == 2 ? 1 : 0;
                 j.lplane = g->rows; j.rplane = g->rows;
                 j.lrow0 = g->row0[k]; j.rrow0 = g->row0[k];
                 j.lk0 = t * g->bpad; j.rk0 = t * g->bpad;
-                j.nkb = tkb;
-                j.ksteps_last = ksl;
+                j.nkb = tkb; j.ksteps_last = ksl;
                 j.m = kb[k].G; j.n = kb[k].G;
-                j.out = (which == 0 ? kb[k].PS : kb[k].PH) + (t % g->tbatch) * kb[k].pstride;
+                j.out = (which == 0 ? kb[k].RS : which == 1 ? kb[k].RHr : kb[k].RHi) + (t % g->tbatch) * kb[k].pstride;
                 j.ldo = kb[k].G;
-                j.el = g->dM.expo + g->row0[k];
-                j.er = (which == 0 ? g->dW.expo : g->dX.expo) + g->row0[k];
                 jsh.push_back(j);
             }
-        if (t == 0) {
-            rc = upload_schedule(jsh, g->d_jobs_sh, g->d_list_sh, g->tiles_sh, tile);
-            if (rc) return fail(rc);
-        } else {
-            int64_t total = 0;
-            for (auto &j : jsh) {
-                j.tiles_n = (j.n + tile - 1) / tile;
-                j.tile_begin = total;
-                total += job_tiles(j, tile);
-            }
-        }
-        all.insert(all.end(), jsh.begin(), jsh.end());
-    }
-    e = cudaMemcpy(g->d_jobs_sh, all.data(), sizeof(OzJob) * all.size(), cudaMemcpyHostToDevice);
+    g->n_jobs_sh = (int)(3 * nk);
+    std::vector<int4> lt, lsh, l0;
+    real_schedule(jt, lt);
+    real_schedule(std::vector<RealJob>(jsh.begin(), jsh.begin() + g->n_jobs_sh), l0);
+    for (int t = 0; t < d.nt; ++t)
+        for (const int4 &x : l0) lsh.push_back(make_int4(t * g->n_jobs_sh + x.x, x.y, x.z, 0));
+    g->tiles_t = (int64_t)lt.size();
+    g->tiles_sh = (int64_t)l0.size();
+    int64_t want_t = 0, want_sh = 0;
+    for (auto &j : jt) want_t += real_job_tiles(j);
+    for (int q = 0; q < g->n_jobs_sh; ++q) want_sh += real_job_tiles(jsh[q]);
+    if (want_t != g->tiles_t || want_sh != g->tiles_sh) { g_oz_err = "tile schedule size mismatch"; return fail(HSDLA_ERR_ARG); }
+    g->d_rjobs_t = keep.take<RealJob>((int64_t)jt.size());
+    g->d_rjobs_sh = keep.take<RealJob>((int64_t)jsh.size());
+    g->d_list_t = keep.take<int4>((int64_t)lt.size() + 1);
+    g->d_list_sh = keep.take<int4>((int64_t)lsh.size() + 1);
+    g->d_list_blk = keep.take<int4>((int64_t)lsh.size() + 1);
+    e = cudaMemcpy(g->d_rjobs_t, jt.data(), sizeof(RealJob) * jt.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(g->d_rjobs_sh, jsh.data(), sizeof(RealJob) * jsh.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(g->d_list_t, lt.data(), sizeof(int4) * lt.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(g->d_list_sh, lsh.data(), sizeof(int4) * lsh.size(), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) { g_oz_err = cudaGetErrorString(e); return fail(HSDLA_ERR_CUDA); }
-    if (g->pair) {
-        rc = build_output_blocks(g, std::vector<OzJob>(all.begin(), all.begin() + g->n_jobs_sh), tile);
-        if (rc) return fail(rc);
-    }
-    g->maps_sh[0] = g->dM.map;
-    g->maps_sh[1] = g->halves == 2 ? g->dW.map64 : g->dW.map;   // right operands
-    g->maps_sh[2] = g->halves == 2 ? g->dX.map64 : g->dX.map;
-    g->maps_sh[3] = g->dM.map;
+    rc = build_output_blocks(g, l0);
+    if (rc) return fail(rc);
+    set_sh_tiles(g, env_int("HSDLA_PAIR_HALVES", 2) == 2 ? 2 : 1, env_int("HSDLA_MERGE", 1) != 0);
     *out = g;
     return HSDLA_OK;
 }
@@ -2316,11 +1989,11 @@ int ozaki_group_prepare(OzakiPlan &oz, const OzGroupDesc &d, const std::vector<O
     cudaError_t e = slice(d.Tfull, d.twoL, nullptr, d.twoL, d.nt * d.twoL, d.twoL, g->bpad, s, g->dT, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) { g_oz_err = cudaGetErrorString(e); return fail(HSDLA_ERR_CUDA); }
-    rc = make_map(g->dC, s);
-    if (!rc) rc = make_map(g->dW, s);
-    if (!rc) rc = make_map(g->dX, s);
-    if (!rc) rc = make_map(g->dT, s);
-    if (!rc && d.hoist) rc = make_map(g->dM, s);
+    rc = make_map(g->dC, 2 * s);
+    if (!rc) rc = make_map(g->dW, 2 * s);
+    if (!rc) rc = make_map(g->dX, 2 * s);
+    if (!rc) rc = make_map(g->dT, 2 * s);
+    if (!rc && d.hoist) rc = make_map(g->dM, 2 * s);
     if (rc) return fail(rc);
     // (b) T application: per type once (hoisted), or per atom of each panel
     if (d.hoist) {
@@ -2374,7 +2047,6 @@ int ozaki_group_prepare(OzakiPlan &oz, const OzGroupDesc &d, const std::vector<O
     g->maps_t[1] = g->maps_t[0]; g->maps_t[2] = g->maps_t[0]; g->maps_t[3] = g->dT.map;
     // (c) S and H jobs of every panel; outputs are patched per run, later panels accumulate
     g->pair = use_pair();
-    g->units = pair_units_plain(g->s);
     const int64_t tile = g->pair ? kPairTile : kTileN;
     g->n_jobs_sh = 2 * g->nk;
     for (int pi = 0; pi < g->panels; ++pi) {
@@ -2413,6 +2085,14 @@ int ozaki_group_prepare(OzakiPlan &oz, const OzGroupDesc &d, const std::vector<O
     return HSDLA_OK;
 }
 
+void ozaki_group_sf_exponents(const OzGroup *g, SfTab &t) {
+    t.frac = g->bands.frac;
+    for (int k = 0; k < g->nk; ++k) {
+        t.e[k].el = g->dM.expo + g->row0[k];
+        t.e[k].ers = g->dW.expo + g->row0[k];
+        t.e[k].erh = g->dX.expo + g->row0[k];
+    }
+}
 void ozaki_group_set_sf(OzGroup *g, const SfTab &t) { g->sft = t; }
 int ozaki_group_last_combine(const OzGroup *g) {
     if (g->side_types > 0) return g->side_types;
@@ -2447,11 +2127,16 @@ static cudaError_t record(cudaEvent_t ev, cudaStream_t st) {
 int ozaki_group_tapply_events(const OzGroup *g) { return (g->sf || g->hoist) ? 1 : g->panels; }
 
 bool ozaki_group_streamable(const OzGroup *g) {
-    return g && g->sf && g->pair && g->nblk > 1 && g->tbatch >= g->nt && g->side_types == 0 &&
+    return g && g->sf && g->nblk > 1 && g->tbatch >= g->nt && g->side_types == 0 &&
            env_int("HSDLA_STREAM_OUTPUT", 1) != 0;
 }
 
 int ozaki_group_output_blocks(const OzGroup *g) { return g ? g->nblk : 0; }
+
+// Products of `tiles` entries of a tile list.
+static cudaError_t launch_sh(const OzGroup *g, const int4 *list, int64_t tiles, cudaStream_t st) {
+    return launch_real_products(g->dM.map, g->dW.map64, g->dX.map64, g->d_rjobs_sh, list, tiles, g->bands, g->d_err, st);
+}
 
 // The streamed host output's S/H part.  Per column block: one pair launch over every type's tiles
 // of the block, then the block's combine on the main stream, which writes the block's diagonal
@@ -2477,9 +2162,7 @@ static cudaError_t run_sh_streamed(OzGroup *g, cudaStream_t st, const cudaEvent_
         const bool last = b + 1 == g->nblk;
         if (b < npair) e = record(ev[2 * b], st);
         if (e == cudaSuccess)
-            e = launch_pair(g->maps_sh, g->s, g->d_err, g->d_jobs_sh, g->n_jobs_sh * g->nt,
-                            g->blk_begin[b + 1] - g->blk_begin[b], g->d_list_blk + g->blk_begin[b], nullptr, st,
-                            g->units, g->halves);
+            e = launch_sh(g, g->d_list_blk + g->blk_begin[b], g->blk_begin[b + 1] - g->blk_begin[b], st);
         if (e == cudaSuccess && b < npair) e = record(ev[2 * b + 1], st);
         SfTab tab = out;
         tab.type = 0;
@@ -2537,15 +2220,13 @@ int ozaki_group_run(OzGroup *g, const DevSystem &sys, const KTable &ktab, cudaSt
     int nl = 0;
     cudaError_t e = cudaSuccess;
     if (g->sf) {
-        e = slice_launch(g->tM, st);                      // M and M diag(w_t)
+        e = launch_real_slice(g->rM, st);                 // R and R diag(w_t)
         if (e == cudaSuccess && tev) e = cudaEventRecord(ev_t[0], st);
         if (e == cudaSuccess)
-            e = g->pair ? launch_pair(g->maps_t, g->s, g->d_err, g->d_jobs_t, g->n_jobs_t, g->tiles_t, g->d_list_t,
-                                      nullptr, st, g->units_t, g->halves_t)
-                        : launch_prepared(g->maps_t, g->s, g->d_err, g->d_jobs_t, g->n_jobs_t, g->tiles_t,
-                                          g->d_list_t, nullptr, st);
+            e = launch_real_products(g->dT.map, g->dM.map64, g->dM.map64, g->d_rjobs_t, g->d_list_t, g->tiles_t,
+                                     g->bands_t, g->d_err, st);
         if (e == cudaSuccess && tev) e = cudaEventRecord(ev_t[1], st);
-        if (e == cudaSuccess) e = slice_launch(g->pan[0].tX, st);    // Z
+        if (e == cudaSuccess) e = launch_real_slice(g->rX, st);      // Z'
         nl += 3;
         if (host_out && ozaki_group_streamable(g)) {
             if (e == cudaSuccess) e = run_sh_streamed(g, st, ev, nev, *host_out, &nl);
@@ -2553,62 +2234,42 @@ int ozaki_group_run(OzGroup *g, const DevSystem &sys, const KTable &ktab, cudaSt
             if (e != cudaSuccess) { g_oz_err = cudaGetErrorString(e); return HSDLA_ERR_CUDA; }
             return HSDLA_OK;
         }
-        for (int t = 0; t < g->nt && e == cudaSuccess; ++t) {
-            const OzJob *jobs = g->d_jobs_sh + (int64_t)g->n_jobs_sh * t;
-            if (nev >= 2 * g->nt) e = record(ev[2 * t], st);
-            // no grid lockstep here: the per-type operands are small enough for L2 without it, and
-            // pairs that drift apart spread their drains over the MMA phases of the others (c2
-            // 34.5 -> 33.8 ms, c3 11.7 -> 11.4 ms, c4 461 -> 442 ms per k-point)
-            if (e == cudaSuccess)
-                e = g->pair ? launch_pair(g->maps_sh, g->s, g->d_err, jobs, g->n_jobs_sh, g->tiles_sh, g->d_list_sh,
-                                          nullptr, st, g->units, g->halves)
-                            : launch_prepared(g->maps_sh, g->s, g->d_err, jobs, g->n_jobs_sh, g->tiles_sh,
-                                              g->d_list_sh, g->d_progress, st);
-            if (e == cudaSuccess && nev >= 2 * g->nt) e = record(ev[2 * t + 1], st);
+        // batches of types: their products in one launch, then their combine into S and H (the
+        // caller combines the group's last batch when it defers it).  With a side stream the one
+        // batch runs in two parts, the first part's combine beside the second part's products.
+        const int step = g->side_types > 0 ? g->side_types : g->tbatch;
+        int p = 0;
+        for (int t0 = 0; t0 < g->nt && e == cudaSuccess; ++p) {
+            const int t1 = g->side_types > 0 && t0 > 0 ? (int)g->nt : (int)std::min<int64_t>(g->nt, t0 + step);
+            const bool last = t1 == g->nt, timed = 2 * p + 1 < nev;
+            if (timed) e = record(ev[2 * p], st);
+            if (e == cudaSuccess) e = launch_sh(g, g->d_list_sh + t0 * g->tiles_sh, (t1 - t0) * g->tiles_sh, st);
+            if (e == cudaSuccess && timed) e = record(ev[2 * p + 1], st);
             nl += 1;
-            if (g->side_types > 0) {
-                // the first side_types types' products into S and H on the side stream, then the
-                // rest (the caller's when it defers the last combine)
-                if (e == cudaSuccess && t + 1 == g->side_types) {
-                    SfTab tab = g->sft;
-                    tab.type = 0;
-                    tab.ntypes = g->side_types;
-                    tab.slot0 = 0;
-                    // plain records: under graph capture they fork the side stream into the graph
-                    // and join it back
-                    e = cudaEventRecord(g->ev_fork, st);
-                    if (e == cudaSuccess) e = cudaStreamWaitEvent(g->side, g->ev_fork, 0);
-                    if (e == cudaSuccess) e = launch_sf_combine(tab, g->sf_tab, true, g->side);
-                    if (e == cudaSuccess) e = cudaEventRecord(g->ev_join, g->side);
+            SfTab tab = g->sft;
+            tab.type = t0;
+            tab.ntypes = t1 - t0;
+            tab.slot0 = t0 % g->tbatch;
+            if (g->side_types > 0 && !last) {
+                // plain records: under graph capture they fork the side stream into the graph
+                // and join it back
+                if (e == cudaSuccess) e = cudaEventRecord(g->ev_fork, st);
+                if (e == cudaSuccess) e = cudaStreamWaitEvent(g->side, g->ev_fork, 0);
+                if (e == cudaSuccess) e = launch_sf_combine(tab, g->sf_tab, true, g->side);
+                if (e == cudaSuccess) e = cudaEventRecord(g->ev_join, g->side);
+                nl += 1;
+            } else {
+                if (e == cudaSuccess && g->side_types > 0) e = cudaStreamWaitEvent(st, g->ev_join, 0);
+                if (e == cudaSuccess && !(defer_last_combine && last)) {
+                    e = launch_sf_combine(tab, g->sf_tab, t0 == 0, st);
                     nl += 1;
                 }
-                if (e == cudaSuccess && t + 1 == g->nt) {
-                    e = cudaStreamWaitEvent(st, g->ev_join, 0);
-                    if (e == cudaSuccess && !defer_last_combine) {
-                        SfTab tab = g->sft;
-                        tab.type = g->side_types;
-                        tab.ntypes = g->nt - g->side_types;
-                        tab.slot0 = g->side_types;
-                        e = launch_sf_combine(tab, g->sf_tab, false, st);
-                        nl += 1;
-                    }
-                }
-                continue;
             }
-            // the batch's last type: its products into S and H (the caller combines the group's last
-            // batch when it defers it)
-            if (e == cudaSuccess && ((t + 1) % g->tbatch == 0 || t + 1 == g->nt) &&
-                !(defer_last_combine && t + 1 == g->nt)) {
-                const int t0 = t / g->tbatch * g->tbatch;
-                g->sft.type = t0;
-                g->sft.ntypes = t + 1 - t0;
-                e = launch_sf_combine(g->sft, g->sf_tab, t0 == 0, st);
-                nl += 1;
-            }
+            t0 = t1;
         }
-        // event pairs past the types (kept for the streamed form's column blocks) span nothing,
-        // after the S/H launches (the last event closes the group's products)
-        for (int p = g->nt; nev >= 2 * g->nt && p < nev / 2 && e == cudaSuccess; ++p) {
+        // event pairs past the batches (kept for the streamed form's column blocks) span nothing,
+        // after the products (the last event closes the group's products)
+        for (; 2 * p + 1 < nev && e == cudaSuccess; ++p) {
             e = record(ev[2 * p], st);
             if (e == cudaSuccess) e = record(ev[2 * p + 1], st);
         }
@@ -2653,7 +2314,7 @@ int ozaki_group_run(OzGroup *g, const DevSystem &sys, const KTable &ktab, cudaSt
         const OzJob *jobs = g->d_jobs_sh + (int64_t)g->n_jobs_sh * pi;
         if (e == cudaSuccess)
             e = g->pair ? launch_pair(g->maps_sh, g->s, g->d_err, jobs, g->n_jobs_sh, g->tiles_sh, g->d_list_sh,
-                                      g->d_progress, st, g->units)
+                                      g->d_progress, st)
                         : launch_prepared(g->maps_sh, g->s, g->d_err, jobs, g->n_jobs_sh, g->tiles_sh, g->d_list_sh,
                                           g->d_progress, st);
         nl += 1;
@@ -2664,18 +2325,7 @@ int ozaki_group_run(OzGroup *g, const DevSystem &sys, const KTable &ktab, cudaSt
     return HSDLA_OK;
 }
 
-// The structure-factor form's S/H tile configuration: tile shape (halves 1: 256 x 256
-// accumulators; 2: two 256 x 128 halves in alternating TMEM buffers) and accumulation split
-// (merged: adjacent digit diagonals share an exact FP32 unit; else one unit per diagonal).
-static void set_sh_tiles(OzGroup *g, int halves, bool merged) {
-    g->halves = halves;
-    g->merged = merged;
-    g->units = pair_units(g->s, g->bpad / kKBlock, merged, g->twoL);
-    g->maps_sh[1] = halves == 2 ? g->dW.map64 : g->dW.map;
-    g->maps_sh[2] = halves == 2 ? g->dX.map64 : g->dX.map;
-}
-
-bool ozaki_group_tunable(const OzGroup *g) { return g && g->sf && g->pair; }
+bool ozaki_group_tunable(const OzGroup *g) { return g && g->sf; }
 
 void ozaki_group_tiles(const OzGroup *g, int *halves, int *merged) {
     *halves = g->halves;
@@ -2686,13 +2336,13 @@ void ozaki_group_set_tiles(OzGroup *g, int halves, int merged) {
     if (ozaki_group_tunable(g)) set_sh_tiles(g, halves == 1 ? 1 : 2, merged != 0);
 }
 
-// Times the first type's S/H launch (every k-point of the group) in each configuration and keeps
+// Times the first type's products (every k-point of the group) in each configuration and keeps
 // the fastest.  The digit planes must hold a completed run's data (the launches only rewrite that
 // type's product slot, which the run has combined already).  Each configuration runs twice, the
 // second timed.
 int ozaki_group_tune_tiles(OzGroup *g, cudaStream_t st, float *ms_best) {
     if (!ozaki_group_tunable(g)) return HSDLA_OK;
-    const int cfg[4][2] = {{2, 1}, {1, 1}, {2, 0}, {1, 0}};
+    const int cfg[2][2] = {{2, 1}, {2, 0}};
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) {
         if (e0) cudaEventDestroy(e0);
@@ -2707,7 +2357,7 @@ int ozaki_group_tune_tiles(OzGroup *g, cudaStream_t st, float *ms_best) {
     float best = -1.f;
     int bi = 0;
     cudaError_t e = cudaSuccess;
-    for (int c = 0; c < 4 && e == cudaSuccess; ++c) {
+    for (int c = 0; c < 2 && e == cudaSuccess; ++c) {
         set_sh_tiles(g, cfg[c][0], cfg[c][1] != 0);
         // one untimed launch, then the faster of two timed ones (a launch slowed by something
         // else on the machine would otherwise fix a worse configuration for the plan)
@@ -2715,8 +2365,7 @@ int ozaki_group_tune_tiles(OzGroup *g, cudaStream_t st, float *ms_best) {
         for (int rep = 0; rep < 3 && e == cudaSuccess; ++rep) {
             if (rep > 0) e = cudaEventRecord(e0, st);
             if (e == cudaSuccess)
-                e = launch_pair(g->maps_sh, g->s, g->d_err, g->d_jobs_sh, g->n_jobs_sh, tiles, g->d_list_sh, nullptr,
-                                st, g->units, g->halves);
+                e = launch_sh(g, g->d_list_sh, tiles, st);
             if (e == cudaSuccess && rep > 0) e = cudaEventRecord(e1, st);
             if (e == cudaSuccess && rep > 0) e = cudaEventSynchronize(e1);
             float t = 0.f;
@@ -2725,8 +2374,7 @@ int ozaki_group_tune_tiles(OzGroup *g, cudaStream_t st, float *ms_best) {
         }
         if (e == cudaSuccess && (best < 0.f || ms < best)) { best = ms; bi = c; }
         if (e == cudaSuccess && env_int("HSDLA_TRACE", 0))
-            fprintf(stderr, "tile tuner: halves %d, %s units: %.3f ms\n", cfg[c][0], cfg[c][1] ? "merged" : "single-diagonal",
-                    ms);
+            fprintf(stderr, "tile tuner: bands of %d: %.3f ms\n", cfg[c][1] ? 2 : 1, ms);
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -2756,7 +2404,7 @@ void ozaki_group_destroy(OzGroup *g) {
 // One k-point through a temporary group (the slice autotuner's probe).
 int64_t ozaki_pipeline_workspace(int s, int64_t twoL, int64_t na, int64_t nt, int64_t G) {
     const std::vector<int64_t> g{G};
-    return ozaki_group_bytes(s, twoL, na, nt, g, 1, true, false) + ozaki_group_persist_bytes(s, twoL, na, nt, g, 1) +
+    return ozaki_group_bytes(s, twoL, na, nt, g, 1, true, false) + ozaki_group_persist_bytes(s, twoL, na, nt, g, 1, false) +
            2048;
 }
 
@@ -2891,8 +2539,8 @@ extern "C" int hsdla_zherkx_lower_noalloc(int32_t num_slices, int64_t n, int64_t
     if (e == cudaSuccess) e = slice(reinterpret_cast<const double2 *>(dP), ldp, nullptr, k, n, Kpad, Kpad, s, dp, st);
     if (e == cudaSuccess) e = slice(reinterpret_cast<const double2 *>(dQ), ldq, dw, k, n, Kpad, Kpad, s, dq, st);
     if (e != cudaSuccess) { g_oz_err = cudaGetErrorString(e); return HSDLA_ERR_CUDA; }
-    rc = make_map(dp, s);
-    if (!rc) rc = make_map(dq, s);
+    rc = make_map(dp, 2 * s);
+    if (!rc) rc = make_map(dq, 2 * s);
     if (rc) return rc;
     OzJob j;
     memset(&j, 0, sizeof(j));

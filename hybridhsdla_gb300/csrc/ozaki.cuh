@@ -43,8 +43,11 @@ struct OzKBufs {
     double2 *M = nullptr;    // per-type rows M (2L nt x G), hoisted T application only
     double2 *Z = nullptr;    // per-type products Z (2L nt x G), hoisted T application only
     int64_t G = 0;
-    double2 *PS = nullptr;   // structure-factor form: per-type products (G x G, ld G), type
-    double2 *PH = nullptr;   // slot b of a combine batch at + b pstride
+    // structure-factor form (real rows, see real_products.cu): rows R (2L nt x G), and as
+    // fixed-point numbers Z' = T' R (4L nt x G; per type the real rows, then the imaginary ones) and
+    // the per-type products S, Re H, Im H (G x G, ld G), type slot b of a combine batch at + b pstride
+    double *R = nullptr;
+    long long *ZR = nullptr, *RS = nullptr, *RHr = nullptr, *RHi = nullptr;
     int64_t pstride = 0;
 };
 struct OzGroupDesc {
@@ -55,7 +58,8 @@ struct OzGroupDesc {
     const int32_t *atom_type = nullptr;    // host [na]
     int panels = 1;                        // atom panels the contraction index is streamed in
     bool sf = false;                       // structure-factor form (requires hoist)
-    const double *wt = nullptr;            // its per-type S weights [nt][2L]
+    const double *wt = nullptr;            // its per-type S weights [nt][2L] (of the real rows)
+    const double *TR = nullptr;            // its real T blocks (launch_treal)
     const double2 *sf_tab = nullptr;       // its structure factors
     int tbatch = 1;                        // its types per combine batch (product slots)
 };
@@ -67,11 +71,13 @@ struct OzGroup;
 int64_t ozaki_group_bytes(int s, int64_t twoL, int64_t na, int64_t nt, const std::vector<int64_t> &G, int panels,
                           bool hoist, bool sf);
 int64_t ozaki_group_persist_bytes(int s, int64_t twoL, int64_t na, int64_t nt, const std::vector<int64_t> &G,
-                                  int panels);
+                                  int panels, bool sf);
 int ozaki_group_prepare(OzakiPlan &oz, const OzGroupDesc &d, const std::vector<OzKBufs> &kb, void *ws,
                         void *persist, cudaStream_t st, OzGroup **out);
 void ozaki_group_set_outputs(OzGroup *g, double2 *const *S, double2 *const *H, const int64_t *ld);
-// Structure-factor form: the group's combine table (outputs of this run, per-type products).
+// Structure-factor form: the group's combine table (outputs of this run, per-type products), and the
+// products' exponents and fixed point filled into one.
+void ozaki_group_sf_exponents(const OzGroup *g, SfTab &t);
 void ozaki_group_set_sf(OzGroup *g, const SfTab &t);
 // Structure-factor form: the first type of the group's last combine (types [t0, nt), adding to
 // S and H unless t0 = 0): what ozaki_group_run leaves to its caller with defer_last_combine.
@@ -97,9 +103,9 @@ int ozaki_group_output_blocks(const OzGroup *g);
 // Event pairs ozaki_group_run records around the group's T application (see ev_t).
 int ozaki_group_tapply_events(const OzGroup *g);
 void ozaki_group_destroy(OzGroup *g);
-// The structure-factor form's S/H tile configuration on CTA-pair tiles: halves 1 (256 x 256
-// accumulators) or 2 (two 256 x 128 halves), merged 1 (adjacent digit diagonals share exact
-// accumulation units) or 0.  Tunable: a structure-factor group on pair tiles.
+// The structure-factor form's S/H configuration: bands of two adjacent digit diagonals (merged 1)
+// or of one, alternating between two TMEM halves (halves 2) or waiting for each other in one.
+// Tunable: a structure-factor group.
 bool ozaki_group_tunable(const OzGroup *g);
 void ozaki_group_tiles(const OzGroup *g, int *halves, int *merged);
 void ozaki_group_set_tiles(OzGroup *g, int halves, int merged);

@@ -1,0 +1,611 @@
+// Real digit products of the structure-factor form on the FP8 tensor cores.
+//
+// The matching rows of one type come in pairs: row (l, -m) is (-1)^m times the complex conjugate
+// of row (l, m) (Y_l,-m = (-1)^m conj Y_lm).  With rho = (Re, Im of the rows m > 0; the real rows
+// m = 0) the rows are M = V rho with V constant per pair, so
+//     S_t[g, g'] = rho(g)^T diag(w'_t) rho(g'),            w' = 2 w on the rows of m != 0,
+//     H_t[g, g'] = rho(g)^T (T'_t rho(g')),                T'_t = V^H T_t V:
+// one real product for S and two for H where the complex rows need four each, over the same 2L
+// rows (the rows rho are the very numbers of M; T' sums four entries of T).
+//
+// oz_real_kernel forms these products exactly as oz_pair_kernel does the complex ones (base-32
+// digits in e4m3, FP32 accumulators that hold exact integers, the triangle i + j <= s + 1), with
+// the work arranged for short real contractions (K = 2L):
+//  * CTA pairs, 256 x 128 tiles, tcgen05.mma.cta_group::2 (M 256, N 128, K 32).
+//  * The contraction runs in chunks of 64 digits.  All digit planes of a chunk (left 8 KB, right 4
+//    KB each) are in shared memory together, so each is loaded once for all its digit pairs: 132 KB
+//    per 8.4k MMA cycles and SM at s = 11 (16 B per cycle), where staging the planes pair by pair
+//    takes 96 B per cycle.  (128-digit chunks leave no room to load ahead.)  Planes arrive and
+//    leave in batches of four: a barrier per plane kept the MMA thread at its waits and commits
+//    (150 cycles per MMA of 64).
+//  * The digit pairs run in bands of two diagonals, so that a step of the left plane feeds two MMAs
+//    (the second takes it from the collector buffer).  The bands alternate between two TMEM halves:
+//    one drains while the next computes.
+//  * The sums over diagonals and chunks stay in registers as 64-bit fixed-point numbers (64 per
+//    thread of the eight epilogue warps): a diagonal's FP32 integer becomes an integer by one FADD
+//    (x + 1.5 2^23 leaves it in the low mantissa bits), and a band's adds with one multiply-add.
+//    Each output element is written once, rather than once per accumulation unit through L2
+//    reductions.  The fixed-point sum is exact down to 2^-frac of a unit of the top diagonal.
+// What bounds it: the MMA thread's issue and the drains share the time (the tensor pipe is busy 0.7
+// of it).  One type of the 8000-column workload (lmax 10, 11 digits): 3.05 ms in the complex form,
+// 1.13 ms here = 2.7 PFLOP/s of e4m3, 0.71 of twice the measured bf16 rate; sixteen epilogue warps
+// with half the sums each: 1.15 ms.
+// Every wait is bounded (ptx.cuh); both CTAs meet at a cluster barrier before TMEM is freed.
+#include <cuda_fp8.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
+#include "ptx.cuh"
+#include "real_products.cuh"
+
+namespace hsdla {
+namespace {
+
+constexpr int kThreads = 384;              // warps 0-3: left TMA, MMA, right TMA, idle; 4-11 epilogue
+constexpr int kEpi = 8;
+constexpr int kCols = kRealTileN / 2;      // columns of an epilogue warp (two warps per lane quadrant)
+constexpr int kABytes = 128 * kRealKBlock, kBBytes = kRealBRows * kRealKBlock;
+// Planes move in batches of kBatch digits.  Left planes: a ring of kRing batches, one more than a
+// chunk has; right planes: a bank per chunk, two banks.
+constexpr int kBatch = 4, kRing = 4, kNA = kRing * kBatch, kBank = kRealMaxSlices, kNB = 2 * kBank;
+static_assert((kRing - 1) * kBatch >= kRealMaxSlices, "the ring holds a chunk's planes");
+constexpr int kSmem = 1024 + kNA * kABytes + kNB * kBBytes;
+static_assert(kSmem <= 226 * 1024, "shared memory (the barriers are static)");
+// Register split: 384 threads are launched with 168 registers each (64512); the control warps keep
+// 56 and the epilogue warps get 216, 62464 in all.  launch_real_products checks the 168.
+constexpr int kRegsLaunch = 168, kRegsControl = 56, kRegsEpilogue = 216;
+static_assert(128 * kRegsControl + 256 * kRegsEpilogue <= kThreads * kRegsLaunch, "register split");
+
+struct __align__(8) RealBarriers {
+    uint64_t full[kRing];              // a batch's left and right planes landed (both CTAs')
+    uint64_t aempty[kRing], bempty[2]; // a left batch, a right bank consumed
+    uint64_t tfull[2], tempty[2];      // a band's accumulators in each TMEM half
+};
+
+__host__ __device__ constexpr uint32_t idesc_real() {
+    return (1u << 4) | ((uint32_t)(kRealTileN >> 3) << 17) | ((uint32_t)(kRealTileM >> 4) << 24);
+}
+
+// After an abort the copies and MMAs in flight have long landed: short waits for them
+constexpr long long kAbortCycles = 100000000LL;
+
+constexpr float kMagic = 12582912.0f;                  // 1.5 2^23
+constexpr uint32_t kMagicBits = 0x4B400000u;
+
+// One band's accumulators (diagonal T - 1 at t0, T at t1) into the sums (RealBands).  One short path
+// per kind of fold: a path per shift and width, and FP64 conversions at the tile's end, overflowed
+// the instruction cache.
+template <int kFold>
+__device__ __forceinline__ void add_band(unsigned long long (&acc)[kCols], uint32_t t0, uint32_t t1, float g, float f,
+                                         uint32_t mul, uint32_t tempty, int lane) {
+#pragma unroll
+    for (int h = 0; h < kCols; h += 32) {
+        uint32_t v0[32], v1[32];
+        tmem_ld32(t0 + h, v0);
+        tmem_ld32(t1 + h, v1);
+        tmem_ld_wait();
+        if (h + 32 >= kCols) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_remote(tempty);
+        }
+#pragma unroll
+        for (int c = 0; c < 32; ++c) {
+            const float x0 = __uint_as_float(v0[c]), x1 = __uint_as_float(v1[c]);
+            const uint32_t b = kFold == kFoldInt
+                                   ? (__float_as_uint(x0 + kMagic) << 5) + __float_as_uint(x1 + kMagic)
+                                   : __float_as_uint(fmaf(fmaf(x0, g, x1), f, kMagic));
+            if (kFold == kFoldHigh) {
+                const uint32_t lo = (uint32_t)acc[h + c], hi = (uint32_t)(acc[h + c] >> 32) + b * mul;
+                acc[h + c] = ((unsigned long long)hi << 32) | lo;
+            } else acc[h + c] += (unsigned long long)b * mul;
+        }
+    }
+}
+
+// MMAs of the pair with operands given by the low words of their descriptors; the high word and the
+// instruction descriptor are constants (fewer registers to move to the uniform file per MMA).
+// kA: the left operand's collector buffer (0 none, 1 fill, 2 last use)
+constexpr uint32_t kDescHi = (512u >> 4) | (1u << 14) | (4u << 29);    // SW64 K-major, 8 rows of 64 bytes
+template <int kA>
+__device__ __forceinline__ void mma_real(uint32_t d, uint32_t a, uint32_t b, uint32_t acc) {
+#define HSDLA_MMA_REAL(coll)                                                                                  \
+    asm volatile(                                                                                             \
+        "{\n .reg .b64 da, db;\n .reg .pred p;\n .reg .b32 h;\n mov.b32 h, %3;\n mov.b64 da, {%1, h};\n"        \
+        " mov.b64 db, {%2, h};\n setp.ne.b32 p, %5, 0;\n"                                                     \
+        " tcgen05.mma.cta_group::2.kind::f8f6f4" coll " [%0], da, db, %4, p;\n}\n" ::"r"(d),                  \
+        "r"(a), "r"(b), "n"(kDescHi), "r"(idesc_real()), "r"(acc)                                             \
+        : "memory")
+    if constexpr (kA == 0) HSDLA_MMA_REAL("");
+    else if constexpr (kA == 1) HSDLA_MMA_REAL(".collector::a::fill");
+    else HSDLA_MMA_REAL(".collector::a::lastuse");
+#undef HSDLA_MMA_REAL
+}
+__device__ __forceinline__ uint32_t desc_lo(uint32_t saddr) { return ((saddr & 0x3FFFF) >> 4) | (1u << 16); }
+
+__global__ void __launch_bounds__(kThreads, 1)
+    oz_real_kernel(const __grid_constant__ CUtensorMap lmap, const __grid_constant__ CUtensorMap rmap0,
+                   const __grid_constant__ CUtensorMap rmap1, const RealJob *__restrict__ jobs, int64_t total_tiles,
+                   const int4 *__restrict__ tile_list, int *err, const __grid_constant__ RealBands bands) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char *smem = reinterpret_cast<unsigned char *>(
+        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    __shared__ RealBarriers bars;
+    __shared__ uint32_t tmem_base_sh;
+    __shared__ volatile int abort_flag;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (cluster_size() != 2) {
+        if (threadIdx.x == 0) atomicCAS(err, 0, kDevBadInput * 16 + 6);
+        return;
+    }
+    const uint32_t rank = cluster_rank();
+    const bool leader = rank == 0;
+    const int s = bands.s;
+    auto pwait = [&](uint64_t *bar, uint32_t parity, int where, int slot, int count) -> bool {
+        if (mbar_wait(bar, parity, &abort_flag, err, where)) return true;
+        if (atomicCAS(err + 7, 0, 1) == 0) {
+            err[1] = blockIdx.x; err[2] = (int)rank; err[3] = slot; err[4] = (int)parity; err[5] = count;
+        }
+        return false;
+    };
+    const int64_t pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
+    unsigned char *abuf = smem, *bbuf = smem + kNA * kABytes;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kRing; ++i) { mbar_init(&bars.full[i], 1); mbar_init(&bars.aempty[i], 1); }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&bars.bempty[i], 1);
+            mbar_init(&bars.tfull[i], 1);
+            mbar_init(&bars.tempty[i], 2 * kEpi);
+        }
+        abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        asm volatile("prefetch.tensormap [%0];\n" ::"l"((uint64_t)&lmap) : "memory");
+        asm volatile("prefetch.tensormap [%0];\n" ::"l"((uint64_t)&rmap0) : "memory");
+        asm volatile("prefetch.tensormap [%0];\n" ::"l"((uint64_t)&rmap1) : "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;\n" ::"r"(smem_u32(&tmem_base_sh))
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;\n" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();          // barriers of both CTAs initialised before any remote arrival
+    tc_fence_after();
+    const uint32_t tmem_base = tmem_base_sh;
+
+    if (warp < 4) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kRegsControl));
+        const bool one = elect_one();
+        if (warp == 0 && one) {
+            // ------------------------------------------------ planes, in batches
+            const uint32_t full_leader = mapa_rank(smem_u32(&bars.full[0]), 0);
+            uint32_t n = 0, chunk = 0;               // batches issued, chunks begun
+            bool ok = true;
+            for (int64_t tile = pair; ok && tile < total_tiles; tile += npairs) {
+                const int4 e = tile_list[tile];
+                const RealJob &j = jobs[e.x];
+                const CUtensorMap *rm = j.rmap ? &rmap1 : &rmap0;
+                const int64_t lstep = j.lplane, rstep = j.rstep * j.rplane, nkb = j.nkb;
+                int64_t yl = j.lrow0 + (int64_t)e.y * kRealTileM + rank * (kRealTileM / 2);
+                int64_t yr = j.rpart * j.rplane + j.rrow0 + (int64_t)e.z * kRealTileN + rank * kRealBRows;
+                const int64_t kl = j.lk0, kr = j.rk0;
+                for (int64_t kb = 0; ok && kb < nkb; ++kb, ++chunk) {
+                    const int xl = (int)(kl + kb * kRealKBlock), xr = (int)(kr + kb * kRealKBlock);
+                    if (!pwait(&bars.bempty[chunk & 1], ((chunk >> 1) & 1) ^ 1, 7, (int)(chunk & 1), (int)chunk)) { ok = false; break; }
+                    unsigned char *bp = bbuf + (chunk & 1) * kBank * kBBytes;
+                    for (int i0 = 0; i0 < s; i0 += kBatch, ++n) {
+                        const int slot = n % kRing, cnt = min(kBatch, s - i0);
+                        if (!pwait(&bars.aempty[slot], ((n / kRing) & 1) ^ 1, 1, slot, (int)n)) { ok = false; break; }
+                        if (leader) mbar_expect_tx(&bars.full[slot], 2 * cnt * (kABytes + kBBytes));
+                        const uint32_t fb = full_leader + slot * 8;
+                        for (int q = 0; q < cnt; ++q) {
+                            tma_load_2d_pair(abuf + (slot * kBatch + q) * kABytes, &lmap, fb, xl, (int)(yl + (i0 + q) * lstep));
+                            tma_load_2d_pair(bp + (i0 + q) * kBBytes, rm, fb, xr, (int)(yr + (i0 + q) * rstep));
+                        }
+                    }
+                }
+            }
+            // every batch issued has been consumed before the CTA may exit (bounded after an abort):
+            // its left planes' release follows the last use of its right planes or precedes their bank's
+            const long long budget = ok ? kWaitCycles : kAbortCycles;
+            for (uint32_t q = n > kRing ? n - kRing : 0; q < n; ++q)
+                mbar_drain_wait(&bars.aempty[q % kRing], (q / kRing) & 1, budget);
+            for (uint32_t c = chunk > 2 ? chunk - 2 : 0; c < chunk; ++c)
+                mbar_drain_wait(&bars.bempty[c & 1], (c >> 1) & 1, budget);
+        } else if (warp == 1 && one && leader) {
+            // ------------------------------------------------ MMA issuer
+            const uint32_t da0 = desc_lo(smem_u32(abuf)), db0 = desc_lo(smem_u32(bbuf));
+            constexpr uint32_t kAStep = kABytes >> 4, kBStep = kBBytes >> 4;
+            uint32_t n = 0, chunk = 0, seq = 0;      // the chunk's first batch; chunks; bands so far
+            const int halves = bands.halves, nbatch = (s + kBatch - 1) / kBatch, nbands = bands.n;
+            bool ok = true, cut = false;
+            for (int64_t tile = pair; ok && tile < total_tiles; tile += npairs) {
+                const RealJob &j = jobs[tile_list[tile].x];
+                const int nkb = (int)j.nkb, ksl = j.ksteps_last;
+                for (int kb = 0; ok && kb < nkb; ++kb, ++chunk, n += nbatch) {
+                    const bool two = kb + 1 < nkb || ksl > 1;      // K steps of the chunk
+                    const uint32_t db = db0 + (chunk & 1) * kBank * kBStep;
+                    int ready = 0;
+                    for (int b = 0; b < nbands; ++b, ++seq) {
+                        const int T = bands.T[b];
+                        const bool last = b + 1 == nbands, pairs = bands.w[b] == 2;
+                        const int h = halves == 2 ? (int)(seq & 1) : 0;
+                        const uint32_t use = halves == 2 ? seq >> 1 : seq;
+                        if (!pwait(&bars.tempty[h], (use & 1) ^ 1, 2, b, (int)seq)) { ok = false; break; }
+                        for (; ready <= (T - 2) / kBatch; ++ready)
+                            if (!pwait(&bars.full[(n + ready) % kRing], ((n + ready) / kRing) & 1, 3, ready, (int)seq)) { ok = false; break; }
+                        if (!ok) break;
+                        tc_fence_after();
+                        cut = true;
+                        const uint32_t d1 = tmem_base + h * 2 * kRealTileN, d2 = d1 + kRealTileN;
+                        // left plane i with right planes T - 1 - i (diagonal T - 1) and T - i (diagonal T)
+                        uint32_t dt = db + (T - 2) * kBStep;
+                        for (int i0 = 1; i0 < T; i0 += kBatch) {
+                            const int slot = (n + (i0 - 1) / kBatch) % kRing;
+                            uint32_t da = da0 + slot * kBatch * kAStep;
+                            const int i1 = min(i0 + kBatch, T);
+                            for (int i = i0; i < i1; ++i, da += kAStep, dt -= kBStep) {
+                                const uint32_t acc = i > 1 ? 1u : 0u;
+                                if (pairs && i + 1 < T) {
+                                    const uint32_t dl = dt - kBStep;
+                                    mma_real<1>(d1, da, dl, acc);
+                                    mma_real<2>(d2, da, dt, acc);
+                                    if (two) {
+                                        mma_real<1>(d1, da + 2, dl + 2, 1u);
+                                        mma_real<2>(d2, da + 2, dt + 2, 1u);
+                                    }
+                                } else {
+                                    mma_real<0>(d2, da, dt, acc);
+                                    if (two) mma_real<0>(d2, da + 2, dt + 2, 1u);
+                                }
+                            }
+                            if (last) mma_commit_pair(&bars.aempty[slot]);     // the batch's last use
+                        }
+                        mma_commit_pair(&bars.tfull[h]);
+                        if (last) mma_commit_pair(&bars.bempty[chunk & 1]);
+                        cut = false;
+                    }
+                }
+            }
+            if (!ok) {
+                // wait (bounded) for the MMAs of a band cut short: the commit tracks all of them
+                if (cut) {
+                    const int h = halves == 2 ? (int)(seq & 1) : 0;
+                    mma_commit_pair(&bars.tfull[h]);
+                    mbar_drain_wait(&bars.tfull[h], (halves == 2 ? seq >> 1 : seq) & 1);
+                }
+            } else {
+                // both CTAs' drains of the last bands
+                for (uint32_t q = seq > 2 ? seq - 2 : 0; q < seq; ++q) {
+                    const int h = halves == 2 ? (int)(q & 1) : 0;
+                    const uint32_t use = halves == 2 ? q >> 1 : q;
+                    if (halves == 1 && q + 1 < seq) continue;
+                    mbar_drain_wait(&bars.tfull[h], use & 1);
+                    mbar_drain_wait(&bars.tempty[h], use & 1);
+                }
+            }
+        }
+        __syncwarp();
+    } else {
+        // ------------------------------------------------ epilogue
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(kRegsEpilogue));
+        const int q4 = warp & 3, cbeg = ((warp - 4) >> 2) * kCols;
+        const uint32_t tempty_leader = mapa_rank(smem_u32(&bars.tempty[0]), 0);
+        const uint32_t tb = tmem_base + ((uint32_t)(q4 * 32) << 16) + cbeg;
+        uint32_t seq = 0;
+        bool ok = true;
+        const int halves = bands.halves;
+        for (int64_t tile = pair; ok && tile < total_tiles; tile += npairs) {
+            const int4 te = tile_list[tile];
+            const RealJob &j = jobs[te.x];
+            const int64_t nkb = j.nkb;
+            unsigned long long acc[kCols];
+            {
+                const unsigned long long a0 = 0ull - bands.bias * (unsigned long long)nkb;
+#pragma unroll
+                for (int c = 0; c < kCols; ++c) acc[c] = a0;
+            }
+            for (int64_t kb = 0; ok && kb < nkb; ++kb) {
+                for (int b = 0; b < bands.n; ++b, ++seq) {
+                    const int h = halves == 2 ? (int)(seq & 1) : 0;
+                    const uint32_t use = halves == 2 ? seq >> 1 : seq;
+                    if (!pwait(&bars.tfull[h], use & 1, 8, warp, (int)seq)) { ok = false; break; }
+                    tc_fence_after();
+                    // (a band of one diagonal has it in the second buffer)
+                    const uint32_t t1 = tb + (2 * h + 1) * kRealTileN, te = tempty_leader + h * 8;
+                    const uint32_t t0 = bands.w[b] == 2 ? t1 - kRealTileN : t1;
+                    const float g = bands.g[b], f = bands.f[b];
+                    const uint32_t mul = bands.mul[b];
+                    const int fold = bands.fold[b];
+                    if (fold == kFoldHigh) add_band<kFoldHigh>(acc, t0, t1, g, f, mul, te, lane);
+                    else if (fold == kFoldFloat) add_band<kFoldFloat>(acc, t0, t1, g, f, mul, te, lane);
+                    else add_band<kFoldInt>(acc, t0, t1, g, f, mul, te, lane);
+                }
+            }
+            if (!ok) break;
+            // the tile: lane = row, so a column's 32 values are 256 consecutive bytes
+            const int64_t row = (int64_t)te.y * kRealTileM + rank * (kRealTileM / 2) + q4 * 32 + lane;
+            const int64_t col0 = (int64_t)te.z * kRealTileN + cbeg;
+            const int64_t n = j.n, ldo = j.ldo;
+            const bool rok = row < j.m;
+            const int64_t cend = j.lower ? min(n, row + 1) : n;
+            long long *out = j.out + row + ldo * col0;
+            const int live = rok ? (int)max((int64_t)0, min((int64_t)kCols, cend - col0)) : 0;
+#pragma unroll
+            for (int c = 0; c < kCols; ++c)
+                if (c < live) out[ldo * c] = (long long)acc[c];
+        }
+        __syncwarp();
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();          // neither CTA frees TMEM or exits while the other may address it
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;\n" ::"r"(tmem_base) : "memory");
+    }
+}
+
+// ------------------------------------------------------------------ slicing of real columns
+// As oz_slice_kernel (the same digits of the same values): one CTA per plane row, first the
+// column's largest magnitude (its exponent), then X = rint(z 2^(5s-1-e)) of eight consecutive
+// contraction bytes per thread and their balanced base-32 digits, one 8-byte store per plane.
+constexpr int kSliceThreads = 256;
+constexpr int kVec = 8;
+
+__device__ __forceinline__ unsigned long long abs_bits(double x) {
+    return (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffull;
+}
+// frexp's exponent of a positive finite double given as bits
+__device__ __forceinline__ int frexp_exp_bits(unsigned long long b) {
+    const int E = (int)(b >> 52) & 0x7ff;
+    if (E) return E - 1022;
+    return -1010 - __clzll((long long)(b & 0xfffffffffffffull));
+}
+// rint(x 2^k), half to even, for |x 2^k| < 2^62
+__device__ __forceinline__ long long rint_pow2(double x, int k) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const int E = (int)((b >> 52) & 0x7ff);
+    const unsigned long long mant = b & 0xfffffffffffffull;
+    const unsigned long long m = E ? (mant | (1ull << 52)) : mant;
+    const int sh = 1075 - (E ? E : 1) - k;
+    unsigned long long q;
+    if (sh <= 0) {
+        q = m << (-sh);
+    } else if (sh >= 54) {
+        q = 0;
+    } else {
+        q = m >> sh;
+        const unsigned long long rem = m & ((1ull << sh) - 1), half = 1ull << (sh - 1);
+        q += (rem > half) | ((rem == half) & (q & 1ull));
+    }
+    return (b >> 63) ? -(long long)q : (long long)q;
+}
+
+__device__ __forceinline__ unsigned long long block_max(unsigned long long m, unsigned long long *red) {
+    for (int o = 16; o > 0; o >>= 1) m = max(m, (unsigned long long)__shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+    __syncthreads();
+    unsigned long long r = 0;
+    for (int i = 0; i < kSliceThreads / 32; ++i) r = max(r, red[i]);
+    return r;
+}
+
+// The s digits of eight values X + B (B = 16 in every lower digit) to planes `step` apart, the
+// least significant first: 5-bit fields, encoded as e4m3 by a table in shared memory.
+__device__ __forceinline__ void write_digits(long long (&u)[kVec], int s, const uint8_t *lut, uint8_t *dst,
+                                             int64_t step) {
+    uint8_t *p = dst + (int64_t)(s - 1) * step;
+#pragma unroll 1
+    for (int i = s - 1; i >= 0; --i, p -= step) {
+        uint32_t w0 = 0, w1 = 0;
+#pragma unroll
+        for (int v = 0; v < kVec; ++v) {
+            // (the top digit of a finite column is in [-16, 16]; the clamp keeps the table read in
+            // bounds for any column)
+            const int idx = i == 0 ? min(max((int)u[v] + 16, 0), 32) : (int)(u[v] & 31);
+            const uint32_t b = (uint32_t)lut[idx] << (8 * (v & 3));
+            if (v < 4) w0 |= b; else w1 |= b;
+            u[v] >>= 5;
+        }
+        *reinterpret_cast<uint2 *>(p) = make_uint2(w0, w1);
+    }
+}
+
+// kFixed: the source is a product's fixed-point numbers (parts rows exponents el, see RealSliceTab)
+template <bool kDual, bool kFixed>
+__global__ void __launch_bounds__(kSliceThreads) oz_slice_real_kernel(const __grid_constant__ RealSliceTab tab) {
+    __shared__ uint8_t lut[33];
+    __shared__ unsigned long long red[2][kSliceThreads / 32];
+    const int64_t r = blockIdx.x;
+    int k = 0;
+    while (k + 1 < tab.nk && tab.e[k + 1].row0 <= r) ++k;
+    const int64_t g = r - tab.e[k].row0;
+    const bool live = g >= 0 && g < tab.e[k].ncols;
+    const int64_t col = tab.ldz * (live ? g : 0);
+    const double *Z = reinterpret_cast<const double *>(tab.e[k].Z) + col;
+    const long long *F = reinterpret_cast<const long long *>(tab.e[k].Z) + col;
+    const int rpb = (int)tab.rpb, bpad = (int)tab.bpad, nblk = (int)tab.blocks, parts = tab.parts, s = tab.s;
+    const int bch = bpad / kVec, nch = bch * nblk;               // chunks of a block and part; of a part
+    if (threadIdx.x < 33) {
+        const float dv = (float)((int)threadIdx.x - 16);
+        lut[threadIdx.x] = (uint8_t)(__nv_cvt_float2_to_fp8x2(make_float2(dv, 0.f), __NV_SATFINITE, __NV_E4M3) & 0xffu);
+    }
+    // (a fixed-point number's bit length and row exponent, offset to stay positive, order as |value|)
+    constexpr int kOff = 1 << 20;
+    unsigned long long mx = 0, mx2 = 0;
+    for (int c = threadIdx.x; live && c < nch * parts; c += kSliceThreads) {
+        const int p = c / nch, cc = c - p * nch, b = cc / bch, r0 = (cc - b * bch) * kVec;
+        const int64_t o = (int64_t)b * tab.bstride + p * tab.pstride + r0;
+#pragma unroll
+        for (int u = 0; u < kVec; ++u)
+            if (r0 + u < rpb) {
+                if constexpr (kFixed) {
+                    const long long x = F[o + u];
+                    if (x) mx = max(mx, (unsigned long long)(kOff + 64 - __clzll(x < 0 ? -x : x) + tab.el[o + u]));
+                } else {
+                    const double x = Z[o + u];
+                    mx = max(mx, abs_bits(x));
+                    if (kDual) mx2 = max(mx2, abs_bits(x * tab.v2[b * rpb + r0 + u]));
+                }
+            }
+    }
+    int e = 0, e2 = 0, q = 0;
+    const unsigned long long m = block_max(mx, red[0]);
+    if constexpr (kFixed) {
+        q = (live ? tab.er[r] : 0) - 8 - tab.frac;               // the column's part of the values' exponent
+        if (m > 0) e = (int)m - kOff + q;
+    } else if (m > 0) e = frexp_exp_bits(m);
+    if (kDual) {
+        const unsigned long long m2 = block_max(mx2, red[1]);
+        if (m2 > 0) e2 = frexp_exp_bits(m2);
+    }
+    if (threadIdx.x == 0) {
+        tab.expo[r] = e;
+        if (kDual) tab.expo2[r] = e2;
+    }
+    const int top = 5 * s - 1;
+    long long B = 0;
+    for (int p = 0; p < s - 1; ++p) B |= 16ll << (5 * p);
+    const int64_t plane = tab.plane_rows * tab.pitch;
+    for (int c = threadIdx.x; c < nch * parts; c += kSliceThreads) {
+        const int p = c / nch, cc = c - p * nch, b = cc / bch, r0 = (cc - b * bch) * kVec;
+        const int64_t o = (int64_t)b * tab.bstride + p * tab.pstride + r0;
+        long long x[kVec];
+#pragma unroll
+        for (int u = 0; u < kVec; ++u) {
+            long long X = 0;
+            if (live && r0 + u < rpb) {
+                if constexpr (kFixed) {
+                    // F 2^(el + q) scaled by 2^(top - e): a shift, rounded half up
+                    const int d = tab.el[o + u] + q + top - e;
+                    const long long f = F[o + u];
+                    X = d >= 0 ? f << min(d, 63) : d < -63 ? 0 : ((f >> (-d - 1)) + 1) >> 1;
+                } else X = rint_pow2(Z[o + u], top - e);
+            }
+            x[u] = B + X;
+        }
+        write_digits(x, s, lut, tab.digits + r * tab.pitch + (int64_t)b * bpad + r0 + p * plane, parts * plane);
+        if (kDual) {
+#pragma unroll
+            for (int u = 0; u < kVec; ++u)
+                x[u] = B + (live && r0 + u < rpb ? rint_pow2(Z[o + u] * tab.v2[b * rpb + r0 + u], top - e2) : 0ll);
+            write_digits(x, s, lut, tab.digits2 + r * tab.pitch + (int64_t)b * bpad + r0, plane);
+        }
+    }
+}
+
+}  // namespace
+
+RealBands real_bands(int s, int width, int halves, int64_t kvalid) {
+    RealBands b;
+    memset(&b, 0, sizeof(b));
+    b.s = s;
+    b.halves = halves;
+    width = std::max(1, std::min(width, 2));
+    // |sum| <= kvalid 2^8 (operands below 2^4 in units of their top digit) stays below 2^(63 - frac)
+    int kb = 0;
+    while (((int64_t)1 << kb) <= kvalid) ++kb;
+    b.frac = 55 - kb;
+    // a single diagonal comes first: the last band (T = s + 1) is full width
+    int T = 2 + ((s - 1) % width);
+    for (int t = 1; t < s + 1; T += width) {
+        const int n = b.n++, sh = b.frac - 5 * (T - 2);
+        b.T[n] = (int8_t)T;
+        b.w[n] = (int8_t)(T - t);
+        // the largest |32 x0 + x1| of a chunk: 64 products of at most 2^8 per digit pair
+        const int64_t big = (int64_t)kRealKBlock * 256 * ((b.w[n] == 2 ? 32 * (T - 2) : 0) + T - 1);
+        const int r = sh < 0 ? -sh : 0;          // below the fixed point the sums are rounded to it
+        b.fold[n] = sh >= 32 ? kFoldHigh : (big >> r) < (1 << 22) ? kFoldFloat : kFoldInt;
+        b.mul[n] = sh >= 32 ? 1u << (sh - 32) : 1u << std::max(sh, 0);
+        b.g[n] = b.w[n] == 2 ? 32.0f : 0.0f;
+        b.f[n] = std::ldexp(1.0f, -r);
+        const uint32_t m = b.fold[n] == kFoldInt ? 33u * kMagicBits : kMagicBits;   // (far from 2^32's ends)
+        b.bias += b.fold[n] == kFoldHigh ? (unsigned long long)(m * b.mul[n]) << 32 : (unsigned long long)m * b.mul[n];
+        t = T;
+    }
+    return b;
+}
+
+int64_t real_job_tiles(const RealJob &j) {
+    const int64_t tm = (j.m + kRealTileM - 1) / kRealTileM, tn = (j.n + kRealTileN - 1) / kRealTileN;
+    if (!j.lower) return tm * tn;
+    int64_t t = 0;
+    for (int64_t i = 0; i < tm; ++i) t += std::min(tn, (i + 1) * (kRealTileM / kRealTileN));
+    return t;
+}
+
+void real_schedule(const std::vector<RealJob> &jobs, std::vector<int4> &list) {
+    // super-blocks of 4 x 8 tiles (1024 rows and columns) keep a wave's operand planes in L2
+    constexpr int64_t kSB = 4, kRatio = kRealTileM / kRealTileN;
+    list.clear();
+    for (size_t a = 0; a < jobs.size();) {
+        const RealJob &ja = jobs[a];
+        const int64_t tm = (ja.m + kRealTileM - 1) / kRealTileM, tn = (ja.n + kRealTileN - 1) / kRealTileN;
+        if (!ja.lower) {
+            for (int64_t c = 0; c < tn; ++c)
+                for (int64_t r = 0; r < tm; ++r) list.push_back(make_int4((int)a, (int)r, (int)c, 0));
+            ++a;
+            continue;
+        }
+        size_t b = a;
+        while (b < jobs.size() && jobs[b].lower && jobs[b].n == ja.n && jobs[b].lrow0 == ja.lrow0 && jobs[b].lk0 == ja.lk0) ++b;
+        for (int64_t I = 0; I < tm; I += kSB)
+            for (int64_t J = 0; J <= I; J += kSB)
+                for (int64_t r = I; r < std::min(tm, I + kSB); ++r)
+                    for (int64_t c = J * kRatio; c < std::min(std::min(tn, (r + 1) * kRatio), (J + kSB) * kRatio); ++c)
+                        for (size_t q = a; q < b; ++q) list.push_back(make_int4((int)q, (int)r, (int)c, 0));
+        a = b;
+    }
+}
+
+cudaError_t launch_real_products(const CUtensorMap &left, const CUtensorMap &right0, const CUtensorMap &right1,
+                                 const RealJob *d_jobs, const int4 *d_list, int64_t tiles, const RealBands &bands,
+                                 int *d_err, cudaStream_t st) {
+    if (tiles <= 0) return cudaSuccess;
+    cudaError_t e = cudaFuncSetAttribute(oz_real_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = kSmem;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    static int max_pairs = 0;
+    if (max_pairs == 0) {
+        // the register split draws on what the block was launched with
+        cudaFuncAttributes fa;
+        e = cudaFuncGetAttributes(&fa, oz_real_kernel);
+        if (e != cudaSuccess) return e;
+        if (fa.numRegs * kThreads < 128 * kRegsControl + 256 * kRegsEpilogue) return cudaErrorInvalidConfiguration;
+        cfg.gridDim = dim3(2);
+        int nc = 0;
+        e = cudaOccupancyMaxActiveClusters(&nc, (const void *)oz_real_kernel, &cfg);
+        if (e != cudaSuccess) return e;
+        if (nc < 1) return cudaErrorInvalidConfiguration;
+        max_pairs = nc;
+    }
+    cfg.gridDim = dim3((unsigned)(2 * std::min<int64_t>(tiles, max_pairs)));
+    return cudaLaunchKernelEx(&cfg, oz_real_kernel, left, right0, right1, d_jobs, tiles, d_list, d_err, bands);
+}
+
+cudaError_t launch_real_slice(const RealSliceTab &t, cudaStream_t st) {
+    if (t.plane_rows <= 0) return cudaSuccess;
+    const unsigned grid = (unsigned)t.plane_rows;
+    if (t.frac) oz_slice_real_kernel<false, true><<<grid, kSliceThreads, 0, st>>>(t);
+    else if (t.digits2) oz_slice_real_kernel<true, false><<<grid, kSliceThreads, 0, st>>>(t);
+    else oz_slice_real_kernel<false, false><<<grid, kSliceThreads, 0, st>>>(t);
+    return cudaGetLastError();
+}
+
+}  // namespace hsdla

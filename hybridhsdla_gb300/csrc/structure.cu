@@ -59,6 +59,28 @@ __global__ void __launch_bounds__(kSfTabThreads) sf_table_kernel(const double2 *
     }
 }
 
+// A 64-bit integer as a double (nearest even) on the integer pipes: GB300's FP64 pipe, which a
+// conversion instruction uses, issues one warp instruction in 16 cycles.
+__device__ __forceinline__ double int_to_f64(long long a) {
+    unsigned long long u = a < 0 ? 0ull - (unsigned long long)a : (unsigned long long)a;
+    const int lz = __clzll((long long)u);
+    u <<= lz & 63;
+    const unsigned long long rem = u & 0x7ffull;
+    // (the mantissa carries the hidden bit into the exponent field)
+    unsigned long long b = ((unsigned long long)(unsigned)(1023 + 62 - lz) << 52) + (u >> 11);
+    b += (rem > 0x400ull) | ((rem == 0x400ull) & (b & 1ull));
+    b |= (unsigned long long)a & 0x8000000000000000ull;
+    return __longlong_as_double((long long)(a ? b : 0ull));
+}
+__device__ __noinline__ double ldexp_call(double v, int k) { return ldexp(v, k); }
+// v 2^k by an exponent add where v and the result are normal, else ldexp
+__device__ __forceinline__ double scale_exp(double v, int k) {
+    const long long b = __double_as_longlong(v);
+    const int E = (int)((b >> 52) & 0x7ff);
+    if (E > 0 && E + k > 0 && E + k < 2047) return __longlong_as_double(b + ((long long)k << 52));
+    return ldexp_call(v, k);
+}
+
 // 128-thread CTAs (32 rows x 4 column lanes): small enough to share an SM with a pair launch
 constexpr int kSfTile = 32, kSfRows = 4;
 
@@ -67,6 +89,7 @@ constexpr int kSfTile = 32, kSfRows = 4;
 // rows of a column.  A batch of several types reads and writes S and H once.  The tiles of an
 // entry are its tile columns [tc0, tc1) (a column range of the launch), each from the diagonal
 // tile down.
+template <bool kReal>
 __global__ void __launch_bounds__(kSfTile * kSfRows) sf_combine_kernel(const __grid_constant__ SfTab tab,
                                                                        const double2 *__restrict__ sf, int first) {
     const int64_t tile = blockIdx.x;
@@ -101,11 +124,27 @@ __global__ void __launch_bounds__(kSfTile * kSfRows) sf_combine_kernel(const __g
         double2 vs = make_double2(0.0, 0.0), vh = make_double2(0.0, 0.0);
         for (int b = 0; b < tab.ntypes; ++b) {
             const double2 f = sft[idx + b * tab.box];
+            if constexpr (kReal) {
+                // S_t real, H_t complex: 6 FMAs (GB300's FP64 rate bounds this kernel)
+                const int64_t o = off + (tab.slot0 + b) * E.pstride;
+                const double ps = int_to_f64(E.RS[o]), hr = int_to_f64(E.RHr[o]), hi = int_to_f64(E.RHi[o]);
+                vs.x = fma(f.x, ps, vs.x);
+                vs.y = fma(f.y, ps, vs.y);
+                vh.x = fma(f.x, hr, fma(-f.y, hi, vh.x));
+                vh.y = fma(f.x, hi, fma(f.y, hr, vh.y));
+                continue;
+            }
             const double2 ps = E.PS[off + (tab.slot0 + b) * E.pstride], ph = E.PH[off + (tab.slot0 + b) * E.pstride];
             vs.x = fma(f.x, ps.x, fma(-f.y, ps.y, vs.x));
             vs.y = fma(f.x, ps.y, fma(f.y, ps.x, vs.y));
             vh.x = fma(f.x, ph.x, fma(-f.y, ph.y, vh.x));
             vh.y = fma(f.x, ph.y, fma(f.y, ph.x, vh.y));
+        }
+        if constexpr (kReal) {
+            // one power of two for every type's products of an element
+            const int k0 = E.el[row] - 8 - tab.frac, ks = k0 + E.ers[col], kh = k0 + E.erh[col];
+            vs = make_double2(scale_exp(vs.x, ks), scale_exp(vs.y, ks));
+            vh = make_double2(scale_exp(vh.x, kh), scale_exp(vh.y, kh));
         }
         const bool x = E.Sx && row < tab.xrow1;
         double2 *so = x ? E.Sx + row + E.ldx * col : E.S + row + E.ldo * col;
@@ -159,7 +198,9 @@ cudaError_t launch_sf_combine(const SfTab &tab, const double2 *sf, bool first, c
     const int64_t tiles = sf_tab_tiles(t);
     if (tiles <= 0) return cudaSuccess;
     if (tiles > 0x7fffffffLL) return cudaErrorInvalidValue;
-    sf_combine_kernel<<<(unsigned)tiles, dim3(kSfTile, kSfRows), 0, st>>>(t, sf, first ? 1 : 0);
+    const dim3 block(kSfTile, kSfRows);
+    if (t.nk > 0 && t.e[0].RS) sf_combine_kernel<true><<<(unsigned)tiles, block, 0, st>>>(t, sf, first ? 1 : 0);
+    else sf_combine_kernel<false><<<(unsigned)tiles, block, 0, st>>>(t, sf, first ? 1 : 0);
     return cudaGetLastError();
 }
 

@@ -131,9 +131,9 @@ typedef struct hsdla_report {
     int32_t num_row_sets;        /* structure-factor form: the row sets contracted (types, or (type, rotation)
                                     classes when atoms carry rotations); 0 = the per-atom form */
     int32_t rotation_classes;    /* 1: the row sets are (type, rotation) classes */
-    int32_t tile_halves;         /* Ozaki, structure-factor form: S/H tiles as 256 x 256 accumulators (1) or */
-                                 /* two 256 x 128 halves in alternating TMEM buffers (2); 0 otherwise */
-    int32_t merged_units;        /* the same launches: 1 = adjacent digit diagonals share exact accumulation units */
+    int32_t tile_halves;         /* Ozaki, structure-factor form: the S/H products' bands of digit diagonals alternate */
+                                 /* between two halves of TMEM (2) or wait for each other in one (1); 0 otherwise */
+    int32_t merged_units;        /* the same launches: 1 = two adjacent digit diagonals share a band, 0 = one each */
     int32_t tile_tuned;          /* 1 = those two were chosen by timing on this plan's data (or a cached result) */
     int32_t output_blocks;       /* hsdla_create_hs, outputs written in place: the column blocks they were written
                                     in while the digit products of the next block ran (0 = after all products) */

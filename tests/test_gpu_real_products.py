@@ -1,0 +1,46 @@
+"""The real digit products of the structure-factor form (csrc/real_products.cu): one real product for
+S and two for H over the real and imaginary parts of the matching rows, against the oracle.
+
+Sizes where the kernels change course: contraction lengths 2L = 2 (lmax + 1)^2 on both sides of the
+64-digit chunks and with one or two K steps in the last (lmax 1: 8, 3: 32, 5: 72, 7: 128, 9: 200, 11:
+288, 14: 450), basis sizes around the 128-column and 256-row tiles, 10, 11 and 12 digits (bands of one
+and of two diagonals first, every fold of the fixed-point sums).  Tolerance: 1e-13 (relative
+Frobenius and max-norm of the lower triangles) for 11 and 12 digits; a digit less multiplies the
+truncation error by 2^5, so 32e-13 for 10."""
+import numpy as np
+import pytest
+
+import oracle
+from hybridhsdla_gb300 import api, synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    c = api.Context()
+    yield c
+    c.close()
+
+
+@pytest.mark.parametrize("lmax,n_g,slices", [
+    (1, 1, 11), (1, 128, 11), (2, 129, 12), (3, 255, 11), (4, 256, 10), (5, 257, 11), (5, 130, 12), (7, 385, 11),
+    (8, 127, 11), (9, 513, 11), (10, 300, 12), (10, 261, 11), (11, 200, 11), (14, 150, 12), (14, 140, 10)])
+def test_real_products_match_oracle(ctx, lmax, n_g, slices):
+    cfg = dict(cell=(10.0, 10.5, 11.0), atoms=5, types=2, rmt=2.0, min_sep=3.9, lmax=lmax,
+               kpts=[(0.1, 0.2, 0.3), (-0.2, 0.35, 0.15)], n_g=n_g, seed=100 * lmax + n_g)
+    s = synth.make_system(cfg)
+    if lmax > 1:
+        s.type_lmax = np.asarray([lmax, lmax - 1], np.int32)      # rows above a type's lmax are zero
+        s.type_lmax_nonsph = s.type_lmax.copy()
+    res, rep = ctx.create_hs(s, precision="ozaki", num_slices=slices)
+    assert rep["num_row_sets"] == 2
+    tol = 1e-13 if slices >= 11 else 32e-13
+    for (H, S), kp in zip(res, s.kpoints):
+        Hr, Sr = oracle.reference_hs(s, kp)
+        for X, R, nm in ((H, Hr, "H"), (S, Sr, "S")):
+            fro, mx = oracle.lower_errors(X, R)
+            assert fro < tol and mx < tol, (nm, lmax, n_g, slices, fro, mx)
