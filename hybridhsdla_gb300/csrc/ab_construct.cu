@@ -316,12 +316,12 @@ __global__ void __launch_bounds__(kThreads) construct_ab_kernel(DevSystem sys, c
     }
 }
 
-// Per-type rows M only (atoms sharing their type's rotation, no per-atom rows), kRowCols G columns
-// per CTA.  The per-column scalar work -- the Bessel recursions per type and the Y_lm sets, FP64
+// Real per-type rows R only (atoms sharing their type's rotation, no per-atom rows), kRowCols G
+// columns per CTA.  The per-column scalar work -- the Bessel recursions per type and the Y_lm sets, FP64
 // code with data-dependent loops -- runs one column per lane, as work items (column, type) and
 // (column, m), instead of on a few lanes of one warp per column: GB300 issues an FP64 warp
 // instruction in 16 cycles however few of its lanes are active.  The same formulas in the same
-// order as construct_ab_kernel, so M is the same to the bit.
+// order as construct_ab_kernel.
 constexpr int kRowCols = 16;
 __global__ void __launch_bounds__(kThreads) construct_rows_kernel(DevSystem sys, const __grid_constant__ KTable tab) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -390,32 +390,13 @@ __global__ void __launch_bounds__(kThreads) construct_rows_kernel(DevSystem sys,
                 }
             }
             __syncthreads();
-            // the rows M_t = [A_t; B_t] / e^{i 2pi K.tau} of each column (types with this rotation)
+            // the rows [A_t; B_t] / e^{i 2pi K.tau} of each column (types with this rotation)
             for (int c = 0; c < ncols; ++c) {
                 const int64_t gc = col0 + c;
                 const KEntry &ent = tab.e[entry_of(tab, gc)];
-                if (ent.R) {
-                    // the real form: Re of the rows m >= 0, Im of the rows m > 0 in place of -m
-                    double *rcol = ent.R + ldm * (gc - ent.col_begin);
-                    for (int idx = threadIdx.x; idx < twoL * nt; idx += blockDim.x) {
-                        const int t = idx / twoL;
-                        if (sys.num_rots > 0 && sys.type_rot[t] != rho) continue;
-                        const int r = idx - t * twoL;
-                        const bool isB = r >= L;
-                        const int lm = isB ? r - L : r;
-                        const int l = l_of[lm];
-                        double out = 0.0;
-                        if (l <= sys.type_lmax[t]) {
-                            const int tl = t * nl + l, l0 = l * (l + 1);
-                            const double y = lm >= l0 ? ylm[c * L + lm].x : -ylm[c * L + 2 * l0 - lm].y;
-                            out = (y * cf[tl]) * (isB ? bu[c * tnl + tl] : au[c * tnl + tl]);
-                        }
-                        rcol[idx] = out;
-                    }
-                    continue;
-                }
-                if (!ent.M) continue;
-                double2 *mcol = ent.M + ldm * (gc - ent.col_begin);
+                if (!ent.R) continue;
+                // Re of the rows m >= 0, Im of the rows m > 0 in place of -m
+                double *rcol = ent.R + ldm * (gc - ent.col_begin);
                 for (int idx = threadIdx.x; idx < twoL * nt; idx += blockDim.x) {
                     const int t = idx / twoL;
                     if (sys.num_rots > 0 && sys.type_rot[t] != rho) continue;
@@ -423,15 +404,13 @@ __global__ void __launch_bounds__(kThreads) construct_rows_kernel(DevSystem sys,
                     const bool isB = r >= L;
                     const int lm = isB ? r - L : r;
                     const int l = l_of[lm];
-                    double2 out = make_double2(0.0, 0.0);
+                    double out = 0.0;
                     if (l <= sys.type_lmax[t]) {
-                        const int tl = t * nl + l;
-                        const double cc = cf[tl];
-                        const double2 y = ylm[c * L + lm];
-                        const double f = isB ? bu[c * tnl + tl] : au[c * tnl + tl];
-                        out = make_double2((y.x * cc) * f, (-y.y * cc) * f);
+                        const int tl = t * nl + l, l0 = l * (l + 1);
+                        const double y = lm >= l0 ? ylm[c * L + lm].x : -ylm[c * L + 2 * l0 - lm].y;
+                        out = (y * cf[tl]) * (isB ? bu[c * tnl + tl] : au[c * tnl + tl]);
                     }
-                    mcol[idx] = out;
+                    rcol[idx] = out;
                 }
             }
         }
@@ -659,13 +638,17 @@ cudaError_t launch_construct_ab(const DevSystem &sys, const DevKpoint &kp, doubl
 
 cudaError_t launch_construct_ab_multi(const DevSystem &sys, const KTable &tab, cudaStream_t st) {
     if (tab.total_cols <= 0) return cudaSuccess;
-    bool anyM = false, anyC = false;
-    for (int k = 0; k < tab.nk; ++k) { anyM = anyM || tab.e[k].M || tab.e[k].R; anyC = anyC || tab.e[k].C; }
+    bool anyM = false, anyC = false, anyR = false;
+    for (int k = 0; k < tab.nk; ++k) {
+        anyM = anyM || tab.e[k].M;
+        anyC = anyC || tab.e[k].C;
+        anyR = anyR || tab.e[k].R;
+    }
     const bool rot = sys.atom_rotmat != nullptr;
     const size_t smem_rows = rows_kernel_smem(sys.L, sys.max_lmax, sys.num_types);
     // (the column-per-CTA kernel below for many types at a high lmax, whose tables do not fit;
     // per-type rows of (type, rotation) classes come only from this kernel)
-    if ((!rot || sys.num_rots > 0) && anyM && !anyC && smem_rows <= kRowsKernelSmemMax) {
+    if ((!rot || sys.num_rots > 0) && anyR && !anyC && !anyM && smem_rows <= kRowsKernelSmemMax) {
         const size_t smem = smem_rows;
         cudaError_t e = cudaFuncSetAttribute(construct_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
@@ -679,7 +662,7 @@ cudaError_t launch_construct_ab_multi(const DevSystem &sys, const KTable &tab, c
     smem = (smem + 15) & ~size_t(15);
     const int64_t grid = std::min<int64_t>(tab.total_cols, (int64_t)sm_count() * 8);
     if (rot) {
-        if (anyM) return cudaErrorInvalidValue;  // per-type rows exist only when atoms share the rotation
+        if (anyM || anyR) return cudaErrorInvalidValue;  // per-type rows exist only when atoms share the rotation
         cudaFuncSetAttribute(construct_ab_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         construct_ab_kernel<true><<<(unsigned)grid, kThreads, smem, st>>>(sys, tab);
     } else {

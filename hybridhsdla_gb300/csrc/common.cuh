@@ -121,14 +121,30 @@ constexpr int kFp64Tile = 64;
 int64_t fp64_job_tiles(const Fp64Job &j);
 cudaError_t launch_fp64_jobs(const Fp64Job *d_jobs, int num_jobs, int64_t total_tiles, cudaStream_t st);
 
+// Real FP64 contraction out = P^T diag(w) Q over a batch of jobs (the structure-factor form's real
+// rows, see real_products.cu): P k x m, Q k x n, out m x n, column-major.
+struct Fp64RealJob {
+    const double *P; int64_t ldp;
+    const double *Q; int64_t ldq;
+    const double *w;                 // k weights or nullptr
+    double *out; int64_t ldo;
+    int64_t m, n, k;
+    int32_t lower;                   // 1: only elements with row >= col (m == n required)
+    int32_t tiles_n;                 // tile columns of this job
+    int64_t tile_begin;              // first global tile index of this job
+};
+// Numbers the jobs' tiles for one launch and returns their count; `edge` receives the tile edge
+// chosen for the launch (what launch_fp64_real needs back).
+int64_t fp64_real_assign(Fp64RealJob *jobs, int num_jobs, int *edge);
+cudaError_t launch_fp64_real(const Fp64RealJob *d_jobs, int num_jobs, int64_t tiles, int edge, cudaStream_t st);
+
 // ---- structure-factor form (atoms sharing their type's rotation)
-// One k-point of a combine: per-type products PS, PH (lower triangles, ld ldp) into the outputs
+// One k-point of a combine: real per-type products (lower triangles, ld ldp) into the outputs
 // S, H (ld ldo); g the k-point's G-vectors [n][3] on the device.
 struct SfEntry {
-    const double2 *PS = nullptr, *PH = nullptr;   // per-type products, type slot b at + b pstride
-    // or (PS and PH NULL) as fixed-point numbers: S, and the real and imaginary parts of H, element
-    // (r, c) times 2^(el[r] + er[c] - 8 - frac) with er = ers for S and erh for H
-    const long long *RS = nullptr, *RHr = nullptr, *RHi = nullptr;
+    // per-type products S, Re H and Im H, type slot b at + b pstride: FP64, or (el set) fixed-point
+    // numbers, element (r, c) times 2^(el[r] + er[c] - 8 - frac) with er = ers for S and erh for H
+    const void *RS = nullptr, *RHr = nullptr, *RHi = nullptr;
     const int32_t *el = nullptr, *ers = nullptr, *erh = nullptr;
     double2 *S = nullptr, *H = nullptr;
     // what a combine that is not the first adds to (NULL: S and H themselves, ldo)
@@ -155,7 +171,7 @@ struct SfTab {
 // per-atom factors ex[a][dGx + dx] = e^{i 2pi dGx tau_a,x} (and y, z); atoms listed by type.
 cudaError_t launch_sf_table(const double2 *ex, const double2 *ey, const double2 *ez, const int32_t *order,
                             const int32_t *type_begin, int nt, int nx, int ny, int nz, double2 *sf, cudaStream_t st);
-// S (+)= sum_b SF_{type+b} (.) PS_b and H (+)= sum_b SF_{type+b} (.) PH_b over the lower triangles
+// S (+)= sum_b SF_{type+b} (.) S_b and H (+)= sum_b SF_{type+b} (.) H_b over the lower triangles
 // of every entry, b over the batch's type slots, in columns [tab.col0, tab.col1) (multiples of 32
 // but for the end); rows below tab.xrow1 into Sx, Hx instead for entries that give them.
 cudaError_t launch_sf_combine(const SfTab &tab, const double2 *sf, bool first, cudaStream_t st);

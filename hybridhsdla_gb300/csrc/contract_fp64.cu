@@ -168,7 +168,135 @@ __global__ void __launch_bounds__(kThreads) fp64_jobs_kernel(const Fp64Job *__re
     }
 }
 
+// ---------------------------------------------------------------- real products
+// Real DMMA products for the structure-factor form's real rows.  GB300's FP64 rate (1.05 TFLOP/s,
+// one m16n8k4 MMA in ~300 cycles and SM) bounds every shape, so there is no staging: fragments come
+// straight from global memory (L1 and L2 serve the reuse, 0.3-0.5 TB/s), four K steps ahead, and what
+// counts is an even share of the MMAs per SM.  A CTA of four warps has a 32 x 32 tile (a 16 x 16
+// quarter each); where a launch has fewer than kSplitBelow of those per SM, a 16 x 16 tile with the
+// contraction split over the warps.  Whole pass, complex 64 x 64 tiles before and this now: 235 columns,
+// lmax 8, two types (host call) 2.96 and 0.64 ms (20 of 152 SMs were busy); 3000 columns of four types
+// 55.7 and 20.6 ms (eight real products and three, each at the FP64 rate).
+constexpr int kRealU = 4;            // K steps loaded ahead
+constexpr int kSplitBelow = 8;
+
+template <bool kSplit>
+__global__ void __launch_bounds__(128) fp64_real_kernel(const Fp64RealJob *__restrict__ jobs, int num_jobs) {
+    constexpr int kT = kSplit ? 16 : 32;
+    const int64_t gt = blockIdx.x;
+    int lo = 0, hi = num_jobs - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (jobs[mid].tile_begin <= gt) lo = mid; else hi = mid - 1;
+    }
+    const Fp64RealJob &j = jobs[lo];
+    const int64_t m = j.m, n = j.n, K = j.k, x = gt - j.tile_begin;
+    int64_t ti, tj;
+    if (j.lower) {
+        ti = (int64_t)((sqrt(8.0 * (double)x + 1.0) - 1.0) * 0.5);
+        while (ti * (ti + 1) / 2 > x) --ti;
+        while ((ti + 1) * (ti + 2) / 2 <= x) ++ti;
+        tj = x - ti * (ti + 1) / 2;
+    } else {
+        ti = x / j.tiles_n;
+        tj = x - ti * j.tiles_n;
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gid = lane >> 2, tig = lane & 3;
+    const int64_t m0 = ti * kT + (kSplit ? 0 : (warp >> 1) * 16), n0 = tj * kT + (kSplit ? 0 : (warp & 1) * 16);
+    double acc[2][4] = {};
+    const int64_t steps = (K + 3) / 4;
+    const int64_t s0 = kSplit ? steps * warp / 4 : 0, s1 = kSplit ? steps * (warp + 1) / 4 : steps;
+    if (m0 < m && n0 < n && !(j.lower && m0 + 15 < n0)) {
+        // rows and columns past the ends repeat the last one (their results are not stored)
+        const double *pa0 = j.P + j.ldp * min(m0 + gid, m - 1), *pa1 = j.P + j.ldp * min(m0 + gid + 8, m - 1);
+        const double *pb0 = j.Q + j.ldq * min(n0 + gid, n - 1), *pb1 = j.Q + j.ldq * min(n0 + gid + 8, n - 1);
+        double a0[2][kRealU], a1[2][kRealU], b0[2][kRealU], b1[2][kRealU];
+        auto load = [&](int buf, int64_t s) {
+#pragma unroll
+            for (int u = 0; u < kRealU; ++u) {
+                const int64_t k = (s + u) * 4 + tig, kc = min(k, K - 1);
+                const bool in = k < K && s + u < s1;
+                a0[buf][u] = in ? pa0[kc] : 0.0;
+                a1[buf][u] = in ? pa1[kc] : 0.0;
+                b0[buf][u] = pb0[kc];
+                b1[buf][u] = pb1[kc];
+                if (j.w) {
+                    const double w = j.w[kc];
+                    a0[buf][u] *= w;
+                    a1[buf][u] *= w;
+                }
+            }
+        };
+        auto mma = [&](int buf) {
+#pragma unroll
+            for (int u = 0; u < kRealU; ++u) {
+                dmma(acc[0], a0[buf][u], a1[buf][u], b0[buf][u]);
+                dmma(acc[1], a0[buf][u], a1[buf][u], b1[buf][u]);
+            }
+        };
+        if (s0 < s1) load(0, s0);
+        for (int64_t s = s0; s < s1; s += 2 * kRealU) {
+            if (s + kRealU < s1) load(1, s + kRealU);
+            mma(0);
+            if (s + 2 * kRealU < s1) load(0, s + 2 * kRealU);
+            if (s + kRealU < s1) mma(1);
+        }
+    }
+    if constexpr (kSplit) {
+        // the warps' parts, added in warp order
+        __shared__ double part[3][2][4][32];
+        if (warp > 0)
+#pragma unroll
+            for (int t = 0; t < 2; ++t)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) part[warp - 1][t][c][lane] = acc[t][c];
+        __syncthreads();
+        if (warp > 0) return;
+#pragma unroll
+        for (int w = 0; w < 3; ++w)
+#pragma unroll
+            for (int t = 0; t < 2; ++t)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[t][c] += part[w][t][c][lane];
+    }
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int64_t row = m0 + gid + ((c >= 2) ? 8 : 0), col = n0 + t * 8 + tig * 2 + (c & 1);
+            if (row < m && col < n && (!j.lower || row >= col)) j.out[row + j.ldo * col] = acc[t][c];
+        }
+}
+
 }  // namespace
+
+int64_t fp64_real_assign(Fp64RealJob *jobs, int num_jobs, int *edge) {
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    int64_t total = 0;
+    for (int e = 32; e >= 16; e /= 2) {
+        total = 0;
+        for (int i = 0; i < num_jobs; ++i) {
+            Fp64RealJob &j = jobs[i];
+            const int64_t tm = (j.m + e - 1) / e, tn = (j.n + e - 1) / e;
+            j.tiles_n = (int32_t)tn;
+            j.tile_begin = total;
+            total += j.lower ? tm * (tm + 1) / 2 : tm * tn;
+        }
+        *edge = e;
+        if (total >= (int64_t)kSplitBelow * nsm) break;
+    }
+    return total;
+}
+
+cudaError_t launch_fp64_real(const Fp64RealJob *d_jobs, int num_jobs, int64_t tiles, int edge, cudaStream_t st) {
+    if (tiles <= 0) return cudaSuccess;
+    if (tiles > 0x7fffffffLL) return cudaErrorInvalidValue;
+    if (edge == 16) fp64_real_kernel<true><<<(unsigned)tiles, 128, 0, st>>>(d_jobs, num_jobs);
+    else fp64_real_kernel<false><<<(unsigned)tiles, 128, 0, st>>>(d_jobs, num_jobs);
+    return cudaGetLastError();
+}
 
 int64_t fp64_job_tiles(const Fp64Job &j) {
     const int64_t tm = (j.m + BM - 1) / BM, tn = (j.n + BN - 1) / BN;

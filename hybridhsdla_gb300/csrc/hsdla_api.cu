@@ -94,6 +94,7 @@ struct hsdla_plan {
     std::vector<Fp64Job> h_jobs;
     OzakiPlan oz{};
     // k-point groups, prepared against the context workspace (re-prepared when it moves)
+    struct RealBatch { int first = 0, jobs = 0, edge = 0; int64_t tiles = 0; };
     struct Group {
         std::vector<int> kidx;           // plan k-point indices
         KTable ktab;                     // construct / phase tables (C, M, Z, X per k-point)
@@ -104,6 +105,10 @@ struct hsdla_plan {
         Fp64Job *d_jobs_sh = nullptr;    // FP64: S/H jobs (device) and their pinned host copy
         Fp64Job *h_jobs_sh = nullptr;
         int64_t tiles_sh = 0;
+        // FP64 structure-factor form: real jobs (device), the products' in one launch per combine batch
+        Fp64RealJob *d_rjobs_t = nullptr, *d_rjobs_sh = nullptr;
+        int edge_t = 0;
+        std::vector<RealBatch> batches;
         void *persist = nullptr;         // prepared tables (not shared with other groups)
         int64_t persist_bytes = 0;
         // event pairs around the S/H product launches (one pair, or one per type in the
@@ -133,10 +138,8 @@ struct hsdla_plan {
     bool tcheck_pending = false;
     const unsigned long long *tcheck_host = nullptr;
     std::vector<int32_t> tcheck_class_type;
-    double *wt = nullptr;
-    double *wt_real = nullptr;       // the same for the real rows (2 wt where m != 0)
-    double *TR = nullptr;            // real T blocks [nt][4L][2L] (Ozaki)
-    bool real = false;               // the structure-factor form runs on real rows (real_products.cu)
+    double *wt = nullptr;            // (of the real rows: doubled where m != 0)
+    double *TR = nullptr;            // real T blocks [nt][4L][2L]
     double2 *sf_tab = nullptr;
     SfTab sf_dims{};                 // box extents and offsets (entries filled per group)
     int tbatch = 1;                  // types whose products are combined into S and H in one pass
@@ -807,14 +810,12 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     // grouped by type and the table itself over the box of G-vector differences g_col - g_row
     const char *sf_env = getenv("HSDLA_SF");
     pl->sf = pl->hoist && !(sf_env && strtol(sf_env, nullptr, 10) == 0);
-    pl->real = pl->sf && pl->opts.precision == HSDLA_PREC_OZAKI_FP8;
     int half[3] = {0, 0, 0}, ext[3] = {1, 1, 1};
     if (pl->sf) {
         for (int i = 0; i < nk; ++i)
             for (int64_t q = 0; q < kpts[i].n_g; ++q)
                 for (int c = 0; c < 3; ++c) half[c] = std::max(half[c], 2 * std::abs(kpts[i].g[3 * q + c]));
         for (int c = 0; c < 3; ++c) ext[c] = 2 * half[c] + 1;
-        add(sizeof(double) * 2 * L * nt);
         add(sizeof(double) * 2 * L * nt);
         add(sizeof(int32_t) * (na + nt + 1));
     }
@@ -827,7 +828,7 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
         add(sizeof(double2) * (int64_t)na * (ext[0] + ext[1] + ext[2]));
         add(sizeof(double2) * (int64_t)nt * ext[0] * ext[1] * ext[2]);
     }
-    if (pl->real) add(sizeof(double) * 2 * tf_elems);
+    if (pl->sf) add(sizeof(double) * 2 * tf_elems);
     const double p_tables = pms();
     rc = ctx_malloc(ctx, &pl->tables, bytes);
     if (rc) { delete pl; return rc; }
@@ -903,17 +904,12 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
         for (int t = 0; t < nt; ++t)
             for (int l = 0; l < nl; ++l)
                 for (int lm = l * l; lm < (l + 1) * (l + 1); ++lm) {
-                    wt[(size_t)2 * L * t + lm] = 1.0;
-                    wt[(size_t)2 * L * t + L + lm] = (l <= s->type_lmax[t]) ? s->type_dE_u_norm[t * nl + l] : 0.0;
+                    // the rows (l, m) and (l, -m) of a real pair carry both complex rows' weight
+                    const double pair = lm == l * (l + 1) ? 1.0 : 2.0;
+                    wt[(size_t)2 * L * t + lm] = pair;
+                    wt[(size_t)2 * L * t + L + lm] = (l <= s->type_lmax[t]) ? pair * s->type_dE_u_norm[t * nl + l] : 0.0;
                 }
         pl->wt = (double *)put(wt.data(), sizeof(double) * wt.size());
-        // the rows (l, m) and (l, -m) of a real pair carry both complex rows' weight
-        for (int t = 0; t < nt; ++t)
-            for (int h = 0; h < 2; ++h)
-                for (int l = 0; l < nl; ++l)
-                    for (int lm = l * l; lm < (l + 1) * (l + 1); ++lm)
-                        if (lm != l * (l + 1)) wt[(size_t)2 * L * t + (size_t)h * L + lm] *= 2.0;
-        pl->wt_real = (double *)put(wt.data(), sizeof(double) * wt.size());
         std::vector<int32_t> ord;
         std::vector<int32_t> tb(nt + 1, 0);
         for (int t = 0; t < nt; ++t) {
@@ -941,7 +937,7 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
         d_ex = (double2 *)dev_only(sizeof(double2) * (int64_t)na * (ext[0] + ext[1] + ext[2]));
         pl->sf_tab = (double2 *)dev_only(sizeof(double2) * (int64_t)nt * ext[0] * ext[1] * ext[2]);
     }
-    if (pl->real) pl->TR = (double *)dev_only(sizeof(double) * 2 * tf_elems);
+    if (pl->sf) pl->TR = (double *)dev_only(sizeof(double) * 2 * tf_elems);
     std::vector<unsigned long long> tstats((size_t)5 * nt, 0);
     {
         // the pending copies as one byte range split evenly over up to four threads (one copying
@@ -976,7 +972,7 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     cudaError_t e = cudaMemcpyAsync(pl->tables, stage, upload_bytes, cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(d_stats, 0, sizeof(unsigned long long) * 5 * nt, ctx->stream);
     if (e == cudaSuccess) e = launch_tfull(d_taa, d_tab, d_tbb, nt, L, pl->Tfull, d_stats, ctx->stream);
-    if (e == cudaSuccess && pl->real) e = launch_treal(pl->Tfull, nt, L, pl->TR, ctx->stream);
+    if (e == cudaSuccess && pl->sf) e = launch_treal(pl->Tfull, nt, L, pl->TR, ctx->stream);
     if (e == cudaSuccess && pl->sf) e = launch_sf_phases(D.atom_pos, na, half, ext, d_ex, ctx->stream);
     if (e == cudaSuccess && pl->sf)
         e = launch_sf_table(d_ex, d_ex + (size_t)na * ext[0], d_ex + (size_t)na * (ext[0] + ext[1]), d_order,
@@ -1025,11 +1021,11 @@ namespace {
 int64_t kpoint_fp64_bytes(const hsdla_plan *pl, int64_t G) {
     const int64_t K = pl->twoLa, ldm = 2 * (int64_t)pl->L * pl->nt;
     auto r = [](int64_t x) { return (x + 1023) / 1024 * 1024; };        // each buffer is 1 KB aligned
-    // structure-factor form: M, Z and the two products of each type of a combine batch (no C, no X)
-    if (pl->real)       // the same on real rows: R, Z' (two parts) and three products
+    // structure-factor form: the real rows R, Z' (two parts) and the three products of each type of a
+    // combine batch (no C, no X)
+    if (pl->sf)
         return r(ldm * G * (int64_t)sizeof(double)) + r(2 * ldm * G * (int64_t)sizeof(double)) +
                3 * r(pl->tbatch * G * G * (int64_t)sizeof(double));
-    if (pl->sf) return 2 * r(ldm * G * (int64_t)sizeof(double2)) + 2 * r(pl->tbatch * G * G * (int64_t)sizeof(double2));
     const int64_t nCX = pl->opts.precision == HSDLA_PREC_FP64 ? 2 : 1;   // FP64 keeps C and X apart
     int64_t b = nCX * r(K * G * (int64_t)sizeof(double2));
     if (pl->hoist) b += 2 * r(ldm * G * (int64_t)sizeof(double2));
@@ -1052,13 +1048,14 @@ int64_t group_persist_bytes(const hsdla_plan *pl, const std::vector<int> &kidx) 
     if (pl->opts.precision == HSDLA_PREC_OZAKI_FP8)
         return ozaki_group_persist_bytes(pl->oz.num_slices, 2 * (int64_t)pl->L, pl->na, pl->nt, G, pl->panels, pl->sf);
     // the FP64 group keeps two job tables, each rounded up to 1 KiB: the T applications (one per
-    // type when hoisted, else one per atom, per k-point) and the S/H products (two per type in
+    // type when hoisted, else one per atom, per k-point) and the S/H products (three per type in
     // the structure-factor form, else two, per k-point)
     const int64_t nk = (int64_t)kidx.size();
     const int64_t n_t = nk * (pl->hoist ? pl->nt : pl->na);
-    const int64_t n_sh = nk * 2 * (pl->sf ? pl->nt : 1);
+    const int64_t n_sh = nk * (pl->sf ? 3 * pl->nt : 2);
     auto up = [](int64_t b) { return (b + 1023) / 1024 * 1024; };
-    return up((int64_t)sizeof(Fp64Job) * n_t) + up((int64_t)sizeof(Fp64Job) * n_sh);
+    const int64_t js = pl->sf ? sizeof(Fp64RealJob) : sizeof(Fp64Job);
+    return up(js * n_t) + up(js * n_sh);
 }
 
 // Device-memory budget for one group's workspace: HSDLA_WORKSPACE_BUDGET (bytes), else 85% of
@@ -1149,6 +1146,7 @@ void release_groups(hsdla_plan *pl) {
         g.ev_dom.clear();
         for (auto &e : g.ev_t) if (e) cudaEventDestroy(e);
         g.ev_t.clear();
+        g.batches.clear();
         g.oz = nullptr;
         g.h_jobs_sh = nullptr;
         g.persist = nullptr;
@@ -1169,9 +1167,9 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
         g.persist_bytes = group_persist_bytes(pl, g.kidx);
         int rcp = ctx_malloc(ctx, &g.persist, g.persist_bytes);
         if (rcp) return rcp;
-        // one pair per S/H product launch: FP64 runs one per type, Ozaki one per combine batch
+        // one pair per S/H product launch: one launch per combine batch in the structure-factor form
         // (streamed host output adds pairs for its column blocks)
-        g.ev_dom.assign(pl->real ? 2 * std::max(2, (pl->nt + pl->tbatch - 1) / pl->tbatch) : pl->sf ? 2 * pl->nt : 2, nullptr);
+        g.ev_dom.assign(pl->sf ? 2 * std::max(2, (pl->nt + pl->tbatch - 1) / pl->tbatch) : 2, nullptr);
         for (auto &e : g.ev_dom) CUDA_TRY(ctx, cudaEventCreate(&e));
         char *pp = reinterpret_cast<char *>(g.persist);
         auto keep = [&](int64_t bytes) { char *r = pp; pp += (bytes + 1023) / 1024 * 1024; return r; };
@@ -1188,7 +1186,7 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
             e.col_begin = col;
             col += G;
             if (pl->sf) {
-                e.C = nullptr;            // structure-factor form: only the per-type rows
+                e.C = nullptr;            // structure-factor form: only the real per-type rows
                 e.X = nullptr;
             } else {
                 e.C = reinterpret_cast<double2 *>(take(K * G * (int64_t)sizeof(double2)));
@@ -1198,7 +1196,7 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
             }
             OzKBufs b;
             b.G = G;
-            if (pl->real) {
+            if (pl->sf) {
                 b.R = reinterpret_cast<double *>(take(ldm * G * (int64_t)sizeof(double)));
                 b.ZR = reinterpret_cast<long long *>(take(2 * ldm * G * (int64_t)sizeof(long long)));
                 b.pstride = G * G;
@@ -1220,13 +1218,6 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
             e.M = pl->hoist ? reinterpret_cast<double2 *>(take(ldm * G * (int64_t)sizeof(double2))) : nullptr;
             double2 *Z = pl->hoist ? reinterpret_cast<double2 *>(take(ldm * G * (int64_t)sizeof(double2))) : nullptr;
             e.Z = Z;
-            if (pl->sf) {
-                SfEntry &f = g.sft.e[q];
-                f = SfEntry();
-                f.PS = reinterpret_cast<double2 *>(take(pl->tbatch * G * G * (int64_t)sizeof(double2)));
-                f.PH = reinterpret_cast<double2 *>(take(pl->tbatch * G * G * (int64_t)sizeof(double2)));
-                f.ldp = G; f.n = G; f.pstride = G * G; f.g = pk.dk.g;
-            }
             b.CX = e.C; b.M = e.M; b.Z = Z;
             kb.push_back(b);
         }
@@ -1242,16 +1233,62 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
             d.twoL = twoL; d.na = pl->na; d.nt = pl->nt; d.hoist = pl->hoist;
             d.w = pl->w; d.Tfull = pl->Tfull; d.atom_type = pl->atom_type.data();
             d.panels = pl->panels;
-            d.sf = pl->sf; d.wt = pl->wt_real; d.TR = pl->TR; d.sf_tab = pl->sf_tab; d.tbatch = pl->tbatch;
+            d.sf = pl->sf; d.wt = pl->wt; d.TR = pl->TR; d.sf_tab = pl->sf_tab; d.tbatch = pl->tbatch;
             char *oz_ws = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(p) + 1023) & ~uintptr_t(1023));
             int rc = ozaki_group_prepare(pl->oz, d, kb, oz_ws, g.persist, st, &g.oz);
             if (rc) return set_err(ctx, rc, "group set-up failed: %s", ozaki_last_error());
-            if (pl->real) ozaki_group_sf_exponents(g.oz, g.sft);
+            if (pl->sf) ozaki_group_sf_exponents(g.oz, g.sft);
             g.ev_t.assign(2 * ozaki_group_tapply_events(g.oz), nullptr);
             for (auto &e : g.ev_t) CUDA_TRY(ctx, cudaEventCreate(&e));
         } else {
             g.ev_t.assign(2, nullptr);
             for (auto &e : g.ev_t) CUDA_TRY(ctx, cudaEventCreate(&e));
+            if (pl->sf) {
+                // Z'_t = T'_t R_t, and per type S_t = R_t^T diag(w_t) R_t and H_t = R_t^T Z'_t (real and
+                // imaginary parts) of every k-point; one launch per combine batch
+                std::vector<Fp64RealJob> rt, rsh;
+                for (int q = 0; q < kt.nk; ++q)
+                    for (int t = 0; t < pl->nt; ++t) {
+                        Fp64RealJob jb{};
+                        jb.P = pl->TR + 2 * twoL * twoL * t; jb.ldp = twoL;
+                        jb.Q = kb[q].R + twoL * t; jb.ldq = ldm;
+                        jb.out = reinterpret_cast<double *>(kb[q].ZR) + 2 * twoL * t; jb.ldo = 2 * ldm;
+                        jb.m = 2 * twoL; jb.n = kb[q].G; jb.k = twoL;
+                        rt.push_back(jb);
+                    }
+                g.tiles_t = fp64_real_assign(rt.data(), (int)rt.size(), &g.edge_t);
+                for (int t0 = 0; t0 < pl->nt; t0 += pl->tbatch) {
+                    const size_t first = rsh.size();
+                    for (int t = t0; t < std::min(pl->nt, t0 + pl->tbatch); ++t)
+                        for (int q = 0; q < kt.nk; ++q)
+                            for (int which = 0; which < 3; ++which) {
+                                Fp64RealJob jb{};
+                                jb.P = kb[q].R + twoL * t; jb.ldp = ldm;
+                                jb.Q = which == 0 ? jb.P : reinterpret_cast<double *>(kb[q].ZR) + 2 * twoL * t + (which - 1) * twoL;
+                                jb.ldq = which == 0 ? ldm : 2 * ldm;
+                                jb.w = which == 0 ? pl->wt + twoL * t : nullptr;
+                                jb.out = reinterpret_cast<double *>(which == 0 ? kb[q].RS : which == 1 ? kb[q].RHr : kb[q].RHi) +
+                                         (int64_t)(t - t0) * kb[q].pstride;
+                                jb.ldo = kb[q].G;
+                                jb.m = kb[q].G; jb.n = kb[q].G; jb.k = twoL; jb.lower = 1;
+                                rsh.push_back(jb);
+                            }
+                    hsdla_plan::RealBatch rb;
+                    rb.first = (int)first;
+                    rb.jobs = (int)(rsh.size() - first);
+                    rb.tiles = fp64_real_assign(rsh.data() + first, rb.jobs, &rb.edge);
+                    g.batches.push_back(rb);
+                }
+                g.n_jobs_t = (int)rt.size();
+                g.d_rjobs_t = reinterpret_cast<Fp64RealJob *>(keep(sizeof(Fp64RealJob) * rt.size()));
+                g.d_rjobs_sh = reinterpret_cast<Fp64RealJob *>(keep(sizeof(Fp64RealJob) * rsh.size()));
+                if (pp - reinterpret_cast<char *>(g.persist) > g.persist_bytes)
+                    return set_err(ctx, HSDLA_ERR_NOMEM, "job tables (%lld bytes) exceed the group's %lld persistent bytes",
+                                   (long long)(pp - reinterpret_cast<char *>(g.persist)), (long long)g.persist_bytes);
+                CUDA_TRY(ctx, cudaMemcpy(g.d_rjobs_t, rt.data(), sizeof(Fp64RealJob) * rt.size(), cudaMemcpyHostToDevice));
+                CUDA_TRY(ctx, cudaMemcpy(g.d_rjobs_sh, rsh.data(), sizeof(Fp64RealJob) * rsh.size(), cudaMemcpyHostToDevice));
+                continue;
+            }
             std::vector<Fp64Job> jt, jsh;
             for (int q = 0; q < kt.nk; ++q) {
                 const KEntry &e = kt.e[q];
@@ -1275,7 +1312,6 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
                         jt.push_back(jb);
                     }
                 }
-                if (pl->sf) continue;
                 Fp64Job js{};
                 js.P = e.C; js.ldp = K; js.Q = e.C; js.ldq = K; js.w = pl->w;
                 js.m = G; js.n = G; js.k = K; js.lower = 1;
@@ -1285,32 +1321,7 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
                 jsh.push_back(jh);
             }
             g.tiles_t = assign_tiles(jt, 0);
-            if (pl->sf) {
-                // per type: S_t = M_t^H diag(w_t) M_t and H_t = M_t^H Z_t of every k-point into the
-                // products; one launch per type (each type's jobs carry their own tile numbering)
-                for (int t = 0; t < pl->nt; ++t) {
-                    std::vector<Fp64Job> jt_sh;
-                    for (int q = 0; q < kt.nk; ++q) {
-                        const KEntry &e = kt.e[q];
-                        const int64_t G = pl->kps[g.kidx[q]].n_g;
-                        Fp64Job js{};
-                        js.P = e.M + twoL * t; js.ldp = ldm; js.Q = e.M + twoL * t; js.ldq = ldm;
-                        js.w = pl->wt + twoL * t;
-                        const int64_t slot = (int64_t)(t % pl->tbatch) * g.sft.e[q].pstride;
-                        js.out = const_cast<double2 *>(g.sft.e[q].PS) + slot; js.ldo = G;
-                        js.m = G; js.n = G; js.k = twoL; js.lower = 1;
-                        Fp64Job jh = js;
-                        jh.Q = e.Z + twoL * t; jh.w = nullptr;
-                        jh.out = const_cast<double2 *>(g.sft.e[q].PH) + slot;
-                        jt_sh.push_back(js);
-                        jt_sh.push_back(jh);
-                    }
-                    g.tiles_sh = assign_tiles(jt_sh, 0);
-                    jsh.insert(jsh.end(), jt_sh.begin(), jt_sh.end());
-                }
-            } else {
-                g.tiles_sh = assign_tiles(jsh, 0);
-            }
+            g.tiles_sh = assign_tiles(jsh, 0);
             g.n_jobs_t = (int)jt.size();
             g.d_jobs_t = reinterpret_cast<Fp64Job *>(keep(sizeof(Fp64Job) * jt.size()));
             g.d_jobs_sh = reinterpret_cast<Fp64Job *>(keep(sizeof(Fp64Job) * jsh.size()));
@@ -1323,8 +1334,6 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
             }
             memcpy(g.h_jobs_sh, jsh.data(), sizeof(Fp64Job) * jsh.size());
             CUDA_TRY(ctx, cudaMemcpy(g.d_jobs_t, jt.data(), sizeof(Fp64Job) * jt.size(), cudaMemcpyHostToDevice));
-            if (pl->sf)     // the products' jobs do not change between runs
-                CUDA_TRY(ctx, cudaMemcpy(g.d_jobs_sh, jsh.data(), sizeof(Fp64Job) * jsh.size(), cudaMemcpyHostToDevice));
         }
     }
     pl->prepared_ws = ws;
@@ -1390,8 +1399,9 @@ void run_groups_flop_one(const hsdla_plan *pl, const hsdla_plan::Group &g, doubl
     for (int q = 0; q < g.ktab.nk; ++q) {
         const double G = (double)g.ktab.e[q].kp.n_g;
         const double lower = 4.0 * G * (G + 1.0) * Klen;
-        // (the real form: three real products where the complex form has eight)
-        *dom_flop += 2.0 * lower * (g.oz ? sl * (sl + 1) / 2 : 1.0) * (pl->real ? 0.375 : 1.0);
+        // (digit products: the real form's three where the complex form has eight; FP64: the flops of
+        // the complex products that the real ones replace)
+        *dom_flop += 2.0 * lower * (g.oz ? sl * (sl + 1) / 2 * (pl->sf ? 0.375 : 1.0) : 1.0);
     }
 }
 
@@ -1523,28 +1533,32 @@ int run_groups(hsdla_plan *pl, cudaStream_t st, bool timed, float *ms_ab, float 
             }
         } else if (pl->sf) {
             if (timed) CUDA_TRY(ctx, cudaEventRecord(g.ev_t[0], st));
-            CUDA_TRY(ctx, launch_fp64_jobs(g.d_jobs_t, g.n_jobs_t, g.tiles_t, st));
+            CUDA_TRY(ctx, launch_fp64_real(g.d_rjobs_t, g.n_jobs_t, g.tiles_t, g.edge_t, st));
             if (timed) CUDA_TRY(ctx, cudaEventRecord(g.ev_t[1], st));
             pl->launches++;
-            const int nj = 2 * g.ktab.nk;
-            for (int t = 0; t < pl->nt; ++t) {
-                CUDA_TRY(ctx, record_event(g.ev_dom[2 * t], st));
-                CUDA_TRY(ctx, launch_fp64_jobs(g.d_jobs_sh + (int64_t)nj * t, nj, g.tiles_sh, st));
-                CUDA_TRY(ctx, record_event(g.ev_dom[2 * t + 1], st));
+            size_t p = 0;
+            for (int t0 = 0; t0 < pl->nt; t0 += pl->tbatch, ++p) {
+                const hsdla_plan::RealBatch &rb = g.batches[p];
+                CUDA_TRY(ctx, record_event(g.ev_dom[2 * p], st));
+                CUDA_TRY(ctx, launch_fp64_real(g.d_rjobs_sh + rb.first, rb.jobs, rb.tiles, rb.edge, st));
+                CUDA_TRY(ctx, record_event(g.ev_dom[2 * p + 1], st));
                 pl->launches++;
-                // the batch's last type: its products into S and H
-                if ((t + 1) % pl->tbatch == 0 || t + 1 == pl->nt) {
-                    const int t0 = t / pl->tbatch * pl->tbatch;
-                    if (t0 == last_t0) {
-                        const int rcc = combine_last(pl, g, t0, t + 1 - t0, st, capturing);
-                        if (rcc) return rcc;
-                        continue;
-                    }
-                    g.sft.type = t0;
-                    g.sft.ntypes = t + 1 - t0;
-                    CUDA_TRY(ctx, launch_sf_combine(g.sft, pl->sf_tab, t0 == 0, st));
-                    pl->launches++;
+                // the batch's products into S and H
+                const int nb = std::min(pl->nt, t0 + pl->tbatch) - t0;
+                if (t0 == last_t0) {
+                    const int rcc = combine_last(pl, g, t0, nb, st, capturing);
+                    if (rcc) return rcc;
+                    continue;
                 }
+                g.sft.type = t0;
+                g.sft.ntypes = nb;
+                CUDA_TRY(ctx, launch_sf_combine(g.sft, pl->sf_tab, t0 == 0, st));
+                pl->launches++;
+            }
+            // (pairs past the batches span nothing; the last event closes the group's products)
+            for (; 2 * p + 1 < g.ev_dom.size(); ++p) {
+                CUDA_TRY(ctx, record_event(g.ev_dom[2 * p], st));
+                CUDA_TRY(ctx, record_event(g.ev_dom[2 * p + 1], st));
             }
         } else {
             if (timed) CUDA_TRY(ctx, cudaEventRecord(g.ev_t[0], st));

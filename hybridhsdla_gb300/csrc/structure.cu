@@ -89,7 +89,8 @@ constexpr int kSfTile = 32, kSfRows = 4;
 // rows of a column.  A batch of several types reads and writes S and H once.  The tiles of an
 // entry are its tile columns [tc0, tc1) (a column range of the launch), each from the diagonal
 // tile down.
-template <bool kReal>
+// kFixed: fixed-point products (of the digit form), else FP64 ones.
+template <bool kFixed>
 __global__ void __launch_bounds__(kSfTile * kSfRows) sf_combine_kernel(const __grid_constant__ SfTab tab,
                                                                        const double2 *__restrict__ sf, int first) {
     const int64_t tile = blockIdx.x;
@@ -124,23 +125,24 @@ __global__ void __launch_bounds__(kSfTile * kSfRows) sf_combine_kernel(const __g
         double2 vs = make_double2(0.0, 0.0), vh = make_double2(0.0, 0.0);
         for (int b = 0; b < tab.ntypes; ++b) {
             const double2 f = sft[idx + b * tab.box];
-            if constexpr (kReal) {
-                // S_t real, H_t complex: 6 FMAs (GB300's FP64 rate bounds this kernel)
-                const int64_t o = off + (tab.slot0 + b) * E.pstride;
-                const double ps = int_to_f64(E.RS[o]), hr = int_to_f64(E.RHr[o]), hi = int_to_f64(E.RHi[o]);
-                vs.x = fma(f.x, ps, vs.x);
-                vs.y = fma(f.y, ps, vs.y);
-                vh.x = fma(f.x, hr, fma(-f.y, hi, vh.x));
-                vh.y = fma(f.x, hi, fma(f.y, hr, vh.y));
-                continue;
+            // S_t real, H_t complex: 6 FMAs (GB300's FP64 rate bounds this kernel)
+            const int64_t o = off + (tab.slot0 + b) * E.pstride;
+            double ps, hr, hi;
+            if constexpr (kFixed) {
+                ps = int_to_f64(static_cast<const long long *>(E.RS)[o]);
+                hr = int_to_f64(static_cast<const long long *>(E.RHr)[o]);
+                hi = int_to_f64(static_cast<const long long *>(E.RHi)[o]);
+            } else {
+                ps = static_cast<const double *>(E.RS)[o];
+                hr = static_cast<const double *>(E.RHr)[o];
+                hi = static_cast<const double *>(E.RHi)[o];
             }
-            const double2 ps = E.PS[off + (tab.slot0 + b) * E.pstride], ph = E.PH[off + (tab.slot0 + b) * E.pstride];
-            vs.x = fma(f.x, ps.x, fma(-f.y, ps.y, vs.x));
-            vs.y = fma(f.x, ps.y, fma(f.y, ps.x, vs.y));
-            vh.x = fma(f.x, ph.x, fma(-f.y, ph.y, vh.x));
-            vh.y = fma(f.x, ph.y, fma(f.y, ph.x, vh.y));
+            vs.x = fma(f.x, ps, vs.x);
+            vs.y = fma(f.y, ps, vs.y);
+            vh.x = fma(f.x, hr, fma(-f.y, hi, vh.x));
+            vh.y = fma(f.x, hi, fma(f.y, hr, vh.y));
         }
-        if constexpr (kReal) {
+        if constexpr (kFixed) {
             // one power of two for every type's products of an element
             const int k0 = E.el[row] - 8 - tab.frac, ks = k0 + E.ers[col], kh = k0 + E.erh[col];
             vs = make_double2(scale_exp(vs.x, ks), scale_exp(vs.y, ks));
@@ -199,7 +201,7 @@ cudaError_t launch_sf_combine(const SfTab &tab, const double2 *sf, bool first, c
     if (tiles <= 0) return cudaSuccess;
     if (tiles > 0x7fffffffLL) return cudaErrorInvalidValue;
     const dim3 block(kSfTile, kSfRows);
-    if (t.nk > 0 && t.e[0].RS) sf_combine_kernel<true><<<(unsigned)tiles, block, 0, st>>>(t, sf, first ? 1 : 0);
+    if (t.nk > 0 && t.e[0].el) sf_combine_kernel<true><<<(unsigned)tiles, block, 0, st>>>(t, sf, first ? 1 : 0);
     else sf_combine_kernel<false><<<(unsigned)tiles, block, 0, st>>>(t, sf, first ? 1 : 0);
     return cudaGetLastError();
 }

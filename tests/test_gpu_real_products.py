@@ -44,3 +44,19 @@ def test_real_products_match_oracle(ctx, lmax, n_g, slices):
         for X, R, nm in ((H, Hr, "H"), (S, Sr, "S")):
             fro, mx = oracle.lower_errors(X, R)
             assert fro < tol and mx < tol, (nm, lmax, n_g, slices, fro, mx)
+
+
+@pytest.mark.parametrize("lmax,n_g,types", [(1, 1, 1), (1, 15, 2), (2, 17, 1), (3, 33, 2), (4, 100, 3), (8, 241, 2),
+                                            (10, 47, 1), (5, 801, 4), (7, 1000, 2)])
+def test_fp64_real_products_match_oracle(ctx, lmax, n_g, types):
+    """Plain FP64 on both tile shapes: small launches (16 x 16 tiles, the contraction split over four
+    warps; contraction lengths 8 to 242 are not multiples of its steps) and large ones (32 x 32)."""
+    cfg = dict(cell=(10.0, 10.5, 11.0), atoms=5, types=types, rmt=2.0, min_sep=3.9, lmax=lmax,
+               kpts=[(0.1, 0.2, 0.3)], n_g=n_g, seed=7 + n_g)
+    s = synth.make_system(cfg)
+    ((H, S),), rep = ctx.create_hs(s, precision="fp64")
+    assert rep["num_row_sets"] == types
+    Hr, Sr = oracle.reference_hs(s, s.kpoints[0])
+    for X, R, nm in ((H, Hr, "H"), (S, Sr, "S")):
+        fro, mx = oracle.lower_errors(X, R)
+        assert fro < 1e-13 and mx < 1e-13, (nm, lmax, n_g, fro, mx)
