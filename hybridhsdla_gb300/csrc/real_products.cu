@@ -26,10 +26,12 @@
 //    (x + 1.5 2^23 leaves it in the low mantissa bits), and a band's adds with one multiply-add.
 //    Each output element is written once, rather than once per accumulation unit through L2
 //    reductions.  The fixed-point sum is exact down to 2^-frac of a unit of the top diagonal.
-// What bounds it: the MMA thread's issue and the drains share the time (the tensor pipe is busy 0.7
-// of it).  One type of the 8000-column workload (lmax 10, 11 digits): 3.05 ms in the complex form,
-// 1.13 ms here = 2.7 PFLOP/s of e4m3, 0.71 of twice the measured bf16 rate; sixteen epilogue warps
-// with half the sums each: 1.15 ms.
+// What bounds it: the drains and the MMA thread, each ~0.85 of the time, in turn where a band's MMAs
+// are shorter than the drain before them.  One type of the 8000-column workload (lmax 10, 11 digits):
+// 3.05 ms in the complex form, 1.07 ms here = 2.9 PFLOP/s of e4m3, 0.75 of twice the measured bf16
+// rate (0.91 ms with the drains' arithmetic left out).  Measured and not kept: sixteen epilogue warps
+// with half the sums each (1.07), TMEM loads ahead of the arithmetic (1.07), shifts and adds in place
+// of the wide multiply-adds (1.10), no collector buffer (1.07).
 // Every wait is bounded (ptx.cuh); both CTAs meet at a cluster barrier before TMEM is freed.
 #include <cuda_fp8.h>
 
@@ -249,19 +251,31 @@ __global__ void __launch_bounds__(kThreads, 1)
                             const int slot = (n + (i0 - 1) / kBatch) % kRing;
                             uint32_t da = da0 + slot * kBatch * kAStep;
                             const int i1 = min(i0 + kBatch, T);
-                            for (int i = i0; i < i1; ++i, da += kAStep, dt -= kBStep) {
-                                const uint32_t acc = i > 1 ? 1u : 0u;
-                                if (pairs && i + 1 < T) {
-                                    const uint32_t dl = dt - kBStep;
+                            if (two && pairs && i0 + kBatch < T) {
+                                // a whole batch of pairs as straight-line code (1.102 -> 1.067 ms, as above)
+#pragma unroll
+                                for (int q = 0; q < kBatch; ++q, da += kAStep, dt -= kBStep) {
+                                    const uint32_t acc = i0 + q > 1 ? 1u : 0u, dl = dt - kBStep;
                                     mma_real<1>(d1, da, dl, acc);
                                     mma_real<2>(d2, da, dt, acc);
-                                    if (two) {
-                                        mma_real<1>(d1, da + 2, dl + 2, 1u);
-                                        mma_real<2>(d2, da + 2, dt + 2, 1u);
+                                    mma_real<1>(d1, da + 2, dl + 2, 1u);
+                                    mma_real<2>(d2, da + 2, dt + 2, 1u);
+                                }
+                            } else {
+                                for (int i = i0; i < i1; ++i, da += kAStep, dt -= kBStep) {
+                                    const uint32_t acc = i > 1 ? 1u : 0u;
+                                    if (pairs && i + 1 < T) {
+                                        const uint32_t dl = dt - kBStep;
+                                        mma_real<1>(d1, da, dl, acc);
+                                        mma_real<2>(d2, da, dt, acc);
+                                        if (two) {
+                                            mma_real<1>(d1, da + 2, dl + 2, 1u);
+                                            mma_real<2>(d2, da + 2, dt + 2, 1u);
+                                        }
+                                    } else {
+                                        mma_real<0>(d2, da, dt, acc);
+                                        if (two) mma_real<0>(d2, da + 2, dt + 2, 1u);
                                     }
-                                } else {
-                                    mma_real<0>(d2, da, dt, acc);
-                                    if (two) mma_real<0>(d2, da + 2, dt + 2, 1u);
                                 }
                             }
                             if (last) mma_commit_pair(&bars.aempty[slot]);     // the batch's last use
@@ -512,9 +526,10 @@ RealBands real_bands(int s, int width, int halves, int64_t kvalid) {
     int kb = 0;
     while (((int64_t)1 << kb) <= kvalid) ++kb;
     b.frac = 55 - kb;
-    // a single diagonal comes first: the last band (T = s + 1) is full width
-    int T = 2 + ((s - 1) % width);
-    for (int t = 1; t < s + 1; T += width) {
+    // pairs, a single diagonal last: a band shorter than a drain holds up the band after the next, so
+    // the first is a pair too (one type of the 8000-column workload 1.128 -> 1.102 ms)
+    for (int t = 1, T; t < s + 1; t = T) {
+        T = std::min(t + width, s + 1);
         const int n = b.n++, sh = b.frac - 5 * (T - 2);
         b.T[n] = (int8_t)T;
         b.w[n] = (int8_t)(T - t);
@@ -527,7 +542,6 @@ RealBands real_bands(int s, int width, int halves, int64_t kvalid) {
         b.f[n] = std::ldexp(1.0f, -r);
         const uint32_t m = b.fold[n] == kFoldInt ? 33u * kMagicBits : kMagicBits;   // (far from 2^32's ends)
         b.bias += b.fold[n] == kFoldHigh ? (unsigned long long)(m * b.mul[n]) << 32 : (unsigned long long)m * b.mul[n];
-        t = T;
     }
     return b;
 }
