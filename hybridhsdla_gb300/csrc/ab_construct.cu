@@ -236,10 +236,10 @@ __global__ void __launch_bounds__(kThreads) construct_ab_kernel(DevSystem sys, c
             // phase-free per-type rows M_t = [A_t; B_t] / e^{i 2pi K.tau} (shared by every atom of type t)
             if (ent.R) {
                 double *rcol = ent.R + ldm * gi;
-                const int nrm = twoL * nt;
+                const int nrm = twoL * sys.num_sets;
                 for (int idx = threadIdx.x; idx < nrm; idx += blockDim.x) {
-                    const int t = idx / twoL;
-                    const int r = idx - t * twoL;
+                    const int set = idx / twoL, t = sys.set_type[set];
+                    const int r = idx - set * twoL;
                     const bool isB = r >= L;
                     const int lm = isB ? r - L : r;
                     const int l = l_of[lm];
@@ -316,29 +316,60 @@ __global__ void __launch_bounds__(kThreads) construct_ab_kernel(DevSystem sys, c
     }
 }
 
-// Real per-type rows R only (atoms sharing their type's rotation, no per-atom rows), kRowCols G
-// columns per CTA.  The per-column scalar work -- the Bessel recursions per type and the Y_lm sets, FP64
-// code with data-dependent loops -- runs one column per lane, as work items (column, type) and
-// (column, m), instead of on a few lanes of one warp per column: GB300 issues an FP64 warp
-// instruction in 16 cycles however few of its lanes are active.  The same formulas in the same
-// order as construct_ab_kernel.
-constexpr int kRowCols = 16;
+// Real rows R of the row sets only (no per-atom rows), kRowCols G columns and a share of the
+// rotations (blockIdx.y of gridDim.y) per CTA.  GB300 issues an FP64 warp instruction in 16 cycles
+// however few of its lanes are active, so the FP64 work is spread over lanes and kept small: work
+// items (column, type) run the Bessel recursions, (column, rotation) the directions, (column, m) the
+// Y_lm recursions -- normalised, so that a step is three multiplies and no division -- and a row costs
+// one multiply.  8000 columns, lmax 10, 8 types: 243 us with the unnormalised recursions and a direction
+// for each (column, m), 120 us now; 3001 columns of 4 types in 5 rotations: 255 and 58 us.
+__device__ __forceinline__ void ylm_real_dev(int lmax, int m, double cth, double sth, double cph, double sph,
+                                             const double *leg, double *y) {
+    const int nl = lmax + 1;
+    const double *a = leg + m * nl, *b = a + nl * nl;
+    // e^{i m phi} and sin^m theta by repeated multiplication (Y_lm to 7.8e-16, where the three-term
+    // recursion in m phi gives 1.0e-15, relative over lmax 10)
+    double cm = 1.0, sm = 0.0, p = a[m];
+    for (int k = 0; k < m; ++k) {
+        const double c2 = fma(cm, cph, -(sm * sph));
+        sm = fma(cm, sph, sm * cph);
+        cm = c2;
+        p *= sth;
+    }
+    double p1 = 0.0;
+    for (int l = m; l <= lmax; ++l) {
+        if (l > m) {
+            const double q = a[l] * fma(cth, p, -(b[l] * p1));
+            p1 = p;
+            p = q;
+        }
+        // the row of conj(Y_lm): its real part, and its imaginary part in place of -m
+        y[l * (l + 1) + m] = p * cm;
+        if (m) y[l * (l + 1) - m] = -(p * sm);
+    }
+}
+
 __global__ void __launch_bounds__(kThreads) construct_rows_kernel(DevSystem sys, const __grid_constant__ KTable tab) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int L = sys.L, nl = sys.max_lmax + 1, nt = sys.num_types, twoL = 2 * L, tnl = nt * nl;
-    double2 *ylm = reinterpret_cast<double2 *>(smem_raw);          // [kRowCols][L]
-    double *au = reinterpret_cast<double *>(ylm + kRowCols * L);    // [kRowCols][nt nl]
+    double *ylm = reinterpret_cast<double *>(smem_raw);             // [kRowCols][L]
+    double *au = ylm + kRowCols * L;                                // [kRowCols][nt nl]
     double *bu = au + kRowCols * tnl;                               // [kRowCols][nt nl]
-    double *cf = bu + kRowCols * tnl;                               // [nt nl] 4 pi / sqrt(Omega) / W
+    double *cf = bu + kRowCols * tnl;                               // [nt nl] 4 pi / sqrt(Omega) / W, 0 past a type's lmax
     double *kv = cf + tnl;                                          // [kRowCols][4]: K, |bmat K|
-    unsigned char *l_of = reinterpret_cast<unsigned char *>(kv + 4 * kRowCols);   // [L]
+    double *dir = kv + 4 * kRowCols;                                // [kRowRots][kRowCols][4]: cos, sin theta; cos, sin phi
+    double **rcol = reinterpret_cast<double **>(dir + 4 * kRowCols * kRowRots);   // [kRowCols]
+    unsigned char *l_of = reinterpret_cast<unsigned char *>(rcol + kRowCols);     // [L]
     for (int lm = threadIdx.x; lm < L; lm += blockDim.x) {
-        int l = (int)sqrt((double)lm);
+        int l = (int)sqrtf((float)lm);
         while (l * l > lm) --l;
         while ((l + 1) * (l + 1) <= lm) ++l;
         l_of[lm] = (unsigned char)l;
     }
-    for (int i = threadIdx.x; i < tnl; i += blockDim.x) cf[i] = sys.vol_prefac * sys.inv_w[i];
+    for (int i = threadIdx.x; i < tnl; i += blockDim.x)
+        cf[i] = i % nl <= sys.type_lmax[i / nl] ? sys.vol_prefac * sys.inv_w[i] : 0.0;
+    const int nrot = sys.num_rots > 0 ? sys.num_rots : 1;
+    const int rho0 = (int)((int64_t)nrot * blockIdx.y / gridDim.y), rho1 = (int)((int64_t)nrot * (blockIdx.y + 1) / gridDim.y);
     const int64_t ldm = tab.ldm;
     for (int64_t col0 = blockIdx.x * (int64_t)kRowCols; col0 < tab.total_cols; col0 += (int64_t)gridDim.x * kRowCols) {
         const int ncols = (int)(tab.total_cols - col0 < kRowCols ? tab.total_cols - col0 : kRowCols);
@@ -355,62 +386,67 @@ __global__ void __launch_bounds__(kThreads) construct_rows_kernel(DevSystem sys,
             }
             double *k4 = kv + 4 * threadIdx.x;
             k4[0] = K[0]; k4[1] = K[1]; k4[2] = K[2]; k4[3] = sqrt(s);
+            rcol[threadIdx.x] = ent.R ? ent.R + ldm * (gc - ent.col_begin) : nullptr;
         }
         __syncthreads();
-        // the columns' Bessel values per type, then their Y_lm sets (one warp per kind, mostly);
-        // with (type, rotation) classes the Y_lm sets come once per rotation, each followed by the
-        // rows of the types (classes) that carry it
-        const int nrot = sys.num_rots > 0 ? sys.num_rots : 1;
-        for (int rho = 0; rho < nrot; ++rho) {
+        // the columns' directions in this CTA's first rotations, then their Bessel values per type
+        // (warps of one kind each, mostly)
+        const int nd = ncols * (rho1 - rho0 < kRowRots ? rho1 - rho0 : kRowRots), nb = ncols * nt;
+        auto direction = [&](int w, int base) {
+            const int q = w / ncols, c = w - q * ncols;
             // R^T K with R = mrot bmat of this rotation (tensor_AB_match.cpp:97), bmat without one
-            const double *R = sys.num_rots > 0 ? sys.rots + 9 * rho : sys.bmat;
-            const int nb = rho == 0 ? ncols * nt : 0, ny = ncols * nl;
-            if (rho > 0) __syncthreads();     // the previous rotation's rows have read ylm
-            for (int w = threadIdx.x; w < nb + ny; w += blockDim.x) {
-                if (w < nb) {
-                    const int c = w / nt, t = w - c * nt;
-                    const double kn = kv[4 * c + 3];
-                    double fj[kMaxLmax + 1], dfj[kMaxLmax + 1];
-                    const double x = sys.type_rmt[t] * kn;
-                    sphbes_dev(sys.max_lmax, x, fj);
-                    dsphbs_dev(sys.max_lmax, x, fj, dfj);
-                    for (int l = 0; l < nl; ++l) {
-                        const int tl = t * nl + l;
-                        au[c * tnl + tl] = sys.dE_u[tl] * kn * dfj[l] - sys.dE_u_dr[tl] * fj[l];
-                        bu[c * tnl + tl] = -sys.u[tl] * kn * dfj[l] + sys.u_dr[tl] * fj[l];
-                    }
-                } else {
-                    const int q = w - nb, c = q / nl, m = q - c * nl;
-                    const double *k4 = kv + 4 * c;
-                    double v[3];
-                    for (int d = 0; d < 3; ++d) v[d] = R[d] * k4[0] + R[3 + d] * k4[1] + R[6 + d] * k4[2];
-                    const double nrm = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-                    if (nrm > 0.0) { v[0] /= nrm; v[1] /= nrm; v[2] /= nrm; }
-                    ylm_column_dev(sys.max_lmax, m, v, sys.ynorm, ylm + c * L);
+            const double *R = sys.num_rots > 0 ? sys.rots + 9 * (base + q) : sys.bmat;
+            const double *k4 = kv + 4 * c;
+            double v[3];
+            for (int d = 0; d < 3; ++d) v[d] = R[d] * k4[0] + R[3 + d] * k4[1] + R[6 + d] * k4[2];
+            const double nrm = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+            if (nrm > 0.0) { v[0] /= nrm; v[1] /= nrm; v[2] /= nrm; }
+            // as ylm4.f:45-60
+            const double small = 1.0e-12, xy = v[0] * v[0] + v[1] * v[1];
+            const double r = sqrt(xy + v[2] * v[2]), rxy = sqrt(xy);
+            double *d4 = dir + 4 * (q * kRowCols + c);
+            if (r > small) { d4[0] = v[2] / r; d4[1] = rxy / r; } else { d4[0] = 1.0; d4[1] = 0.0; }
+            if (rxy > small) { d4[2] = v[0] / rxy; d4[3] = v[1] / rxy; } else { d4[2] = 1.0; d4[3] = 0.0; }
+        };
+        for (int w = threadIdx.x; w < nd + nb; w += blockDim.x) {
+            if (w < nd) {
+                direction(w, rho0);
+            } else {
+                const int q = w - nd, c = q / nt, t = q - c * nt;
+                const double kn = kv[4 * c + 3];
+                double fj[kMaxLmax + 1], dfj[kMaxLmax + 1];
+                const double x = sys.type_rmt[t] * kn;
+                sphbes_dev(sys.max_lmax, x, fj);
+                dsphbs_dev(sys.max_lmax, x, fj, dfj);
+                for (int l = 0; l < nl; ++l) {
+                    const int tl = t * nl + l;
+                    au[c * tnl + tl] = (sys.dE_u[tl] * kn * dfj[l] - sys.dE_u_dr[tl] * fj[l]) * cf[tl];
+                    bu[c * tnl + tl] = (-sys.u[tl] * kn * dfj[l] + sys.u_dr[tl] * fj[l]) * cf[tl];
                 }
             }
+        }
+        for (int rho = rho0; rho < rho1; ++rho) {
+            const int q = (rho - rho0) % kRowRots;
+            __syncthreads();                  // directions ready; the previous rotation's rows have read ylm
+            if (q == 0 && rho > rho0) {
+                for (int w = threadIdx.x; w < ncols * min(kRowRots, rho1 - rho); w += blockDim.x) direction(w, rho);
+                __syncthreads();
+            }
+            for (int w = threadIdx.x; w < ncols * nl; w += blockDim.x) {
+                // (m slowest, so that a warp's lanes run recursions of about one length)
+                const int m = w / ncols, c = w - m * ncols;
+                const double *d4 = dir + 4 * (q * kRowCols + c);
+                ylm_real_dev(sys.max_lmax, m, d4[0], d4[1], d4[2], d4[3], sys.legendre, ylm + c * L);
+            }
             __syncthreads();
-            // the rows [A_t; B_t] / e^{i 2pi K.tau} of each column (types with this rotation)
-            for (int c = 0; c < ncols; ++c) {
-                const int64_t gc = col0 + c;
-                const KEntry &ent = tab.e[entry_of(tab, gc)];
-                if (!ent.R) continue;
-                // Re of the rows m >= 0, Im of the rows m > 0 in place of -m
-                double *rcol = ent.R + ldm * (gc - ent.col_begin);
-                for (int idx = threadIdx.x; idx < twoL * nt; idx += blockDim.x) {
-                    const int t = idx / twoL;
-                    if (sys.num_rots > 0 && sys.type_rot[t] != rho) continue;
-                    const int r = idx - t * twoL;
-                    const bool isB = r >= L;
-                    const int lm = isB ? r - L : r;
-                    const int l = l_of[lm];
-                    double out = 0.0;
-                    if (l <= sys.type_lmax[t]) {
-                        const int tl = t * nl + l, l0 = l * (l + 1);
-                        const double y = lm >= l0 ? ylm[c * L + lm].x : -ylm[c * L + 2 * l0 - lm].y;
-                        out = (y * cf[tl]) * (isB ? bu[c * tnl + tl] : au[c * tnl + tl]);
-                    }
-                    rcol[idx] = out;
+            // the rows [A; B] / e^{i 2pi K.tau} of the rotation's sets, every column
+            const int q0 = sys.num_rots > 0 ? sys.rot_begin[rho] : 0, q1 = sys.num_rots > 0 ? sys.rot_begin[rho + 1] : sys.num_sets;
+            for (int set = q0; set < q1; ++set) {
+                const int t = sys.set_type[set];
+                const double *a = au + t * nl, *b = bu + t * nl;
+                for (int w = threadIdx.x; w < ncols * twoL; w += blockDim.x) {
+                    const int c = w / twoL, r = w - c * twoL, lm = r >= L ? r - L : r;
+                    if (rcol[c]) rcol[c][(int64_t)set * twoL + r] = ylm[c * L + lm] * (r >= L ? b : a)[c * tnl + l_of[lm]];
                 }
             }
         }
@@ -652,8 +688,10 @@ cudaError_t launch_construct_ab_multi(const DevSystem &sys, const KTable &tab, c
         const size_t smem = smem_rows;
         cudaError_t e = cudaFuncSetAttribute(construct_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        const int64_t grid = std::min<int64_t>((tab.total_cols + kRowCols - 1) / kRowCols, (int64_t)sm_count() * 4);
-        construct_rows_kernel<<<(unsigned)grid, kThreads, smem, st>>>(sys, tab);
+        // a few CTAs per SM: over the columns, and over the rotations where the columns give too few
+        const int64_t want = (int64_t)sm_count() * 4, nx = std::min<int64_t>((tab.total_cols + kRowCols - 1) / kRowCols, want);
+        const int64_t ny = std::min<int64_t>(std::max(sys.num_rots, 1), std::max<int64_t>(1, want / nx));
+        construct_rows_kernel<<<dim3((unsigned)nx, (unsigned)ny), kThreads, smem, st>>>(sys, tab);
         return cudaGetLastError();
     }
     const int nl = sys.max_lmax + 1;

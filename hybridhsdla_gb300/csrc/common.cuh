@@ -11,6 +11,7 @@ namespace hsdla {
 constexpr int kMaxLmax = 14;                 // (14+1)^2 = 225 lm per atom
 constexpr int kMaxL = (kMaxLmax + 1) * (kMaxLmax + 1);
 constexpr int kMaxTypes = 64;
+constexpr int kMaxSets = 4096;               // row sets of the structure-factor form
 constexpr double kPi = 3.14159265358979323846;
 
 // Device error word: kernels with bounded waits write a code here instead of trapping.
@@ -35,19 +36,27 @@ struct DevSystem {
     const double *u, *u_dr, *dE_u, *dE_u_dr;
     const double *inv_w;        // 1 / (udot u' - u udot')
     const double *ynorm;        // [L] Y_lm normalisation (ylm4.f:111-137)
-    // Per-type rows of (type, rotation) classes: the types are the classes, type t's atoms share
-    // the rotation rots[9 type_rot[t] ..] (row-major mrot bmat).  num_rots = 0: every type's rows
-    // use R = bmat (no atom carries its own rotation).
-    int num_rots;
+    // The row sets of the structure-factor form: the types, or (type, rotation) classes, whose atoms
+    // share the rotation.  Set q is of type set_type[q]; the sets of rotation rho (row-major mrot bmat
+    // at rots[9 rho]) are [rot_begin[rho], rot_begin[rho + 1]).  num_rots = 0: every set's rows use
+    // R = bmat (no atom carries its own rotation).
+    int num_sets, num_rots;
+    const int32_t *set_type;    // [num_sets]
     const double *rots;         // [num_rots][9]
-    const int32_t *type_rot;    // [t]
+    const int32_t *rot_begin;   // [num_rots + 1]
+    // normalised Legendre recursion, [2][max_lmax + 1 (m)][max_lmax + 1 (l)]: P_l^m = a_lm (cos P_{l-1}^m -
+    // b_lm P_{l-2}^m), with a_mm the factor of sin^m in P_m^m
+    const double *legendre;
 };
 
-// Shared memory of the per-type rows kernel (construct_rows_kernel) for L lm, lmax max_lmax and
-// nt types; the kernel runs only where it fits (160 KB).
+// Shared memory of the rows kernel (construct_rows_kernel) for L lm, lmax max_lmax and nt types; the
+// kernel runs only where it fits (160 KB).
+constexpr int kRowCols = 16;    // G columns of a CTA
+constexpr int kRowRots = 16;    // rotations of a CTA at most
 inline size_t rows_kernel_smem(int L, int max_lmax, int nt) {
-    const int kRowCols = 16, nl = max_lmax + 1, tnl = nt * nl;
-    size_t b = sizeof(double) * 2 * kRowCols * L + sizeof(double) * (2 * kRowCols * tnl + tnl + 4 * kRowCols) + L + 16;
+    const int nl = max_lmax + 1, tnl = nt * nl;
+    size_t b = sizeof(double) * (kRowCols * L + 2 * kRowCols * tnl + tnl + 4 * kRowCols + 4 * kRowCols * kRowRots) +
+               sizeof(double *) * kRowCols + L + 16;
     return (b + 15) & ~size_t(15);
 }
 constexpr size_t kRowsKernelSmemMax = 160 * 1024;

@@ -77,7 +77,9 @@ struct PlanKpoint {
 struct hsdla_plan {
     hsdla_context *ctx = nullptr;
     hsdla_opts opts{};
-    int L = 0, na = 0, nt = 0, max_lmax = 0;
+    int L = 0, na = 0, nt = 0, max_lmax = 0;    // nt: row sets (types, or (type, rotation) classes)
+    int ntypes = 0;                  // types of the T blocks
+    std::vector<int32_t> set_type;   // type of each row set
     int64_t twoLa = 0;
     DevSystem dsys{};
     std::vector<PlanKpoint> kps;
@@ -137,7 +139,6 @@ struct hsdla_plan {
     // statistics land in the context's page-locked staging, checked once the stream is idle
     bool tcheck_pending = false;
     const unsigned long long *tcheck_host = nullptr;
-    std::vector<int32_t> tcheck_class_type;
     double *wt = nullptr;            // (of the real rows: doubled where m != 0)
     double *TR = nullptr;            // real T blocks [nt][4L][2L]
     double2 *sf_tab = nullptr;
@@ -327,6 +328,24 @@ std::vector<double> ylm_norms(int lmax) {
     return yn;
 }
 
+// Coefficients of the normalised Legendre recursion (DevSystem::legendre): with the Condon-Shortley
+// phase and the Y_lm norm sqrt((2l+1)/(4 pi) (l-m)!/(l+m)!) in P_l^m.
+std::vector<double> legendre_table(int lmax) {
+    const int nl = lmax + 1;
+    std::vector<double> t(2 * (size_t)nl * nl, 0.0);
+    double d = std::sqrt(1.0 / (4.0 * 3.1415926535897932));
+    for (int m = 0; m <= lmax; ++m) {
+        if (m > 0) d *= -std::sqrt((2.0 * m + 1.0) / (2.0 * m));
+        t[(size_t)m * nl + m] = d;
+        for (int l = m + 1; l <= lmax; ++l) {
+            const double l2 = (double)l * l, m2 = (double)m * m, k2 = (l - 1.0) * (l - 1.0);
+            t[(size_t)m * nl + l] = std::sqrt((4.0 * l2 - 1.0) / (l2 - m2));
+            t[(size_t)(nl + m) * nl + l] = std::sqrt((k2 - m2) / (4.0 * k2 - 1.0));
+        }
+    }
+    return t;
+}
+
 int validate(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoint *kpts, int nk) {
     if (!s) return set_err(ctx, HSDLA_ERR_ARG, "system is NULL");
     if (s->num_atoms < 1 || s->num_types < 1 || s->num_types > kMaxTypes)
@@ -379,89 +398,63 @@ int validate(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoint *kpts
 // (FleurData.cpp:52-62, 453-455) and builds its rows with it (tensor_AB_match.cpp:97) while its
 // type supplies the radial data and T blocks.  Atoms of one type whose rotations are equal have
 // the same rows up to their structure phase, so the structure-factor form runs per class instead
-// of per type: a derived system whose types are the classes (each with its type's tables) and
-// whose rows carry the class's rotation.
-struct ClassSystem {
-    hsdla_system sys{};
-    int n = 0;                            // classes
-    std::vector<int32_t> atom_class, class_type, class_rot, lmax;
-    std::vector<double> rots, rmt, u, u_dr, dE_u, dE_u_dr, dE_u_norm;
-    std::vector<hsdla_cx> taa, tab, tbb;
+// of per type; each class's rows carry its rotation.
+struct RowSets {
+    int n = 0;                                  // sets, numbered by rotation
+    std::vector<int32_t> atom_set, set_type;
+    std::vector<int32_t> rot_begin;             // sets of each rotation
+    std::vector<double> rots;
 };
 
-// Builds the class system when it shrinks the work: the classes' rows (2L per class) are few
-// enough against the per-atom rows (2L per atom) to pay for the structure-factor combine, and
-// their table fits the per-type rows kernel.  Returns false otherwise (per-atom form).
-bool make_classes(const hsdla_system *s, ClassSystem &cs) {
+// Builds the classes when they shrink the work: their rows (2L per class) are few enough against
+// the per-atom rows (2L per atom) to pay for the structure-factor combine, and the types' tables
+// fit the rows kernel.  Returns false otherwise (per-atom form).
+bool make_classes(const hsdla_system *s, RowSets &rs) {
     if (!s->atom_rotmat) return false;
-    const int na = s->num_atoms, nt = s->num_types, nl = s->max_lmax + 1, L = nl * nl;
+    const int na = s->num_atoms, nl = s->max_lmax + 1;
     std::map<std::vector<uint64_t>, int> rot_id;
-    std::map<std::pair<int, int>, int> cls;
-    cs.atom_class.resize(na);
+    std::map<std::pair<int, int>, int> cls;     // (rotation, type)
+    std::vector<std::pair<int, int>> of(na);
     for (int j = 0; j < na; ++j) {
         std::vector<uint64_t> bits(9);
         memcpy(bits.data(), s->atom_rotmat + 9 * (size_t)j, 9 * sizeof(double));
         auto r = rot_id.find(bits);
         if (r == rot_id.end()) {
             r = rot_id.emplace(bits, (int)rot_id.size()).first;
-            cs.rots.insert(cs.rots.end(), s->atom_rotmat + 9 * (size_t)j, s->atom_rotmat + 9 * (size_t)j + 9);
+            rs.rots.insert(rs.rots.end(), s->atom_rotmat + 9 * (size_t)j, s->atom_rotmat + 9 * (size_t)j + 9);
         }
-        const auto key = std::make_pair((int)s->atom_type[j], r->second);
-        auto c = cls.find(key);
-        if (c == cls.end()) {
-            c = cls.emplace(key, (int)cls.size()).first;
-            cs.class_type.push_back(key.first);
-            cs.class_rot.push_back(key.second);
-        }
-        cs.atom_class[j] = c->second;
+        of[j] = std::make_pair(r->second, (int)s->atom_type[j]);
+        cls.emplace(of[j], 0);
     }
-    cs.n = (int)cls.size();
-    if (4 * cs.n > 3 * na || cs.n > kMaxTypes || rows_kernel_smem(L, s->max_lmax, cs.n) > kRowsKernelSmemMax)
+    rs.n = (int)cls.size();
+    if (4 * rs.n > 3 * na || rs.n > kMaxSets || rows_kernel_smem(nl * nl, s->max_lmax, s->num_types) > kRowsKernelSmemMax)
         return false;
-    const int n = cs.n;
-    cs.rmt.resize(n); cs.lmax.resize(n);
-    for (auto *v : {&cs.u, &cs.u_dr, &cs.dE_u, &cs.dE_u_dr, &cs.dE_u_norm}) v->resize((size_t)n * nl);
-    for (auto *v : {&cs.taa, &cs.tab, &cs.tbb}) v->resize((size_t)n * L * L);
-    for (int c = 0; c < n; ++c) {
-        const int t = cs.class_type[c];
-        cs.rmt[c] = s->type_rmt[t];
-        cs.lmax[c] = s->type_lmax[t];
-        const double *src[5] = {s->type_u, s->type_u_dr, s->type_dE_u, s->type_dE_u_dr, s->type_dE_u_norm};
-        std::vector<double> *dst[5] = {&cs.u, &cs.u_dr, &cs.dE_u, &cs.dE_u_dr, &cs.dE_u_norm};
-        for (int q = 0; q < 5; ++q) memcpy(dst[q]->data() + (size_t)c * nl, src[q] + (size_t)t * nl, nl * sizeof(double));
-        const hsdla_cx *tsrc[3] = {s->type_t_aa, s->type_t_ab, s->type_t_bb};
-        std::vector<hsdla_cx> *tdst[3] = {&cs.taa, &cs.tab, &cs.tbb};
-        for (int q = 0; q < 3; ++q)
-            memcpy(tdst[q]->data() + (size_t)c * L * L, tsrc[q] + (size_t)t * L * L, (size_t)L * L * sizeof(hsdla_cx));
+    int q = 0;
+    rs.rot_begin.assign(rot_id.size() + 1, 0);
+    for (auto &c : cls) {
+        c.second = q++;
+        rs.set_type.push_back(c.first.second);
+        rs.rot_begin[c.first.first + 1] = q;
     }
-    hsdla_system &d = cs.sys;
-    d = *s;
-    d.num_types = n;
-    d.atom_type = cs.atom_class.data();
-    d.type_rmt = cs.rmt.data();
-    d.type_lmax = cs.lmax.data();
-    d.type_u = cs.u.data(); d.type_u_dr = cs.u_dr.data(); d.type_dE_u = cs.dE_u.data();
-    d.type_dE_u_dr = cs.dE_u_dr.data(); d.type_dE_u_norm = cs.dE_u_norm.data();
-    d.type_t_aa = cs.taa.data(); d.type_t_ab = cs.tab.data(); d.type_t_bb = cs.tbb.data();
+    rs.atom_set.resize(na);
+    for (int j = 0; j < na; ++j) rs.atom_set[j] = cls[of[j]];
     return true;
 }
 
 // The T blocks' checks, made on the device while they were assembled (launch_tfull): finite
 // values, and T_AA and T_BB Hermitian (AtomData.cpp:138-139 asserts it), |T - T^H|^2 against
 // |T|^2 over the lower triangle (its mirror element is the pair's other half).
-int check_tmats(hsdla_context *ctx, const std::vector<unsigned long long> &st, int nt,
-                const std::vector<int32_t> *class_type = nullptr) {
+int check_tmats(hsdla_context *ctx, const std::vector<unsigned long long> &st, int nt) {
     auto as_double = [](unsigned long long b) { double d; memcpy(&d, &b, sizeof(d)); return d; };
     for (int t = 0; t < nt; ++t) {
-        const int ty = class_type ? (*class_type)[t] : t;    // the caller's type of a class
         const unsigned long long fl = st[5 * (size_t)t];
         for (int q = 0; q < 3; ++q)
-            if (fl & (1ull << q)) return set_err(ctx, HSDLA_ERR_INPUT, "T block %d of type %d not finite", q, ty);
+            if (fl & (1ull << q)) return set_err(ctx, HSDLA_ERR_INPUT, "T block %d of type %d not finite", q, t);
         for (int q = 0; q < 2; ++q) {
             const double mx2 = as_double(st[5 * (size_t)t + 1 + 2 * q]), dev2 = as_double(st[5 * (size_t)t + 2 + 2 * q]);
             if (dev2 > 1e-24 * std::max(mx2, 1e-300))
                 return set_err(ctx, HSDLA_ERR_INPUT, "T_%s of type %d is not Hermitian (|T-T^H| = %.3g)",
-                               q == 0 ? "AA" : "BB", ty, std::sqrt(dev2));
+                               q == 0 ? "AA" : "BB", t, std::sqrt(dev2));
         }
     }
     return HSDLA_OK;
@@ -543,7 +536,7 @@ int autotune_slices(hsdla_plan *pl, double2 *C, cudaStream_t st) {
     int rc = ozaki_plan_init(probe, kProbe, pl->opts.target_rel_err);
     if (rc) return set_err(ctx, rc, "autotune: %s", ozaki_last_error());
     const int64_t bytes_sample = 2 * K * ns * (int64_t)sizeof(double2) + 4 * ns * ns * (int64_t)sizeof(double2);
-    const int64_t bytes_oz = ozaki_pipeline_workspace(kProbe, twoL, pl->na, pl->nt, ns) + 1024;
+    const int64_t bytes_oz = ozaki_pipeline_workspace(kProbe, twoL, pl->na, pl->ntypes, ns) + 1024;
     void *buf = nullptr;
     rc = ctx_malloc(ctx, &buf, bytes_sample + bytes_oz);
     if (rc) { ozaki_plan_release(probe); return rc; }
@@ -586,7 +579,7 @@ int autotune_slices(hsdla_plan *pl, double2 *C, cudaStream_t st) {
     // Ozaki at the probe slice count (overwrites Xs after the FP64 H job, in stream order)
     OzakiInputs in;
     in.C = Cs; in.Tfull = pl->Tfull; in.w = pl->w; in.atom_type = pl->atom_type.data(); in.X = Xs;
-    in.twoL = twoL; in.na = pl->na; in.nt = pl->nt; in.G = ns;
+    in.twoL = twoL; in.na = pl->na; in.nt = pl->ntypes; in.G = ns;
     int nl = 0;
     rc = ozaki_pipeline(probe, in, So, Ho, ns, wz, st, &nl);
     if (rc) return fail(rc, ozaki_last_error());
@@ -754,13 +747,18 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     // atoms with rotations: (type, rotation) classes keep the structure-factor form where they
     // shrink the work (HSDLA_SF=0 or HSDLA_CLASSES=0 keeps the per-atom form)
     const char *sf_env0 = getenv("HSDLA_SF");
-    ClassSystem cls;
+    RowSets sets;
     const bool use_classes = s->atom_rotmat && !(sf_env0 && strtol(sf_env0, nullptr, 10) == 0) &&
-                             env_flag("HSDLA_CLASSES", true) && make_classes(s, cls);
-    if (use_classes) s = &cls.sys;
+                             env_flag("HSDLA_CLASSES", true) && make_classes(s, sets);
+    if (!use_classes) {      // the types, no rotations
+        sets = RowSets();
+        sets.n = s->num_types;
+        sets.atom_set.assign(s->atom_type, s->atom_type + s->num_atoms);
+        for (int t = 0; t < sets.n; ++t) sets.set_type.push_back(t);
+    }
     auto *pl = new hsdla_plan();
     pl->ctx = ctx;
-    pl->classes = use_classes ? cls.n : 0;
+    pl->classes = use_classes ? sets.n : 0;
     if (opts) pl->opts = *opts;
     if (pl->opts.precision != HSDLA_PREC_FP64 && pl->opts.precision != HSDLA_PREC_OZAKI_FP8) {
         delete pl;
@@ -768,7 +766,9 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     }
     if (pl->opts.target_rel_err <= 0.0) pl->opts.target_rel_err = 1e-13;
     const int na = s->num_atoms, nt = s->num_types, nl = s->max_lmax + 1, L = nl * nl;
-    pl->L = L; pl->na = na; pl->nt = nt; pl->max_lmax = s->max_lmax;
+    const int ns = sets.n;
+    pl->L = L; pl->na = na; pl->nt = ns; pl->ntypes = nt; pl->max_lmax = s->max_lmax;
+    pl->set_type = sets.set_type;
     pl->hoist = s->atom_rotmat == nullptr || use_classes;
     pl->twoLa = 2 * (int64_t)L * na;
     pl->atom_type.assign(s->atom_type, s->atom_type + na);
@@ -799,7 +799,9 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     int64_t bytes = 0;
     auto add = [&](int64_t b) { bytes += (b + 255) & ~int64_t(255); };
     add(sizeof(int32_t) * na); add(sizeof(double) * 3 * na); add(s->atom_rotmat ? sizeof(double) * 9 * na : 0);
-    add(use_classes ? sizeof(double) * cls.rots.size() : 0); add(use_classes ? sizeof(int32_t) * nt : 0);
+    add(sizeof(int32_t) * ns);
+    add(sizeof(double) * sets.rots.size()); add(sizeof(int32_t) * sets.rot_begin.size());
+    add(sizeof(double) * 2 * nl * nl);
     add(sizeof(double) * nt); add(sizeof(int32_t) * nt);
     for (int q = 0; q < 5; ++q) add(sizeof(double) * nt * nl);
     add(sizeof(double) * L);
@@ -816,8 +818,8 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
             for (int64_t q = 0; q < kpts[i].n_g; ++q)
                 for (int c = 0; c < 3; ++c) half[c] = std::max(half[c], 2 * std::abs(kpts[i].g[3 * q + c]));
         for (int c = 0; c < 3; ++c) ext[c] = 2 * half[c] + 1;
-        add(sizeof(double) * 2 * L * nt);
-        add(sizeof(int32_t) * (na + nt + 1));
+        add(sizeof(double) * 2 * L * ns);
+        add(sizeof(int32_t) * (na + ns + 1));
     }
     const int64_t upload_bytes = bytes;
     // filled on the device: the assembled T blocks and their checks; the structure-factor form's
@@ -826,7 +828,7 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     add(sizeof(unsigned long long) * 5 * nt);
     if (pl->sf) {
         add(sizeof(double2) * (int64_t)na * (ext[0] + ext[1] + ext[2]));
-        add(sizeof(double2) * (int64_t)nt * ext[0] * ext[1] * ext[2]);
+        add(sizeof(double2) * (int64_t)ns * ext[0] * ext[1] * ext[2]);
     }
     if (pl->sf) add(sizeof(double) * 2 * tf_elems);
     const double p_tables = pms();
@@ -869,11 +871,15 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     D.atom_type = (const int32_t *)put(s->atom_type, sizeof(int32_t) * na);
     D.atom_pos = (const double *)put(s->atom_pos, sizeof(double) * 3 * na);
     D.atom_rotmat = s->atom_rotmat ? (const double *)put(s->atom_rotmat, sizeof(double) * 9 * na) : nullptr;
+    D.num_sets = ns;
+    D.set_type = (const int32_t *)put(sets.set_type.data(), sizeof(int32_t) * ns);
     if (use_classes) {
-        D.num_rots = (int)(cls.rots.size() / 9);
-        D.rots = (const double *)put(cls.rots.data(), sizeof(double) * cls.rots.size());
-        D.type_rot = (const int32_t *)put(cls.class_rot.data(), sizeof(int32_t) * nt);
+        D.num_rots = (int)(sets.rots.size() / 9);
+        D.rots = (const double *)put(sets.rots.data(), sizeof(double) * sets.rots.size());
+        D.rot_begin = (const int32_t *)put(sets.rot_begin.data(), sizeof(int32_t) * sets.rot_begin.size());
     }
+    const std::vector<double> leg = legendre_table(s->max_lmax);
+    D.legendre = (const double *)put(leg.data(), sizeof(double) * leg.size());
     D.type_rmt = (const double *)put(s->type_rmt, sizeof(double) * nt);
     D.type_lmax = (const int32_t *)put(s->type_lmax, sizeof(int32_t) * nt);
     D.u = (const double *)put(s->type_u, sizeof(double) * nt * nl);
@@ -900,24 +906,24 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     double2 *d_ex = nullptr;
     const int32_t *d_order = nullptr;
     if (pl->sf) {
-        std::vector<double> wt((size_t)2 * L * nt);
-        for (int t = 0; t < nt; ++t)
+        std::vector<double> wt((size_t)2 * L * ns);
+        for (int q = 0; q < ns; ++q)
             for (int l = 0; l < nl; ++l)
                 for (int lm = l * l; lm < (l + 1) * (l + 1); ++lm) {
+                    const int t = sets.set_type[q];
                     // the rows (l, m) and (l, -m) of a real pair carry both complex rows' weight
                     const double pair = lm == l * (l + 1) ? 1.0 : 2.0;
-                    wt[(size_t)2 * L * t + lm] = pair;
-                    wt[(size_t)2 * L * t + L + lm] = (l <= s->type_lmax[t]) ? pair * s->type_dE_u_norm[t * nl + l] : 0.0;
+                    wt[(size_t)2 * L * q + lm] = pair;
+                    wt[(size_t)2 * L * q + L + lm] = (l <= s->type_lmax[t]) ? pair * s->type_dE_u_norm[t * nl + l] : 0.0;
                 }
         pl->wt = (double *)put(wt.data(), sizeof(double) * wt.size());
-        std::vector<int32_t> ord;
-        std::vector<int32_t> tb(nt + 1, 0);
-        for (int t = 0; t < nt; ++t) {
-            tb[t] = (int32_t)ord.size();
-            for (int j = 0; j < na; ++j)
-                if (s->atom_type[j] == t) ord.push_back(j);
-        }
-        tb[nt] = (int32_t)ord.size();
+        // the atoms set by set
+        std::vector<int32_t> ord, tb(ns + 1, 0);
+        for (int j = 0; j < na; ++j) ++tb[sets.atom_set[j] + 1];
+        for (int q = 0; q < ns; ++q) tb[q + 1] += tb[q];
+        ord.resize(na);
+        std::vector<int32_t> at(tb.begin(), tb.end() - 1);
+        for (int j = 0; j < na; ++j) ord[at[sets.atom_set[j]]++] = j;
         ord.insert(ord.end(), tb.begin(), tb.end());
         d_order = (const int32_t *)put(ord.data(), sizeof(int32_t) * ord.size());
         SfTab &dm = pl->sf_dims;
@@ -935,7 +941,7 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     unsigned long long *d_stats = (unsigned long long *)dev_only(sizeof(unsigned long long) * 5 * nt);
     if (pl->sf) {
         d_ex = (double2 *)dev_only(sizeof(double2) * (int64_t)na * (ext[0] + ext[1] + ext[2]));
-        pl->sf_tab = (double2 *)dev_only(sizeof(double2) * (int64_t)nt * ext[0] * ext[1] * ext[2]);
+        pl->sf_tab = (double2 *)dev_only(sizeof(double2) * (int64_t)ns * ext[0] * ext[1] * ext[2]);
     }
     if (pl->sf) pl->TR = (double *)dev_only(sizeof(double) * 2 * tf_elems);
     std::vector<unsigned long long> tstats((size_t)5 * nt, 0);
@@ -976,7 +982,7 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     if (e == cudaSuccess && pl->sf) e = launch_sf_phases(D.atom_pos, na, half, ext, d_ex, ctx->stream);
     if (e == cudaSuccess && pl->sf)
         e = launch_sf_table(d_ex, d_ex + (size_t)na * ext[0], d_ex + (size_t)na * (ext[0] + ext[1]), d_order,
-                            d_order + na, nt, ext[0], ext[1], ext[2], pl->sf_tab, ctx->stream);
+                            d_order + na, ns, ext[0], ext[1], ext[2], pl->sf_tab, ctx->stream);
     const bool defer = defer_tcheck && ctx->staging != nullptr;
     unsigned long long *stats_host =
         defer ? reinterpret_cast<unsigned long long *>(reinterpret_cast<char *>(ctx->staging) + stats_off) : tstats.data();
@@ -998,9 +1004,8 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     if (defer) {
         pl->tcheck_pending = true;
         pl->tcheck_host = stats_host;
-        if (use_classes) pl->tcheck_class_type = cls.class_type;
     } else {
-        rc = check_tmats(ctx, tstats, nt, use_classes ? &cls.class_type : nullptr);
+        rc = check_tmats(ctx, tstats, nt);
         if (rc) { hsdla_plan_destroy(pl); return rc; }
     }
     if (pl->opts.precision == HSDLA_PREC_OZAKI_FP8) {
@@ -1046,7 +1051,8 @@ int64_t group_persist_bytes(const hsdla_plan *pl, const std::vector<int> &kidx) 
     std::vector<int64_t> G;
     for (int i : kidx) G.push_back(pl->kps[i].n_g);
     if (pl->opts.precision == HSDLA_PREC_OZAKI_FP8)
-        return ozaki_group_persist_bytes(pl->oz.num_slices, 2 * (int64_t)pl->L, pl->na, pl->nt, G, pl->panels, pl->sf);
+        return ozaki_group_persist_bytes(pl->oz.num_slices, 2 * (int64_t)pl->L, pl->na, pl->nt, G, pl->panels, pl->sf,
+                                         pl->ntypes);
     // the FP64 group keeps two job tables, each rounded up to 1 KiB: the T applications (one per
     // type when hoisted, else one per atom, per k-point) and the S/H products (three per type in
     // the structure-factor form, else two, per k-point)
@@ -1231,6 +1237,7 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
         if (pl->opts.precision == HSDLA_PREC_OZAKI_FP8) {
             OzGroupDesc d;
             d.twoL = twoL; d.na = pl->na; d.nt = pl->nt; d.hoist = pl->hoist;
+            d.ntypes = pl->ntypes; d.set_type = pl->set_type.data(); d.d_set_type = pl->dsys.set_type;
             d.w = pl->w; d.Tfull = pl->Tfull; d.atom_type = pl->atom_type.data();
             d.panels = pl->panels;
             d.sf = pl->sf; d.wt = pl->wt; d.TR = pl->TR; d.sf_tab = pl->sf_tab; d.tbatch = pl->tbatch;
@@ -1250,7 +1257,7 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
                 for (int q = 0; q < kt.nk; ++q)
                     for (int t = 0; t < pl->nt; ++t) {
                         Fp64RealJob jb{};
-                        jb.P = pl->TR + 2 * twoL * twoL * t; jb.ldp = twoL;
+                        jb.P = pl->TR + 2 * twoL * twoL * pl->set_type[t]; jb.ldp = twoL;
                         jb.Q = kb[q].R + twoL * t; jb.ldq = ldm;
                         jb.out = reinterpret_cast<double *>(kb[q].ZR) + 2 * twoL * t; jb.ldo = 2 * ldm;
                         jb.m = 2 * twoL; jb.n = kb[q].G; jb.k = twoL;
@@ -1865,7 +1872,7 @@ int hsdla_contract_ab(hsdla_context *ctx, int32_t L, int32_t a, int64_t G, const
         return set_err(ctx, HSDLA_ERR_ARG, "unknown precision %d", pl->opts.precision);
     }
     if (pl->opts.target_rel_err <= 0.0) pl->opts.target_rel_err = 1e-13;
-    pl->L = L; pl->na = a; pl->nt = a; pl->max_lmax = max_lmax;
+    pl->L = L; pl->na = a; pl->nt = a; pl->ntypes = a; pl->max_lmax = max_lmax;
     pl->hoist = false;
     pl->external = true;
     pl->twoLa = twoL * a;
@@ -2053,9 +2060,9 @@ int hsdla_create_hs(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoin
     if (rc == HSDLA_OK && es != cudaSuccess) rc = set_err(ctx, HSDLA_ERR_CUDA, "sync failed: %s", cudaGetErrorString(es));
     if (pl->tcheck_pending && (rc == HSDLA_OK || es == cudaSuccess)) {
         // the T blocks' check, deferred past the launches (their statistics are on the host now)
-        const int nt = pl->nt;
+        const int nt = pl->ntypes;
         const std::vector<unsigned long long> st(pl->tcheck_host, pl->tcheck_host + 5 * (size_t)nt);
-        const int rct = check_tmats(ctx, st, nt, pl->tcheck_class_type.empty() ? nullptr : &pl->tcheck_class_type);
+        const int rct = check_tmats(ctx, st, nt);
         if (rct) rc = rct;
     }
     if (rc == HSDLA_OK && rep) {

@@ -1661,7 +1661,7 @@ int64_t ozaki_group_bytes(int s, int64_t twoL, int64_t na, int64_t nt, const std
 }
 
 int64_t ozaki_group_persist_bytes(int s, int64_t twoL, int64_t na, int64_t nt, const std::vector<int64_t> &G,
-                                  int panels, bool sf) {
+                                  int panels, bool sf, int64_t ntypes) {
     const int64_t bpad = round_up(atom_stride(twoL), kKBlock);    // T operand: one atom's rows per plane row
     const int64_t nk = (int64_t)G.size();
     if (sf) {
@@ -1671,7 +1671,7 @@ int64_t ozaki_group_persist_bytes(int s, int64_t twoL, int64_t na, int64_t nt, c
             tiles_t += nt * ((2 * twoL + kRealTileM - 1) / kRealTileM) * tn;
             tiles_sh += 3 * nt * tm * tn;                // (more than the lower triangle's)
         }
-        return operand_bytes(s, 2 * nt * twoL, bpad, s) + round_up(sizeof(RealJob) * nk * nt, 1024) +
+        return operand_bytes(s, 2 * ntypes * twoL, bpad, s) + round_up(sizeof(RealJob) * nk * nt, 1024) +
                round_up(sizeof(RealJob) * 3 * nk * nt, 1024) + round_up(sizeof(int4) * (tiles_t + 1), 1024) +
                2 * round_up(sizeof(int4) * (tiles_sh + 1), 1024) + 8192;
     }
@@ -1795,7 +1795,7 @@ static int group_prepare_sf(OzakiPlan &oz, const OzGroupDesc &d, const std::vect
     carve_rows(g->dM, s);        // R
     carve_rows(g->dW, s);        // R diag(w_t)
     carve_rows(g->dX, 2 * s);    // Z'
-    carve_operand(keep, g->dT, s, 2 * d.nt * d.twoL, round_up(g->bpad, kKBlock), s);
+    carve_operand(keep, g->dT, s, 2 * d.ntypes * d.twoL, round_up(g->bpad, kKBlock), s);
     const int64_t nk = g->nk;
     auto fail = [&](int code) { ozaki_group_destroy(g); return code; };
     auto table = [&](const DigitOperand &o, int parts) {
@@ -1816,12 +1816,13 @@ static int group_prepare_sf(OzakiPlan &oz, const OzGroupDesc &d, const std::vect
     g->rX = table(g->dX, 2);
     g->rX.frac = g->bands_t.frac;         // Z' in fixed point, with T's row and R's column exponents
     g->rX.el = g->dT.expo;
+    g->rX.set_type = d.d_set_type;
     g->rX.er = g->dM.expo;
     g->panels = 1;
     RealSliceTab tT;
     tT.nk = 1; tT.s = s; tT.ldz = d.twoL; tT.blocks = 1; tT.rpb = d.twoL; tT.bstride = d.twoL; tT.bpad = g->bpad;
     tT.digits = g->dT.digits; tT.plane_rows = g->dT.plane_rows; tT.pitch = g->dT.pitch; tT.expo = g->dT.expo;
-    tT.e[0] = RealSliceEntry{d.TR, 2 * d.nt * d.twoL, 0};
+    tT.e[0] = RealSliceEntry{d.TR, 2 * d.ntypes * d.twoL, 0};
     cudaError_t e = launch_real_slice(tT, st);    // stream-ordered before every use of the T digits
     if (e != cudaSuccess) { g_oz_err = cudaGetErrorString(e); return fail(HSDLA_ERR_CUDA); }
     // left operands in boxes of a CTA's 128 rows, right operands of its 64 rows
@@ -1839,7 +1840,7 @@ static int group_prepare_sf(OzakiPlan &oz, const OzGroupDesc &d, const std::vect
             memset(&j, 0, sizeof(j));
             j.rmap = 0; j.rstep = 1;
             j.lplane = g->dT.plane_rows; j.rplane = g->rows;
-            j.lrow0 = 2 * t * d.twoL; j.rrow0 = g->row0[k];
+            j.lrow0 = 2 * d.set_type[t] * d.twoL; j.rrow0 = g->row0[k];
             j.rk0 = t * g->bpad;
             j.nkb = tkb; j.ksteps_last = ksl;
             j.m = 2 * d.twoL; j.n = kb[k].G;
@@ -2404,7 +2405,7 @@ void ozaki_group_destroy(OzGroup *g) {
 // One k-point through a temporary group (the slice autotuner's probe).
 int64_t ozaki_pipeline_workspace(int s, int64_t twoL, int64_t na, int64_t nt, int64_t G) {
     const std::vector<int64_t> g{G};
-    return ozaki_group_bytes(s, twoL, na, nt, g, 1, true, false) + ozaki_group_persist_bytes(s, twoL, na, nt, g, 1, false) +
+    return ozaki_group_bytes(s, twoL, na, nt, g, 1, true, false) + ozaki_group_persist_bytes(s, twoL, na, nt, g, 1, false, nt) +
            2048;
 }
 
@@ -2412,7 +2413,7 @@ int ozaki_pipeline(OzakiPlan &oz, const OzakiInputs &in, double2 *S, double2 *H,
                    cudaStream_t st, int *launches) {
     OzGroupDesc d;
     d.twoL = in.twoL; d.na = in.na; d.nt = in.nt; d.hoist = in.M != nullptr;
-    d.w = in.w; d.Tfull = in.Tfull; d.atom_type = in.atom_type;
+    d.w = in.w; d.Tfull = in.Tfull; d.atom_type = in.atom_type; d.ntypes = in.nt;
     std::vector<OzKBufs> kb(1);
     // the probe keeps C and X apart: C is its input, X is written by the T application
     kb[0].CX = const_cast<double2 *>(in.C);

@@ -61,7 +61,10 @@ struct OzGroupDesc {
     const double *wt = nullptr;            // its per-type S weights [nt][2L] (of the real rows)
     const double *TR = nullptr;            // its real T blocks (launch_treal)
     const double2 *sf_tab = nullptr;       // its structure factors
-    int tbatch = 1;                        // its types per combine batch (product slots)
+    int tbatch = 1;                        // its row sets per combine batch (product slots)
+    int64_t ntypes = 0;                    // types of Tfull and TR (row sets: nt)
+    const int32_t *set_type = nullptr;     // type of each row set: host [nt],
+    const int32_t *d_set_type = nullptr;   // and device
 };
 struct OzGroup;
 // scratch: rewritten by every run (may be shared by the groups of a plan); persist: owned by
@@ -71,7 +74,7 @@ struct OzGroup;
 int64_t ozaki_group_bytes(int s, int64_t twoL, int64_t na, int64_t nt, const std::vector<int64_t> &G, int panels,
                           bool hoist, bool sf);
 int64_t ozaki_group_persist_bytes(int s, int64_t twoL, int64_t na, int64_t nt, const std::vector<int64_t> &G,
-                                  int panels, bool sf);
+                                  int panels, bool sf, int64_t ntypes);
 int ozaki_group_prepare(OzakiPlan &oz, const OzGroupDesc &d, const std::vector<OzKBufs> &kb, void *ws,
                         void *persist, cudaStream_t st, OzGroup **out);
 void ozaki_group_set_outputs(OzGroup *g, double2 *const *S, double2 *const *H, const int64_t *ld);

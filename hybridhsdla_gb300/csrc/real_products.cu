@@ -456,12 +456,13 @@ __global__ void __launch_bounds__(kSliceThreads) oz_slice_real_kernel(const __gr
     for (int c = threadIdx.x; live && c < nch * parts; c += kSliceThreads) {
         const int p = c / nch, cc = c - p * nch, b = cc / bch, r0 = (cc - b * bch) * kVec;
         const int64_t o = (int64_t)b * tab.bstride + p * tab.pstride + r0;
+        const int32_t *el = kFixed ? tab.el + (int64_t)tab.set_type[b] * tab.bstride + p * tab.pstride + r0 : nullptr;
 #pragma unroll
         for (int u = 0; u < kVec; ++u)
             if (r0 + u < rpb) {
                 if constexpr (kFixed) {
                     const long long x = F[o + u];
-                    if (x) mx = max(mx, (unsigned long long)(kOff + 64 - __clzll(x < 0 ? -x : x) + tab.el[o + u]));
+                    if (x) mx = max(mx, (unsigned long long)(kOff + 64 - __clzll(x < 0 ? -x : x) + el[u]));
                 } else {
                     const double x = Z[o + u];
                     mx = max(mx, abs_bits(x));
@@ -490,6 +491,7 @@ __global__ void __launch_bounds__(kSliceThreads) oz_slice_real_kernel(const __gr
     for (int c = threadIdx.x; c < nch * parts; c += kSliceThreads) {
         const int p = c / nch, cc = c - p * nch, b = cc / bch, r0 = (cc - b * bch) * kVec;
         const int64_t o = (int64_t)b * tab.bstride + p * tab.pstride + r0;
+        const int32_t *el = kFixed ? tab.el + (int64_t)tab.set_type[b] * tab.bstride + p * tab.pstride + r0 : nullptr;
         long long x[kVec];
 #pragma unroll
         for (int u = 0; u < kVec; ++u) {
@@ -497,7 +499,7 @@ __global__ void __launch_bounds__(kSliceThreads) oz_slice_real_kernel(const __gr
             if (live && r0 + u < rpb) {
                 if constexpr (kFixed) {
                     // F 2^(el + q) scaled by 2^(top - e): a shift, rounded half up
-                    const int d = tab.el[o + u] + q + top - e;
+                    const int d = el[u] + q + top - e;
                     const long long f = F[o + u];
                     X = d >= 0 ? f << min(d, 63) : d < -63 ? 0 : ((f >> (-d - 1)) + 1) >> 1;
                 } else X = rint_pow2(Z[o + u], top - e);

@@ -83,7 +83,8 @@ struct RealSliceTab {
     int64_t plane_rows = 0, pitch = 0;
     int32_t *expo = nullptr;
     int frac = 0;                      // fixed-point source: its fraction bits (0: an FP64 source),
-    const int32_t *el = nullptr;       // row exponents,
+    const int32_t *el = nullptr;       // row exponents (those of block b from set_type[b] bstride on),
+    const int32_t *set_type = nullptr;
     const int32_t *er = nullptr;       // and the column exponents (per plane row)
     // a second operand of the same source with row weights v2[b rpb + r] (parts = 1)
     const double *v2 = nullptr;
