@@ -135,6 +135,7 @@ struct hsdla_plan {
     // the structure factors SF_t over the box of G-vector differences
     bool sf = false;
     int classes = 0;                 // (type, rotation) classes the structure-factor form runs over (0: types)
+    bool per_atom_sets = false;      // ... more than 3/4 as many as atoms (reported as the per-atom form)
     // T-block check read after the call's own synchronisation (hsdla_create_hs): the device's
     // statistics land in the context's page-locked staging, checked once the stream is idle
     bool tcheck_pending = false;
@@ -401,14 +402,19 @@ int validate(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoint *kpts
 // of per type; each class's rows carry its rotation.
 struct RowSets {
     int n = 0;                                  // sets, numbered by rotation
+    bool shared = true;                         // atoms share them: at most 3/4 as many sets as atoms
     std::vector<int32_t> atom_set, set_type;
     std::vector<int32_t> rot_begin;             // sets of each rotation
     std::vector<double> rots;
 };
 
-// Builds the classes when they shrink the work: their rows (2L per class) are few enough against
-// the per-atom rows (2L per atom) to pay for the structure-factor combine, and the types' tables
-// fit the rows kernel.  Returns false otherwise (per-atom form).
+// Builds the classes of a system whose atoms carry rotations, down to one atom each; returns false
+// where the types' tables do not fit the rows kernel.  Row sets pay even where no two atoms share
+// one: a set takes three real digit products over 2L rows, the per-atom form eight over the same rows
+// plus a T application per atom.  One pass, per-atom form and row sets of one atom each (ms): 32 atoms,
+// lmax 8, 230 columns 3.8 and 0.62, 2003 columns 6.6 and 3.5; 5 atoms, lmax 4, 150 columns 0.68 and
+// 0.19; 100 atoms, lmax 10, 2003 columns 26.1 and 12.9; plain FP64, 32 atoms, 1000 columns 57.2 and 21.3
+// (1.5 to 8 times, 2.6 to 42 in FP64, over 2 to 100 atoms and 60 to 2003 columns).
 bool make_classes(const hsdla_system *s, RowSets &rs) {
     if (!s->atom_rotmat) return false;
     const int na = s->num_atoms, nl = s->max_lmax + 1;
@@ -427,7 +433,8 @@ bool make_classes(const hsdla_system *s, RowSets &rs) {
         cls.emplace(of[j], 0);
     }
     rs.n = (int)cls.size();
-    if (4 * rs.n > 3 * na || rs.n > kMaxSets || rows_kernel_smem(nl * nl, s->max_lmax, s->num_types) > kRowsKernelSmemMax)
+    rs.shared = 4 * rs.n <= 3 * na;
+    if (rs.n > kMaxSets || rows_kernel_smem(nl * nl, s->max_lmax, s->num_types) > kRowsKernelSmemMax)
         return false;
     int q = 0;
     rs.rot_begin.assign(rot_id.size() + 1, 0);
@@ -729,6 +736,22 @@ int hsdla_plan_create(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpo
 }  // extern "C"
 
 namespace {
+int64_t workspace_budget(hsdla_context *ctx);
+
+// Device bytes of one k-point (the largest) over `ns` row sets, with one product slot: real rows, Z',
+// digit planes of 12 slices, products, structure factors.
+int64_t sets_bytes(const hsdla_system *s, const hsdla_kpoint *kpts, int nk, int64_t ns) {
+    const int64_t L = (int64_t)(s->max_lmax + 1) * (s->max_lmax + 1);
+    int64_t G = 0, half[3] = {0, 0, 0};
+    for (int i = 0; i < nk; ++i) {
+        G = std::max(G, kpts[i].n_g);
+        for (int64_t q = 0; q < kpts[i].n_g; ++q)
+            for (int c = 0; c < 3; ++c) half[c] = std::max<int64_t>(half[c], 2 * std::abs((int64_t)kpts[i].g[3 * q + c]));
+    }
+    const int64_t box = (2 * half[0] + 1) * (2 * half[1] + 1) * (2 * half[2] + 1);
+    return 8 * 3 * 2 * L * ns * G + 4 * 12 * (G + 256) * (ns * (2 * L + 64) + 256) + 24 * G * G + 16 * ns * box;
+}
+
 // defer_tcheck: leave the T-block check to the caller (after its own synchronisation), so that the
 // device runs on while the host sets up the execution
 int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoint *kpts, int32_t nk,
@@ -748,8 +771,12 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     // shrink the work (HSDLA_SF=0 or HSDLA_CLASSES=0 keeps the per-atom form)
     const char *sf_env0 = getenv("HSDLA_SF");
     RowSets sets;
-    const bool use_classes = s->atom_rotmat && !(sf_env0 && strtol(sf_env0, nullptr, 10) == 0) &&
+    bool use_classes = s->atom_rotmat && !(sf_env0 && strtol(sf_env0, nullptr, 10) == 0) &&
                              env_flag("HSDLA_CLASSES", true) && make_classes(s, sets);
+    // many sets: only where one k-point's workspace (one product slot) fits, else the per-atom form,
+    // which can stream its contraction in atom panels
+    if (use_classes && (!sets.shared || sets.n > kMaxTypes) && sets_bytes(s, kpts, nk, sets.n) > workspace_budget(ctx))
+        use_classes = false;
     if (!use_classes) {      // the types, no rotations
         sets = RowSets();
         sets.n = s->num_types;
@@ -759,6 +786,7 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     auto *pl = new hsdla_plan();
     pl->ctx = ctx;
     pl->classes = use_classes ? sets.n : 0;
+    pl->per_atom_sets = use_classes && !sets.shared;
     if (opts) pl->opts = *opts;
     if (pl->opts.precision != HSDLA_PREC_FP64 && pl->opts.precision != HSDLA_PREC_OZAKI_FP8) {
         delete pl;
@@ -1111,7 +1139,9 @@ void choose_type_batch(hsdla_plan *pl, int64_t budget) {
         if (pl->kps[i].n_g > 0 && (big < 0 || pl->kps[i].n_g > pl->kps[big].n_g)) big = i;
     if (big < 0) return;
     const std::vector<int> one{big};
-    pl->tbatch = pl->nt;
+    // (many sets: a batch of 16 reads and writes S and H rarely enough; its products stay a fraction
+    // of the device memory)
+    pl->tbatch = pl->per_atom_sets || pl->nt > kMaxTypes ? std::min(pl->nt, 16) : pl->nt;
     while (pl->tbatch > 1 && group_bytes(pl, one) > budget) --pl->tbatch;
 }
 
@@ -1797,8 +1827,8 @@ int hsdla_plan_execute(hsdla_plan *pl, hsdla_cx *const *dH, hsdla_cx *const *dS,
         rep->est_rel_err = pl->est_err;
         rep->kernel_launches = pl->launches;
         rep->num_panels = pl->opts.precision == HSDLA_PREC_OZAKI_FP8 ? pl->panels : 0;
-        rep->num_row_sets = pl->sf ? pl->nt : 0;
-        rep->rotation_classes = pl->classes > 0 ? 1 : 0;
+        rep->num_row_sets = pl->sf && !pl->per_atom_sets ? pl->nt : 0;
+        rep->rotation_classes = pl->classes > 0 && !pl->per_atom_sets ? 1 : 0;
         if (!pl->groups.empty() && pl->groups[0].oz && ozaki_group_tunable(pl->groups[0].oz)) {
             int h = 0, m = 0;
             ozaki_group_tiles(pl->groups[0].oz, &h, &m);

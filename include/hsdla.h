@@ -129,7 +129,8 @@ typedef struct hsdla_report {
     int32_t num_panels;          /* Ozaki: atom panels the contraction was streamed in (1 = resident) */
     int32_t outputs_in_place;    /* hsdla_create_hs: 1 = the GPU wrote the page-locked host H, S itself */
     int32_t num_row_sets;        /* structure-factor form: the row sets contracted (types, or (type, rotation)
-                                    classes when atoms carry rotations); 0 = the per-atom form */
+                                    classes when atoms carry rotations); 0 = rows per atom (also where more than
+                                    three quarters as many classes as atoms are contracted) */
     int32_t rotation_classes;    /* 1: the row sets are (type, rotation) classes */
     int32_t tile_halves;         /* Ozaki, structure-factor form: the S/H products' bands of digit diagonals alternate */
                                  /* between two halves of TMEM (2) or wait for each other in one (1); 0 otherwise */

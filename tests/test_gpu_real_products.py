@@ -60,3 +60,24 @@ def test_fp64_real_products_match_oracle(ctx, lmax, n_g, types):
     for X, R, nm in ((H, Hr, "H"), (S, Sr, "S")):
         fro, mx = oracle.lower_errors(X, R)
         assert fro < 1e-13 and mx < 1e-13, (nm, lmax, n_g, fro, mx)
+
+
+@pytest.mark.parametrize("precision", ["ozaki", "fp64"])
+@pytest.mark.parametrize("atoms,lmax,n_g", [(1, 2, 40), (3, 6, 130), (18, 3, 257), (35, 1, 300)])
+def test_every_atom_its_own_rotation_on_row_sets(ctx, monkeypatch, precision, atoms, lmax, n_g):
+    """Every atom a row set of its own (one atom; more sets than a combine batch of 16, with a partial
+    last batch; more rotations than the rows kernel's 16 at a time): the oracle, and the per-atom form."""
+    edge = (125.0 * max(atoms, 2)) ** (1.0 / 3.0)
+    cfg = dict(cell=(edge, edge, edge), atoms=atoms, types=min(atoms, 2), rmt=2.0, min_sep=3.6, lmax=lmax,
+               kpts=[(0.1, 0.2, 0.3), (0.0, 0.0, 0.0)], n_g=n_g, seed=31 + atoms)
+    s = synth.with_rotations(synth.make_system(cfg))
+    res, rep = ctx.create_hs(s, precision=precision, num_slices=11 if precision == "ozaki" else 0)
+    assert rep["num_row_sets"] == 0 and rep["rotation_classes"] == 0
+    monkeypatch.setenv("HSDLA_CLASSES", "0")
+    per_atom, rep_pa = ctx.create_hs(s, precision=precision, num_slices=11 if precision == "ozaki" else 0)
+    for (H, S), (Hp, Sp), kp in zip(res, per_atom, s.kpoints):
+        Hr, Sr = oracle.reference_hs(s, kp)
+        for X, P, R, nm in ((H, Hp, Hr, "H"), (S, Sp, Sr, "S")):
+            fro, mx = oracle.lower_errors(X, R)
+            assert fro < 1e-13 and mx < 1e-13, (nm, atoms, lmax, fro, mx)
+            assert oracle.lower_errors(X, P)[0] < 1e-13
