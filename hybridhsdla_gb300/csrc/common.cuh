@@ -173,17 +173,22 @@ struct SfTab {
     int64_t xrow1 = 0;                            // rows below it go to the entries' Sx, Hx when set
 
     int dx = 0, dy = 0, dz = 0, ny = 0, nz = 0;   // box offsets (half widths) and extents
-    int64_t box = 0;                              // entries per type
+    int64_t box = 0;                              // entries
+    int nt = 1;                                   // row sets of the structure-factor table
+    int sfbits = 0;                               // its fixed point (launch_sf_table), 0: FP64
     SfEntry e[kMaxGroup];
 };
 // SF_t(dG) = sum_{a of type t} e^{i 2pi dG.tau_a} over the box of G-vector differences, from
-// per-atom factors ex[a][dGx + dx] = e^{i 2pi dGx tau_a,x} (and y, z); atoms listed by type.
+// per-atom factors ex[a][dGx + dx] = e^{i 2pi dGx tau_a,x} (and y, z); atoms listed by type.  The table
+// holds entry dG's types together (type fastest), 16 bytes each: FP64 (re, im), or with sfbits > 0
+// each part as the limbs {f >> 28, f & (2^28 - 1)} of f = rint(part 2^sfbits), |f| < 2^55.
 cudaError_t launch_sf_table(const double2 *ex, const double2 *ey, const double2 *ez, const int32_t *order,
-                            const int32_t *type_begin, int nt, int nx, int ny, int nz, double2 *sf, cudaStream_t st);
+                            const int32_t *type_begin, int nt, int nx, int ny, int nz, int sfbits, void *sf,
+                            cudaStream_t st);
 // S (+)= sum_b SF_{type+b} (.) S_b and H (+)= sum_b SF_{type+b} (.) H_b over the lower triangles
 // of every entry, b over the batch's type slots, in columns [tab.col0, tab.col1) (multiples of 32
 // but for the end); rows below tab.xrow1 into Sx, Hx instead for entries that give them.
-cudaError_t launch_sf_combine(const SfTab &tab, const double2 *sf, bool first, cudaStream_t st);
+cudaError_t launch_sf_combine(const SfTab &tab, const void *sf, bool first, cudaStream_t st);
 
 // BLAS-shaped plugin (blas_plugin.cu).  Operand in the 'C' layout: dst rows [r0, r0 + k) of every
 // column c < n (ld ldd) = s * src[r, c] (src k x n, transpose false) or s * conj(src[c, r]) (src

@@ -142,7 +142,7 @@ struct hsdla_plan {
     const unsigned long long *tcheck_host = nullptr;
     double *wt = nullptr;            // (of the real rows: doubled where m != 0)
     double *TR = nullptr;            // real T blocks [nt][4L][2L]
-    double2 *sf_tab = nullptr;
+    void *sf_tab = nullptr;
     SfTab sf_dims{};                 // box extents and offsets (entries filled per group)
     int tbatch = 1;                  // types whose products are combined into S and H in one pass
     // hsdla_create_hs: the host outputs the last combine of each group downloads column block by
@@ -958,6 +958,14 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
         dm.dx = half[0]; dm.dy = half[1]; dm.dz = half[2];
         dm.ny = ext[1]; dm.nz = ext[2];
         dm.box = (int64_t)ext[0] * ext[1] * ext[2];
+        dm.nt = ns;
+        if (pl->opts.precision == HSDLA_PREC_OZAKI_FP8) {
+            // |SF_t| <= atoms of the set < 2^(55 - sfbits)
+            int most = 0, b = 0;
+            for (int q = 0; q < ns; ++q) most = std::max(most, tb[q + 1] - tb[q]);
+            while ((1 << b) <= most) ++b;
+            dm.sfbits = 55 - b;
+        }
     }
     // past the uploaded part: what the device fills
     auto dev_only = [&](int64_t b) -> void * {
@@ -969,7 +977,7 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     unsigned long long *d_stats = (unsigned long long *)dev_only(sizeof(unsigned long long) * 5 * nt);
     if (pl->sf) {
         d_ex = (double2 *)dev_only(sizeof(double2) * (int64_t)na * (ext[0] + ext[1] + ext[2]));
-        pl->sf_tab = (double2 *)dev_only(sizeof(double2) * (int64_t)ns * ext[0] * ext[1] * ext[2]);
+        pl->sf_tab = dev_only(sizeof(double2) * (int64_t)ns * ext[0] * ext[1] * ext[2]);
     }
     if (pl->sf) pl->TR = (double *)dev_only(sizeof(double) * 2 * tf_elems);
     std::vector<unsigned long long> tstats((size_t)5 * nt, 0);
@@ -1010,7 +1018,7 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     if (e == cudaSuccess && pl->sf) e = launch_sf_phases(D.atom_pos, na, half, ext, d_ex, ctx->stream);
     if (e == cudaSuccess && pl->sf)
         e = launch_sf_table(d_ex, d_ex + (size_t)na * ext[0], d_ex + (size_t)na * (ext[0] + ext[1]), d_order,
-                            d_order + na, ns, ext[0], ext[1], ext[2], pl->sf_tab, ctx->stream);
+                            d_order + na, ns, ext[0], ext[1], ext[2], pl->sf_dims.sfbits, pl->sf_tab, ctx->stream);
     const bool defer = defer_tcheck && ctx->staging != nullptr;
     unsigned long long *stats_host =
         defer ? reinterpret_cast<unsigned long long *>(reinterpret_cast<char *>(ctx->staging) + stats_off) : tstats.data();
@@ -1263,6 +1271,7 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
             const SfTab &dm = pl->sf_dims;
             ft.nk = kt.nk;
             ft.dx = dm.dx; ft.dy = dm.dy; ft.dz = dm.dz; ft.ny = dm.ny; ft.nz = dm.nz; ft.box = dm.box;
+            ft.nt = dm.nt; ft.sfbits = dm.sfbits;
         }
         if (pl->opts.precision == HSDLA_PREC_OZAKI_FP8) {
             OzGroupDesc d;

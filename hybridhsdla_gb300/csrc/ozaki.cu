@@ -1463,7 +1463,7 @@ struct OzGroup {
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     SfTab sft{};                // its combine table (outputs patched per run)
-    const double2 *sf_tab = nullptr;
+    const void *sf_tab = nullptr;
     // Streamed host output (structure-factor form on pair tiles, every type in one combine batch):
     // the S/H products of all types in column blocks, one launch per block, each block combined
     // into the caller's page-locked outputs on blk_side while the next block's products run.

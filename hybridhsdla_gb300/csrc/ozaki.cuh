@@ -60,7 +60,7 @@ struct OzGroupDesc {
     bool sf = false;                       // structure-factor form (requires hoist)
     const double *wt = nullptr;            // its per-type S weights [nt][2L] (of the real rows)
     const double *TR = nullptr;            // its real T blocks (launch_treal)
-    const double2 *sf_tab = nullptr;       // its structure factors
+    const void *sf_tab = nullptr;          // its structure factors
     int tbatch = 1;                        // its row sets per combine batch (product slots)
     int64_t ntypes = 0;                    // types of Tfull and TR (row sets: nt)
     const int32_t *set_type = nullptr;     // type of each row set: host [nt],

@@ -81,3 +81,30 @@ def test_every_atom_its_own_rotation_on_row_sets(ctx, monkeypatch, precision, at
             fro, mx = oracle.lower_errors(X, R)
             assert fro < 1e-13 and mx < 1e-13, (nm, atoms, lmax, fro, mx)
             assert oracle.lower_errors(X, P)[0] < 1e-13
+
+
+@pytest.mark.parametrize("precision", ["ozaki", "fp64"])
+@pytest.mark.parametrize("types", [1, 2, 3, 4, 5, 6, 7, 8, 9, 13, 16, 17])
+def test_combine_over_type_counts(ctx, monkeypatch, precision, types):
+    """Every chunk of the combine (4, 2 and 1 types) and sums of more than the eight types that the
+    integers hold, whole and cut into batches of three types; a ragged basis of one and a half tiles,
+    and many atoms of one type beside single ones (the structure factors' fixed point)."""
+    atoms = types + 14
+    edge = (125.0 * atoms) ** (1.0 / 3.0)
+    cfg = dict(cell=(edge, edge * 1.05, edge * 0.95), atoms=atoms, types=types, rmt=2.0, min_sep=3.6, lmax=3,
+               kpts=[(0.1, 0.2, 0.3), (-0.25, 0.0, 0.5)], n_g=49, seed=53 + types)
+    s = synth.make_system(cfg)
+    first = np.arange(types)
+    s.atom_type = np.concatenate([first, np.full(14, types - 1)]).astype(s.atom_type.dtype)
+    n_slices = 11 if precision == "ozaki" else 0
+    whole, rep = ctx.create_hs(s, precision=precision, num_slices=n_slices)
+    assert rep["num_row_sets"] == types
+    monkeypatch.setenv("HSDLA_TYPE_BATCH", "3")
+    cut, _ = ctx.create_hs(s, precision=precision, num_slices=n_slices)
+    for (H, S), (Hc, Sc), kp in zip(whole, cut, s.kpoints):
+        Hr, Sr = oracle.reference_hs(s, kp)
+        for X, C, R, nm in ((H, Hc, Hr, "H"), (S, Sc, Sr, "S")):
+            fro, mx = oracle.lower_errors(X, R)
+            assert fro < 1e-13 and mx < 1e-13, (nm, types, fro, mx)
+            fro, mx = oracle.lower_errors(C, R)
+            assert fro < 1e-13 and mx < 1e-13, (nm, types, fro, mx)
