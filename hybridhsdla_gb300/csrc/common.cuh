@@ -87,6 +87,9 @@ struct KTable {
     KEntry e[kMaxGroup];
 };
 
+// dst[2L u + i] = src[L u + i] for u < units, i < L: rows of A (or, dst + L, of B) into [A; B].
+cudaError_t launch_stack_rows(const double2 *src, int L, int64_t units, double2 *dst, cudaStream_t st);
+
 // ----------------------------------------------------------- kernels (host)
 // (a) for every k-point of a table in one launch (C always; M when the entries give it)
 cudaError_t launch_construct_ab_multi(const DevSystem &sys, const KTable &tab, cudaStream_t st);

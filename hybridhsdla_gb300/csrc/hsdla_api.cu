@@ -11,7 +11,11 @@
 // in either plain FP64 or the Ozaki FP8 form.  Errors are returned as status
 // codes with a message in the context (the reference prints and exits,
 // h_and_s.cpp:712-723).
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <complex>
@@ -31,6 +35,10 @@
 #include "ozaki.cuh"
 
 using namespace hsdla;
+
+namespace {
+class OutputPages;
+}
 
 struct hsdla_context {
     int device = 0;
@@ -150,6 +158,7 @@ struct hsdla_plan {
     struct Download {
         std::vector<hsdla_cx *> H, S;
         std::vector<int64_t> ld;
+        OutputPages *pages = nullptr;   // to wait for before the first copy
         bool direct = false;   // every output is page-locked host memory the GPU can write
         bool done = false;
         bool in_place = false;   // the combine wrote the host outputs
@@ -275,6 +284,80 @@ int ctx_host_out(hsdla_context *ctx, int64_t bytes, void **out) {
     return HSDLA_OK;
 }
 
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+
+// Pages of pageable host outputs that are not in memory yet (a fresh allocation), made present by up
+// to four threads while the GPU computes.  A copy into an absent page has the GPU fault on it: an
+// otherwise untouched H of 1501 (3000) columns took 34 (134) ms to download, 0.17 (0.52) ms when its
+// pages were there; one thread makes them in 1.2 (7.4) ms.  Contents stay as they are; where the
+// kernel lacks the request the copies fault as they did.
+class OutputPages {
+    struct Piece {
+        uintptr_t lo;
+        size_t bytes;
+    };
+    static constexpr size_t kPiece = (size_t)2 << 20;
+    std::vector<Piece> todo_;
+    std::vector<std::thread> threads_;
+    std::atomic<size_t> next_{0};
+    const size_t page_ = (size_t)sysconf(_SC_PAGESIZE);
+
+    void span(uintptr_t lo, size_t bytes) {
+        const uintptr_t hi = (lo + bytes + page_ - 1) / page_ * page_;
+        lo = lo / page_ * page_;
+        std::vector<unsigned char> in((hi - lo) / page_);
+        if (mincore(reinterpret_cast<void *>(lo), hi - lo, in.data()) != 0) return;
+        for (size_t a = 0; a < in.size();) {
+            size_t b = a;
+            while (b < in.size() && !(in[b] & 1) && (b - a) * page_ < kPiece) ++b;
+            if (b > a) todo_.push_back({lo + a * page_, (b - a) * page_});
+            else ++b;
+            a = b;
+        }
+    }
+    void work() {
+        for (size_t i; (i = next_++) < todo_.size();)
+            madvise(reinterpret_cast<void *>(todo_[i].lo), todo_[i].bytes, MADV_POPULATE_WRITE);
+    }
+
+  public:
+    OutputPages() = default;
+    OutputPages(const OutputPages &) = delete;
+    OutputPages &operator=(const OutputPages &) = delete;
+    ~OutputPages() { wait(); }
+    // `cols` columns of `width` bytes, `pitch` bytes apart
+    void add(void *p, int64_t pitch, int64_t width, int64_t cols) {
+        cudaPointerAttributes pa{};
+        if (cols < 1 || width < 1) return;
+        if (cudaPointerGetAttributes(&pa, p) != cudaSuccess) {
+            cudaGetLastError();
+            return;
+        }
+        if (pa.type != cudaMemoryTypeUnregistered) return;
+        const uintptr_t lo = reinterpret_cast<uintptr_t>(p);
+        try {
+            if (pitch - width < 2 * (int64_t)page_) span(lo, (size_t)((cols - 1) * pitch + width));
+            else
+                for (int64_t c = 0; c < cols; ++c) span(lo + (size_t)(c * pitch), (size_t)width);
+        } catch (...) {          // (no memory for the list: the copies fault)
+        }
+    }
+    void start() {
+        const size_t n = std::min<size_t>(4, todo_.size());
+        try {
+            while (threads_.size() < n) threads_.emplace_back(&OutputPages::work, this);
+        } catch (...) {          // a thread that cannot start leaves its share to the others and wait()
+        }
+    }
+    void wait() {
+        work();
+        for (auto &t : threads_) t.join();
+        threads_.clear();
+    }
+};
+
 // Download of the lower triangle of a column-major n x n device matrix into a host matrix of
 // leading dimension ld: column blocks of kDownBlock, each from its first row down (the strict
 // upper triangle outside the diagonal blocks is not copied; ~half the bytes of the full matrix).
@@ -288,6 +371,12 @@ cudaError_t download_lower(hsdla_cx *host, int64_t ld, const hsdla_cx *dev, int6
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
+}
+
+// The pages that download_lower writes.
+void add_lower(OutputPages &pages, hsdla_cx *host, int64_t ld, int64_t n) {
+    for (int64_t c0 = 0; c0 < n; c0 += kDownBlock)
+        pages.add(host + c0 + ld * c0, ld * sizeof(hsdla_cx), (n - c0) * sizeof(hsdla_cx), std::min(kDownBlock, n - c0));
 }
 
 int ctx_workspace(hsdla_context *ctx, int64_t bytes, void **out) {
@@ -1507,6 +1596,7 @@ int combine_last(hsdla_plan *pl, hsdla_plan::Group &g, int t0, int ntypes, cudaS
         pl->launches++;
         CUDA_TRY(ctx, cudaEventRecord(ctx->ev_copy, st));
         CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->copy_stream, ctx->ev_copy, 0));
+        if (c0 == 0 && pl->dl->pages) pl->dl->pages->wait();
         for (int q = 0; q < g.ktab.nk; ++q) {
             const int i = g.kidx[q];
             const int64_t n = pl->kps[i].n_g;
@@ -1932,6 +2022,7 @@ int hsdla_contract_ab(hsdla_context *ctx, int32_t L, int32_t a, int64_t G, const
     pl->kps.push_back(pk);
     pl->flop = 20.0 * (double)G * G * L * a + 24.0 * (double)L * L * a * G;
     cudaStream_t st = ctx->stream;
+    OutputPages pages;
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -1964,19 +2055,38 @@ int hsdla_contract_ab(hsdla_context *ctx, int32_t L, int32_t a, int64_t G, const
     if (rc) return done(rc);
     hsdla_cx *dH = reinterpret_cast<hsdla_cx *>(dout), *dS = dH + G * G;
     const int64_t ldd = G;
-    // A, B (L x a x G, column-major) straight into C's per-atom [A_a; B_a] row blocks
+    for (hsdla_cx *hp : {H, S}) add_lower(pages, hp, ld, G);
+    pages.start();
+    // A, B (L x a x G, column-major) into C's per-atom [A_a; B_a] row blocks, through the output
+    // buffer in as many pieces as it takes: a strided copy of L-element rows reaches 32 GB/s, a plain
+    // one 145 (8 atoms, lmax 8, 1501 columns: 0.49 and 0.11 ms each for A and B).  Bases so small that
+    // this takes many pieces are copied strided.
     const KEntry &e = pl->groups[0].ktab.e[0];
-    if (cudaMemsetAsync(dout, 0, 2 * G * G * sizeof(double2), st) != cudaSuccess ||
-        cudaMemcpy2DAsync(e.C, twoL * sizeof(double2), A, L * sizeof(double2), L * sizeof(double2), (size_t)a * G,
-                          cudaMemcpyHostToDevice, st) != cudaSuccess ||
-        cudaMemcpy2DAsync(e.C + L, twoL * sizeof(double2), B, L * sizeof(double2), L * sizeof(double2), (size_t)a * G,
-                          cudaMemcpyHostToDevice, st) != cudaSuccess)
+    const int64_t units = (int64_t)a * G, cap = 2 * G * G / L;
+    cudaError_t eu = cudaSuccess;
+    for (int m = 0; m < 2; ++m) {
+        const hsdla_cx *src = m == 0 ? A : B;
+        double2 *dst = e.C + m * L;
+        if (cap * 8 < units) {
+            if (eu == cudaSuccess)
+                eu = cudaMemcpy2DAsync(dst, twoL * sizeof(double2), src, L * sizeof(double2), L * sizeof(double2),
+                                       (size_t)units, cudaMemcpyHostToDevice, st);
+            continue;
+        }
+        for (int64_t u0 = 0; eu == cudaSuccess && u0 < units; u0 += cap) {
+            const int64_t nu = std::min(cap, units - u0);
+            eu = cudaMemcpyAsync(dout, src + L * u0, sizeof(double2) * (size_t)(L * nu), cudaMemcpyHostToDevice, st);
+            if (eu == cudaSuccess) eu = launch_stack_rows(reinterpret_cast<const double2 *>(dout), L, nu, dst + twoL * u0, st);
+        }
+    }
+    if (eu != cudaSuccess || cudaMemsetAsync(dout, 0, 2 * G * G * sizeof(double2), st) != cudaSuccess)
         return done(set_err(ctx, HSDLA_ERR_CUDA, "A/B upload failed"));
     set_outputs(pl, &dH, &dS, &ldd);
     float ms_ab = 0.f, ms_tap = 0.f;
     double dom_flop = 0.0;
     rc = run_groups(pl, st, true, &ms_ab, &ms_tap, &dom_flop);
     if (rc) return done(rc);
+    pages.wait();
     if (download_lower(H, ld, dH, G, st) != cudaSuccess || download_lower(S, ld, dS, G, st) != cudaSuccess)
         return done(set_err(ctx, HSDLA_ERR_CUDA, "H/S download failed"));
     cudaEventRecord(e1, st);
@@ -2033,6 +2143,11 @@ int hsdla_create_hs(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoin
     void *dout = nullptr;
     rc = ctx_host_out(ctx, std::max<int64_t>(out_elems, 1) * (int64_t)sizeof(double2), &dout);
     if (rc) { hsdla_plan_destroy(pl); cudaEventDestroy(e0); cudaEventDestroy(e1); return rc; }
+    OutputPages pages;
+    for (int i = 0; i < nk; ++i)
+        if (ng[i] > 0)
+            for (hsdla_cx *hp : {H[i], S[i]}) add_lower(pages, hp, ld[i], ng[i]);
+    pages.start();
     std::vector<hsdla_cx *> dH(nk), dS(nk);
     std::vector<int64_t> dld(nk);
     hsdla_cx *p = reinterpret_cast<hsdla_cx *>(dout);
@@ -2053,6 +2168,7 @@ int hsdla_create_hs(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoin
             }
     // structure-factor form: the last combine downloads each column block as soon as it is done
     hsdla_plan::Download dl;
+    dl.pages = &pages;
     dl.H.assign(H, H + nk);
     dl.S.assign(S, S + nk);
     dl.ld.assign(ld, ld + nk);
@@ -2085,6 +2201,7 @@ int hsdla_create_hs(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoin
         if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->stream, ctx->ev_copy, 0);
         if (e != cudaSuccess) rc = set_err(ctx, HSDLA_ERR_CUDA, "D2H copy failed: %s", cudaGetErrorString(e));
     }
+    pages.wait();
     for (int i = 0; rc == HSDLA_OK && !dl.done && i < nk; ++i) {
         if (ng[i] == 0) continue;
         e = download_lower(H[i], ld[i], dH[i], ng[i], ctx->stream);
@@ -2304,6 +2421,10 @@ int plugin_contract(hsdla_context *ctx, int kind, int32_t precision, int32_t num
         dldb = rows;
     }
     if (hC) {
+        OutputPages pages;
+        pages.add(C, ldc * e16, n * e16, n);
+        pages.start();
+        pages.wait();
         // the whole n x n block travels (the other triangle comes back as it went)
         CUDA_TRY(ctx, cudaMemcpy2DAsync(ws + oC, n * e16, C, ldc * e16, n * e16, n, cudaMemcpyHostToDevice, st));
         dC = reinterpret_cast<double2 *>(ws + oC);
