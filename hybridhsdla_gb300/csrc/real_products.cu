@@ -18,20 +18,26 @@
 //    takes 96 B per cycle.  (128-digit chunks leave no room to load ahead.)  Planes arrive and
 //    leave in batches of four: a barrier per plane kept the MMA thread at its waits and commits
 //    (150 cycles per MMA of 64).
-//  * The digit pairs run in bands of two diagonals, so that a step of the left plane feeds two MMAs
-//    (the second takes it from the collector buffer).  The bands alternate between two TMEM halves:
-//    one drains while the next computes.
+//  * The digit pairs run in bands of two diagonals (RealBands) summed in one accumulator: the products
+//    of the upper diagonal carry a factor 32, as the left operand's block scale (mxf8f6f4; the scale
+//    factors 1 and 32 fill TMEM columns of their own).  A band leaves 128 columns of TMEM instead of 256
+//    and takes one FP32 operation less per element.  Three accumulators take the bands in turn.
+//  * Two threads issue the MMAs, every other band each: one takes ~75 cycles per MMA, of which it
+//    must not take more than 80 and did not keep to with the epilogue's warps on its scheduler.
 //  * The sums over diagonals and chunks stay in registers as 64-bit fixed-point numbers (64 per
-//    thread of the eight epilogue warps): a diagonal's FP32 integer becomes an integer by one FADD
-//    (x + 1.5 2^23 leaves it in the low mantissa bits), and a band's adds with one multiply-add.
-//    Each output element is written once, rather than once per accumulation unit through L2
-//    reductions.  The fixed-point sum is exact down to 2^-frac of a unit of the top diagonal.
-// What bounds it: the drains and the MMA thread, each ~0.85 of the time, in turn where a band's MMAs
-// are shorter than the drain before them.  One type of the 8000-column workload (lmax 10, 11 digits):
-// 3.05 ms in the complex form, 1.07 ms here = 2.9 PFLOP/s of e4m3, 0.75 of twice the measured bf16
-// rate (0.91 ms with the drains' arithmetic left out).  Measured and not kept: sixteen epilogue warps
-// with half the sums each (1.07), TMEM loads ahead of the arithmetic (1.07), shifts and adds in place
-// of the wide multiply-adds (1.10), no collector buffer (1.07).
+//    thread of the eight epilogue warps): a band's FP32 integer becomes an integer by one FMA
+//    (x + 1.5 2^23 leaves it in the low mantissa bits) and adds with one multiply-add.  Each output
+//    element is written once, rather than once per accumulation unit through L2 reductions.  The
+//    fixed-point sum is exact down to 2^-frac of a unit of the top diagonal.
+//  * A tile is stored only when the next one's first band has left its accumulator, so the MMAs run
+//    four bands ahead meanwhile.
+// What bounds it: the tensor pipe, 0.93 of the time (0.83 ms with neither stores nor sums).  One type of
+// the 8000-column workload (lmax 10, 11 digits): 3.05 ms in the complex form, 0.863 ms here = 3.56
+// PFLOP/s of e4m3, 0.93 of twice the measured bf16 rate.  On the way: two accumulators a band, summed by
+// the epilogue, and one issuer 1.067; block scales 1.059; the next tile's chunk count fetched ahead
+// 1.033; the delayed store 1.004; two issuers 0.863.  Measured and not kept: sixteen epilogue warps with
+// half the sums each, TMEM loads ahead of the arithmetic, shifts and adds in place of the wide
+// multiply-adds, large bands first in a tile, right planes a chunk at a time ahead of the left ones.
 // Every wait is bounded (ptx.cuh); both CTAs meet at a cluster barrier before TMEM is freed.
 #include <cuda_fp8.h>
 
@@ -45,7 +51,7 @@
 namespace hsdla {
 namespace {
 
-constexpr int kThreads = 384;              // warps 0-3: left TMA, MMA, right TMA, idle; 4-11 epilogue
+constexpr int kThreads = 384;              // warps 0-3: TMA, MMA, idle, MMA; 4-11 epilogue
 constexpr int kEpi = 8;
 constexpr int kCols = kRealTileN / 2;      // columns of an epilogue warp (two warps per lane quadrant)
 constexpr int kABytes = 128 * kRealKBlock, kBBytes = kRealBRows * kRealKBlock;
@@ -55,6 +61,10 @@ constexpr int kBatch = 4, kRing = 4, kNA = kRing * kBatch, kBank = kRealMaxSlice
 static_assert((kRing - 1) * kBatch >= kRealMaxSlices, "the ring holds a chunk's planes");
 constexpr int kSmem = 1024 + kNA * kABytes + kNB * kBBytes;
 static_assert(kSmem <= 226 * 1024, "shared memory (the barriers are static)");
+// TMEM: buffers of one FP32 accumulator, then the scale factors 1 and 32 (all bytes of 32 columns each)
+constexpr int kBufs = 3;
+constexpr uint32_t kScaleOne = kBufs * kRealTileN, kScale32 = kScaleOne + 32;
+constexpr uint32_t kOneBytes = 0x7F7F7F7Fu, k32Bytes = 0x84848484u;    // ue8m0
 // Register split: 384 threads are launched with 168 registers each (64512); the control warps keep
 // 56 and the epilogue warps get 216, 62464 in all.  launch_real_products checks the 168.
 constexpr int kRegsLaunch = 168, kRegsControl = 56, kRegsEpilogue = 216;
@@ -63,11 +73,16 @@ static_assert(128 * kRegsControl + 256 * kRegsEpilogue <= kThreads * kRegsLaunch
 struct __align__(8) RealBarriers {
     uint64_t full[kRing];              // a batch's left and right planes landed (both CTAs')
     uint64_t aempty[kRing], bempty[2]; // a left batch, a right bank consumed
-    uint64_t tfull[2], tempty[2];      // a band's accumulators in each TMEM half
+    uint64_t tfull[kBufs], tempty[kBufs];   // a band's accumulators in each TMEM buffer
 };
 
 __host__ __device__ constexpr uint32_t idesc_real() {
     return (1u << 4) | ((uint32_t)(kRealTileN >> 3) << 17) | ((uint32_t)(kRealTileM >> 4) << 24);
+}
+
+// The same with block scales (mxf8f6f4; scale factors in ue8m0, byte 0 of each TMEM word)
+__host__ __device__ constexpr uint32_t idesc_scaled() {
+    return ((uint32_t)(kRealTileN >> 3) << 17) | (1u << 23) | ((uint32_t)(kRealTileM >> 4) << 24);
 }
 
 // After an abort the copies and MMAs in flight have long landed: short waits for them
@@ -76,54 +91,48 @@ constexpr long long kAbortCycles = 100000000LL;
 constexpr float kMagic = 12582912.0f;                  // 1.5 2^23
 constexpr uint32_t kMagicBits = 0x4B400000u;
 
-// One band's accumulators (diagonal T - 1 at t0, T at t1) into the sums (RealBands).  One short path
-// per kind of fold: a path per shift and width, and FP64 conversions at the tile's end, overflowed
-// the instruction cache.
+// One band's accumulators into the sums (RealBands).  One short path per kind of fold: a path per shift
+// and width, and FP64 conversions at the tile's end, overflowed the instruction cache.
 template <int kFold>
-__device__ __forceinline__ void add_band(unsigned long long (&acc)[kCols], uint32_t t0, uint32_t t1, float g, float f,
-                                         uint32_t mul, uint32_t tempty, int lane) {
+__device__ __forceinline__ void add_band(unsigned long long (&acc)[kCols], const uint32_t (&v)[2][32], float f,
+                                         uint32_t mul) {
 #pragma unroll
-    for (int h = 0; h < kCols; h += 32) {
-        uint32_t v0[32], v1[32];
-        tmem_ld32(t0 + h, v0);
-        tmem_ld32(t1 + h, v1);
-        tmem_ld_wait();
-        if (h + 32 >= kCols) {
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_remote(tempty);
-        }
-#pragma unroll
-        for (int c = 0; c < 32; ++c) {
-            const float x0 = __uint_as_float(v0[c]), x1 = __uint_as_float(v1[c]);
-            const uint32_t b = kFold == kFoldInt
-                                   ? (__float_as_uint(x0 + kMagic) << 5) + __float_as_uint(x1 + kMagic)
-                                   : __float_as_uint(fmaf(fmaf(x0, g, x1), f, kMagic));
-            if (kFold == kFoldHigh) {
-                const uint32_t lo = (uint32_t)acc[h + c], hi = (uint32_t)(acc[h + c] >> 32) + b * mul;
-                acc[h + c] = ((unsigned long long)hi << 32) | lo;
-            } else acc[h + c] += (unsigned long long)b * mul;
-        }
+    for (int c = 0; c < kCols; ++c) {
+        const uint32_t b = __float_as_uint(fmaf(__uint_as_float(v[c / 32][c % 32]), f, kMagic));
+        if (kFold == kFoldHigh) {
+            const uint32_t lo = (uint32_t)acc[c], hi = (uint32_t)(acc[c] >> 32) + b * mul;
+            acc[c] = ((unsigned long long)hi << 32) | lo;
+        } else acc[c] += (unsigned long long)b * mul;
     }
 }
 
 // MMAs of the pair with operands given by the low words of their descriptors; the high word and the
 // instruction descriptor are constants (fewer registers to move to the uniform file per MMA).
-// kA: the left operand's collector buffer (0 none, 1 fill, 2 last use)
 constexpr uint32_t kDescHi = (512u >> 4) | (1u << 14) | (4u << 29);    // SW64 K-major, 8 rows of 64 bytes
-template <int kA>
 __device__ __forceinline__ void mma_real(uint32_t d, uint32_t a, uint32_t b, uint32_t acc) {
-#define HSDLA_MMA_REAL(coll)                                                                                  \
-    asm volatile(                                                                                             \
-        "{\n .reg .b64 da, db;\n .reg .pred p;\n .reg .b32 h;\n mov.b32 h, %3;\n mov.b64 da, {%1, h};\n"        \
-        " mov.b64 db, {%2, h};\n setp.ne.b32 p, %5, 0;\n"                                                     \
-        " tcgen05.mma.cta_group::2.kind::f8f6f4" coll " [%0], da, db, %4, p;\n}\n" ::"r"(d),                  \
-        "r"(a), "r"(b), "n"(kDescHi), "r"(idesc_real()), "r"(acc)                                             \
-        : "memory")
-    if constexpr (kA == 0) HSDLA_MMA_REAL("");
-    else if constexpr (kA == 1) HSDLA_MMA_REAL(".collector::a::fill");
-    else HSDLA_MMA_REAL(".collector::a::lastuse");
-#undef HSDLA_MMA_REAL
+    asm volatile(
+        "{\n .reg .b64 da, db;\n .reg .pred p;\n .reg .b32 h;\n mov.b32 h, %3;\n mov.b64 da, {%1, h};\n"
+        " mov.b64 db, {%2, h};\n setp.ne.b32 p, %5, 0;\n"
+        " tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], da, db, %4, p;\n}\n" ::"r"(d),
+        "r"(a), "r"(b), "n"(kDescHi), "r"(idesc_real()), "r"(acc)
+        : "memory");
+}
+// ... with the left operand scaled by the factors at sa (those at sb are 1)
+__device__ __forceinline__ void mma_scaled(uint32_t d, uint32_t a, uint32_t b, uint32_t acc, uint32_t sa, uint32_t sb) {
+    asm volatile(
+        "{\n .reg .b64 da, db;\n .reg .pred p;\n .reg .b32 h;\n mov.b32 h, %3;\n mov.b64 da, {%1, h};\n"
+        " mov.b64 db, {%2, h};\n setp.ne.b32 p, %5, 0;\n"
+        " tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale.scale_vec::1X [%0], da, db, %4, [%6], [%7], p;\n}\n" ::"r"(d),
+        "r"(a), "r"(b), "n"(kDescHi), "r"(idesc_scaled()), "r"(acc), "r"(sa), "r"(sb)
+        : "memory");
+}
+// 32 columns of this warp's lane quadrant set to one word
+__device__ __forceinline__ void tmem_fill32(uint32_t taddr, uint32_t v) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,"
+        "%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};\n" ::"r"(taddr),
+        "r"(v)
+        : "memory");
 }
 __device__ __forceinline__ uint32_t desc_lo(uint32_t saddr) { return ((saddr & 0x3FFFF) >> 4) | (1u << 16); }
 
@@ -157,9 +166,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     unsigned char *abuf = smem, *bbuf = smem + kNA * kABytes;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < kRing; ++i) { mbar_init(&bars.full[i], 1); mbar_init(&bars.aempty[i], 1); }
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(&bars.bempty[i], 1);
+        for (int i = 0; i < kRing; ++i) { mbar_init(&bars.full[i], 1); mbar_init(&bars.aempty[i], 2); }
+        for (int i = 0; i < 2; ++i) mbar_init(&bars.bempty[i], 2);
+        for (int i = 0; i < kBufs; ++i) {
             mbar_init(&bars.tfull[i], 1);
             mbar_init(&bars.tempty[i], 2 * kEpi);
         }
@@ -176,9 +185,18 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     tc_fence_before();
     __syncthreads();
-    cluster_sync_all();          // barriers of both CTAs initialised before any remote arrival
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_sh;
+    if (warp >= 4 && warp < 8) {
+        const uint32_t t = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
+        tmem_fill32(t + kScaleOne, kOneBytes);
+        tmem_fill32(t + kScale32, k32Bytes);
+        asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();          // barriers and scale factors of both CTAs in place
+    tc_fence_after();
 
     if (warp < 4) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;\n" ::"n"(kRegsControl));
@@ -219,86 +237,123 @@ __global__ void __launch_bounds__(kThreads, 1)
                 mbar_drain_wait(&bars.aempty[q % kRing], (q / kRing) & 1, budget);
             for (uint32_t c = chunk > 2 ? chunk - 2 : 0; c < chunk; ++c)
                 mbar_drain_wait(&bars.bempty[c & 1], (c >> 1) & 1, budget);
-        } else if (warp == 1 && one && leader) {
-            // ------------------------------------------------ MMA issuer
+        } else if ((warp & 1) && one && leader) {
+            const uint32_t me = warp >> 1;           // the bands seq = me (mod 2) are this issuer's
+            // ------------------------------------------------ MMA issuers
             const uint32_t da0 = desc_lo(smem_u32(abuf)), db0 = desc_lo(smem_u32(bbuf));
             constexpr uint32_t kAStep = kABytes >> 4, kBStep = kBBytes >> 4;
             uint32_t n = 0, chunk = 0, seq = 0;      // the chunk's first batch; chunks; bands so far
-            const int halves = bands.halves, nbatch = (s + kBatch - 1) / kBatch, nbands = bands.n;
+            const int nbuf = bands.halves == 2 ? kBufs : 1, nbatch = (s + kBatch - 1) / kBatch, nbands = bands.n;
+            const int step = nbuf == 1 ? 1 : 2;
             bool ok = true, cut = false;
+            // (a tile's chunk count is fetched while the tile before runs)
+            int nkb = 0, ksl = 0, nkb1 = 0, ksl1 = 0;
+            if (pair < total_tiles) {
+                const RealJob &j = jobs[tile_list[pair].x];
+                nkb1 = (int)j.nkb;
+                ksl1 = j.ksteps_last;
+            }
             for (int64_t tile = pair; ok && tile < total_tiles; tile += npairs) {
-                const RealJob &j = jobs[tile_list[tile].x];
-                const int nkb = (int)j.nkb, ksl = j.ksteps_last;
+                nkb = nkb1;
+                ksl = ksl1;
+                if (tile + npairs < total_tiles) {
+                    const RealJob &j = jobs[tile_list[tile + npairs].x];
+                    nkb1 = (int)j.nkb;
+                    ksl1 = j.ksteps_last;
+                }
                 for (int kb = 0; ok && kb < nkb; ++kb, ++chunk, n += nbatch) {
                     const bool two = kb + 1 < nkb || ksl > 1;      // K steps of the chunk
                     const uint32_t db = db0 + (chunk & 1) * kBank * kBStep;
-                    int ready = 0;
-                    for (int b = 0; b < nbands; ++b, ++seq) {
+                    int ready = 0;                                 // left batches seen to have landed
+                    // this issuer's bands of the chunk; the last one also frees the planes (a chunk without a
+                    // band of its own is only signed off), all of them seen to have landed before, so that no
+                    // barrier is signed twice in a phase.  One buffer has one issuer: the other could not tell
+                    // its phases apart
+                    const int b0 = nbuf == 1 ? (me ? nbands : 0) : (int)((seq ^ me) & 1);
+                    const uint32_t seq0 = seq;
+                    seq += b0;
+                    if (b0 >= nbands) {
+                        for (; ready < nbatch; ++ready)
+                            if (!pwait(&bars.full[(n + ready) % kRing], ((n + ready) / kRing) & 1, 3, ready, (int)seq)) { ok = false; break; }
+                        if (!ok) break;
+                        for (int q = 0; q < nbatch; ++q) mma_commit_pair(&bars.aempty[(n + q) % kRing]);
+                        mma_commit_pair(&bars.bempty[chunk & 1]);
+                    }
+                    for (int b = b0; b < nbands; b += step, seq += step) {
                         const int T = bands.T[b];
-                        const bool last = b + 1 == nbands, pairs = bands.w[b] == 2;
-                        const int h = halves == 2 ? (int)(seq & 1) : 0;
-                        const uint32_t use = halves == 2 ? seq >> 1 : seq;
+                        const bool last = b + step >= nbands, pairs = bands.w[b] == 2;
+                        const uint32_t use = nbuf == 1 ? seq : seq / kBufs;
+                        const int h = (int)(seq - use * nbuf);
                         if (!pwait(&bars.tempty[h], (use & 1) ^ 1, 2, b, (int)seq)) { ok = false; break; }
-                        for (; ready <= (T - 2) / kBatch; ++ready)
+                        for (; ready <= (last ? nbatch - 1 : (T - 2) / kBatch); ++ready)
                             if (!pwait(&bars.full[(n + ready) % kRing], ((n + ready) / kRing) & 1, 3, ready, (int)seq)) { ok = false; break; }
                         if (!ok) break;
                         tc_fence_after();
                         cut = true;
-                        const uint32_t d1 = tmem_base + h * 2 * kRealTileN, d2 = d1 + kRealTileN;
-                        // left plane i with right planes T - 1 - i (diagonal T - 1) and T - i (diagonal T)
+                        const uint32_t d = tmem_base + h * kRealTileN, one = tmem_base + kScaleOne, x32 = tmem_base + kScale32;
+                        // left plane i with right planes T - 1 - i (diagonal T - 1, times 32) and T - i (diagonal T)
                         uint32_t dt = db + (T - 2) * kBStep;
                         for (int i0 = 1; i0 < T; i0 += kBatch) {
                             const int slot = (n + (i0 - 1) / kBatch) % kRing;
                             uint32_t da = da0 + slot * kBatch * kAStep;
                             const int i1 = min(i0 + kBatch, T);
-                            if (two && pairs && i0 + kBatch < T) {
-                                // a whole batch of pairs as straight-line code (1.102 -> 1.067 ms, as above)
+                            if (two && i0 + kBatch < T) {
+                                // a whole batch as straight-line code
+                                if (pairs) {
 #pragma unroll
-                                for (int q = 0; q < kBatch; ++q, da += kAStep, dt -= kBStep) {
-                                    const uint32_t acc = i0 + q > 1 ? 1u : 0u, dl = dt - kBStep;
-                                    mma_real<1>(d1, da, dl, acc);
-                                    mma_real<2>(d2, da, dt, acc);
-                                    mma_real<1>(d1, da + 2, dl + 2, 1u);
-                                    mma_real<2>(d2, da + 2, dt + 2, 1u);
+                                    for (int q = 0; q < kBatch; ++q, da += kAStep, dt -= kBStep) {
+                                        const uint32_t dl = dt - kBStep;
+                                        mma_scaled(d, da, dl, q > 0 || i0 > 1 ? 1u : 0u, x32, one);
+                                        mma_scaled(d, da, dt, 1u, one, one);
+                                        mma_scaled(d, da + 2, dl + 2, 1u, x32, one);
+                                        mma_scaled(d, da + 2, dt + 2, 1u, one, one);
+                                    }
+                                } else {
+#pragma unroll
+                                    for (int q = 0; q < kBatch; ++q, da += kAStep, dt -= kBStep) {
+                                        mma_real(d, da, dt, q > 0 || i0 > 1 ? 1u : 0u);
+                                        mma_real(d, da + 2, dt + 2, 1u);
+                                    }
                                 }
                             } else {
                                 for (int i = i0; i < i1; ++i, da += kAStep, dt -= kBStep) {
                                     const uint32_t acc = i > 1 ? 1u : 0u;
-                                    if (pairs && i + 1 < T) {
-                                        const uint32_t dl = dt - kBStep;
-                                        mma_real<1>(d1, da, dl, acc);
-                                        mma_real<2>(d2, da, dt, acc);
-                                        if (two) {
-                                            mma_real<1>(d1, da + 2, dl + 2, 1u);
-                                            mma_real<2>(d2, da + 2, dt + 2, 1u);
+                                    if (pairs) {
+                                        if (i + 1 < T) {
+                                            const uint32_t dl = dt - kBStep;
+                                            mma_scaled(d, da, dl, acc, x32, one);
+                                            if (two) mma_scaled(d, da + 2, dl + 2, 1u, x32, one);
                                         }
+                                        mma_scaled(d, da, dt, i + 1 < T ? 1u : acc, one, one);
+                                        if (two) mma_scaled(d, da + 2, dt + 2, 1u, one, one);
                                     } else {
-                                        mma_real<0>(d2, da, dt, acc);
-                                        if (two) mma_real<0>(d2, da + 2, dt + 2, 1u);
+                                        mma_real(d, da, dt, acc);
+                                        if (two) mma_real(d, da + 2, dt + 2, 1u);
                                     }
                                 }
                             }
                             if (last) mma_commit_pair(&bars.aempty[slot]);     // the batch's last use
                         }
+                        if (last)
+                            for (int q = (T + kBatch - 2) / kBatch; q < nbatch; ++q) mma_commit_pair(&bars.aempty[(n + q) % kRing]);
                         mma_commit_pair(&bars.tfull[h]);
                         if (last) mma_commit_pair(&bars.bempty[chunk & 1]);
                         cut = false;
                     }
+                    if (ok) seq = seq0 + nbands;
                 }
             }
             if (!ok) {
                 // wait (bounded) for the MMAs of a band cut short: the commit tracks all of them
                 if (cut) {
-                    const int h = halves == 2 ? (int)(seq & 1) : 0;
+                    const uint32_t use = nbuf == 1 ? seq : seq / kBufs, h = seq - use * nbuf;
                     mma_commit_pair(&bars.tfull[h]);
-                    mbar_drain_wait(&bars.tfull[h], (halves == 2 ? seq >> 1 : seq) & 1);
+                    mbar_drain_wait(&bars.tfull[h], use & 1);
                 }
             } else {
                 // both CTAs' drains of the last bands
-                for (uint32_t q = seq > 2 ? seq - 2 : 0; q < seq; ++q) {
-                    const int h = halves == 2 ? (int)(q & 1) : 0;
-                    const uint32_t use = halves == 2 ? q >> 1 : q;
-                    if (halves == 1 && q + 1 < seq) continue;
+                for (uint32_t q = seq > (uint32_t)nbuf ? seq - nbuf : 0; q < seq; ++q) {
+                    const uint32_t use = nbuf == 1 ? q : q / kBufs, h = q - use * nbuf;
                     mbar_drain_wait(&bars.tfull[h], use & 1);
                     mbar_drain_wait(&bars.tempty[h], use & 1);
                 }
@@ -313,47 +368,55 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint32_t tb = tmem_base + ((uint32_t)(q4 * 32) << 16) + cbeg;
         uint32_t seq = 0;
         bool ok = true;
-        const int halves = bands.halves;
-        for (int64_t tile = pair; ok && tile < total_tiles; tile += npairs) {
-            const int4 te = tile_list[tile];
-            const RealJob &j = jobs[te.x];
-            const int64_t nkb = j.nkb;
-            unsigned long long acc[kCols];
-            {
-                const unsigned long long a0 = 0ull - bands.bias * (unsigned long long)nkb;
-#pragma unroll
-                for (int c = 0; c < kCols; ++c) acc[c] = a0;
-            }
-            for (int64_t kb = 0; ok && kb < nkb; ++kb) {
-                for (int b = 0; b < bands.n; ++b, ++seq) {
-                    const int h = halves == 2 ? (int)(seq & 1) : 0;
-                    const uint32_t use = halves == 2 ? seq >> 1 : seq;
-                    if (!pwait(&bars.tfull[h], use & 1, 8, warp, (int)seq)) { ok = false; break; }
-                    tc_fence_after();
-                    // (a band of one diagonal has it in the second buffer)
-                    const uint32_t t1 = tb + (2 * h + 1) * kRealTileN, te = tempty_leader + h * 8;
-                    const uint32_t t0 = bands.w[b] == 2 ? t1 - kRealTileN : t1;
-                    const float g = bands.g[b], f = bands.f[b];
-                    const uint32_t mul = bands.mul[b];
-                    const int fold = bands.fold[b];
-                    if (fold == kFoldHigh) add_band<kFoldHigh>(acc, t0, t1, g, f, mul, te, lane);
-                    else if (fold == kFoldFloat) add_band<kFoldFloat>(acc, t0, t1, g, f, mul, te, lane);
-                    else add_band<kFoldInt>(acc, t0, t1, g, f, mul, te, lane);
-                }
-            }
-            if (!ok) break;
-            // the tile: lane = row, so a column's 32 values are 256 consecutive bytes
-            const int64_t row = (int64_t)te.y * kRealTileM + rank * (kRealTileM / 2) + q4 * 32 + lane;
-            const int64_t col0 = (int64_t)te.z * kRealTileN + cbeg;
-            const int64_t n = j.n, ldo = j.ldo;
-            const bool rok = row < j.m;
-            const int64_t cend = j.lower ? min(n, row + 1) : n;
-            long long *out = j.out + row + ldo * col0;
-            const int live = rok ? (int)max((int64_t)0, min((int64_t)kCols, cend - col0)) : 0;
+        const uint32_t nbuf = bands.halves == 2 ? kBufs : 1;
+        unsigned long long acc[kCols];
+        long long *out = nullptr;                 // the tile whose sums acc holds: where they go
+        int64_t ldo = 0;
+        int live = 0;
+        auto store = [&]() {
 #pragma unroll
             for (int c = 0; c < kCols; ++c)
                 if (c < live) out[ldo * c] = (long long)acc[c];
+        };
+        for (int64_t tile = pair; ok && tile < total_tiles; tile += npairs) {
+            const int4 te = tile_list[tile];
+            const RealJob &j = jobs[te.x];
+            const int nkb = (int)j.nkb;
+            for (int kb = 0; ok && kb < nkb; ++kb) {
+                for (int b = 0; b < bands.n; ++b, ++seq) {
+                    const uint32_t use = nbuf == 1 ? seq : seq / kBufs, h = seq - use * nbuf;
+                    if (!pwait(&bars.tfull[h], use & 1, 8, warp, (int)seq)) { ok = false; break; }
+                    tc_fence_after();
+                    const float f = bands.f[b];
+                    const uint32_t mul = bands.mul[b], t = tb + h * kRealTileN;
+                    uint32_t v[2][32];
+                    tmem_ld32(t, v[0]);
+                    tmem_ld32(t + 32, v[1]);
+                    tmem_ld_wait();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_remote(tempty_leader + h * 8);
+                    if (kb == 0 && b == 0) {
+                        // the tile before leaves only here, after this band has left its buffer: the MMAs
+                        // run ahead by one more band while it is being stored
+                        store();
+                        const unsigned long long a0 = 0ull - bands.bias * (unsigned long long)nkb;
+#pragma unroll
+                        for (int c = 0; c < kCols; ++c) acc[c] = a0;
+                        // lane = row, so a column's 32 values are 256 consecutive bytes
+                        const int64_t row = (int64_t)te.y * kRealTileM + rank * (kRealTileM / 2) + q4 * 32 + lane;
+                        const int64_t col0 = (int64_t)te.z * kRealTileN + cbeg;
+                        const int64_t cend = j.lower ? min(j.n, row + 1) : j.n;
+                        ldo = j.ldo;
+                        out = j.out + row + ldo * col0;
+                        live = row < j.m ? (int)max((int64_t)0, min((int64_t)kCols, cend - col0)) : 0;
+                    }
+                    if (bands.fold[b] == kFoldHigh) add_band<kFoldHigh>(acc, v, f, mul);
+                    else add_band<kFoldLow>(acc, v, f, mul);
+                }
+            }
         }
+        if (ok) store();
         __syncwarp();
     }
     tc_fence_before();
@@ -528,22 +591,19 @@ RealBands real_bands(int s, int width, int halves, int64_t kvalid) {
     int kb = 0;
     while (((int64_t)1 << kb) <= kvalid) ++kb;
     b.frac = 55 - kb;
-    // pairs, a single diagonal last: a band shorter than a drain holds up the band after the next, so
-    // the first is a pair too (one type of the 8000-column workload 1.128 -> 1.102 ms)
+    // Pairs while the largest |32 x0 + x1| of a chunk (64 products of at most 2^8 per digit pair) stays
+    // below 2^22, from the first diagonals on: theirs are the bands shorter than a drain.
     for (int t = 1, T; t < s + 1; t = T) {
         T = std::min(t + width, s + 1);
+        if (T - t == 2 && (int64_t)kRealKBlock * 256 * (32 * (T - 2) + T - 1) >= 1 << 22) T = t + 1;
         const int n = b.n++, sh = b.frac - 5 * (T - 2);
         b.T[n] = (int8_t)T;
         b.w[n] = (int8_t)(T - t);
-        // the largest |32 x0 + x1| of a chunk: 64 products of at most 2^8 per digit pair
-        const int64_t big = (int64_t)kRealKBlock * 256 * ((b.w[n] == 2 ? 32 * (T - 2) : 0) + T - 1);
-        const int r = sh < 0 ? -sh : 0;          // below the fixed point the sums are rounded to it
-        b.fold[n] = sh >= 32 ? kFoldHigh : (big >> r) < (1 << 22) ? kFoldFloat : kFoldInt;
+        b.fold[n] = sh >= 32 ? kFoldHigh : kFoldLow;
         b.mul[n] = sh >= 32 ? 1u << (sh - 32) : 1u << std::max(sh, 0);
-        b.g[n] = b.w[n] == 2 ? 32.0f : 0.0f;
-        b.f[n] = std::ldexp(1.0f, -r);
-        const uint32_t m = b.fold[n] == kFoldInt ? 33u * kMagicBits : kMagicBits;   // (far from 2^32's ends)
-        b.bias += b.fold[n] == kFoldHigh ? (unsigned long long)(m * b.mul[n]) << 32 : (unsigned long long)m * b.mul[n];
+        b.f[n] = std::ldexp(1.0f, std::min(sh, 0));       // below the fixed point the sums are rounded to it
+        b.bias += b.fold[n] == kFoldHigh ? (unsigned long long)(kMagicBits * b.mul[n]) << 32
+                                         : (unsigned long long)kMagicBits * b.mul[n];
     }
     return b;
 }

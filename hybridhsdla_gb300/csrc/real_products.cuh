@@ -34,25 +34,22 @@ struct RealJob {
 };
 
 // The order in which a chunk's digit pairs (i, j), i + j = t, run: bands of one or two adjacent
-// diagonals ending at T, ascending, and how a band's FP32 sums x0 (diagonal T - 1) and x1 (T) enter
-// the fixed-point sums.  With bits(x) those of the FP32 number x + 1.5 2^23 (an integer plus a
-// constant, |x| < 2^22):
-//     kFoldFloat: b = bits((32 x0 + x1) f)            (32 x0 + x1 exact: below 2^24; g = 32, or 0 for
-//                                                      a band of one diagonal)
-//     kFoldInt:   b = 32 bits(x0) + bits(x1)          (where 32 x0 + x1 may reach 2^22)
-// and sum += b mul (into the high word only for kFoldHigh, kFoldFloat's form for the first bands);
-// the constants are taken off at the start (bias per chunk).
-enum { kFoldHigh = 0, kFoldFloat = 1, kFoldInt = 2 };
+// diagonals ending at T, ascending, each summed in one FP32 accumulator x (diagonal T - 1 times 32,
+// diagonal T) that enters the fixed-point sums as
+//     sum += bits(x f) mul        bits(y): those of the FP32 number y + 1.5 2^23 (an integer plus a
+//                                 constant, |y| < 2^22)
+// (kFoldHigh: into the high word only); the constants are taken off at the start (bias per chunk).
+enum { kFoldHigh = 0, kFoldLow = 1 };
 struct RealBands {
     int32_t s;                         // digits per operand
     int32_t frac;                      // fraction bits of the fixed-point sums
-    int32_t halves;                    // TMEM halves the bands alternate between (1: they wait for each other)
+    int32_t halves;                    // 2: the bands alternate between TMEM buffers, 1: they wait for each other
     int32_t n;                         // bands
     unsigned long long bias;
     int8_t T[kRealMaxSlices];          // last diagonal of each band
     int8_t w[kRealMaxSlices];          // its diagonals (1-2)
     int8_t fold[kRealMaxSlices];
-    float g[kRealMaxSlices], f[kRealMaxSlices];
+    float f[kRealMaxSlices];
     uint32_t mul[kRealMaxSlices];
 };
 // Bands of at most `width` diagonals for s digits and a contraction over kvalid digits.

@@ -108,3 +108,23 @@ def test_combine_over_type_counts(ctx, monkeypatch, precision, types):
             assert fro < 1e-13 and mx < 1e-13, (nm, types, fro, mx)
             fro, mx = oracle.lower_errors(C, R)
             assert fro < 1e-13 and mx < 1e-13, (nm, types, fro, mx)
+
+
+@pytest.mark.parametrize("slices", [2, 3, 4, 6, 8, 9, 10, 11, 12])
+@pytest.mark.parametrize("halves,merge", [("2", "1"), ("2", "0"), ("1", "1"), ("1", "0")])
+def test_bands_and_issuers(ctx, monkeypatch, slices, halves, merge):
+    """Every number of digits (bands of one and two diagonals, odd and even counts of them, chunks in
+    which an issuer has no band) with one accumulator and with all of them: the tolerance grows by 2^5 per
+    digit left out."""
+    monkeypatch.setenv("HSDLA_PAIR_HALVES", halves)
+    monkeypatch.setenv("HSDLA_MERGE", merge)
+    cfg = dict(cell=(10.0, 10.5, 11.0), atoms=5, types=2, rmt=2.0, min_sep=3.9, lmax=5,
+               kpts=[(0.1, 0.2, 0.3)], n_g=700, seed=slices)
+    s = synth.make_system(cfg)
+    ((H, S),), rep = ctx.create_hs(s, precision="ozaki", num_slices=slices)
+    assert rep["tile_halves"] == int(halves) and rep["merged_units"] == int(merge)
+    Hr, Sr = oracle.reference_hs(s, s.kpoints[0])
+    tol = 1e-13 * 32.0 ** max(0, 11 - slices)
+    for X, R, nm in ((H, Hr, "H"), (S, Sr, "S")):
+        fro, mx = oracle.lower_errors(X, R)
+        assert fro < tol and mx < tol, (nm, slices, fro, mx)
