@@ -165,6 +165,8 @@ struct hsdla_plan {
         int blocks = 0;          // ... in column blocks while the products of the next ran (0: after them)
     };
     Download *dl = nullptr;
+    void *split = nullptr;           // memory for splitting the S/H products (hsdla_contract_ab), or null
+    int64_t split_bytes = 0;
     double est_err = 0.0;            // autotuner's predicted relative error
     int launches = 0;
     bool tiles_tuned = false;        // the S/H tile configuration came from the tile tuner
@@ -392,6 +394,18 @@ int ctx_workspace(hsdla_context *ctx, int64_t bytes, void **out) {
     ctx->ws_bytes = bytes;
     *out = ctx->ws;
     return HSDLA_OK;
+}
+
+// ctx_workspace with `extra` bytes behind the `bytes` (rounded to 1 KB) that a call needs: `tail` gets them,
+// or null where they cannot be had or the context has a cap (a capped one keeps to what it needs).
+int ctx_workspace_tail(hsdla_context *ctx, int64_t bytes, int64_t extra, void **out, void **tail) {
+    *tail = nullptr;
+    bytes = (bytes + 1023) / 1024 * 1024;
+    if (extra > 0 && ctx->mem_cap <= 0 && ctx_workspace(ctx, bytes + extra, out) == HSDLA_OK) {
+        *tail = reinterpret_cast<char *>(*out) + bytes;
+        return HSDLA_OK;
+    }
+    return ctx_workspace(ctx, bytes, out);
 }
 
 bool finite_all(const double *p, int64_t n) {
@@ -1368,6 +1382,7 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
             d.ntypes = pl->ntypes; d.set_type = pl->set_type.data(); d.d_set_type = pl->dsys.set_type;
             d.w = pl->w; d.Tfull = pl->Tfull; d.atom_type = pl->atom_type.data();
             d.panels = pl->panels;
+            d.split = pl->split; d.split_bytes = pl->split_bytes;
             d.sf = pl->sf; d.wt = pl->wt; d.TR = pl->TR; d.sf_tab = pl->sf_tab; d.tbatch = pl->tbatch;
             char *oz_ws = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(p) + 1023) & ~uintptr_t(1023));
             int rc = ozaki_group_prepare(pl->oz, d, kb, oz_ws, g.persist, st, &g.oz);
@@ -2047,7 +2062,9 @@ int hsdla_contract_ab(hsdla_context *ctx, int32_t L, int32_t a, int64_t G, const
         if (rc) return done(set_err(ctx, rc, "bad slice count"));
     }
     form_groups(pl, workspace_budget(ctx));
-    rc = ctx_workspace(ctx, hsdla_plan_workspace_bytes(pl), &ws);
+    if (pl->opts.precision == HSDLA_PREC_OZAKI_FP8)
+        pl->split_bytes = ozaki_split_bytes(pl->oz.num_slices, (twoL + 15) / 16 * 16 * a, G, 2);
+    rc = ctx_workspace_tail(ctx, hsdla_plan_workspace_bytes(pl), pl->split_bytes, &ws, &pl->split);
     if (rc) return done(rc);
     rc = prepare_groups(pl, ws, st);
     if (rc) return done(rc);
@@ -2314,12 +2331,13 @@ int hsdla_zherkx_lower(hsdla_context *ctx, int32_t precision, int32_t num_slices
         OzakiPlan oz{};
         int rc = ozaki_plan_init(oz, num_slices, 1e-13);
         if (rc) return set_err(ctx, rc, "bad slice count");
-        void *ws = nullptr;
-        rc = ctx_workspace(ctx, ozaki_herkx_workspace(oz.num_slices, k, n), &ws);
+        void *ws = nullptr, *split = nullptr;
+        const int64_t extra = ozaki_split_bytes(oz.num_slices, k, n, 1);
+        rc = ctx_workspace_tail(ctx, ozaki_herkx_workspace(oz.num_slices, k, n), extra, &ws, &split);
         if (rc) return rc;
         int nl = 0;
         rc = ozaki_herkx(oz, reinterpret_cast<const double2 *>(dP), ldp, reinterpret_cast<const double2 *>(dQ), ldq,
-                         dw, k, n, reinterpret_cast<double2 *>(dOut), ldo, ws, st, &nl);
+                         dw, k, n, reinterpret_cast<double2 *>(dOut), ldo, ws, st, &nl, split, extra);
         if (rc) { ozaki_plan_release(oz); return set_err(ctx, rc, "Ozaki zherkx failed: %s", ozaki_last_error()); }
         cudaError_t e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) { ozaki_plan_release(oz); return set_err(ctx, HSDLA_ERR_CUDA, "zherkx ozaki: %s", cudaGetErrorString(e)); }
@@ -2402,8 +2420,9 @@ int plugin_contract(hsdla_context *ctx, int kind, int32_t precision, int32_t num
     const int64_t oR = slot(product && !direct, n * n * e16);
     const int64_t oJ = slot(product && precision == HSDLA_PREC_FP64, sizeof(Fp64Job));
     const int64_t oZ = slot(product && precision == HSDLA_PREC_OZAKI_FP8, s ? ozaki_herkx_workspace(s, K, n) : 0);
-    void *wsv = nullptr;
-    int rc = ctx_workspace(ctx, std::max<int64_t>(off, 1024), &wsv);
+    void *wsv = nullptr, *split = nullptr;
+    const int64_t extra = product && s ? ozaki_split_bytes(s, K, n, 1) : 0;
+    int rc = ctx_workspace_tail(ctx, std::max<int64_t>(off, 1024), extra, &wsv, &split);
     if (rc) return rc;
     char *ws = reinterpret_cast<char *>(wsv);
     // ---- stage host memory
@@ -2466,7 +2485,7 @@ int plugin_contract(hsdla_context *ctx, int kind, int32_t precision, int32_t num
             rc = ozaki_plan_init(ctx->plugin_oz, s, 1e-13);
             if (rc) return set_err(ctx, rc, "%s: %s", nm, ozaki_last_error());
             int nl = 0;
-            rc = ozaki_herkx(ctx->plugin_oz, P, ldp, Q, ldq, nullptr, K, n, R, ldr, ws + oZ, st, &nl);
+            rc = ozaki_herkx(ctx->plugin_oz, P, ldp, Q, ldq, nullptr, K, n, R, ldr, ws + oZ, st, &nl, split, extra);
             if (rc) return set_err(ctx, rc, "%s: %s", nm, ozaki_last_error());
         }
     }

@@ -515,7 +515,8 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     oz_pair_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap map1,
                    const __grid_constant__ CUtensorMap map2, const __grid_constant__ CUtensorMap map3,
                    const OzJob *__restrict__ jobs, int num_jobs, int64_t total_tiles, int s, int *err,
-                   const int4 *__restrict__ tile_list, int *progress, int sync_every, int slack) {
+                   const int4 *__restrict__ tile_list, int *progress, int sync_every, int slack,
+                   const int4 *__restrict__ parts, double2 *slabs) {
     constexpr int kStages = kPairStages;
     constexpr int kStageB = kStageBytes;
     constexpr int kN = kPairTile;
@@ -569,6 +570,8 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     const uint32_t tmem_base = tmem_base_sh;
     const uint32_t full0_leader = mapa_rank(smem_u32(&bars.full[0]), 0);
     const uint32_t tempty_leader = mapa_rank(smem_u32(&bars.tempty), 0);
+    // the steps (digit pair and k-block, in the order of the loops) [x, y) of an entry, and its slab z
+    auto part_of = [&](int64_t tile) { return parts ? parts[tile] : make_int4(0, INT_MAX, -1, 0); };
     const int64_t half = (int64_t)rank * (kPairTile / 2);     // this CTA's rows of a tile, and of the right operand
 
     if (warp == 0) {
@@ -582,13 +585,18 @@ __global__ void __launch_bounds__(kPairThreads, 1)
                 int64_t tm, tn;
                 const OzJob &j = resolve_tile(jobs, num_jobs, tile_list, tile, tm, tn);
                 const CUtensorMap *lm = map_of(j.lmap), *rm = map_of(j.rmap);
+                const int4 part = part_of(tile);
+                int step = 0;
                 for (int t = 2; ok && t <= s + 1; ++t) {
                     const int ilo = max(1, t - s), ihi = min(s, t - 1);
                     const int64_t ck = chunk_kblocks(ihi - ilo + 1);
                     for (int64_t cb = 0; ok && cb < j.nkb; cb += ck) {
                         const int64_t ce = min(j.nkb, cb + ck);
+                        const int end = step + (int)(ce - cb) * (ihi - ilo + 1);
+                        if (end <= part.x || step >= part.y) { step = end; continue; }
                         for (int64_t kb = cb; ok && kb < ce; ++kb) {
-                            for (int i = ilo; i <= ihi; ++i) {
+                            for (int i = ilo; i <= ihi; ++i, ++step) {
+                                if (step < part.x || step >= part.y) continue;
                                 const int jj = t - i;
                                 if (leader && progress && issued > 0 && issued % sync_every == 0 &&
                                     !grid_lockstep(progress, (int)npairs, (int)(issued / sync_every), &abort_flag, err,
@@ -636,16 +644,21 @@ __global__ void __launch_bounds__(kPairThreads, 1)
                 // the job's fields in registers: the asm statements below clobber memory, and the
                 // issuer must not reload them between MMAs
                 const int64_t jnkb = j.nkb;
+                const int4 part = part_of(tile);
+                int step = 0;
                 for (int t = 2; ok && t <= s + 1; ++t) {
                     const int ilo = max(1, t - s), ihi = min(s, t - 1);
                     const int64_t ck = chunk_kblocks(ihi - ilo + 1);
                     for (int64_t cb = 0; ok && cb < jnkb; cb += ck) {
                         const int64_t ce = min(jnkb, cb + ck);
+                        const int end = step + (int)(ce - cb) * (ihi - ilo + 1);
+                        if (end <= part.x || step >= part.y) { step = end; continue; }
                         if (!pwait(&bars.tempty, (uint32_t)((unit & 1) ^ 1), 2, stage, (int)unit)) { ok = false; break; }
                         tc_fence_after();
                         bool first = true;
                         for (int64_t kb = cb; ok && kb < ce; ++kb) {
-                            for (int i = ilo; i <= ihi; ++i) {
+                            for (int i = ilo; i <= ihi; ++i, ++step) {
+                                if (step < part.x || step >= part.y) continue;
                                 if (!pwait(&bars.full[stage], phase, 3, stage, (int)unit)) { ok = false; break; }
                                 tc_fence_after();
                                 const uint32_t a_re = sbase + stage * kStageB, a_im = a_re + 16384;
@@ -718,10 +731,26 @@ __global__ void __launch_bounds__(kPairThreads, 1)
             int64_t tm, tn;
             const OzJob &j = resolve_tile(jobs, num_jobs, tile_list, tile, tm, tn);
             const int64_t r0 = tm * kPairTile + half + q * 32, row = r0 + lane;
-            const int64_t m = j.m, n = j.n, ldo = j.ldo, nkb = j.nkb;
-            const bool lower = j.lower != 0, accum = j.accum != 0;
+            const int64_t m = j.m, n = j.n;
+            const int nkb = (int)j.nkb;
+            const bool lower = j.lower != 0;
             const int erow = row < m ? j.el[row] : 0;
+            // a later part of a tile goes to a slab of its own
+            int64_t ldo = j.ldo;
             double2 *out = j.out;
+            bool fresh = j.accum == 0;
+            int from = 0, to = INT_MAX;
+            if (parts) {
+                const int4 part = parts[tile];
+                from = part.x;
+                to = part.y;
+                if (part.z >= 0) {
+                    ldo = kPairTile;
+                    out = slabs + (int64_t)part.z * kPairTile * kPairTile - tm * kPairTile - tn * kPairTile * ldo;
+                    fresh = true;
+                }
+            }
+            int step = 0;
             // The tile's column exponents, loaded once for all its units: lane l holds column
             // tn*256 + cbeg + 32c + l of chunk c in ex[c], with each chunk's
             // range for the fast-path test.  The registers rotate after each chunk, so the current
@@ -739,13 +768,19 @@ __global__ void __launch_bounds__(kPairThreads, 1)
                 exhi[x] = __reduce_max_sync(0xffffffffu, ex[x]);
             }
             for (int t = 2; ok && t <= s + 1; ++t) {
-                const int64_t ck = chunk_kblocks(min(s, t - 1) - max(1, t - s) + 1);
+                const int cnt = min(s, t - 1) - max(1, t - s) + 1;
+                const int ck = (int)min((int64_t)nkb, chunk_kblocks(cnt));
                 const int kb = 2 - 5 * t + erow;
                 // 2^(kb + e_col) as an FP64 exponent bias: the row's part plus e_col << 20
                 const uint32_t rbias = pow2_ebias(kb);
-                for (int64_t cb = 0; ok && cb < nkb; cb += ck) {
-                    const bool first = (t == 2 && cb == 0) && !accum;
-                    const uint64_t pol = (t == s + 1 && cb + ck >= nkb) ? pol_first : pol_last;
+                for (int cb = 0; ok && cb < nkb; cb += ck) {
+                    const int end = step + (min(nkb, cb + ck) - cb) * cnt;
+                    const bool none = end <= from || step >= to;
+                    step = end;
+                    if (none) continue;
+                    const bool first = fresh;
+                    fresh = false;
+                    const uint64_t pol = ((t == s + 1 && cb + ck >= nkb) || end >= to) ? pol_first : pol_last;
                     {
                         if (!pwait(&bars.tfull, (uint32_t)(unit & 1), 4, warp, (int)unit)) { ok = false; break; }
                         tc_fence_after();
@@ -830,6 +865,29 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;\n" ::"r"(tmem_base) : "memory");
+    }
+}
+
+// The slabs of a split tile into the output, in the order of its parts (adds: job, tile row, tile
+// column, first slab; then their number).  A warp's lanes walk rows.
+__global__ void __launch_bounds__(kPairTile) oz_slab_add_kernel(const OzJob *__restrict__ jobs, const int4 *__restrict__ adds,
+                                                                const double2 *__restrict__ slabs) {
+    const int4 a = adds[2 * blockIdx.x];
+    const int count = adds[2 * blockIdx.x + 1].x;
+    const OzJob &j = jobs[a.x];
+    const int64_t row = (int64_t)a.y * kPairTile + threadIdx.x;
+    if (row >= j.m) return;
+    for (int c = blockIdx.y; c < kPairTile; c += gridDim.y) {
+        const int64_t col = (int64_t)a.z * kPairTile + c;
+        if (col >= j.n || (j.lower && row < col)) break;
+        const double2 *p = slabs + ((int64_t)a.w * kPairTile + c) * kPairTile + threadIdx.x;
+        double2 v = j.out[row + j.ldo * col];
+        for (int q = 0; q < count; ++q, p += kPairTile * kPairTile) {
+            const double2 x = __ldcs(p);
+            v.x += x.x;
+            v.y += x.y;
+        }
+        j.out[row + j.ldo * col] = v;
     }
 }
 
@@ -1433,6 +1491,16 @@ struct OzPanel {
     int64_t tiles_t = 0;
 };
 
+// A split of the tiles that do not fill a wave of CTA pairs: each pair takes an equal run of their steps
+// (a step: one digit pair of one k-block), so a tile is made by one pair or by several.  The part with a
+// tile's first step adds into the output as an unsplit tile does, the others into slabs of their own,
+// which oz_slab_add_kernel adds in the order of the parts (results repeat bit for bit).
+struct PairSplit {
+    int4 *list = nullptr, *parts = nullptr, *adds = nullptr;
+    double2 *slabs = nullptr;
+    int64_t total = 0;             // entries
+    int pairs = 0, n_adds = 0;     // CTA pairs; split tiles
+};
 struct OzGroup {
     int s = 0, nk = 0, panels = 1;
     bool hoist = false;
@@ -1450,6 +1518,7 @@ struct OzGroup {
     int *d_progress = nullptr;
     int *d_err = nullptr;
     bool pair = false;          // S/H on CTA-pair tiles
+    PairSplit split;
     bool sf = false;            // structure-factor form, on real rows:
     RealSliceTab rM, rX;        // the slicing of R (and R diag(w)) and of Z'
     RealJob *d_rjobs_t = nullptr, *d_rjobs_sh = nullptr;   // T application; 3 nk products per type
@@ -1486,34 +1555,15 @@ int64_t group_rows(const std::vector<int64_t> &G) {
     return r + kTileM;
 }
 
-int upload_schedule(std::vector<OzJob> &jobs, OzJob *d_jobs, int4 *d_list, int64_t &tiles, int64_t tile = kTileN) {
-    int64_t total = 0;
-    for (auto &j : jobs) {
-        j.tiles_n = (j.n + tile - 1) / tile;
-        j.tile_begin = total;
-        total += job_tiles(j, tile);
-    }
-    std::vector<int4> list;
-    build_schedule(jobs, list, tile);
-    if ((int64_t)list.size() != total) { g_oz_err = "tile schedule size mismatch"; return HSDLA_ERR_ARG; }
-    cudaError_t e = cudaMemcpy(d_jobs, jobs.data(), sizeof(OzJob) * jobs.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && total > 0)
-        e = cudaMemcpy(d_list, list.data(), sizeof(int4) * list.size(), cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) { g_oz_err = cudaGetErrorString(e); return HSDLA_ERR_CUDA; }
-    tiles = total;
-    return HSDLA_OK;
-}
+constexpr int64_t kSlabBytes = (int64_t)kPairTile * kPairTile * sizeof(double2);
 
 // Launch of a prepared pair-tile job table: clusters of two CTAs, one per SM, as many pairs as
 // can be resident (at most one per tile); cooperative when the lockstep slots are given.
-cudaError_t launch_pair(const CUtensorMap *maps, int s, int *d_err, const OzJob *d_jobs, int n_jobs, int64_t total,
-                        const int4 *d_list, int *d_progress, cudaStream_t st) {
-    if (total <= 0) return cudaSuccess;
+// With a split (make_split) its entries run in place of the tiles, then the slabs are added up.
+cudaError_t pair_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, int &max_out, cudaStream_t st) {
     const size_t smem = kPairSmem;
     cudaError_t e = cudaFuncSetAttribute(oz_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = 2;
     at[0].val.clusterDim.y = 1;
@@ -1532,7 +1582,21 @@ cudaError_t launch_pair(const CUtensorMap *maps, int s, int *d_err, const OzJob 
         if (nc < 1) return cudaErrorInvalidConfiguration;
         max_pairs = nc;
     }
-    const int64_t pairs = std::min<int64_t>(total, max_pairs);
+    max_out = max_pairs;
+    return cudaSuccess;
+}
+
+cudaError_t launch_pair(const CUtensorMap *maps, int s, int *d_err, const OzJob *d_jobs, int n_jobs, int64_t total,
+                        const int4 *d_list, int *d_progress, cudaStream_t st, const PairSplit *split = nullptr) {
+    if (total <= 0) return cudaSuccess;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[2];
+    int max_pairs = 0;
+    cudaError_t e = pair_config(cfg, at, max_pairs, st);
+    if (e != cudaSuccess) return e;
+    const bool cut = split && split->n_adds > 0;
+    if (cut) { total = split->total; d_list = split->list; }
+    const int64_t pairs = cut ? split->pairs : std::min<int64_t>(total, max_pairs);
     cfg.gridDim = dim3((unsigned)(2 * pairs));
     const bool lockstep = d_progress && pairs > 1 && pairs <= kProgressCap && env_int("HSDLA_LOCKSTEP", 1) != 0;
     if (lockstep) {
@@ -1553,8 +1617,112 @@ cudaError_t launch_pair(const CUtensorMap *maps, int s, int *d_err, const OzJob 
     // lockstep epoch (stages) and how many epochs a pair may lead the slowest one
     static const int sync_every = (int)std::max<int64_t>(8, env_int("HSDLA_SYNC_EVERY", kSyncEvery));
     static const int slack = (int)std::max<int64_t>(1, env_int("HSDLA_SYNC_SLACK", 1));
-    return cudaLaunchKernelEx(&cfg, oz_pair_kernel, maps[0], maps[1], maps[2], maps[3], d_jobs, n_jobs, total,
-                              s, d_err, d_list, lockstep ? d_progress : (int *)nullptr, sync_every, slack);
+    e = cudaLaunchKernelEx(&cfg, oz_pair_kernel, maps[0], maps[1], maps[2], maps[3], d_jobs, n_jobs, total,
+                           s, d_err, d_list, lockstep ? d_progress : (int *)nullptr, sync_every, slack,
+                           cut ? (const int4 *)split->parts : (const int4 *)nullptr, cut ? split->slabs : (double2 *)nullptr);
+    if (e != cudaSuccess || !cut) return e;
+    oz_slab_add_kernel<<<dim3((unsigned)split->n_adds, 32), kPairTile, 0, st>>>(d_jobs, split->adds, split->slabs);
+    return cudaGetLastError();
+}
+
+// The rule: of N tiles of `steps` steps (~1.3 us each) on np pairs, the R = N mod np beyond whole waves are
+// cut where that shortens the last wave by at least kSplitGain steps and a quarter; below, the slabs (1 MB
+// each, written and read), the additional drains and operand panels that fewer pairs share at a time take
+// as much.  Whole and cut, us: 3 tiles of 66 steps (57 saved) 488 and 383 of a call, 21 of 66 (47 saved) 524 and
+// 484, 78 of 66 (57 saved) 747 and 662, 21 of 726 (525 saved) 1255 and 729; but 36 of 66 (34 saved) 550 and
+// 553, 66 of 528 (69 saved) 1155 and 1173.  Parts have at least kSplitMin steps.
+constexpr int64_t kSplitGain = 40, kSplitMin = 8;
+struct SplitRule {
+    int np = 0;
+    int64_t R = 0, P = 0, per = 0;       // tiles cut, over P pairs, steps of each
+};
+bool split_rule(int64_t N, int64_t steps, SplitRule &r) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[2];
+    if (N < 1 || steps > INT_MAX || !use_pair() || pair_config(cfg, at, r.np, nullptr) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    r.R = N % r.np;
+    r.P = std::min<int64_t>(r.np, r.R * steps / kSplitMin);
+    if (r.R == 0 || r.P <= r.R) return false;
+    r.per = (r.R * steps + r.P - 1) / r.P;
+    return steps - r.per >= std::max(kSplitGain, steps / 4);
+}
+
+// `mem`, `bytes`: as ozaki_split_bytes says, or none (no split).
+int make_split(PairSplit &sp, const std::vector<int4> &list, int64_t steps, void *mem, int64_t bytes) {
+    sp = PairSplit();
+    SplitRule rule;
+    const int64_t N = (int64_t)list.size();
+    if (!mem || !split_rule(N, steps, rule)) return HSDLA_OK;
+    const int64_t np = rule.np, W = N / np, R = rule.R, P = rule.P, per = rule.per;
+    std::vector<std::vector<std::pair<int4, int4>>> of(P);
+    std::vector<int4> adds;
+    int slab = 0;
+    size_t rounds = 0;
+    for (int64_t p = 0; p < P; ++p) {
+        int64_t a = std::min(p * per, R * steps);
+        const int64_t b = std::min(a + per, R * steps);
+        for (; a < b;) {
+            const int64_t r = a / steps, lo = a - r * steps, hi = std::min(steps, b - r * steps);
+            const int4 e = list[W * np + r];
+            if (lo > 0) {
+                if (adds.empty() || adds[adds.size() - 2].x != e.x || adds[adds.size() - 2].y != e.y || adds[adds.size() - 2].z != e.z) {
+                    adds.push_back(make_int4(e.x, e.y, e.z, slab));
+                    adds.push_back(make_int4(0, 0, 0, 0));
+                }
+                ++adds.back().x;
+            }
+            of[p].push_back({e, make_int4((int)lo, (int)hi, lo > 0 ? slab++ : -1, 0)});
+            a = r * steps + hi;
+        }
+        rounds = std::max(rounds, of[p].size());
+    }
+    const int64_t G = W > 0 ? np : P, total = (W + (int64_t)rounds) * G;
+    if (slab * kSlabBytes + 32 * total + 16 * (int64_t)adds.size() > bytes) return HSDLA_OK;
+    std::vector<int4> up(2 * total, make_int4(0, 0, 0, 0));
+    for (int64_t i = 0; i < total; ++i) up[total + i] = make_int4(0, 0, -1, 0);
+    for (int64_t i = 0; i < W * np; ++i) {
+        up[i] = list[i];
+        up[total + i] = make_int4(0, INT_MAX, -1, 0);
+    }
+    for (int64_t p = 0; p < P; ++p)
+        for (size_t q = 0; q < of[p].size(); ++q) {
+            const int64_t i = (W + (int64_t)q) * G + p;
+            up[i] = of[p][q].first;
+            up[total + i] = of[p][q].second;
+        }
+    up.insert(up.end(), adds.begin(), adds.end());
+    sp.slabs = reinterpret_cast<double2 *>(mem);
+    sp.list = reinterpret_cast<int4 *>(reinterpret_cast<char *>(mem) + slab * kSlabBytes);
+    sp.parts = sp.list + total;
+    sp.adds = sp.parts + total;
+    sp.total = total;
+    sp.pairs = (int)G;
+    sp.n_adds = (int)adds.size() / 2;
+    const cudaError_t e = cudaMemcpy(sp.list, up.data(), sizeof(int4) * up.size(), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) { g_oz_err = cudaGetErrorString(e); return HSDLA_ERR_CUDA; }
+    return HSDLA_OK;
+}
+
+int upload_schedule(std::vector<OzJob> &jobs, OzJob *d_jobs, int4 *d_list, int64_t &tiles, int64_t tile = kTileN,
+                    PairSplit *split = nullptr, int64_t steps = 0, void *split_mem = nullptr, int64_t split_size = 0) {
+    int64_t total = 0;
+    for (auto &j : jobs) {
+        j.tiles_n = (j.n + tile - 1) / tile;
+        j.tile_begin = total;
+        total += job_tiles(j, tile);
+    }
+    std::vector<int4> list;
+    build_schedule(jobs, list, tile);
+    if ((int64_t)list.size() != total) { g_oz_err = "tile schedule size mismatch"; return HSDLA_ERR_ARG; }
+    cudaError_t e = cudaMemcpy(d_jobs, jobs.data(), sizeof(OzJob) * jobs.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && total > 0)
+        e = cudaMemcpy(d_list, list.data(), sizeof(int4) * list.size(), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) { g_oz_err = cudaGetErrorString(e); return HSDLA_ERR_CUDA; }
+    tiles = total;
+    return split ? make_split(*split, list, steps, split_mem, split_size) : HSDLA_OK;
 }
 
 // Launch of a prepared job table (no host synchronisation; capturable).
@@ -1593,10 +1761,21 @@ cudaError_t launch_prepared(const CUtensorMap *maps, int s, int *d_err, const Oz
 
 }  // namespace
 
+// Memory with which ozaki_herkx, or a group, splits the tiles of a partial last wave: `jobs` lower products
+// of n columns over K rows (0: they would not be split).
+int64_t ozaki_split_bytes(int s, int64_t K, int64_t n, int64_t jobs) {
+    const int64_t T = (n + kPairTile - 1) / kPairTile, N = jobs * T * (T + 1) / 2;
+    SplitRule r;
+    if (!split_rule(N, round_up(std::max<int64_t>(K, 1), kKBlock) / kKBlock * s * (s + 1) / 2, r)) return 0;
+    // at most P - 1 parts do not begin a tile; entries of whole waves and of up to P tiles a pair in the last
+    return r.P * kSlabBytes + round_up(32 * (N + (2 + (r.R + r.P - 1) / r.P) * r.np) + 32 * r.R, 1024);
+}
+
 // P^H diag(w) Q (lower triangle) for one pair of K x n operands: the contraction behind
 // hsdla_zherkx_lower and the BLAS-shaped plugin.
 int ozaki_herkx(OzakiPlan &oz, const double2 *P, int64_t ldp, const double2 *Q, int64_t ldq, const double *w,
-                int64_t K, int64_t n, double2 *out, int64_t ldo, void *ws, cudaStream_t st, int *launches) {
+                int64_t K, int64_t n, double2 *out, int64_t ldo, void *ws, cudaStream_t st, int *launches, void *split,
+                int64_t split_size) {
     const int s = oz.num_slices;
     const int64_t Kpad = round_up(std::max<int64_t>(K, 1), kKBlock);
     Arena ar{reinterpret_cast<char *>(ws)};
@@ -1623,9 +1802,10 @@ int ozaki_herkx(OzakiPlan &oz, const double2 *P, int64_t ldp, const double2 *Q, 
         // CTA-pair 256 x 256 tiles, one exact unit per diagonal and K chunk, pairs in lockstep
         int *d_progress = ar.take<int>(kProgressCap);
         int64_t tiles = 0;
-        rc = upload_schedule(jobs, d_jobs, d_list, tiles, kPairTile);
+        PairSplit sp;
+        rc = upload_schedule(jobs, d_jobs, d_list, tiles, kPairTile, &sp, j.nkb * s * (s + 1) / 2, split, split_size);
         if (rc) return rc;
-        const cudaError_t el = launch_pair(maps, s, oz.d_error, d_jobs, 1, tiles, d_list, d_progress, st);
+        const cudaError_t el = launch_pair(maps, s, oz.d_error, d_jobs, 1, tiles, d_list, d_progress, st, &sp);
         if (el != cudaSuccess) { g_oz_err = cudaGetErrorString(el); return HSDLA_ERR_CUDA; }
     } else {
         rc = launch_gemm(jobs, maps, s, oz.d_error, d_jobs, st, nullptr, nullptr, d_list);
@@ -2069,7 +2249,8 @@ int ozaki_group_prepare(OzakiPlan &oz, const OzGroupDesc &d, const std::vector<O
             }
         // the tile list is the same for every panel: upload it once
         if (pi == 0) {
-            rc = upload_schedule(jsh, g->d_jobs_sh, g->d_list_sh, g->tiles_sh, tile);
+            rc = upload_schedule(jsh, g->d_jobs_sh, g->d_list_sh, g->tiles_sh, tile, &g->split, jsh[0].nkb * s * (s + 1) / 2,
+                                 g->pair && g->panels == 1 ? d.split : nullptr, d.split_bytes);
             if (rc) return fail(rc);
         } else {
             int64_t total = 0;
@@ -2315,7 +2496,7 @@ int ozaki_group_run(OzGroup *g, const DevSystem &sys, const KTable &ktab, cudaSt
         const OzJob *jobs = g->d_jobs_sh + (int64_t)g->n_jobs_sh * pi;
         if (e == cudaSuccess)
             e = g->pair ? launch_pair(g->maps_sh, g->s, g->d_err, jobs, g->n_jobs_sh, g->tiles_sh, g->d_list_sh,
-                                      g->d_progress, st)
+                                      g->d_progress, st, &g->split)
                         : launch_prepared(g->maps_sh, g->s, g->d_err, jobs, g->n_jobs_sh, g->tiles_sh, g->d_list_sh,
                                           g->d_progress, st);
         nl += 1;

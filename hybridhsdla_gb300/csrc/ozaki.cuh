@@ -65,6 +65,8 @@ struct OzGroupDesc {
     int64_t ntypes = 0;                    // types of Tfull and TR (row sets: nt)
     const int32_t *set_type = nullptr;     // type of each row set: host [nt],
     const int32_t *d_set_type = nullptr;   // and device
+    void *split = nullptr;                 // ozaki_split_bytes for the S/H products, or null
+    int64_t split_bytes = 0;
 };
 struct OzGroup;
 // scratch: rewritten by every run (may be shared by the groups of a plan); persist: owned by
@@ -119,13 +121,15 @@ int ozaki_group_tune_tiles(OzGroup *g, cudaStream_t st, float *ms_best);
 int ozaki_plan_init(OzakiPlan &oz, int num_slices, double target);
 void ozaki_plan_release(OzakiPlan &oz);
 int64_t ozaki_pipeline_workspace(int s, int64_t twoL, int64_t na, int64_t nt, int64_t G);
+int64_t ozaki_split_bytes(int s, int64_t K, int64_t n, int64_t jobs);
 int64_t ozaki_herkx_workspace(int s, int64_t K, int64_t n);
 // S = C^H diag(w) C and H = C^H (T C) (lower triangles) with the T application emulated too.
 int ozaki_pipeline(OzakiPlan &oz, const OzakiInputs &in, double2 *S, double2 *H, int64_t ldo, void *ws,
                    cudaStream_t st, int *launches);
 // OUT = P^H diag(w) Q, lower triangle (standalone component).
 int ozaki_herkx(OzakiPlan &oz, const double2 *P, int64_t ldp, const double2 *Q, int64_t ldq, const double *w,
-                int64_t K, int64_t n, double2 *out, int64_t ldo, void *ws, cudaStream_t st, int *launches);
+                int64_t K, int64_t n, double2 *out, int64_t ldo, void *ws, cudaStream_t st, int *launches, void *split = nullptr,
+                int64_t split_size = 0);
 int ozaki_check_device_error(OzakiPlan &oz);
 // Lets one bounded wait expire on purpose (0: an mbarrier nothing arrives on, 1: a lockstep slot
 // that never advances) after budget_cycles; returns the status the host reads (HSDLA_ERR_TIMEOUT).
