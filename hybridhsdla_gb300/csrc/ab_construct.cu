@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(kThreads) construct_ab_kernel(DevSystem sys, c
     __shared__ double knorm;
 
     for (int lm = threadIdx.x; lm < L; lm += blockDim.x) {
-        int l = (int)sqrt((double)lm);
+        int l = (int)sqrtf((float)lm);
         while (l * l > lm) --l;
         while ((l + 1) * (l + 1) <= lm) ++l;
         l_of[lm] = (unsigned char)l;
@@ -563,7 +563,7 @@ __global__ void __launch_bounds__(kTfThreads) treal_kernel(const double2 *__rest
     // the indices of rows (l, |m|) and (l, -|m|), m's sign and parity of row x of a type
     auto split = [&](int x, int &p, int &q, int &m) {
         const int h = x >= L ? L : 0, lm = x - h;
-        int l = (int)sqrt((double)lm);
+        int l = (int)sqrtf((float)lm);
         while (l * l > lm) --l;
         while ((l + 1) * (l + 1) <= lm) ++l;
         m = lm - l * (l + 1);

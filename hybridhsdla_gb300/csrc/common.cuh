@@ -8,6 +8,16 @@
 
 namespace hsdla {
 
+// Row r of element x of a triangle stored row by row (r (r + 1) / 2 <= x), x < 2^31.  The estimate is
+// FP32: a double square root takes GB300's FP64 pipe ~1000 cycles per block of 256 threads.
+__device__ __forceinline__ int64_t triangle_row(int64_t x) {
+    int64_t r = (int64_t)((sqrtf(8.0f * (float)x + 1.0f) - 1.0f) * 0.5f);
+    while (r * (r + 1) / 2 > x) --r;
+    while ((r + 1) * (r + 2) / 2 <= x) ++r;
+    return r;
+}
+
+
 constexpr int kMaxLmax = 14;                 // (14+1)^2 = 225 lm per atom
 constexpr int kMaxL = (kMaxLmax + 1) * (kMaxLmax + 1);
 constexpr int kMaxTypes = 64;
@@ -200,6 +210,7 @@ cudaError_t launch_plugin_operand(const double2 *src, int64_t lds, bool transpos
                                   double2 *dst, int64_t ldd, int64_t r0, cudaStream_t st);
 // On C's uplo triangle: C = a T(R) + beta C, T(R)[i, j] = R[i, j] (lower) or conj(R[j, i]) (upper),
 // R's lower triangle read (R may be NULL: C = beta C); herm: real diagonal.
+cudaError_t launch_plugin_diagonal(double2 *C, int64_t ldc, int64_t n, cudaStream_t st);
 cudaError_t launch_plugin_epilogue(const double2 *R, int64_t ldr, double2 *C, int64_t ldc, int64_t n, double2 a,
                                    double beta, bool upper, bool herm, cudaStream_t st);
 

@@ -45,11 +45,8 @@ __device__ __forceinline__ void dmma(double (&d)[4], double a0, double a1, doubl
 
 __device__ __forceinline__ void tile_of(const Fp64Job &j, int64_t x, int64_t &ti, int64_t &tj) {
     if (j.lower) {
-        int64_t r = (int64_t)((sqrt(8.0 * (double)x + 1.0) - 1.0) * 0.5);
-        while (r * (r + 1) / 2 > x) --r;
-        while ((r + 1) * (r + 2) / 2 <= x) ++r;
-        ti = r;
-        tj = x - r * (r + 1) / 2;
+        ti = triangle_row(x);
+        tj = x - ti * (ti + 1) / 2;
     } else {
         ti = x / j.tiles_n;
         tj = x - ti * j.tiles_n;
@@ -193,9 +190,7 @@ __global__ void __launch_bounds__(128) fp64_real_kernel(const Fp64RealJob *__res
     const int64_t m = j.m, n = j.n, K = j.k, x = gt - j.tile_begin;
     int64_t ti, tj;
     if (j.lower) {
-        ti = (int64_t)((sqrt(8.0 * (double)x + 1.0) - 1.0) * 0.5);
-        while (ti * (ti + 1) / 2 > x) --ti;
-        while ((ti + 1) * (ti + 2) / 2 <= x) ++ti;
+        ti = triangle_row(x);
         tj = x - ti * (ti + 1) / 2;
     } else {
         ti = x / j.tiles_n;

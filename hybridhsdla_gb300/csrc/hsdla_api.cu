@@ -2490,7 +2490,9 @@ int plugin_contract(hsdla_context *ctx, int kind, int32_t precision, int32_t num
         }
     }
     // ---- epilogue on C's triangle (in place for the direct form: only the real diagonal)
-    if (!direct || herm) {
+    if (direct && product) {
+        if (herm) CUDA_TRY(ctx, launch_plugin_diagonal(dC, dldc, n, st));
+    } else if (!direct || herm) {
         const double2 a = kind == kPluginHer2k ? one : alpha;
         CUDA_TRY(ctx, launch_plugin_epilogue(product ? R : nullptr, ldr, dC, dldc, n, a, beta, upper, herm, st));
     }

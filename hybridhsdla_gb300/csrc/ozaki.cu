@@ -102,11 +102,8 @@ __device__ __forceinline__ int job_of(const OzJob *jobs, int num_jobs, int64_t t
 }
 __device__ __forceinline__ void tile_coords(const OzJob &j, int64_t x, int64_t &tm, int64_t &tn) {
     if (j.lower) {
-        int64_t r = (int64_t)((sqrt(8.0 * (double)x + 1.0) - 1.0) * 0.5);
-        while (r * (r + 1) / 2 > x) --r;
-        while ((r + 1) * (r + 2) / 2 <= x) ++r;
-        tm = r;
-        tn = x - r * (r + 1) / 2;
+        tm = triangle_row(x);
+        tn = x - tm * (tm + 1) / 2;
     } else {
         tm = x / j.tiles_n;
         tn = x - tm * j.tiles_n;
@@ -869,7 +866,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
 }
 
 // The slabs of a split tile into the output, in the order of its parts (adds: job, tile row, tile
-// column, first slab; then their number).  A warp's lanes walk rows.
+// column, first slab; then their number).  A block per column of a tile, lanes along its rows.
 __global__ void __launch_bounds__(kPairTile) oz_slab_add_kernel(const OzJob *__restrict__ jobs, const int4 *__restrict__ adds,
                                                                 const double2 *__restrict__ slabs) {
     const int4 a = adds[2 * blockIdx.x];
@@ -877,18 +874,17 @@ __global__ void __launch_bounds__(kPairTile) oz_slab_add_kernel(const OzJob *__r
     const OzJob &j = jobs[a.x];
     const int64_t row = (int64_t)a.y * kPairTile + threadIdx.x;
     if (row >= j.m) return;
-    for (int c = blockIdx.y; c < kPairTile; c += gridDim.y) {
-        const int64_t col = (int64_t)a.z * kPairTile + c;
-        if (col >= j.n || (j.lower && row < col)) break;
-        const double2 *p = slabs + ((int64_t)a.w * kPairTile + c) * kPairTile + threadIdx.x;
-        double2 v = j.out[row + j.ldo * col];
-        for (int q = 0; q < count; ++q, p += kPairTile * kPairTile) {
-            const double2 x = __ldcs(p);
-            v.x += x.x;
-            v.y += x.y;
-        }
-        j.out[row + j.ldo * col] = v;
+    const int64_t col = (int64_t)a.z * kPairTile + blockIdx.y;
+    if (col >= j.n || (j.lower && row < col)) return;
+    const double2 *p = slabs + ((int64_t)a.w * kPairTile + blockIdx.y) * kPairTile + threadIdx.x;
+    double2 v = j.out[row + j.ldo * col];
+#pragma unroll 8
+    for (int q = 0; q < count; ++q, p += kPairTile * kPairTile) {
+        const double2 x = __ldcs(p);
+        v.x += x.x;
+        v.y += x.y;
     }
+    j.out[row + j.ldo * col] = v;
 }
 
 // --------------------------------------------------------------- slicing
@@ -1621,7 +1617,7 @@ cudaError_t launch_pair(const CUtensorMap *maps, int s, int *d_err, const OzJob 
                            s, d_err, d_list, lockstep ? d_progress : (int *)nullptr, sync_every, slack,
                            cut ? (const int4 *)split->parts : (const int4 *)nullptr, cut ? split->slabs : (double2 *)nullptr);
     if (e != cudaSuccess || !cut) return e;
-    oz_slab_add_kernel<<<dim3((unsigned)split->n_adds, 32), kPairTile, 0, st>>>(d_jobs, split->adds, split->slabs);
+    oz_slab_add_kernel<<<dim3((unsigned)split->n_adds, kPairTile), kPairTile, 0, st>>>(d_jobs, split->adds, split->slabs);
     return cudaGetLastError();
 }
 
