@@ -70,8 +70,6 @@ __global__ void __launch_bounds__(kSfTabThreads) sf_table_kernel(const double2 *
     }
 }
 
-__device__ __noinline__ double ldexp_call(double v, int k) { return ldexp(v, k); }
-
 // Exact sums of products p f of 64-bit fixed-point products p and 55-bit structure factors f, in four
 // 64-bit sums of the limb products: p = p1 2^32 + p0 with p0 in [-2^31, 2^31), f = f1 2^28 + f0 with f0
 // in (-2^28, 2^28).  With |p1| < 2^31 and |f1| <= 2^27, kSumTypes types of two terms each overflow none
@@ -90,28 +88,31 @@ struct LimbSum {
         a00 += (long long)p.lo * f0;
     }
     // the sum times 2^k as a double: the bits below 2^36 dropped (the terms' own last places are above
-    // 2^50), the rest rounded on the integer pipes (the FP64 pipe, which a conversion instruction
-    // uses, issues one warp instruction in 16 cycles)
+    // 2^50), the rest rounded on the integer pipes (the FP64 pipe, which a conversion instruction uses
+    // too, takes 64 cycles per warp instruction and scheduler: with three conversions the 2 k-points of
+    // the kernel's comment took 1.88 ms)
     __device__ __forceinline__ double value(int k) const {
-        const long long m = (a10 >> 4) + (a01 >> 8) + (a00 >> 36);
-        const long long top = a11 + (m >> 24);
-        const unsigned low = (unsigned)m & 0xffffffu;
-        const int s = min(__clzll(top ^ (top >> 63)) - 1, 24);
-        const long long x = (top << s) | (long long)(low >> (24 - s));
-        // x to nearest even
-        const unsigned long long sign = (unsigned long long)x & 0x8000000000000000ull;
-        unsigned long long u = x < 0 ? 0ull - (unsigned long long)x : (unsigned long long)x;
-        const int lz = __clzll((long long)u);
-        u <<= lz & 63;
-        const unsigned long long rem = u & 0x7ffull;
-        unsigned long long b = ((unsigned long long)(unsigned)(1023 + 62 - lz) << 52) + (u >> 11);   // (hidden bit carries)
-        b += (rem > 0x400ull) | ((rem == 0x400ull) & (b & 1ull));
-        if (!x) return 0.0;
-        k += 60 - s;
-        const int E = (int)(b >> 52) + k;
-        if (E > 0 && E < 2047) return __longlong_as_double((long long)((b + ((unsigned long long)(unsigned)k << 52)) | sign));
-        return ldexp_call(__longlong_as_double((long long)(b | sign)), k);
+        const long long m = (a10 >> 4) + (a01 >> 8) + (a00 >> 36), top = a11 + (m >> 24);
+        const int sign = (int)(top >> 63);
+        // the magnitude's 96 bits (less one place of 2^36 where negative), its leading one to the top
+        uint32_t w2 = (uint32_t)(top >> 32) ^ sign, w1 = (uint32_t)top ^ sign, w0 = ((uint32_t)m << 8) ^ sign;
+        k += 1022 + 36 + 24 + 63;
+        if (w2 == 0) { w2 = w1; w1 = w0; w0 = 0; k -= 32; }
+        const int lz = __clz((int)w2);
+        const uint32_t hi = __funnelshift_l(w1, w2, lz), lo = __funnelshift_l(w0, w1, lz);
+        k -= lz;
+        if (w2 == 0 || k <= 0 || k >= 2046) return small_or_large(top, (uint32_t)m & 0xffffffu, k + lz);
+        // 53 bits, the next one rounding; the leading one counts in the exponent
+        const unsigned long long b = (((unsigned long long)hi << 32) | lo) >> 11;
+        const unsigned long long r = b + ((lo >> 10) & 1u) + ((unsigned long long)(uint32_t)k << 52);
+        return __longlong_as_double((long long)(r | ((unsigned long long)(uint32_t)(sign & 0x80000000) << 32)));
     }
+    // sums that the exponent range or 32 leading zeros take out of the path above (`k` as there)
+    static __device__ __noinline__ double small_or_large(long long top, uint32_t low, int k) {
+        if (top == 0 && low == 0) return 0.0;
+        return ldexp((double)top + (double)low * 5.9604644775390625e-8, k - (1022 + 63) + (k_small(top) ? 32 : 0));
+    }
+    static __device__ __forceinline__ bool k_small(long long top) { return ((uint32_t)((top ^ (top >> 63)) >> 32)) == 0; }
 };
 
 constexpr int kSfTile = 32;
@@ -125,76 +126,57 @@ constexpr int kSfTile = 32;
 // together; the warp fetches them with lanes side by side on an element's types and hands them over in
 // shared memory (a lane fetching its own element's cost a cache line per lane and type, which bounded
 // the kernel).
+// A warp's work is cut into items, four types of one column: an item's structure factors and products
+// arrive in one of two stages of shared memory by asynchronous copies while the item before is summed.
 // kFixed: fixed-point products and structure factors, summed exactly in integers.  GB300's FP64 pipe
 // (2 multiply-adds per cycle and SM) bounded this kernel at 0.95 of its rate.  8000 columns of 8 types:
-// FP64 2.60 ms, integers 1.59 ms (0.57 of the DRAM rate, 24 warps an SM); 2 k-points of 6300 columns and 4
-// types: 1.74 and 1.41 ms.
-//
-// combine_chunk: kNT types from t0 on of one element per lane into its sums.  All loads -- the lanes'
-// share of the warp's structure factors and the element's 3 kNT products -- go out before the first
-// use: the kernel lives on bytes in flight.  Four types at a time leave registers for 24 warps an SM;
-// eight at a time on 16 warps took 1.66 and 1.60 ms.
+// FP64 2.60 ms, integers 1.44 ms (0.63 of the DRAM rate); 2 k-points of 6300 columns and 4 types: 1.74 and 1.18
+// ms.  Bound now by the wide multiply-adds (a warp's takes four cycles; 24 an element and type) on 16 warps an
+// SM; 20 warps leave too little L1 beside the stages (1.67 and 1.44 ms).  Loads into registers, four types
+// ahead of their use on 24 warps, took 1.59 and 1.41 ms.
+constexpr int kChunk = 4, kSumItems = kSumTypes / kChunk;        // types of an item; items of a sum
+constexpr int kSfPitch = kChunk + 1;                             // 16-byte words of an element's structure factors
+constexpr int kStageSf = kSfTile * kSfPitch * 16, kStageBytesWarp = kStageSf + 3 * kChunk * kSfTile * 8;
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_but_one() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
+
 template <bool kFixed>
 struct Sums {
     double2 s = make_double2(0.0, 0.0), h = make_double2(0.0, 0.0);
+    __device__ __forceinline__ void add(int2 a, int2 c, int2 d, int4 w) {
+        auto dbl = [](int lo, int hi) { return __hiloint2double(hi, lo); };
+        const double fr = dbl(w.x, w.y), fi = dbl(w.z, w.w), x = dbl(a.x, a.y), y = dbl(c.x, c.y), z = dbl(d.x, d.y);
+        s.x = fma(fr, x, s.x);
+        s.y = fma(fi, x, s.y);
+        h.x = fma(fr, y, fma(-fi, z, h.x));
+        h.y = fma(fr, z, fma(fi, y, h.y));
+    }
 };
 template <>
 struct Sums<true> {
     LimbSum sr, si, hr, hi;
+    __device__ __forceinline__ void add(int2 a, int2 c, int2 d, int4 w) {
+        const Limbs x(a), y(c), z(d);
+        sr.add(x, w.x, w.y);
+        si.add(x, w.z, w.w);
+        hr.add(y, w.x, w.y);
+        hr.add(z, -w.z, -w.w);
+        hi.add(z, w.x, w.y);
+        hi.add(y, w.z, w.w);
+    }
 };
-template <bool kFixed, int kNT>
-__device__ __forceinline__ void combine_chunk(Sums<kFixed> &v, const SfEntry &E, const int4 *__restrict__ sf, int64_t idx,
-                                              int64_t off, int t0, int4 (*st)[kSumTypes]) {
-    const int lane = threadIdx.x;
-    const int64_t ps = E.pstride;
-    int4 g[kNT];
-    int2 a[kNT], c[kNT], d[kNT];
-#pragma unroll
-    for (int i = 0; i < kNT; ++i) {
-        const int w = lane + 32 * i;
-        g[i] = sf[__shfl_sync(0xffffffffu, idx, w / kNT) + t0 + w % kNT];
-    }
-    const int2 *pa = static_cast<const int2 *>(E.RS) + off + t0 * ps;
-    const int2 *pc = static_cast<const int2 *>(E.RHr) + off + t0 * ps, *pd = static_cast<const int2 *>(E.RHi) + off + t0 * ps;
-#pragma unroll
-    for (int t = 0; t < kNT; ++t) {
-        a[t] = __ldcs(pa + t * ps);
-        c[t] = __ldcs(pc + t * ps);
-        d[t] = __ldcs(pd + t * ps);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < kNT; ++i) {
-        const int w = lane + 32 * i, e = w / kNT, t = w % kNT;
-        st[e][(t + e) % kSumTypes] = g[i];     // (rotated: rows of 128 bytes would share banks)
-    }
-    __syncwarp();
-#pragma unroll
-    for (int t = 0; t < kNT; ++t) {
-        const int4 w = st[lane][(t + lane) % kSumTypes];
-        if constexpr (kFixed) {
-            const Limbs x(a[t]), y(c[t]), z(d[t]);
-            v.sr.add(x, w.x, w.y);
-            v.si.add(x, w.z, w.w);
-            v.hr.add(y, w.x, w.y);
-            v.hr.add(z, -w.z, -w.w);
-            v.hi.add(z, w.x, w.y);
-            v.hi.add(y, w.z, w.w);
-        } else {
-            auto dbl = [](int lo, int hi) { return __hiloint2double(hi, lo); };
-            const double fr = dbl(w.x, w.y), fi = dbl(w.z, w.w), x = dbl(a[t].x, a[t].y), y = dbl(c[t].x, c[t].y), z = dbl(d[t].x, d[t].y);
-            v.s.x = fma(fr, x, v.s.x);
-            v.s.y = fma(fi, x, v.s.y);
-            v.h.x = fma(fr, y, fma(-fi, z, v.h.x));
-            v.h.y = fma(fr, z, fma(fi, y, v.h.y));
-        }
-    }
-}
 
 template <bool kFixed, int kRows>
-__global__ void __launch_bounds__(kSfTile *kRows, 768 / (kSfTile * kRows)) sf_combine_kernel(const __grid_constant__ SfTab tab,
-                                                                                     const void *__restrict__ sf, int first) {
-    __shared__ int4 stage[kRows][kSfTile][kSumTypes];
+__global__ void __launch_bounds__(kSfTile *kRows, 512 / (kSfTile * kRows)) sf_combine_kernel(const __grid_constant__ SfTab tab,
+                                                                                     const int4 *__restrict__ sf, int first) {
+    extern __shared__ __align__(16) unsigned char stages[];
     const int64_t tile = blockIdx.x;
     int k = 0;
     while (k + 1 < tab.nk && tab.e[k + 1].tile_begin <= tile) ++k;
@@ -212,45 +194,94 @@ __global__ void __launch_bounds__(kSfTile *kRows, 768 / (kSfTile * kRows)) sf_co
     }
     const int64_t tc = lo, tr = tc + (b - before(tc));
     const int lane = threadIdx.x;
-    const int64_t row = tr * kSfTile + lane, rowc = min(row, E.n - 1);
-    const int32_t *gr = E.g + 3 * rowc;
-    const int gr0 = gr[0], gr1 = gr[1], gr2 = gr[2];
-    int4 (*st)[kSumTypes] = stage[threadIdx.y];
-#pragma unroll 1
-    for (int q = 0; q < kSfTile; q += kRows) {
-        const int64_t col = tc * kSfTile + threadIdx.y + q;
-        if (col >= E.n || col > tr * kSfTile + kSfTile - 1) break;      // (warp-uniform)
-        const bool live = row < E.n && col <= row;
-        const int32_t *gc = E.g + 3 * col;
-        const int64_t idx = (((int64_t)(gc[0] - gr0 + tab.dx) * tab.ny + (gc[1] - gr1 + tab.dy)) * tab.nz +
-                             (gc[2] - gr2 + tab.dz)) * tab.nt + tab.type;
-        const int64_t off = rowc + E.ldp * col + tab.slot0 * E.pstride;
-        double2 vs = make_double2(0.0, 0.0), vh = make_double2(0.0, 0.0);
-        for (int t0 = 0; t0 < tab.ntypes; t0 += kSumTypes) {
-            const int nt = min(tab.ntypes - t0, kSumTypes);
-            const int4 *f = static_cast<const int4 *>(sf);
-            Sums<kFixed> v;
-            if constexpr (!kFixed) { v.s = vs; v.h = vh; }
-            int t = t0;
-            if (nt == kSumTypes) { combine_chunk<kFixed, 4>(v, E, f, idx, off, t, st); t += 4; }
-            if (nt >= 4) { combine_chunk<kFixed, 4>(v, E, f, idx, off, t, st); t += 4; }
-            if (nt & 2) { combine_chunk<kFixed, 2>(v, E, f, idx, off, t, st); t += 2; }
-            if (nt & 1) combine_chunk<kFixed, 1>(v, E, f, idx, off, t, st);
-            if constexpr (kFixed) {
-                // one power of two for every type's products of an element
-                const int k0 = E.el[rowc] - 8 - tab.frac - tab.sfbits, ks = k0 + E.ers[col], kh = k0 + E.erh[col];
-                const double2 s = make_double2(v.sr.value(ks), v.si.value(ks)), h = make_double2(v.hr.value(kh), v.hi.value(kh));
-                if (t0 == 0) { vs = s; vh = h; }
-                else { vs.x += s.x; vs.y += s.y; vh.x += h.x; vh.y += h.y; }
-            } else {
-                vs = v.s;
-                vh = v.h;
+    const int64_t row = tr * kSfTile + lane, rowc = min(row, E.n - 1), colc = min(tc * kSfTile + lane, E.n - 1);
+    // the table's place of dG = g_col - g_row is linear in both: this lane's row's and column's parts, and
+    // the rows' of the elements whose structure factors it fetches
+    auto place = [&](int64_t x) {
+        const int32_t *g = E.g + 3 * x;
+        return (((int64_t)g[0] * tab.ny + g[1]) * tab.nz + g[2]) * tab.nt;
+    };
+    const int64_t prow = place(rowc);
+    const int64_t pcol = place(colc) + (((int64_t)tab.dx * tab.ny + tab.dy) * tab.nz + tab.dz) * tab.nt + tab.type;
+    int64_t from[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) from[i] = __shfl_sync(0xffffffffu, prow, lane / 4 + 8 * i) - lane % 4;
+    const int kr = kFixed ? E.el[rowc] - 8 - tab.frac - tab.sfbits : 0;
+    const int kcs = kFixed ? E.ers[colc] : 0, kch = kFixed ? E.erh[colc] : 0;
+    // the warp's columns of the tile: threadIdx.y, + kRows, ... below cend (those of the lower triangle)
+    const int cend = (int)min((int64_t)kSfTile, (tr == tc ? E.n : min(E.n, tc * kSfTile + kSfTile)) - tc * kSfTile);
+    const int ntypes = tab.ntypes, nchunk = (ntypes + kChunk - 1) / kChunk;
+    const int64_t ps = E.pstride, ldp = E.ldp, ldo = E.ldo;
+    unsigned char *mem = stages + threadIdx.y * 2 * kStageBytesWarp;
+    const uint32_t smem = (uint32_t)__cvta_generic_to_shared(mem);
+    // the item to be fetched next: column ic, chunk it; its column's first product
+    int ic = threadIdx.y, it = 0;
+    int64_t o = rowc + tab.slot0 * ps + ldp * (tc * kSfTile + ic);
+    auto fetch = [&](uint32_t st) {
+        if (ic < cend) {
+            const int n = min(kChunk, ntypes - kChunk * it);
+            const int4 *base = sf + __shfl_sync(0xffffffffu, pcol, ic) + kChunk * it;
+            const uint32_t ds = st + (lane / 4 * kSfPitch + lane % 4) * 16;
+            if (lane % 4 < n) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) cp_async16(ds + i * (8 * kSfPitch * 16), base - from[i]);
+            }
+            const uint32_t dp = st + kStageSf + lane * 8;
+            int64_t x = o + kChunk * it * ps;
+#pragma unroll
+            for (int t = 0; t < kChunk; ++t, x += ps)
+                if (t < n) {
+                    cp_async8(dp + (3 * t) * (kSfTile * 8), static_cast<const int2 *>(E.RS) + x);
+                    cp_async8(dp + (3 * t + 1) * (kSfTile * 8), static_cast<const int2 *>(E.RHr) + x);
+                    cp_async8(dp + (3 * t + 2) * (kSfTile * 8), static_cast<const int2 *>(E.RHi) + x);
+                }
+            if (++it == nchunk) {
+                it = 0;
+                ic += kRows;
+                o += kRows * ldp;
             }
         }
-        if (!live) continue;
+        cp_async_commit();
+    };
+    int stage = 0;
+    fetch(smem);
+    int64_t oo = row + ldo * (tc * kSfTile + threadIdx.y);
+#pragma unroll 1
+    for (int c = threadIdx.y; c < cend; c += kRows, oo += kRows * ldo) {
+        double2 vs = make_double2(0.0, 0.0), vh = make_double2(0.0, 0.0);
+        Sums<kFixed> v;
+        const int ks = kFixed ? kr + __shfl_sync(0xffffffffu, kcs, c) : 0, kh = kFixed ? kr + __shfl_sync(0xffffffffu, kch, c) : 0;
+#pragma unroll 1
+        for (int q = 0; q < nchunk; ++q) {
+            fetch(smem + (stage ^ 1) * kStageBytesWarp);
+            cp_async_wait_but_one();
+            __syncwarp();
+            const int n = min(kChunk, ntypes - kChunk * q);
+            const int4 *w = reinterpret_cast<const int4 *>(mem + stage * kStageBytesWarp) + lane * kSfPitch;
+            const int2 *p = reinterpret_cast<const int2 *>(mem + stage * kStageBytesWarp + kStageSf) + lane;
+#pragma unroll
+            for (int t = 0; t < kChunk; ++t)
+                if (t < n) v.add(p[3 * t * kSfTile], p[(3 * t + 1) * kSfTile], p[(3 * t + 2) * kSfTile], w[t]);
+            __syncwarp();
+            stage ^= 1;
+            if constexpr (kFixed) {
+                if (q % kSumItems == kSumItems - 1 || q + 1 == nchunk) {
+                    // one power of two for every type's products of an element
+                    const double2 s = make_double2(v.sr.value(ks), v.si.value(ks)), h = make_double2(v.hr.value(kh), v.hi.value(kh));
+                    if (q < kSumItems) { vs = s; vh = h; }
+                    else { vs.x += s.x; vs.y += s.y; vh.x += h.x; vh.y += h.y; }
+                    v = Sums<kFixed>();
+                }
+            }
+        }
+        if constexpr (!kFixed) {
+            vs = v.s;
+            vh = v.h;
+        }
+        const int64_t col = tc * kSfTile + c;
+        if (row >= E.n || col > row) continue;
         const bool x = E.Sx && row < tab.xrow1;
-        double2 *so = x ? E.Sx + row + E.ldx * col : E.S + row + E.ldo * col;
-        double2 *ho = x ? E.Hx + row + E.ldx * col : E.H + row + E.ldo * col;
+        double2 *so = x ? E.Sx + row + E.ldx * col : E.S + oo, *ho = x ? E.Hx + row + E.ldx * col : E.H + oo;
         if (!first) {
             const double2 s0 = E.Si[row + E.ldi * col], h0 = E.Hi[row + E.ldi * col];
             vs.x += s0.x; vs.y += s0.y;
@@ -262,13 +293,20 @@ __global__ void __launch_bounds__(kSfTile *kRows, 768 / (kSfTile * kRows)) sf_co
 }
 
 template <bool kFixed>
-void combine_launch(const SfTab &t, const void *sf, bool first, int64_t tiles, cudaStream_t st) {
+cudaError_t combine_launch(const SfTab &t, const void *sf, bool first, int64_t tiles, cudaStream_t st) {
     // 4 columns of a tile at a time where there are tiles enough, 8 where not
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (tiles < 8 * (int64_t)nsm) sf_combine_kernel<kFixed, 8><<<(unsigned)tiles, dim3(kSfTile, 8), 0, st>>>(t, sf, first ? 1 : 0);
-    else sf_combine_kernel<kFixed, 4><<<(unsigned)tiles, dim3(kSfTile, 4), 0, st>>>(t, sf, first ? 1 : 0);
+    const bool few = tiles < 8 * (int64_t)nsm;
+    const void *kernel = few ? (const void *)sf_combine_kernel<kFixed, 8> : (const void *)sf_combine_kernel<kFixed, 4>;
+    const int rows = few ? 8 : 4, smem = rows * 2 * kStageBytesWarp;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    const int4 *f = static_cast<const int4 *>(sf);
+    if (few) sf_combine_kernel<kFixed, 8><<<(unsigned)tiles, dim3(kSfTile, 8), smem, st>>>(t, f, first ? 1 : 0);
+    else sf_combine_kernel<kFixed, 4><<<(unsigned)tiles, dim3(kSfTile, 4), smem, st>>>(t, f, first ? 1 : 0);
+    return cudaGetLastError();
 }
 
 }  // namespace
@@ -311,9 +349,7 @@ cudaError_t launch_sf_combine(const SfTab &tab, const void *sf, bool first, cuda
     const int64_t tiles = sf_tab_tiles(t);
     if (tiles <= 0) return cudaSuccess;
     if (tiles > 0x7fffffffLL) return cudaErrorInvalidValue;
-    if (t.nk > 0 && t.e[0].el) combine_launch<true>(t, sf, first, tiles, st);
-    else combine_launch<false>(t, sf, first, tiles, st);
-    return cudaGetLastError();
+    return t.nk > 0 && t.e[0].el ? combine_launch<true>(t, sf, first, tiles, st) : combine_launch<false>(t, sf, first, tiles, st);
 }
 
 }  // namespace hsdla
