@@ -41,6 +41,7 @@
 #include <cstring>
 #include <vector>
 
+#include "digits.cuh"
 #include "ozaki.cuh"
 #include "ptx.cuh"
 #include "real_products.cuh"
@@ -924,42 +925,12 @@ struct SliceTab {
     SliceEntry e[kMaxGroup];
 };
 
-// e4m3 byte of the digit idx - 16 (idx in [0, 32]), per CTA of the slicing kernel: a digit is
-// one shared-memory load instead of an integer-to-float conversion and half a packing conversion
-__shared__ uint8_t g_e4m3_lut[33];
-// The planes of U = X + B from the least significant: plane i (0 = most significant) holds
-// ((U >> 5 (s-1-i)) & 31) - 16 for i >= 1, and the top plane the rest, U >> 5 (s-1) in
-// [-16, 16].  A running arithmetic shift by 5 leaves each field in the low bits in turn (the low
-// bits are the same for arithmetic and logical shifts).
-template <int kVec>
-__device__ __forceinline__ void write_part(const long long (&x)[kVec], int part, int s, uint8_t *row, int64_t plane) {
-    long long u[kVec];
-#pragma unroll
-    for (int v = 0; v < kVec; ++v) u[v] = x[v];
-#pragma unroll 1
-    for (int step = 0; step < s; ++step) {
-        const int i = s - 1 - step;
-        uint32_t w0 = 0, w1 = 0;
-#pragma unroll
-        for (int v = 0; v < kVec; ++v) {
-            // (the top digit of a finite row is in [-16, 16]; the clamp keeps the table read in
-            // bounds for any row)
-            const int idx = i == 0 ? min(max((int)u[v] + 16, 0), 32) : (int)(u[v] & 31);
-            const uint32_t b = (uint32_t)g_e4m3_lut[idx] << (8 * (v & 3));
-            if (v < 4) w0 |= b; else w1 |= b;
-            u[v] >>= 5;
-        }
-        uint8_t *dst = row + (int64_t)(2 * i + part) * plane;
-        if (kVec == 8) *reinterpret_cast<uint2 *>(dst) = make_uint2(w0, w1);
-        else *reinterpret_cast<uint32_t *>(dst) = w0;
-    }
-}
-
+// The planes of U = X + B: plane 2 i + part holds digit i of the real (part 0) or imaginary part.
 template <int kVec>
 __device__ __forceinline__ void write_planes(const long long (&ur)[kVec], const long long (&ui)[kVec], int s,
                                              uint8_t *row, int64_t plane) {
-    write_part<kVec>(ur, 0, s, row, plane);
-    write_part<kVec>(ui, 1, s, row, plane);
+    write_digits<kVec>(ur, s, row, 2 * plane);
+    write_digits<kVec>(ui, s, row + plane, 2 * plane);
 }
 
 // Maximum over the block of non-negative doubles given as bit patterns (which order like the
@@ -1048,29 +1019,28 @@ __global__ void __launch_bounds__(kSliceThreads, HSDLA_SLICE_CTAS) oz_slice_kern
     const int64_t pitch = tab.pitch, plane_rows = tab.plane_rows;
     const int s = tab.s;
     __shared__ unsigned long long red[2][kSliceThreads / 32];
-    // the digit table (read in pass 2, after the barrier of the row maximum)
-    if (threadIdx.x < 33) {
-        const float dv = (float)((int)threadIdx.x - 16);
-        g_e4m3_lut[threadIdx.x] = (uint8_t)(__nv_cvt_float2_to_fp8x2(make_float2(dv, 0.f), __NV_SATFINITE, __NV_E4M3) & 0xffu);
-    }
     // pass 1: column max of max(|re|, |im|) (times the row weight; the only FP64 multiply here)
-    // Each thread reads 8 consecutive values per step (all loads of a step in flight together):
-    // one value per thread and step kept too few bytes in flight to cover the memory latency.
+    // Each thread reads 8 values per step (all loads of a step in flight together: one kept too few
+    // bytes in flight to cover the memory latency), lanes on consecutive ones.
     // (the weighted and unweighted forms as separate loops: GB300 issues the FP64 multiplies of a
     // predicated-off branch all the same, at 16 cycles per warp instruction)
     unsigned long long mx = 0, mx2 = 0;
     auto pass1 = [&](auto weighted) {
-        for (int k0 = threadIdx.x * kSliceVec; k0 < Kin; k0 += kSliceThreads * kSliceVec) {
+        for (int k0 = threadIdx.x; k0 < Kin; k0 += kSliceThreads * kSliceVec) {
             double2 z[kSliceVec];
 #pragma unroll
-            for (int u = 0; u < kSliceVec; ++u) z[u] = k0 + u < Kin ? Zc[k0 + u] : make_double2(0.0, 0.0);
+            for (int u = 0; u < kSliceVec; ++u) {
+                const int i = k0 + u * kSliceThreads;
+                z[u] = i < Kin ? Zc[i] : make_double2(0.0, 0.0);
+            }
 #pragma unroll
             for (int u = 0; u < kSliceVec; ++u) {
                 const unsigned long long a = max(abs_bits(z[u].x), abs_bits(z[u].y));
-                if (k0 + u < Kin) {
-                    if constexpr (decltype(weighted)::value) mx = max(mx, abs_bits(__longlong_as_double((long long)a) * v[k0 + u]));
+                const int i = k0 + u * kSliceThreads;
+                if (i < Kin) {
+                    if constexpr (decltype(weighted)::value) mx = max(mx, abs_bits(__longlong_as_double((long long)a) * v[i]));
                     else mx = max(mx, a);
-                    if (kDual) mx2 = max(mx2, abs_bits(__longlong_as_double((long long)a) * v2[k0 + u]));
+                    if (kDual) mx2 = max(mx2, abs_bits(__longlong_as_double((long long)a) * v2[i]));
                 }
             }
         }

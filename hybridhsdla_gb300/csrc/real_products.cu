@@ -45,6 +45,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "digits.cuh"
 #include "ptx.cuh"
 #include "real_products.cuh"
 
@@ -444,24 +445,14 @@ __device__ __forceinline__ int frexp_exp_bits(unsigned long long b) {
     if (E) return E - 1022;
     return -1010 - __clzll((long long)(b & 0xfffffffffffffull));
 }
-// rint(x 2^k), half to even, for |x 2^k| < 2^62
+// x 2^k rounded to nearest (halves away from zero), for |x 2^k| < 2^62
 __device__ __forceinline__ long long rint_pow2(double x, int k) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-    const int E = (int)((b >> 52) & 0x7ff);
-    const unsigned long long mant = b & 0xfffffffffffffull;
-    const unsigned long long m = E ? (mant | (1ull << 52)) : mant;
-    const int sh = 1075 - (E ? E : 1) - k;
-    unsigned long long q;
-    if (sh <= 0) {
-        q = m << (-sh);
-    } else if (sh >= 54) {
-        q = 0;
-    } else {
-        q = m >> sh;
-        const unsigned long long rem = m & ((1ull << sh) - 1), half = 1ull << (sh - 1);
-        q += (rem > half) | ((rem == half) & (q & 1ull));
-    }
-    return (b >> 63) ? -(long long)q : (long long)q;
+    const int hi = __double2hiint(x), E = (hi >> 20) & 0x7ff;
+    const unsigned long long m = ((unsigned long long)(uint32_t)((hi & 0xfffff) | (E ? 0x100000 : 0)) << 32) | (uint32_t)__double2loint(x);
+    const int sh = 1084 - max(E, 1) - k;
+    // (sh < 0: a column of subnormal numbers)
+    const long long q = (long long)(sh < 0 ? m << min(9 - sh, 63) : (((m << 10) >> min(sh, 63)) + 1) >> 1);
+    return hi < 0 ? -q : q;
 }
 
 __device__ __forceinline__ unsigned long long block_max(unsigned long long m, unsigned long long *red) {
@@ -469,57 +460,17 @@ __device__ __forceinline__ unsigned long long block_max(unsigned long long m, un
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
     __syncthreads();
     unsigned long long r = 0;
-    for (int i = 0; i < kSliceThreads / 32; ++i) r = max(r, red[i]);
+    for (int i = 0; i < (int)blockDim.x / 32; ++i) r = max(r, red[i]);
     return r;
 }
 
-// The s digits of eight values X + B (B = 16 in every lower digit) to planes `step` apart (dst: the
-// first digit's).  The lower digits are 5-bit fields: 15 bits of two values side by side, a field of each
-// at a time into FP16 (1024 + field, less 1040) and both to e4m3 in one conversion (a field and a table
-// read at a time took 237 us where this takes 207, the fixed-point columns of the 8000-column workload).
-__device__ __forceinline__ uint32_t e4m3_pair(uint32_t h) {          // two FP16 numbers, low half first
-    __half2_raw r;
-    r.x = (unsigned short)h;
-    r.y = (unsigned short)(h >> 16);
-    return __nv_cvt_halfraw2_to_fp8x2(r, __NV_SATFINITE, __NV_E4M3);
-}
-__device__ __forceinline__ uint32_t sub_1040(uint32_t h) {
-    uint32_t d;
-    asm("sub.f16x2 %0, %1, %2;\n" : "=r"(d) : "r"(h), "r"(0x64106410u));
-    return d;
-}
-__device__ __forceinline__ void write_digits(const long long (&u)[kVec], int s, uint8_t *dst, int64_t step) {
-    // the first digit: in [-16, 16] for a finite column (clamped for any)
-    {
-        uint32_t w[kVec / 2];
-        const int sh = 5 * (s - 1);
-#pragma unroll
-        for (int v = 0; v < kVec; v += 2) {
-            const int d0 = min(max((int)(u[v] >> sh), -16), 16), d1 = min(max((int)(u[v + 1] >> sh), -16), 16);
-            w[v / 2] = e4m3_pair(sub_1040(__byte_perm(d0 + 0x6410, d1 + 0x6410, 0x5410)));
-        }
-        *reinterpret_cast<uint2 *>(dst) = make_uint2(__byte_perm(w[0], w[1], 0x5410), __byte_perm(w[2], w[3], 0x5410));
-    }
-    uint8_t *p = dst + (int64_t)(s - 1) * step;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        if (3 * c >= s - 1) break;
-        uint32_t w[kVec / 2];
-#pragma unroll
-        for (int v = 0; v < kVec; v += 2)
-            w[v / 2] = __byte_perm((uint32_t)(u[v] >> (15 * c)), (uint32_t)(u[v + 1] >> (15 * c)), 0x5410);
-#pragma unroll
-        for (int f = 0; f < 3; ++f, p -= step) {
-            if (3 * c + f >= s - 1) break;
-            uint32_t d[kVec / 2];
-#pragma unroll
-            for (int v = 0; v < kVec / 2; ++v) d[v] = e4m3_pair(sub_1040(((w[v] >> (5 * f)) & 0x001f001fu) | 0x64006400u));
-            *reinterpret_cast<uint2 *>(p) = make_uint2(__byte_perm(d[0], d[1], 0x5410), __byte_perm(d[2], d[3], 0x5410));
-        }
-    }
-}
-
-// kFixed: the source is a product's fixed-point numbers (parts rows exponents el, see RealSliceTab)
+// kFixed: the source is a product's fixed-point numbers (parts rows exponents el, see RealSliceTab).
+// One thread per eight contraction bytes up to kSliceThreads; a thread's first eight values (all of them up to
+// 2048 bytes) stay in registers between the two passes; they and their exponents and weights come in pairs
+// (launch_real_slice checks that they can).  Bound by the integer pipe.  The 8000-column workload's (8
+// types, lmax 10, 12 digits) columns with their weighted copy take 167 us, its fixed-point ones 160 (both passes
+// reading single values, 256 threads a column: 209 and 207; with 768 contraction bytes a column: 278 and 253
+// us, now 187 and 204).
 template <bool kDual, bool kFixed>
 __global__ void __launch_bounds__(kSliceThreads) oz_slice_real_kernel(const __grid_constant__ RealSliceTab tab) {
     __shared__ unsigned long long red[2][kSliceThreads / 32];
@@ -528,33 +479,73 @@ __global__ void __launch_bounds__(kSliceThreads) oz_slice_real_kernel(const __gr
     while (k + 1 < tab.nk && tab.e[k + 1].row0 <= r) ++k;
     const int64_t g = r - tab.e[k].row0;
     const bool live = g >= 0 && g < tab.e[k].ncols;
-    const int64_t col = tab.ldz * (live ? g : 0);
-    const double *Z = reinterpret_cast<const double *>(tab.e[k].Z) + col;
-    const long long *F = reinterpret_cast<const long long *>(tab.e[k].Z) + col;
-    const int rpb = (int)tab.rpb, bpad = (int)tab.bpad, nblk = (int)tab.blocks, parts = tab.parts, s = tab.s;
+    const long long *Z = reinterpret_cast<const long long *>(tab.e[k].Z) + tab.ldz * (live ? g : 0);
+    const int rpb = live ? (int)tab.rpb : 0, bpad = (int)tab.bpad, nblk = (int)tab.blocks, parts = tab.parts, s = tab.s;
     const int bch = bpad / kVec, nch = bch * nblk;               // chunks of a block and part; of a part
+    struct Place {
+        int b, p, r0;
+    };
+    auto place = [&](int c) {
+        const int p = c / nch, cc = c - p * nch, b = cc / bch;
+        return Place{b, p, (cc - b * bch) * kVec};
+    };
+    // eight values of a chunk, and their weighted copies or row exponents (zeros past the rows)
+    auto load = [&](const Place &q, long long (&z)[kVec], double (&y)[kVec], int (&el)[kVec]) {
+        const longlong2 *src = reinterpret_cast<const longlong2 *>(Z + (int64_t)q.b * tab.bstride + q.p * tab.pstride + q.r0);
+        const int2 *ex = kFixed ? reinterpret_cast<const int2 *>(tab.el + (int64_t)tab.set_type[q.b] * tab.bstride + q.p * tab.pstride + q.r0)
+                                : nullptr;
+        const double2 *w = kDual ? reinterpret_cast<const double2 *>(tab.v2 + q.b * rpb + q.r0) : nullptr;
+#pragma unroll
+        for (int u = 0; u < kVec; u += 2) {
+            const bool in = q.r0 + u < rpb;
+            const longlong2 x = in ? src[u / 2] : make_longlong2(0, 0);
+            z[u] = x.x;
+            z[u + 1] = x.y;
+            if constexpr (kFixed) {
+                const int2 e = in ? ex[u / 2] : make_int2(0, 0);
+                el[u] = e.x;
+                el[u + 1] = e.y;
+            }
+            if constexpr (kDual) {
+                const double2 v = in ? w[u / 2] : make_double2(0.0, 0.0);
+                y[u] = __longlong_as_double(x.x) * v.x;
+                y[u + 1] = __longlong_as_double(x.y) * v.y;
+            }
+        }
+    };
     // (a fixed-point number's bit length and row exponent, offset to stay positive, order as |value|)
     constexpr int kOff = 1 << 20;
     unsigned long long mx = 0, mx2 = 0;
-    for (int c = threadIdx.x; live && c < nch * parts; c += kSliceThreads) {
-        const int p = c / nch, cc = c - p * nch, b = cc / bch, r0 = (cc - b * bch) * kVec;
-        const int64_t o = (int64_t)b * tab.bstride + p * tab.pstride + r0;
-        const int32_t *el = kFixed ? tab.el + (int64_t)tab.set_type[b] * tab.bstride + p * tab.pstride + r0 : nullptr;
+    int mxf = 0;
+    auto largest = [&](const long long (&z)[kVec], const double (&y)[kVec], const int (&el)[kVec]) {
 #pragma unroll
-        for (int u = 0; u < kVec; ++u)
-            if (r0 + u < rpb) {
-                if constexpr (kFixed) {
-                    const long long x = F[o + u];
-                    if (x) mx = max(mx, (unsigned long long)(kOff + 64 - __clzll(x < 0 ? -x : x) + el[u]));
-                } else {
-                    const double x = Z[o + u];
-                    mx = max(mx, abs_bits(x));
-                    if (kDual) mx2 = max(mx2, abs_bits(x * tab.v2[b * rpb + r0 + u]));
-                }
+        for (int u = 0; u < kVec; ++u) {
+            if constexpr (kFixed) {
+                if (z[u]) mxf = max(mxf, kOff + 64 - __clzll(z[u] < 0 ? -z[u] : z[u]) + el[u]);
+            } else {
+                mx = max(mx, (unsigned long long)z[u] & 0x7fffffffffffffffull);
+                if (kDual) mx2 = max(mx2, abs_bits(y[u]));
             }
+        }
+    };
+    long long z[kVec];
+    double y[kVec];
+    int el[kVec];
+    const Place first = place((int)threadIdx.x);
+    const bool any = threadIdx.x < nch * parts;
+    if (any) {
+        load(first, z, y, el);
+        largest(z, y, el);
+    }
+    for (int c = threadIdx.x + blockDim.x; c < nch * parts; c += blockDim.x) {
+        long long zc[kVec];
+        double yc[kVec];
+        int ec[kVec];
+        load(place(c), zc, yc, ec);
+        largest(zc, yc, ec);
     }
     int e = 0, e2 = 0, q = 0;
-    const unsigned long long m = block_max(mx, red[0]);
+    const unsigned long long m = block_max(kFixed ? (unsigned long long)mxf : mx, red[0]);
     if constexpr (kFixed) {
         q = (live ? tab.er[r] : 0) - 8 - tab.frac;               // the column's part of the values' exponent
         if (m > 0) e = (int)m - kOff + q;
@@ -571,31 +562,29 @@ __global__ void __launch_bounds__(kSliceThreads) oz_slice_real_kernel(const __gr
     long long B = 0;
     for (int p = 0; p < s - 1; ++p) B |= 16ll << (5 * p);
     const int64_t plane = tab.plane_rows * tab.pitch;
-    for (int c = threadIdx.x; c < nch * parts; c += kSliceThreads) {
-        const int p = c / nch, cc = c - p * nch, b = cc / bch, r0 = (cc - b * bch) * kVec;
-        const int64_t o = (int64_t)b * tab.bstride + p * tab.pstride + r0;
-        const int32_t *el = kFixed ? tab.el + (int64_t)tab.set_type[b] * tab.bstride + p * tab.pstride + r0 : nullptr;
+    auto digits = [&](const Place &at, const long long (&z)[kVec], const double (&y)[kVec], const int (&el)[kVec]) {
         long long x[kVec];
 #pragma unroll
         for (int u = 0; u < kVec; ++u) {
-            long long X = 0;
-            if (live && r0 + u < rpb) {
-                if constexpr (kFixed) {
-                    // F 2^(el + q) scaled by 2^(top - e): a shift, rounded half up
-                    const int d = el[u] + q + top - e;
-                    const long long f = F[o + u];
-                    X = d >= 0 ? f << min(d, 63) : d < -63 ? 0 : ((f >> (-d - 1)) + 1) >> 1;
-                } else X = rint_pow2(Z[o + u], top - e);
-            }
-            x[u] = B + X;
+            if constexpr (kFixed) {
+                // F 2^(el + q) scaled by 2^(top - e): a shift, rounded half up
+                const int d = el[u] + q + top - e;
+                x[u] = B + (d >= 0 ? z[u] << min(d, 63) : d < -63 ? 0 : ((z[u] >> (-d - 1)) + 1) >> 1);
+            } else x[u] = B + rint_pow2(__longlong_as_double(z[u]), top - e);
         }
-        write_digits(x, s, tab.digits + r * tab.pitch + (int64_t)b * bpad + r0 + p * plane, parts * plane);
-        if (kDual) {
+        const int64_t o = r * tab.pitch + (int64_t)at.b * bpad + at.r0;
+        write_digits<kVec>(x, s, tab.digits + o + at.p * plane, parts * plane);
+        if constexpr (kDual) {
 #pragma unroll
-            for (int u = 0; u < kVec; ++u)
-                x[u] = B + (live && r0 + u < rpb ? rint_pow2(Z[o + u] * tab.v2[b * rpb + r0 + u], top - e2) : 0ll);
-            write_digits(x, s, tab.digits2 + r * tab.pitch + (int64_t)b * bpad + r0, plane);
+            for (int u = 0; u < kVec; ++u) x[u] = B + rint_pow2(y[u], top - e2);
+            write_digits<kVec>(x, s, tab.digits2 + o, plane);
         }
+    };
+    if (any) digits(first, z, y, el);
+    for (int c = threadIdx.x + blockDim.x; c < nch * parts; c += blockDim.x) {
+        const Place at = place(c);
+        load(at, z, y, el);
+        digits(at, z, y, el);
     }
 }
 
@@ -697,10 +686,16 @@ cudaError_t launch_real_products(const CUtensorMap &left, const CUtensorMap &rig
 
 cudaError_t launch_real_slice(const RealSliceTab &t, cudaStream_t st) {
     if (t.plane_rows <= 0) return cudaSuccess;
+    // pairs of values, weights and exponents: 2L rows a block and aligned arrays, as every caller has them
+    if ((t.rpb | t.ldz | t.bstride | t.pstride) & 1 || reinterpret_cast<uintptr_t>(t.v2) % 16 || reinterpret_cast<uintptr_t>(t.el) % 8)
+        return cudaErrorInvalidValue;
+    for (int k = 0; k < t.nk; ++k)
+        if (reinterpret_cast<uintptr_t>(t.e[k].Z) % 16) return cudaErrorInvalidValue;
     const unsigned grid = (unsigned)t.plane_rows;
-    if (t.frac) oz_slice_real_kernel<false, true><<<grid, kSliceThreads, 0, st>>>(t);
-    else if (t.digits2) oz_slice_real_kernel<true, false><<<grid, kSliceThreads, 0, st>>>(t);
-    else oz_slice_real_kernel<false, false><<<grid, kSliceThreads, 0, st>>>(t);
+    const unsigned threads = (unsigned)std::min<int64_t>(kSliceThreads, (t.bpad / kVec * t.blocks * t.parts + 31) / 32 * 32);
+    if (t.frac) oz_slice_real_kernel<false, true><<<grid, threads, 0, st>>>(t);
+    else if (t.digits2) oz_slice_real_kernel<true, false><<<grid, threads, 0, st>>>(t);
+    else oz_slice_real_kernel<false, false><<<grid, threads, 0, st>>>(t);
     return cudaGetLastError();
 }
 
