@@ -2143,6 +2143,8 @@ int ozaki_group_prepare(OzakiPlan &oz, const OzGroupDesc &d, const std::vector<O
     if (!rc && d.hoist) rc = make_map(g->dM, 2 * s);
     if (rc) return fail(rc);
     // (b) T application: per type once (hoisted), or per atom of each panel
+    g->pair = use_pair();
+    const int64_t tile = g->pair ? kPairTile : kTileN;
     if (d.hoist) {
         std::vector<OzJob> jt;
         for (int k = 0; k < g->nk; ++k)
@@ -2160,7 +2162,7 @@ int ozaki_group_prepare(OzakiPlan &oz, const OzGroupDesc &d, const std::vector<O
                 jt.push_back(j);
             }
         g->n_jobs_t = (int)jt.size();
-        rc = upload_schedule(jt, g->d_jobs_t, g->d_list_t, g->tiles_t);
+        rc = upload_schedule(jt, g->d_jobs_t, g->d_list_t, g->tiles_t, tile);
         if (rc) return fail(rc);
     } else {
         int64_t joff = 0, loff = 0;
@@ -2184,7 +2186,7 @@ int ozaki_group_prepare(OzakiPlan &oz, const OzGroupDesc &d, const std::vector<O
             p.jt_off = joff;
             p.lt_off = loff;
             p.n_jobs_t = (int)jt.size();
-            rc = upload_schedule(jt, g->d_jobs_t + joff, g->d_list_t + loff, p.tiles_t);
+            rc = upload_schedule(jt, g->d_jobs_t + joff, g->d_list_t + loff, p.tiles_t, tile);
             if (rc) return fail(rc);
             joff += p.n_jobs_t;
             loff += p.tiles_t;
@@ -2193,8 +2195,6 @@ int ozaki_group_prepare(OzakiPlan &oz, const OzGroupDesc &d, const std::vector<O
     g->maps_t[0] = d.hoist ? g->dM.map : g->dC.map;
     g->maps_t[1] = g->maps_t[0]; g->maps_t[2] = g->maps_t[0]; g->maps_t[3] = g->dT.map;
     // (c) S and H jobs of every panel; outputs are patched per run, later panels accumulate
-    g->pair = use_pair();
-    const int64_t tile = g->pair ? kPairTile : kTileN;
     g->n_jobs_sh = 2 * g->nk;
     for (int pi = 0; pi < g->panels; ++pi) {
         const OzPanel &p = g->pan[pi];
@@ -2257,6 +2257,13 @@ void ozaki_group_set_outputs(OzGroup *g, double2 *const *S, double2 *const *H, c
             j[2 * k + 1].ldo = ld[k];
         }
     }
+}
+
+// The T application of the complex forms, on CTA-pair tiles as well: 272 us for 8 atoms, lmax 8, 1501 columns (507
+// on single-CTA tiles), 161 for 2 atoms, lmax 1, 100 columns (207), 602 for 16, lmax 10, 1500 (813).
+static cudaError_t launch_t(const OzGroup *g, const OzJob *jobs, int n_jobs, int64_t tiles, const int4 *list, cudaStream_t st) {
+    return g->pair ? launch_pair(g->maps_t, g->s, g->d_err, jobs, n_jobs, tiles, list, nullptr, st)
+                   : launch_prepared(g->maps_t, g->s, g->d_err, jobs, n_jobs, tiles, list, nullptr, st);
 }
 
 // Events around the S/H launch; under stream capture they become external event-record nodes
@@ -2429,8 +2436,7 @@ int ozaki_group_run(OzGroup *g, const DevSystem &sys, const KTable &ktab, cudaSt
         e = slice_launch(g->tM, st);
         if (e == cudaSuccess && tev) e = cudaEventRecord(ev_t[0], st);
         if (e == cudaSuccess)
-            e = launch_prepared(g->maps_t, g->s, g->d_err, g->d_jobs_t, g->n_jobs_t, g->tiles_t, g->d_list_t, nullptr,
-                                st);
+            e = launch_t(g, g->d_jobs_t, g->n_jobs_t, g->tiles_t, g->d_list_t, st);
         if (e == cudaSuccess && tev) e = cudaEventRecord(ev_t[1], st);
         nl += 2;
     }
@@ -2451,8 +2457,7 @@ int ozaki_group_run(OzGroup *g, const DevSystem &sys, const KTable &ktab, cudaSt
             } else {
                 if (tev) e = cudaEventRecord(ev_t[2 * pi], st);
                 if (e == cudaSuccess)
-                    e = launch_prepared(g->maps_t, g->s, g->d_err, g->d_jobs_t + p.jt_off, p.n_jobs_t, p.tiles_t,
-                                        g->d_list_t + p.lt_off, nullptr, st);
+                    e = launch_t(g, g->d_jobs_t + p.jt_off, p.n_jobs_t, p.tiles_t, g->d_list_t + p.lt_off, st);
                 if (e == cudaSuccess && tev) e = cudaEventRecord(ev_t[2 * pi + 1], st);
             }
             nl += 1;

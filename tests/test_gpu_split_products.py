@@ -45,3 +45,27 @@ def test_split_matches_whole(torch, n, k, slices):
     for X in (a.T, c.T):
         fro, mx = oracle.lower_errors(X, R)
         assert fro < tol and mx < tol, (n, k, fro, mx)
+
+
+@pytest.mark.parametrize("lmax,types,n_g", [(1, 2, 40), (3, 3, 257), (7, 2, 300), (8, 2, 130), (10, 2, 513)])
+def test_t_application_on_pair_tiles(torch, monkeypatch, lmax, types, n_g):
+    """T applied per type and per atom on 256 x 256 tiles that reach past a type's 2L rows (8, 32, 128, 162 and 242:
+    the rows of the next type or plane, or past the last)."""
+    from hybridhsdla_gb300 import synth
+    cfg = dict(cell=(10.0, 10.5, 11.0), atoms=5, types=types, rmt=2.0, min_sep=3.9, lmax=lmax,
+               kpts=[(0.1, 0.2, 0.3)], n_g=n_g, seed=lmax)
+    ctx = api.Context()
+    try:
+        for rot in (False, True):
+            s = synth.make_system(cfg)
+            s = synth.with_rotations(s) if rot else s
+            monkeypatch.setenv("HSDLA_SF", "0")
+            monkeypatch.setenv("HSDLA_CLASSES", "0")
+            ((H, S),), rep = ctx.create_hs(s, precision="ozaki", num_slices=11)
+            assert rep["num_row_sets"] == 0
+            Hr, Sr = oracle.reference_hs(s, s.kpoints[0])
+            for X, R in ((H, Hr), (S, Sr)):
+                fro, mx = oracle.lower_errors(X, R)
+                assert fro < 1e-13 and mx < 1e-13, (lmax, rot, fro, mx)
+    finally:
+        ctx.close()
