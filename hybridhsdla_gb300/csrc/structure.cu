@@ -130,7 +130,7 @@ constexpr int kSfTile = 32;
 // arrive in one of two stages of shared memory by asynchronous copies while the item before is summed.
 // kFixed: fixed-point products and structure factors, summed exactly in integers.  GB300's FP64 pipe
 // (2 multiply-adds per cycle and SM) bounded this kernel at 0.95 of its rate.  8000 columns of 8 types:
-// FP64 2.60 ms, integers 1.44 ms (0.63 of the DRAM rate); 2 k-points of 6300 columns and 4 types: 1.74 and 1.18
+// FP64 2.60 ms, integers 1.42 ms (0.64 of the DRAM rate); 2 k-points of 6300 columns and 4 types: 1.74 and 1.16
 // ms.  Bound now by the wide multiply-adds (a warp's takes four cycles; 24 an element and type) on 16 warps an
 // SM; 20 warps leave too little L1 beside the stages (1.67 and 1.44 ms).  Loads into registers, four types
 // ahead of their use on 24 warps, took 1.59 and 1.41 ms.
@@ -172,6 +172,10 @@ struct Sums<true> {
         hi.add(y, w.z, w.w);
     }
 };
+
+// (a call: the additions that a batch does not need would issue all the same, predicated off: 1.42 ms of the
+// 8000 columns above, 1.44 inlined)
+__device__ __noinline__ double2 sum2(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 
 template <bool kFixed, int kRows>
 __global__ void __launch_bounds__(kSfTile *kRows, 512 / (kSfTile * kRows)) sf_combine_kernel(const __grid_constant__ SfTab tab,
@@ -269,7 +273,7 @@ __global__ void __launch_bounds__(kSfTile *kRows, 512 / (kSfTile * kRows)) sf_co
                     // one power of two for every type's products of an element
                     const double2 s = make_double2(v.sr.value(ks), v.si.value(ks)), h = make_double2(v.hr.value(kh), v.hi.value(kh));
                     if (q < kSumItems) { vs = s; vh = h; }
-                    else { vs.x += s.x; vs.y += s.y; vh.x += h.x; vh.y += h.y; }
+                    else { vs = sum2(vs, s); vh = sum2(vh, h); }
                     v = Sums<kFixed>();
                 }
             }
@@ -284,8 +288,8 @@ __global__ void __launch_bounds__(kSfTile *kRows, 512 / (kSfTile * kRows)) sf_co
         double2 *so = x ? E.Sx + row + E.ldx * col : E.S + oo, *ho = x ? E.Hx + row + E.ldx * col : E.H + oo;
         if (!first) {
             const double2 s0 = E.Si[row + E.ldi * col], h0 = E.Hi[row + E.ldi * col];
-            vs.x += s0.x; vs.y += s0.y;
-            vh.x += h0.x; vh.y += h0.y;
+            vs = sum2(vs, s0);
+            vh = sum2(vh, h0);
         }
         *so = vs;
         *ho = vh;
