@@ -48,7 +48,7 @@ WORKLOAD_TEXT = {
     "c2t1": "c2t1: c2's cell and n_G 8000 with 16 atoms of one type (one per-type S/H launch of c2's shape)",
     "c2r": "c2r: c2 with per-atom rotations, the atoms of each type in two rotation classes (16 classes)",
 }
-PROFILE_SUMMARY = os.path.join(ROOT, "profiles", "oz_pair_c2.md")
+PROFILE_SUMMARY = os.path.join(ROOT, "profiles", "structure_factor_form_c2.md")
 
 
 def _peaks():
@@ -408,8 +408,8 @@ def run_ours(args):
     traffic = _traffic_from_profile() if args.workload == "c2" else None
     roof = {"bound": "tensor", "achieved": achieved, "peak": fp8_peak, "unit": "TFLOP/s",
             "frac": achieved / fp8_peak, "traffic": traffic,
-            "kernel": "oz_pair_kernel (one type's S and H lower-triangle digit products per launch, "
-                      "CTA-pair 256x256 tiles; achieved and traffic per launch)",
+            "kernel": "oz_real_kernel (the types' S and H lower-triangle digit products, CTA-pair 256x128 tiles; "
+                      "achieved and traffic per launch)",
             "peak_source": f"2 x {src} bf16 burst (FP8 e4m3 dense rate = 2x bf16 on tcgen05)"}
 
     cpu = None

@@ -11,7 +11,7 @@
 //        z ~= sum_i d_i 2^(1-5i),  d_1 in [-16,16],  d_i in [-16,15]  (i >= 2).
 //    Every digit is an integer of magnitude <= 16, exactly representable in
 //    e4m3; one byte plane per (digit, re/im).  The digit extraction runs in
-//    64-bit integer arithmetic (one FP64 multiply and one conversion per value):
+//    64-bit integer arithmetic (one FP64 multiply per weighted value):
 //    GB300's FP64 pipe delivers ~1 TFLOP/s, its integer pipes far more.
 //  * products (oz_gemm_kernel): for the output tile (rows g, cols g') and each
 //    diagonal t = i + j of the digit-product triangle (t = 2..s+1), the FP32
@@ -22,8 +22,11 @@
 //    partial sum an exactly representable integer; chunks are drained into the
 //    FP64 output tile with weight 2^(2-5t), and the last drain applies
 //    2^(e_g + e_g').
+//  * the structure-factor form's products are real ones (real_products.cu); here are the complex products of
+//    the per-atom form, the contraction entry and the plugin (oz_pair_kernel on CTA pairs; oz_gemm_kernel
+//    where no pairs are to be used), and the groups' set-up and runs.
 //
-// GB300 mapping: persistent CTAs (one per SM, 512 TMEM columns = two 128x(128
+// oz_gemm_kernel: persistent CTAs (one per SM, 512 TMEM columns = two 128x(128
 // re + 128 im) FP32 accumulators), warp-specialised: one TMA producer warp
 // (SW128 K-major 128x128-byte boxes, 64 KB per stage, 3 stages), one MMA warp
 // (single elected issuer, tcgen05.commit to release stages and publish
