@@ -130,7 +130,7 @@ constexpr int kSfTile = 32;
 // arrive in one of two stages of shared memory by asynchronous copies while the item before is summed.
 // kFixed: fixed-point products and structure factors, summed exactly in integers.  GB300's FP64 pipe
 // (2 multiply-adds per cycle and SM) bounded this kernel at 0.95 of its rate.  8000 columns of 8 types:
-// FP64 2.60 ms, integers 1.42 ms (0.64 of the DRAM rate); 2 k-points of 6300 columns and 4 types: 1.74 and 1.16
+// FP64 2.60 ms, integers 1.39 ms (0.66 of the DRAM rate); 2 k-points of 6300 columns and 4 types: 1.74 and 1.13
 // ms.  Bound now by the wide multiply-adds (a warp's takes four cycles; 24 an element and type) on 16 warps an
 // SM; 20 warps leave too little L1 beside the stages (1.67 and 1.44 ms).  Loads into registers, four types
 // ahead of their use on 24 warps, took 1.59 and 1.41 ms.
@@ -173,8 +173,8 @@ struct Sums<true> {
     }
 };
 
-// (a call: the additions that a batch does not need would issue all the same, predicated off: 1.42 ms of the
-// 8000 columns above, 1.44 inlined)
+// (a call: the additions that a batch does not need would issue all the same, predicated off: 1.44 ms of the
+// 8000 columns above where this took 1.42)
 __device__ __noinline__ double2 sum2(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 
 template <bool kFixed, int kRows>
@@ -263,9 +263,14 @@ __global__ void __launch_bounds__(kSfTile *kRows, 512 / (kSfTile * kRows)) sf_co
             const int n = min(kChunk, ntypes - kChunk * q);
             const int4 *w = reinterpret_cast<const int4 *>(mem + stage * kStageBytesWarp) + lane * kSfPitch;
             const int2 *p = reinterpret_cast<const int2 *>(mem + stage * kStageBytesWarp + kStageSf) + lane;
+            if (n == kChunk) {
+                // (no branch between the types: their multiply-adds interleave; 1.42 and 1.16 ms with one)
 #pragma unroll
-            for (int t = 0; t < kChunk; ++t)
-                if (t < n) v.add(p[3 * t * kSfTile], p[(3 * t + 1) * kSfTile], p[(3 * t + 2) * kSfTile], w[t]);
+                for (int t = 0; t < kChunk; ++t) v.add(p[3 * t * kSfTile], p[(3 * t + 1) * kSfTile], p[(3 * t + 2) * kSfTile], w[t]);
+            } else {
+#pragma unroll 1
+                for (int t = 0; t < n; ++t) v.add(p[3 * t * kSfTile], p[(3 * t + 1) * kSfTile], p[(3 * t + 2) * kSfTile], w[t]);
+            }
             __syncwarp();
             stage ^= 1;
             if constexpr (kFixed) {
