@@ -139,9 +139,9 @@ struct Fp64Job {
     int32_t tiles_n;                 // tile columns of this job
     int64_t tile_begin;              // first global tile index of this job
 };
-constexpr int kFp64Tile = 64;
-int64_t fp64_job_tiles(const Fp64Job &j);
-cudaError_t launch_fp64_jobs(const Fp64Job *d_jobs, int num_jobs, int64_t total_tiles, cudaStream_t st);
+// As fp64_real_assign, below.
+int64_t fp64_assign(Fp64Job *jobs, int num_jobs, int *edge);
+cudaError_t launch_fp64_jobs(const Fp64Job *d_jobs, int num_jobs, int64_t total_tiles, int edge, cudaStream_t st);
 
 // Real FP64 contraction out = P^T diag(w) Q over a batch of jobs (the structure-factor form's real
 // rows, see real_products.cu): P k x m, Q k x n, out m x n, column-major.

@@ -117,7 +117,7 @@ struct hsdla_plan {
         int64_t tiles_sh = 0;
         // FP64 structure-factor form: real jobs (device), the products' in one launch per combine batch
         Fp64RealJob *d_rjobs_t = nullptr, *d_rjobs_sh = nullptr;
-        int edge_t = 0;
+        int edge_t = 0, edge_sh = 0;
         std::vector<RealBatch> batches;
         void *persist = nullptr;         // prepared tables (not shared with other groups)
         int64_t persist_bytes = 0;
@@ -593,16 +593,6 @@ int upload_jobs(hsdla_plan *pl, cudaStream_t st) {
     return HSDLA_OK;
 }
 
-int64_t assign_tiles(std::vector<Fp64Job> &jobs, size_t first) {
-    int64_t t = 0;
-    for (size_t i = first; i < jobs.size(); ++i) {
-        jobs[i].tiles_n = (int32_t)((jobs[i].n + kFp64Tile - 1) / kFp64Tile);
-        jobs[i].tile_begin = t;
-        t += fp64_job_tiles(jobs[i]);
-    }
-    return t;
-}
-
 // Lower-triangle relative errors (Frobenius, max) of X against R, both n x n column-major.
 void lower_errors(const std::vector<std::complex<double>> &X, const std::vector<std::complex<double>> &R, int64_t n,
                   double &fro, double &mx) {
@@ -672,7 +662,8 @@ int autotune_slices(hsdla_plan *pl, double2 *C, cudaStream_t st) {
         jb.m = twoL; jb.n = ns; jb.k = twoL;
         pl->h_jobs.push_back(jb);
     }
-    const int64_t t1 = assign_tiles(pl->h_jobs, 0);
+    int e1 = 0, e2 = 0;
+    const int64_t t1 = fp64_assign(pl->h_jobs.data(), (int)pl->h_jobs.size(), &e1);
     const size_t nb = pl->h_jobs.size();
     Fp64Job js{};
     js.P = Cs; js.ldp = K; js.Q = Cs; js.ldq = K; js.w = pl->w; js.out = Sr; js.ldo = ns;
@@ -681,10 +672,10 @@ int autotune_slices(hsdla_plan *pl, double2 *C, cudaStream_t st) {
     jh.Q = Xs; jh.w = nullptr; jh.out = Hr;
     pl->h_jobs.push_back(js);
     pl->h_jobs.push_back(jh);
-    const int64_t t2 = assign_tiles(pl->h_jobs, nb);
+    const int64_t t2 = fp64_assign(pl->h_jobs.data() + nb, 2, &e2);
     if (upload_jobs(pl, st)) return fail(HSDLA_ERR_CUDA, "job upload");
-    if (launch_fp64_jobs(pl->d_jobs, (int)nb, t1, st) != cudaSuccess ||
-        launch_fp64_jobs(pl->d_jobs + nb, 2, t2, st) != cudaSuccess)
+    if (launch_fp64_jobs(pl->d_jobs, (int)nb, t1, e1, st) != cudaSuccess ||
+        launch_fp64_jobs(pl->d_jobs + nb, 2, t2, e2, st) != cudaSuccess)
         return fail(HSDLA_ERR_CUDA, "fp64 sample");
     // Ozaki at the probe slice count (overwrites Xs after the FP64 H job, in stream order)
     OzakiInputs in;
@@ -1470,8 +1461,8 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
                 jsh.push_back(js);
                 jsh.push_back(jh);
             }
-            g.tiles_t = assign_tiles(jt, 0);
-            g.tiles_sh = assign_tiles(jsh, 0);
+            g.tiles_t = fp64_assign(jt.data(), (int)jt.size(), &g.edge_t);
+            g.tiles_sh = fp64_assign(jsh.data(), (int)jsh.size(), &g.edge_sh);
             g.n_jobs_t = (int)jt.size();
             g.d_jobs_t = reinterpret_cast<Fp64Job *>(keep(sizeof(Fp64Job) * jt.size()));
             g.d_jobs_sh = reinterpret_cast<Fp64Job *>(keep(sizeof(Fp64Job) * jsh.size()));
@@ -1713,7 +1704,7 @@ int run_groups(hsdla_plan *pl, cudaStream_t st, bool timed, float *ms_ab, float 
             }
         } else {
             if (timed) CUDA_TRY(ctx, cudaEventRecord(g.ev_t[0], st));
-            CUDA_TRY(ctx, launch_fp64_jobs(g.d_jobs_t, g.n_jobs_t, g.tiles_t, st));
+            CUDA_TRY(ctx, launch_fp64_jobs(g.d_jobs_t, g.n_jobs_t, g.tiles_t, g.edge_t, st));
             if (timed) CUDA_TRY(ctx, cudaEventRecord(g.ev_t[1], st));
             pl->launches++;
             if (pl->hoist) {
@@ -1723,7 +1714,7 @@ int run_groups(hsdla_plan *pl, cudaStream_t st, bool timed, float *ms_ab, float 
             CUDA_TRY(ctx, cudaMemcpyAsync(g.d_jobs_sh, g.h_jobs_sh, sizeof(Fp64Job) * 2 * g.ktab.nk,
                                           cudaMemcpyHostToDevice, st));
             CUDA_TRY(ctx, record_event(g.ev_dom[0], st));
-            CUDA_TRY(ctx, launch_fp64_jobs(g.d_jobs_sh, 2 * g.ktab.nk, g.tiles_sh, st));
+            CUDA_TRY(ctx, launch_fp64_jobs(g.d_jobs_sh, 2 * g.ktab.nk, g.tiles_sh, g.edge_sh, st));
             CUDA_TRY(ctx, record_event(g.ev_dom[1], st));
             pl->launches++;
         }
@@ -2316,12 +2307,13 @@ int hsdla_zherkx_lower(hsdla_context *ctx, int32_t precision, int32_t num_slices
         j.Q = reinterpret_cast<const double2 *>(dQ); j.ldq = ldq;
         j.w = dw; j.out = reinterpret_cast<double2 *>(dOut); j.ldo = ldo;
         j.m = n; j.n = n; j.k = k; j.lower = 1;
-        const int64_t tiles = assign_tiles(jobs, 0);
+        int edge = 0;
+        const int64_t tiles = fp64_assign(jobs.data(), 1, &edge);
         void *dj = nullptr;
         int rc = ctx_malloc(ctx, &dj, sizeof(Fp64Job));
         if (rc) return rc;
         cudaError_t e = cudaMemcpyAsync(dj, jobs.data(), sizeof(Fp64Job), cudaMemcpyHostToDevice, st);
-        if (e == cudaSuccess) e = launch_fp64_jobs((Fp64Job *)dj, 1, tiles, st);
+        if (e == cudaSuccess) e = launch_fp64_jobs((Fp64Job *)dj, 1, tiles, edge, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         ctx_free(ctx, dj, sizeof(Fp64Job));
         if (e != cudaSuccess) return set_err(ctx, HSDLA_ERR_CUDA, "zherkx fp64: %s", cudaGetErrorString(e));
@@ -2477,10 +2469,11 @@ int plugin_contract(hsdla_context *ctx, int kind, int32_t precision, int32_t num
             Fp64Job &j = jobs[0];
             j.P = P; j.ldp = ldp; j.Q = Q; j.ldq = ldq; j.w = nullptr;
             j.out = R; j.ldo = ldr; j.m = n; j.n = n; j.k = K; j.lower = 1;
-            const int64_t tiles = assign_tiles(jobs, 0);
+            int edge = 0;
+            const int64_t tiles = fp64_assign(jobs.data(), 1, &edge);
             Fp64Job *dj = reinterpret_cast<Fp64Job *>(ws + oJ);
             CUDA_TRY(ctx, cudaMemcpyAsync(dj, jobs.data(), sizeof(Fp64Job), cudaMemcpyHostToDevice, st));
-            CUDA_TRY(ctx, launch_fp64_jobs(dj, 1, tiles, st));
+            CUDA_TRY(ctx, launch_fp64_jobs(dj, 1, tiles, edge, st));
         } else {
             rc = ozaki_plan_init(ctx->plugin_oz, s, 1e-13);
             if (rc) return set_err(ctx, rc, "%s: %s", nm, ozaki_last_error());

@@ -1,0 +1,38 @@
+"""The complex FP64 products (csrc/contract_fp64.cu) on both tile shapes: small launches on 16 x 16 tiles with the
+contraction split over four warps, large ones on 32 x 32.  Ends of tiles and of the contraction's steps of four
+(and fewer steps than warps), with and without row weights, against numpy.  Tolerance: 1e-13 (relative
+Frobenius and max-norm of the lower triangle), as for every FP64 product here."""
+import numpy as np
+import pytest
+
+import oracle
+from hybridhsdla_gb300 import api
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no GPU")
+    c = api.Context()
+    yield c
+    c.close()
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+@pytest.mark.parametrize("n,k", [(1, 1), (15, 3), (16, 4), (17, 13), (31, 162), (33, 98), (250, 17), (481, 242),
+                                 (1552, 6), (1601, 33), (2113, 50)])
+def test_fp64_tiles(ctx, n, k, weighted):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    P, Q = (torch.complex(torch.randn((n, k), generator=g, device="cuda", dtype=torch.float64),
+                          torch.randn((n, k), generator=g, device="cuda", dtype=torch.float64)) for _ in range(2))
+    w = torch.rand(k, generator=g, device="cuda", dtype=torch.float64) + 0.5 if weighted else None
+    X = ctx.zherkx_lower(P, Q, w, precision="fp64").cpu().numpy().T
+    Pn, Qn = P.cpu().numpy().T, Q.cpu().numpy().T
+    R = Pn.conj().T @ (w.cpu().numpy()[:, None] * Qn if weighted else Qn)
+    fro, mx = oracle.lower_errors(X, R)
+    assert fro < 1e-13 and mx < 1e-13, (n, k, fro, mx)
+    assert not np.triu(X, 1).any()
