@@ -165,8 +165,9 @@ struct hsdla_plan {
         int blocks = 0;          // ... in column blocks while the products of the next ran (0: after them)
     };
     Download *dl = nullptr;
-    void *split = nullptr;           // memory for splitting the S/H products (hsdla_contract_ab), or null
-    int64_t split_bytes = 0;
+    // memory for splitting the S/H products' and the T application's tiles (hsdla_contract_ab), or null
+    void *split = nullptr, *split_t = nullptr;
+    int64_t split_bytes = 0, split_t_bytes = 0;
     double est_err = 0.0;            // autotuner's predicted relative error
     int launches = 0;
     bool tiles_tuned = false;        // the S/H tile configuration came from the tile tuner
@@ -1374,6 +1375,7 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
             d.w = pl->w; d.Tfull = pl->Tfull; d.atom_type = pl->atom_type.data();
             d.panels = pl->panels;
             d.split = pl->split; d.split_bytes = pl->split_bytes;
+            d.split_t = pl->split_t; d.split_t_bytes = pl->split_t_bytes;
             d.sf = pl->sf; d.wt = pl->wt; d.TR = pl->TR; d.sf_tab = pl->sf_tab; d.tbatch = pl->tbatch;
             char *oz_ws = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(p) + 1023) & ~uintptr_t(1023));
             int rc = ozaki_group_prepare(pl->oz, d, kb, oz_ws, g.persist, st, &g.oz);
@@ -2053,10 +2055,14 @@ int hsdla_contract_ab(hsdla_context *ctx, int32_t L, int32_t a, int64_t G, const
         if (rc) return done(set_err(ctx, rc, "bad slice count"));
     }
     form_groups(pl, workspace_budget(ctx));
-    if (pl->opts.precision == HSDLA_PREC_OZAKI_FP8)
+    if (pl->opts.precision == HSDLA_PREC_OZAKI_FP8) {
         pl->split_bytes = ozaki_split_bytes(pl->oz.num_slices, (twoL + 15) / 16 * 16 * a, G, 2);
-    rc = ctx_workspace_tail(ctx, hsdla_plan_workspace_bytes(pl), pl->split_bytes, &ws, &pl->split);
+        pl->split_t_bytes = ozaki_split_bytes_t(pl->oz.num_slices, twoL, G, a);
+    }
+    rc = ctx_workspace_tail(ctx, hsdla_plan_workspace_bytes(pl), pl->split_bytes + pl->split_t_bytes, &ws, &pl->split);
     if (rc) return done(rc);
+    if (pl->split && pl->split_t_bytes > 0) pl->split_t = static_cast<char *>(pl->split) + pl->split_bytes;
+    if (pl->split_bytes == 0) pl->split = nullptr;
     rc = prepare_groups(pl, ws, st);
     if (rc) return done(rc);
     rc = ctx_host_out(ctx, 2 * G * G * (int64_t)sizeof(double2), &dout);

@@ -1487,7 +1487,7 @@ struct OzGroup {
     int *d_progress = nullptr;
     int *d_err = nullptr;
     bool pair = false;          // S/H on CTA-pair tiles
-    PairSplit split;
+    PairSplit split, split_t;   // of the S/H products' and the T application's tiles
     bool sf = false;            // structure-factor form, on real rows:
     RealSliceTab rM, rX;        // the slicing of R (and R diag(w)) and of Z'
     RealJob *d_rjobs_t = nullptr, *d_rjobs_sh = nullptr;   // T application; 3 nk products per type
@@ -1730,14 +1730,26 @@ cudaError_t launch_prepared(const CUtensorMap *maps, int s, int *d_err, const Oz
 
 }  // namespace
 
+namespace {
+int64_t split_bytes(int64_t N, int64_t steps) {
+    SplitRule r;
+    if (!split_rule(N, steps, r)) return 0;
+    // at most P - 1 parts do not begin a tile; entries of whole waves and of up to P tiles a pair in the last
+    return round_up(r.P * kSlabBytes + 32 * (N + (2 + (r.R + r.P - 1) / r.P) * r.np) + 32 * r.R, 1024);
+}
+int64_t pair_steps(int s, int64_t K) { return round_up(std::max<int64_t>(K, 1), kKBlock) / kKBlock * s * (s + 1) / 2; }
+}  // namespace
+
 // Memory with which ozaki_herkx, or a group, splits the tiles of a partial last wave: `jobs` lower products
 // of n columns over K rows (0: they would not be split).
 int64_t ozaki_split_bytes(int s, int64_t K, int64_t n, int64_t jobs) {
-    const int64_t T = (n + kPairTile - 1) / kPairTile, N = jobs * T * (T + 1) / 2;
-    SplitRule r;
-    if (!split_rule(N, round_up(std::max<int64_t>(K, 1), kKBlock) / kKBlock * s * (s + 1) / 2, r)) return 0;
-    // at most P - 1 parts do not begin a tile; entries of whole waves and of up to P tiles a pair in the last
-    return r.P * kSlabBytes + round_up(32 * (N + (2 + (r.R + r.P - 1) / r.P) * r.np) + 32 * r.R, 1024);
+    const int64_t T = (n + kPairTile - 1) / kPairTile;
+    return split_bytes(jobs * T * (T + 1) / 2, pair_steps(s, K));
+}
+// ... or `jobs` T applications of m rows and n columns.
+int64_t ozaki_split_bytes_t(int s, int64_t m, int64_t n, int64_t jobs) {
+    const int64_t tm = (m + kPairTile - 1) / kPairTile, tn = (n + kPairTile - 1) / kPairTile;
+    return split_bytes(jobs * tm * tn, pair_steps(s, m));
 }
 
 // P^H diag(w) Q (lower triangle) for one pair of K x n operands: the contraction behind
@@ -2189,7 +2201,8 @@ int ozaki_group_prepare(OzakiPlan &oz, const OzGroupDesc &d, const std::vector<O
             p.jt_off = joff;
             p.lt_off = loff;
             p.n_jobs_t = (int)jt.size();
-            rc = upload_schedule(jt, g->d_jobs_t + joff, g->d_list_t + loff, p.tiles_t, tile);
+            rc = upload_schedule(jt, g->d_jobs_t + joff, g->d_list_t + loff, p.tiles_t, tile, &g->split_t, tkb * s * (s + 1) / 2,
+                                 g->pair && g->panels == 1 ? d.split_t : nullptr, d.split_t_bytes);
             if (rc) return fail(rc);
             joff += p.n_jobs_t;
             loff += p.tiles_t;
@@ -2264,8 +2277,10 @@ void ozaki_group_set_outputs(OzGroup *g, double2 *const *S, double2 *const *H, c
 
 // The T application of the complex forms, on CTA-pair tiles as well: 272 us for 8 atoms, lmax 8, 1501 columns (507
 // on single-CTA tiles), 161 for 2 atoms, lmax 1, 100 columns (207), 602 for 16, lmax 10, 1500 (813).
+// Cut over the idle pairs (the contraction entry): 236 us of the first; 1 atom, lmax 7, 232 columns 184 -> 68, 4 atoms,
+// lmax 8, 400 columns 268 -> 91.
 static cudaError_t launch_t(const OzGroup *g, const OzJob *jobs, int n_jobs, int64_t tiles, const int4 *list, cudaStream_t st) {
-    return g->pair ? launch_pair(g->maps_t, g->s, g->d_err, jobs, n_jobs, tiles, list, nullptr, st)
+    return g->pair ? launch_pair(g->maps_t, g->s, g->d_err, jobs, n_jobs, tiles, list, nullptr, st, &g->split_t)
                    : launch_prepared(g->maps_t, g->s, g->d_err, jobs, n_jobs, tiles, list, nullptr, st);
 }
 

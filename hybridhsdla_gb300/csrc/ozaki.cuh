@@ -67,6 +67,8 @@ struct OzGroupDesc {
     const int32_t *d_set_type = nullptr;   // and device
     void *split = nullptr;                 // ozaki_split_bytes for the S/H products, or null
     int64_t split_bytes = 0;
+    void *split_t = nullptr;               // ozaki_split_bytes_t for the per-atom T application, or null
+    int64_t split_t_bytes = 0;
 };
 struct OzGroup;
 // scratch: rewritten by every run (may be shared by the groups of a plan); persist: owned by
@@ -122,6 +124,7 @@ int ozaki_plan_init(OzakiPlan &oz, int num_slices, double target);
 void ozaki_plan_release(OzakiPlan &oz);
 int64_t ozaki_pipeline_workspace(int s, int64_t twoL, int64_t na, int64_t nt, int64_t G);
 int64_t ozaki_split_bytes(int s, int64_t K, int64_t n, int64_t jobs);
+int64_t ozaki_split_bytes_t(int s, int64_t m, int64_t n, int64_t jobs);
 int64_t ozaki_herkx_workspace(int s, int64_t K, int64_t n);
 // S = C^H diag(w) C and H = C^H (T C) (lower triangles) with the T application emulated too.
 int ozaki_pipeline(OzakiPlan &oz, const OzakiInputs &in, double2 *S, double2 *H, int64_t ldo, void *ws,

@@ -69,3 +69,33 @@ def test_t_application_on_pair_tiles(torch, monkeypatch, lmax, types, n_g):
                 assert fro < 1e-13 and mx < 1e-13, (lmax, rot, fro, mx)
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("lmax,atoms,G", [(1, 1, 9), (6, 1, 200), (8, 2, 300), (9, 7, 257), (10, 3, 600)])
+def test_contraction_with_split_t(torch, lmax, atoms, G):
+    """T applications of few tiles cut over the pairs (one and two k-blocks), then S and H, against the oracle, a
+    capped context (nothing cut) and a second call, bit for bit."""
+    from hybridhsdla_gb300 import flapw_data
+    L = (lmax + 1) ** 2
+    rng = np.random.default_rng(lmax * 1000 + G)
+    cx = lambda *sh: rng.standard_normal(sh) + 1j * rng.standard_normal(sh)
+    blocks = []
+    for _ in range(atoms):
+        aa, bb = cx(L, L), cx(L, L)
+        blocks.append((aa + aa.conj().T, cx(L, L), bb + bb.conj().T))
+    d = flapw_data.DataIn(L, atoms, G, np.asfortranarray(cx(L * atoms, G)), np.asfortranarray(cx(L * atoms, G)), blocks,
+                          np.full(atoms, lmax, np.int32), lmax, np.sqrt(rng.uniform(0.1, 1.0, (atoms, lmax + 1))))
+    ctx, capped = api.Context(), api.Context()
+    try:
+        capped.set_mem_cap(1 << 34)
+        H, S, _ = ctx.contract_ab(d, precision="ozaki", num_slices=11)
+        H2, S2, _ = ctx.contract_ab(d, precision="ozaki", num_slices=11)
+        Hc, Sc, _ = capped.contract_ab(d, precision="ozaki", num_slices=11)
+    finally:
+        ctx.close()
+        capped.close()
+    assert np.array_equal(H, H2) and np.array_equal(S, S2)
+    Hr, Sr = oracle.stripped_v2(d.L, d.a, d.A, d.B, d.blocks, d.lmaxs, d.max_lmax, d.sqrt_u_norms)
+    for X, R in ((H, Hr), (S, Sr), (Hc, Hr), (Sc, Sr)):
+        fro, mx = oracle.lower_errors(X, R)
+        assert fro < 1e-13 and mx < 1e-13, (lmax, atoms, G, fro, mx)
