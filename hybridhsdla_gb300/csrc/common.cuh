@@ -139,8 +139,10 @@ struct Fp64Job {
     int32_t tiles_n;                 // tile columns of this job
     int64_t tile_begin;              // first global tile index of this job
 };
-// As fp64_real_assign, below.
-int64_t fp64_assign(Fp64Job *jobs, int num_jobs, int *edge);
+// The tile edge for a launch (or all launches that are to sum in one order) of `tiles32` tiles of edge 32.
+int fp64_edge(int64_t tiles32);
+// Numbers the jobs' tiles for one launch and returns their count.
+int64_t fp64_assign(Fp64Job *jobs, int num_jobs, int edge);
 cudaError_t launch_fp64_jobs(const Fp64Job *d_jobs, int num_jobs, int64_t total_tiles, int edge, cudaStream_t st);
 
 // Real FP64 contraction out = P^T diag(w) Q over a batch of jobs (the structure-factor form's real
@@ -155,9 +157,7 @@ struct Fp64RealJob {
     int32_t tiles_n;                 // tile columns of this job
     int64_t tile_begin;              // first global tile index of this job
 };
-// Numbers the jobs' tiles for one launch and returns their count; `edge` receives the tile edge
-// chosen for the launch (what launch_fp64_real needs back).
-int64_t fp64_real_assign(Fp64RealJob *jobs, int num_jobs, int *edge);
+int64_t fp64_real_assign(Fp64RealJob *jobs, int num_jobs, int edge);
 cudaError_t launch_fp64_real(const Fp64RealJob *d_jobs, int num_jobs, int64_t tiles, int edge, cudaStream_t st);
 
 // ---- structure-factor form (atoms sharing their type's rotation)

@@ -42,7 +42,7 @@ __device__ __forceinline__ void tile_of(const Fp64Job &j, int64_t x, int64_t &ti
 // Complex DMMA products (the per-atom form, the contraction entry, the plugin), as fp64_real_kernel (below) with
 // both parts of an element in one CTA: bound by GB300's FP64 rate at every shape, so fragments come straight
 // from global memory and what counts is an even share of the MMAs per SM.  A tile of 32 x 32, a 16 x 16 quarter per
-// warp, or of 16 x 16 with the contraction split over the warps (fp64_assign).  Lower triangle of P^H Q of n columns
+// warp, or of 16 x 16 with the contraction split over the warps (fp64_edge).  Lower triangle of P^H Q of n columns
 // over k rows, ms, here and on the staged 64 x 64 tiles before: n 200, k 400 0.18 and 1.94; n 200, k 1200 0.42 and
 // 5.69; n 700, k 1200 2.6 and 5.7; n 2200, k 1200 22.5 and 27.7; n 6000, k 1000 136 and 140.  Relative error (Frobenius,
 // against extended precision, k 700) 6.5e-16 and 1.3e-15.
@@ -242,25 +242,31 @@ __global__ void __launch_bounds__(128) fp64_real_kernel(const Fp64RealJob *__res
 
 }  // namespace
 
-int64_t fp64_real_assign(Fp64RealJob *jobs, int num_jobs, int *edge) {
-    int dev = 0, nsm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+namespace {
+template <typename Job>
+int64_t assign(Job *jobs, int num_jobs, int edge) {
     int64_t total = 0;
-    for (int e = 32; e >= 16; e /= 2) {
-        total = 0;
-        for (int i = 0; i < num_jobs; ++i) {
-            Fp64RealJob &j = jobs[i];
-            const int64_t tm = (j.m + e - 1) / e, tn = (j.n + e - 1) / e;
-            j.tiles_n = (int32_t)tn;
-            j.tile_begin = total;
-            total += j.lower ? tm * (tm + 1) / 2 : tm * tn;
-        }
-        *edge = e;
-        if (total >= (int64_t)kSplitBelow * nsm) break;
+    for (int i = 0; i < num_jobs; ++i) {
+        Job &j = jobs[i];
+        const int64_t tm = (j.m + edge - 1) / edge, tn = (j.n + edge - 1) / edge;
+        j.tiles_n = (int32_t)tn;
+        j.tile_begin = total;
+        total += j.lower ? tm * (tm + 1) / 2 : tm * tn;
     }
     return total;
 }
+}  // namespace
+
+// Tiles of 32 from kSplitBelow of them per SM on (complex products, n 2200: 22.5 ms, 22.9 on tiles of 16), else of 16
+// (n 1500, k 1200: 10.8 ms, 11.3 on tiles of 32; n 200, k 1200: 0.42, 1.48).
+int fp64_edge(int64_t tiles32) {
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    return tiles32 >= (int64_t)kSplitBelow * nsm ? 32 : 16;
+}
+int64_t fp64_assign(Fp64Job *jobs, int num_jobs, int edge) { return assign(jobs, num_jobs, edge); }
+int64_t fp64_real_assign(Fp64RealJob *jobs, int num_jobs, int edge) { return assign(jobs, num_jobs, edge); }
 
 cudaError_t launch_fp64_real(const Fp64RealJob *d_jobs, int num_jobs, int64_t tiles, int edge, cudaStream_t st) {
     if (tiles <= 0) return cudaSuccess;
@@ -268,28 +274,6 @@ cudaError_t launch_fp64_real(const Fp64RealJob *d_jobs, int num_jobs, int64_t ti
     if (edge == 16) fp64_real_kernel<true><<<(unsigned)tiles, 128, 0, st>>>(d_jobs, num_jobs);
     else fp64_real_kernel<false><<<(unsigned)tiles, 128, 0, st>>>(d_jobs, num_jobs);
     return cudaGetLastError();
-}
-
-// Tiles of 32 from kSplitBelow of them per SM on (n 2200: 22.5 ms, 22.9 on tiles of 16), else of 16 (n 1500, k 1200:
-// 10.8 ms, 11.3 on tiles of 32; n 200, k 1200: 0.42, 1.48).
-int64_t fp64_assign(Fp64Job *jobs, int num_jobs, int *edge) {
-    int dev = 0, nsm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    int64_t total = 0;
-    for (int e = 32; e >= 16; e /= 2) {
-        total = 0;
-        for (int i = 0; i < num_jobs; ++i) {
-            Fp64Job &j = jobs[i];
-            const int64_t tm = (j.m + e - 1) / e, tn = (j.n + e - 1) / e;
-            j.tiles_n = (int32_t)tn;
-            j.tile_begin = total;
-            total += j.lower ? tm * (tm + 1) / 2 : tm * tn;
-        }
-        *edge = e;
-        if (total >= (int64_t)kSplitBelow * nsm) break;
-    }
-    return total;
 }
 
 cudaError_t launch_fp64_jobs(const Fp64Job *d_jobs, int num_jobs, int64_t total_tiles, int edge, cudaStream_t st) {

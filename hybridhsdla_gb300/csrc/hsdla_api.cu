@@ -663,8 +663,9 @@ int autotune_slices(hsdla_plan *pl, double2 *C, cudaStream_t st) {
         jb.m = twoL; jb.n = ns; jb.k = twoL;
         pl->h_jobs.push_back(jb);
     }
-    int e1 = 0, e2 = 0;
-    const int64_t t1 = fp64_assign(pl->h_jobs.data(), (int)pl->h_jobs.size(), &e1);
+    const int64_t ns32 = (ns + 31) / 32;
+    const int e1 = fp64_edge((int64_t)pl->h_jobs.size() * ((2 * (int64_t)pl->L + 31) / 32) * ns32), e2 = fp64_edge(ns32 * (ns32 + 1));
+    const int64_t t1 = fp64_assign(pl->h_jobs.data(), (int)pl->h_jobs.size(), e1);
     const size_t nb = pl->h_jobs.size();
     Fp64Job js{};
     js.P = Cs; js.ldp = K; js.Q = Cs; js.ldq = K; js.w = pl->w; js.out = Sr; js.ldo = ns;
@@ -673,7 +674,7 @@ int autotune_slices(hsdla_plan *pl, double2 *C, cudaStream_t st) {
     jh.Q = Xs; jh.w = nullptr; jh.out = Hr;
     pl->h_jobs.push_back(js);
     pl->h_jobs.push_back(jh);
-    const int64_t t2 = fp64_assign(pl->h_jobs.data() + nb, 2, &e2);
+    const int64_t t2 = fp64_assign(pl->h_jobs.data() + nb, 2, e2);
     if (upload_jobs(pl, st)) return fail(HSDLA_ERR_CUDA, "job upload");
     if (launch_fp64_jobs(pl->d_jobs, (int)nb, t1, e1, st) != cudaSuccess ||
         launch_fp64_jobs(pl->d_jobs + nb, 2, t2, e2, st) != cudaSuccess)
@@ -1300,6 +1301,16 @@ void release_groups(hsdla_plan *pl) {
 int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
     hsdla_context *ctx = pl->ctx;
     const int64_t K = pl->twoLa, twoL = 2 * (int64_t)pl->L, ldm = twoL * pl->nt;
+    // FP64 tile edges by all of the plan's k-points, so that a group's results do not depend on which it holds:
+    // `jobs` products a k-point of m rows (0: lower triangles)
+    auto edge_of = [&](int64_t jobs, int64_t m) {
+        int64_t tiles = 0;
+        for (const auto &k : pl->kps) {
+            const int64_t tn = (k.n_g + 31) / 32;
+            tiles += jobs * (m > 0 ? (m + 31) / 32 * tn : tn * (tn + 1) / 2);
+        }
+        return fp64_edge(tiles);
+    };
     for (auto &g : pl->groups) {
         char *p = reinterpret_cast<char *>(ws);
         auto take = [&](int64_t bytes) { char *r = p; p += (bytes + 1023) / 1024 * 1024; return r; };
@@ -1399,7 +1410,8 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
                         jb.m = 2 * twoL; jb.n = kb[q].G; jb.k = twoL;
                         rt.push_back(jb);
                     }
-                g.tiles_t = fp64_real_assign(rt.data(), (int)rt.size(), &g.edge_t);
+                g.edge_t = edge_of(pl->nt, 2 * twoL);
+                g.tiles_t = fp64_real_assign(rt.data(), (int)rt.size(), g.edge_t);
                 for (int t0 = 0; t0 < pl->nt; t0 += pl->tbatch) {
                     const size_t first = rsh.size();
                     for (int t = t0; t < std::min(pl->nt, t0 + pl->tbatch); ++t)
@@ -1419,7 +1431,8 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
                     hsdla_plan::RealBatch rb;
                     rb.first = (int)first;
                     rb.jobs = (int)(rsh.size() - first);
-                    rb.tiles = fp64_real_assign(rsh.data() + first, rb.jobs, &rb.edge);
+                    rb.edge = edge_of(3 * (std::min(pl->nt, t0 + pl->tbatch) - t0), 0);
+                    rb.tiles = fp64_real_assign(rsh.data() + first, rb.jobs, rb.edge);
                     g.batches.push_back(rb);
                 }
                 g.n_jobs_t = (int)rt.size();
@@ -1463,8 +1476,10 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
                 jsh.push_back(js);
                 jsh.push_back(jh);
             }
-            g.tiles_t = fp64_assign(jt.data(), (int)jt.size(), &g.edge_t);
-            g.tiles_sh = fp64_assign(jsh.data(), (int)jsh.size(), &g.edge_sh);
+            g.edge_t = edge_of(pl->hoist ? pl->nt : pl->na, twoL);
+            g.edge_sh = edge_of(2, 0);
+            g.tiles_t = fp64_assign(jt.data(), (int)jt.size(), g.edge_t);
+            g.tiles_sh = fp64_assign(jsh.data(), (int)jsh.size(), g.edge_sh);
             g.n_jobs_t = (int)jt.size();
             g.d_jobs_t = reinterpret_cast<Fp64Job *>(keep(sizeof(Fp64Job) * jt.size()));
             g.d_jobs_sh = reinterpret_cast<Fp64Job *>(keep(sizeof(Fp64Job) * jsh.size()));
@@ -2313,8 +2328,9 @@ int hsdla_zherkx_lower(hsdla_context *ctx, int32_t precision, int32_t num_slices
         j.Q = reinterpret_cast<const double2 *>(dQ); j.ldq = ldq;
         j.w = dw; j.out = reinterpret_cast<double2 *>(dOut); j.ldo = ldo;
         j.m = n; j.n = n; j.k = k; j.lower = 1;
-        int edge = 0;
-        const int64_t tiles = fp64_assign(jobs.data(), 1, &edge);
+        const int64_t t32 = (n + 31) / 32;
+        const int edge = fp64_edge(t32 * (t32 + 1) / 2);
+        const int64_t tiles = fp64_assign(jobs.data(), 1, edge);
         void *dj = nullptr;
         int rc = ctx_malloc(ctx, &dj, sizeof(Fp64Job));
         if (rc) return rc;
@@ -2475,8 +2491,9 @@ int plugin_contract(hsdla_context *ctx, int kind, int32_t precision, int32_t num
             Fp64Job &j = jobs[0];
             j.P = P; j.ldp = ldp; j.Q = Q; j.ldq = ldq; j.w = nullptr;
             j.out = R; j.ldo = ldr; j.m = n; j.n = n; j.k = K; j.lower = 1;
-            int edge = 0;
-            const int64_t tiles = fp64_assign(jobs.data(), 1, &edge);
+            const int64_t t32 = (n + 31) / 32;
+            const int edge = fp64_edge(t32 * (t32 + 1) / 2);
+            const int64_t tiles = fp64_assign(jobs.data(), 1, edge);
             Fp64Job *dj = reinterpret_cast<Fp64Job *>(ws + oJ);
             CUDA_TRY(ctx, cudaMemcpyAsync(dj, jobs.data(), sizeof(Fp64Job), cudaMemcpyHostToDevice, st));
             CUDA_TRY(ctx, launch_fp64_jobs(dj, 1, tiles, edge, st));

@@ -36,3 +36,29 @@ def test_fp64_tiles(ctx, n, k, weighted):
     fro, mx = oracle.lower_errors(X, R)
     assert fro < 1e-13 and mx < 1e-13, (n, k, fro, mx)
     assert not np.triu(X, 1).any()
+
+
+@pytest.mark.parametrize("sf", ["1", "0"])
+def test_groups_sum_in_one_order(ctx, monkeypatch, sf):
+    """Three k-points whose launches take 32 x 32 tiles together and would take split ones alone: the same bits in one
+    group and in groups of one k-point."""
+    import torch
+    from hybridhsdla_gb300 import synth
+    cfg = dict(cell=(10.0, 10.5, 11.0), atoms=2, types=1, rmt=2.0, min_sep=3.9, lmax=2,
+               kpts=[(0.1, 0.2, 0.3), (0.0, 0.25, -0.1), (0.4, 0.1, 0.2)], n_g=700, seed=3)
+    s = synth.make_system(cfg)
+    monkeypatch.setenv("HSDLA_SF", sf)
+    monkeypatch.setenv("HSDLA_TYPE_BATCH", "1")
+    monkeypatch.setenv("HSDLA_PANELS", "1")
+    outs = []
+    for budget in (None, "1"):
+        if budget:
+            monkeypatch.setenv("HSDLA_WORKSPACE_BUDGET", budget)
+        pl = ctx.plan(s, precision="fp64")
+        o = pl.alloc_outputs()
+        pl.execute(o)
+        torch.cuda.synchronize()
+        outs.append([(h.cpu().numpy(), v.cpu().numpy()) for h, v in o])
+        pl.close()
+    for (h1, s1), (h2, s2) in zip(*outs):
+        assert np.array_equal(h1, h2) and np.array_equal(s1, s2)
