@@ -91,9 +91,10 @@ __global__ void __launch_bounds__(128) fp64_jobs_kernel(const Fp64Job *__restric
             }
         };
         // conj(P) Q: Re += Pr Qr + Pi Qi, Im += Pr Qi - Pi Qr
-        auto mma = [&](int buf) {
+        auto mma = [&](int buf, int64_t left) {
 #pragma unroll
             for (int u = 0; u < kJobsU; ++u) {
+                if (u >= left) break;           // no MMA for a step past the end
                 const double2 x0 = a0[buf][u], x1 = a1[buf][u], y0 = b0[buf][u], y1 = b1[buf][u];
                 dmma(re[0], x0.x, x1.x, y0.x);
                 dmma(re[1], x0.x, x1.x, y1.x);
@@ -108,9 +109,9 @@ __global__ void __launch_bounds__(128) fp64_jobs_kernel(const Fp64Job *__restric
         if (s0 < s1) load(0, s0);
         for (int64_t s = s0; s < s1; s += 2 * kJobsU) {
             if (s + kJobsU < s1) load(1, s + kJobsU);
-            mma(0);
+            mma(0, s1 - s);
             if (s + 2 * kJobsU < s1) load(0, s + 2 * kJobsU);
-            if (s + kJobsU < s1) mma(1);
+            if (s + kJobsU < s1) mma(1, s1 - s - kJobsU);
         }
     }
     if constexpr (kSplit) {
@@ -149,8 +150,8 @@ __global__ void __launch_bounds__(128) fp64_jobs_kernel(const Fp64Job *__restric
 // counts is an even share of the MMAs per SM.  A CTA of four warps has a 32 x 32 tile (a 16 x 16
 // quarter each); where a launch has fewer than kSplitBelow of those per SM, a 16 x 16 tile with the
 // contraction split over the warps.  Whole pass, complex 64 x 64 tiles before and this now: 235 columns,
-// lmax 8, two types (host call) 2.96 and 0.64 ms (20 of 152 SMs were busy); 3000 columns of four types
-// 55.7 and 20.6 ms (eight real products and three, each at the FP64 rate).
+// lmax 8, two types (host call) 2.96 and 0.60 ms (20 of 152 SMs were busy); 3000 columns of four types
+// 55.7 and 19.7 ms (eight real products and three, each at the FP64 rate).
 constexpr int kRealU = 4;            // K steps loaded ahead
 constexpr int kSplitBelow = 8;
 
@@ -199,19 +200,27 @@ __global__ void __launch_bounds__(128) fp64_real_kernel(const Fp64RealJob *__res
                 }
             }
         };
-        auto mma = [&](int buf) {
-#pragma unroll
-            for (int u = 0; u < kRealU; ++u) {
-                dmma(acc[0], a0[buf][u], a1[buf][u], b0[buf][u]);
-                dmma(acc[1], a0[buf][u], a1[buf][u], b1[buf][u]);
+        auto step = [&](int buf, int u) {
+            dmma(acc[0], a0[buf][u], a1[buf][u], b0[buf][u]);
+            dmma(acc[1], a0[buf][u], a1[buf][u], b1[buf][u]);
+        };
+        // the last steps by number: MMAs of steps past the end, even predicated off, would take their time
+        // (whole pass, 235 columns 0.241 and 0.212 ms, 3000 of four types 20.4 and 19.6, 256 of three 0.368 and 0.309)
+        auto mma = [&](int buf, int64_t left) {
+            switch (left < kRealU ? (int)left : kRealU) {
+                case 1: step(buf, 0); break;
+                case 2: step(buf, 0); step(buf, 1); break;
+                case 3: step(buf, 0); step(buf, 1); step(buf, 2); break;
+                default: step(buf, 0); step(buf, 1); step(buf, 2); step(buf, 3);
             }
         };
+        static_assert(kRealU == 4, "steps by number");
         if (s0 < s1) load(0, s0);
         for (int64_t s = s0; s < s1; s += 2 * kRealU) {
             if (s + kRealU < s1) load(1, s + kRealU);
-            mma(0);
+            mma(0, s1 - s);
             if (s + 2 * kRealU < s1) load(0, s + 2 * kRealU);
-            if (s + kRealU < s1) mma(1);
+            if (s + kRealU < s1) mma(1, s1 - s - kRealU);
         }
     }
     if constexpr (kSplit) {
