@@ -145,12 +145,13 @@ int fp64_edge(int64_t tiles32);
 int64_t fp64_assign(Fp64Job *jobs, int num_jobs, int edge);
 cudaError_t launch_fp64_jobs(const Fp64Job *d_jobs, int num_jobs, int64_t total_tiles, int edge, cudaStream_t st);
 
-// Real FP64 contraction out = P^T diag(w) Q over a batch of jobs (the structure-factor form's real
-// rows, see real_products.cu): P k x m, Q k x n, out m x n, column-major.
+// Real FP64 contraction out = P^T Q over a batch of jobs (the structure-factor form's real rows, see
+// real_products.cu): P k x m, Q k x n, out m x n, column-major.
 struct Fp64RealJob {
     const double *P; int64_t ldp;
     const double *Q; int64_t ldq;
-    const double *w;                 // k weights or nullptr
+    const double *w;                 // k weights, with
+    double *wq;                      // diag(w) Q, also written (ld ldq; m >= k, not lower), or nullptr
     double *out; int64_t ldo;
     int64_t m, n, k;
     int32_t lower;                   // 1: only elements with row >= col (m == n required)

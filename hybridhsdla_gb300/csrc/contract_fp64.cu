@@ -144,14 +144,17 @@ __global__ void __launch_bounds__(128) fp64_jobs_kernel(const Fp64Job *__restric
 }
 
 // ---------------------------------------------------------------- real products
-// Real DMMA products for the structure-factor form's real rows.  GB300's FP64 rate (1.05 TFLOP/s,
+// Real DMMA products for the structure-factor form's real rows.  GB300's FP64 rate (~1.1 TFLOP/s,
 // one m16n8k4 MMA in ~300 cycles and SM) bounds every shape, so there is no staging: fragments come
 // straight from global memory (L1 and L2 serve the reuse, 0.3-0.5 TB/s), four K steps ahead, and what
 // counts is an even share of the MMAs per SM.  A CTA of four warps has a 32 x 32 tile (a 16 x 16
 // quarter each); where a launch has fewer than kSplitBelow of those per SM, a 16 x 16 tile with the
 // contraction split over the warps.  Whole pass, complex 64 x 64 tiles before and this now: 235 columns,
 // lmax 8, two types (host call) 2.96 and 0.60 ms (20 of 152 SMs were busy); 3000 columns of four types
-// 55.7 and 19.7 ms (eight real products and three, each at the FP64 rate).
+// 55.7 and 18.5 ms (eight real products and three, each at the FP64 rate).
+// The multiplications by S's row weights share the pipe, at a sixth of an MMA each: done once, by the T application
+// (Fp64RealJob::wq), not for every fragment: 3001 columns of four types 19.6 and 18.4 ms, 400 columns of two 0.232 and
+// 0.226.  Split tiles write diag(w) Q with the warps whose parts are handed over.
 constexpr int kRealU = 4;            // K steps loaded ahead
 constexpr int kSplitBelow = 8;
 
@@ -193,11 +196,6 @@ __global__ void __launch_bounds__(128) fp64_real_kernel(const Fp64RealJob *__res
                 a1[buf][u] = in ? pa1[kc] : 0.0;
                 b0[buf][u] = pb0[kc];
                 b1[buf][u] = pb1[kc];
-                if (j.w) {
-                    const double w = j.w[kc];
-                    a0[buf][u] *= w;
-                    a1[buf][u] *= w;
-                }
             }
         };
         auto step = [&](int buf, int u) {
@@ -232,7 +230,14 @@ __global__ void __launch_bounds__(128) fp64_real_kernel(const Fp64RealJob *__res
 #pragma unroll
                 for (int c = 0; c < 4; ++c) part[warp - 1][t][c][lane] = acc[t][c];
         __syncthreads();
-        if (warp > 0) return;
+        if (warp > 0) {
+            if (j.wq)
+                for (int e = threadIdx.x - 32; e < kT * kT; e += 96) {
+                    const int64_t row = m0 + (e & 15), col = n0 + (e >> 4);
+                    if (row < K && col < n) j.wq[row + j.ldq * col] = j.w[row] * j.Q[row + j.ldq * col];
+                }
+            return;
+        }
 #pragma unroll
         for (int w = 0; w < 3; ++w)
 #pragma unroll
@@ -246,6 +251,7 @@ __global__ void __launch_bounds__(128) fp64_real_kernel(const Fp64RealJob *__res
         for (int c = 0; c < 4; ++c) {
             const int64_t row = m0 + gid + ((c >= 2) ? 8 : 0), col = n0 + t * 8 + tig * 2 + (c & 1);
             if (row < m && col < n && (!j.lower || row >= col)) j.out[row + j.ldo * col] = acc[t][c];
+            if (!kSplit && j.wq && row < K && col < n) j.wq[row + j.ldq * col] = j.w[row] * j.Q[row + j.ldq * col];
         }
 }
 

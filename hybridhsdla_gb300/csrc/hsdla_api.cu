@@ -1158,11 +1158,11 @@ namespace {
 int64_t kpoint_fp64_bytes(const hsdla_plan *pl, int64_t G) {
     const int64_t K = pl->twoLa, ldm = 2 * (int64_t)pl->L * pl->nt;
     auto r = [](int64_t x) { return (x + 1023) / 1024 * 1024; };        // each buffer is 1 KB aligned
-    // structure-factor form: the real rows R, Z' (two parts) and the three products of each type of a
-    // combine batch (no C, no X)
+    // structure-factor form: the real rows R (FP64: and diag(w) R), Z' (two parts) and the three products of each
+    // type of a combine batch (no C, no X)
     if (pl->sf)
-        return r(ldm * G * (int64_t)sizeof(double)) + r(2 * ldm * G * (int64_t)sizeof(double)) +
-               3 * r(pl->tbatch * G * G * (int64_t)sizeof(double));
+        return (pl->opts.precision == HSDLA_PREC_FP64 ? 2 : 1) * r(ldm * G * (int64_t)sizeof(double)) +
+               r(2 * ldm * G * (int64_t)sizeof(double)) + 3 * r(pl->tbatch * G * G * (int64_t)sizeof(double));
     const int64_t nCX = pl->opts.precision == HSDLA_PREC_FP64 ? 2 : 1;   // FP64 keeps C and X apart
     int64_t b = nCX * r(K * G * (int64_t)sizeof(double2));
     if (pl->hoist) b += 2 * r(ldm * G * (int64_t)sizeof(double2));
@@ -1348,6 +1348,8 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
             b.G = G;
             if (pl->sf) {
                 b.R = reinterpret_cast<double *>(take(ldm * G * (int64_t)sizeof(double)));
+                if (pl->opts.precision == HSDLA_PREC_FP64)
+                    b.WR = reinterpret_cast<double *>(take(ldm * G * (int64_t)sizeof(double)));
                 b.ZR = reinterpret_cast<long long *>(take(2 * ldm * G * (int64_t)sizeof(long long)));
                 b.pstride = G * G;
                 const int64_t pb = pl->tbatch * G * G * (int64_t)sizeof(double);
@@ -1398,14 +1400,15 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
             g.ev_t.assign(2, nullptr);
             for (auto &e : g.ev_t) CUDA_TRY(ctx, cudaEventCreate(&e));
             if (pl->sf) {
-                // Z'_t = T'_t R_t, and per type S_t = R_t^T diag(w_t) R_t and H_t = R_t^T Z'_t (real and
-                // imaginary parts) of every k-point; one launch per combine batch
+                // Z'_t = T'_t R_t (and diag(w_t) R_t), and per type S_t = (diag(w_t) R_t)^T R_t and H_t = R_t^T Z'_t
+                // (real and imaginary parts) of every k-point; one launch per combine batch
                 std::vector<Fp64RealJob> rt, rsh;
                 for (int q = 0; q < kt.nk; ++q)
                     for (int t = 0; t < pl->nt; ++t) {
                         Fp64RealJob jb{};
                         jb.P = pl->TR + 2 * twoL * twoL * pl->set_type[t]; jb.ldp = twoL;
                         jb.Q = kb[q].R + twoL * t; jb.ldq = ldm;
+                        jb.w = pl->wt + twoL * t; jb.wq = kb[q].WR + twoL * t;
                         jb.out = reinterpret_cast<double *>(kb[q].ZR) + 2 * twoL * t; jb.ldo = 2 * ldm;
                         jb.m = 2 * twoL; jb.n = kb[q].G; jb.k = twoL;
                         rt.push_back(jb);
@@ -1418,10 +1421,10 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
                         for (int q = 0; q < kt.nk; ++q)
                             for (int which = 0; which < 3; ++which) {
                                 Fp64RealJob jb{};
-                                jb.P = kb[q].R + twoL * t; jb.ldp = ldm;
-                                jb.Q = which == 0 ? jb.P : reinterpret_cast<double *>(kb[q].ZR) + 2 * twoL * t + (which - 1) * twoL;
+                                const double *R = kb[q].R + twoL * t;
+                                jb.P = which == 0 ? kb[q].WR + twoL * t : R; jb.ldp = ldm;
+                                jb.Q = which == 0 ? R : reinterpret_cast<double *>(kb[q].ZR) + 2 * twoL * t + (which - 1) * twoL;
                                 jb.ldq = which == 0 ? ldm : 2 * ldm;
-                                jb.w = which == 0 ? pl->wt + twoL * t : nullptr;
                                 jb.out = reinterpret_cast<double *>(which == 0 ? kb[q].RS : which == 1 ? kb[q].RHr : kb[q].RHi) +
                                          (int64_t)(t - t0) * kb[q].pstride;
                                 jb.ldo = kb[q].G;

@@ -47,6 +47,7 @@ struct OzKBufs {
     // fixed-point numbers Z' = T' R (4L nt x G; per type the real rows, then the imaginary ones) and
     // the per-type products S, Re H, Im H (G x G, ld G), type slot b of a combine batch at + b pstride
     double *R = nullptr;
+    double *WR = nullptr;    // FP64: diag(w) R
     long long *ZR = nullptr, *RS = nullptr, *RHr = nullptr, *RHi = nullptr;
     int64_t pstride = 0;
 };

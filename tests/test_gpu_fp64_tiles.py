@@ -62,3 +62,18 @@ def test_groups_sum_in_one_order(ctx, monkeypatch, sf):
         pl.close()
     for (h1, s1), (h2, s2) in zip(*outs):
         assert np.array_equal(h1, h2) and np.array_equal(s1, s2)
+
+
+@pytest.mark.parametrize("lmax,n_g", [(4, 2017), (3, 3903)])
+def test_weighted_rows_of_whole_tiles(ctx, lmax, n_g):
+    """T applications on 32 x 32 tiles (1216 of them on 152 SMs), which also write the weighted rows of S."""
+    from hybridhsdla_gb300 import synth
+    cfg = dict(cell=(14.0, 14.5, 15.0), atoms=5, types=5, rmt=2.0, min_sep=4.1, lmax=lmax, kpts=[(0.1, 0.2, 0.3)], n_g=n_g,
+               seed=n_g)
+    s = synth.make_system(cfg)
+    ((H, S),), rep = ctx.create_hs(s, precision="fp64")
+    assert rep["num_row_sets"] == 5
+    Hr, Sr = oracle.reference_hs(s, s.kpoints[0])
+    for X, R, nm in ((H, Hr, "H"), (S, Sr, "S")):
+        fro, mx = oracle.lower_errors(X, R)
+        assert fro < 1e-13 and mx < 1e-13, (nm, lmax, n_g, fro, mx)
