@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(128) fp64_jobs_kernel(const Fp64Job *__restric
 // counts is an even share of the MMAs per SM.  A CTA of four warps has a 32 x 32 tile (a 16 x 16
 // quarter each); where a launch has fewer than kSplitBelow of those per SM, a 16 x 16 tile with the
 // contraction split over the warps.  Whole pass, complex 64 x 64 tiles before and this now: 235 columns,
-// lmax 8, two types (host call) 2.96 and 0.60 ms (20 of 152 SMs were busy); 3000 columns of four types
+// lmax 8, two types (host call) 2.98 and 0.62 ms (20 of 152 SMs were busy); 3000 columns of four types
 // 55.7 and 18.5 ms (eight real products and three, each at the FP64 rate).
 // The multiplications by S's row weights share the pipe, at a sixth of an MMA each: done once, by the T application
 // (Fp64RealJob::wq), not for every fragment: 3001 columns of four types 19.6 and 18.4 ms, 400 columns of two 0.232 and
