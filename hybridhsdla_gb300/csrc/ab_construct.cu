@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(kThreads) construct_rows_kernel(DevSystem sys,
     double *ylm = reinterpret_cast<double *>(smem_raw);             // [kRowCols][L]
     double *au = ylm + kRowCols * L;                                // [kRowCols][nt nl]
     double *bu = au + kRowCols * tnl;                               // [kRowCols][nt nl]
-    double *cf = bu + kRowCols * tnl;                               // [nt nl] 4 pi / sqrt(Omega) / W, 0 past a type's lmax
+    double *cf = bu + kRowCols * tnl;                               // [nt nl] 4 pi / sqrt(Omega) / W
     double *kv = cf + tnl;                                          // [kRowCols][4]: K, |bmat K|
     double *dir = kv + 4 * kRowCols;                                // [kRowRots][kRowCols][4]: cos, sin theta; cos, sin phi
     double **rcol = reinterpret_cast<double **>(dir + 4 * kRowCols * kRowRots);   // [kRowCols]
@@ -366,8 +366,7 @@ __global__ void __launch_bounds__(kThreads) construct_rows_kernel(DevSystem sys,
         while ((l + 1) * (l + 1) <= lm) ++l;
         l_of[lm] = (unsigned char)l;
     }
-    for (int i = threadIdx.x; i < tnl; i += blockDim.x)
-        cf[i] = i % nl <= sys.type_lmax[i / nl] ? sys.vol_prefac * sys.inv_w[i] : 0.0;
+    for (int i = threadIdx.x; i < tnl; i += blockDim.x) cf[i] = sys.vol_prefac * sys.inv_w[i];
     const int nrot = sys.num_rots > 0 ? sys.num_rots : 1;
     const int rho0 = (int)((int64_t)nrot * blockIdx.y / gridDim.y), rho1 = (int)((int64_t)nrot * (blockIdx.y + 1) / gridDim.y);
     const int64_t ldm = tab.ldm;
@@ -418,10 +417,14 @@ __global__ void __launch_bounds__(kThreads) construct_rows_kernel(DevSystem sys,
                 const double x = sys.type_rmt[t] * kn;
                 sphbes_dev(sys.max_lmax, x, fj);
                 dsphbs_dev(sys.max_lmax, x, fj, dfj);
+                // (zero past the type's lmax, whatever the radial arrays hold there)
+                const int lt = sys.type_lmax[t];
                 for (int l = 0; l < nl; ++l) {
                     const int tl = t * nl + l;
-                    au[c * tnl + tl] = (sys.dE_u[tl] * kn * dfj[l] - sys.dE_u_dr[tl] * fj[l]) * cf[tl];
-                    bu[c * tnl + tl] = (-sys.u[tl] * kn * dfj[l] + sys.u_dr[tl] * fj[l]) * cf[tl];
+                    const double a = (sys.dE_u[tl] * kn * dfj[l] - sys.dE_u_dr[tl] * fj[l]) * cf[tl];
+                    const double b = (-sys.u[tl] * kn * dfj[l] + sys.u_dr[tl] * fj[l]) * cf[tl];
+                    au[c * tnl + tl] = l <= lt ? a : 0.0;
+                    bu[c * tnl + tl] = l <= lt ? b : 0.0;
                 }
             }
         }
