@@ -2508,10 +2508,11 @@ int plugin_contract(hsdla_context *ctx, int kind, int32_t precision, int32_t num
             if (rc) return set_err(ctx, rc, "%s: %s", nm, ozaki_last_error());
         }
     }
-    // ---- epilogue on C's triangle (in place for the direct form: only the real diagonal)
+    // ---- epilogue on C's triangle (a product in place needs only the real diagonal; without a product the
+    // triangle is beta C)
     if (direct && product) {
         if (herm) CUDA_TRY(ctx, launch_plugin_diagonal(dC, dldc, n, st));
-    } else if (!direct || herm) {
+    } else {
         const double2 a = kind == kPluginHer2k ? one : alpha;
         CUDA_TRY(ctx, launch_plugin_epilogue(product ? R : nullptr, ldr, dC, dldc, n, a, beta, upper, herm, st));
     }
