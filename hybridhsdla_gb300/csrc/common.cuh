@@ -136,14 +136,15 @@ struct Fp64Job {
     double2 *out; int64_t ldo;       // m x n
     int64_t m, n, k;
     int32_t lower;                   // 1: only elements with row >= col (m == n required)
+    int32_t edge;                    // tile edge, 32 or 16 (fp64_edge)
     int32_t tiles_n;                 // tile columns of this job
     int64_t tile_begin;              // first global tile index of this job
 };
-// The tile edge for a launch (or all launches that are to sum in one order) of `tiles32` tiles of edge 32.
+// The edge of jobs that come to `tiles32` tiles of edge 32.
 int fp64_edge(int64_t tiles32);
 // Numbers the jobs' tiles for one launch and returns their count.
-int64_t fp64_assign(Fp64Job *jobs, int num_jobs, int edge);
-cudaError_t launch_fp64_jobs(const Fp64Job *d_jobs, int num_jobs, int64_t total_tiles, int edge, cudaStream_t st);
+int64_t fp64_assign(Fp64Job *jobs, int num_jobs);
+cudaError_t launch_fp64_jobs(const Fp64Job *d_jobs, int num_jobs, int64_t total_tiles, cudaStream_t st);
 
 // Real FP64 contraction out = P^T Q over a batch of jobs (the structure-factor form's real rows, see
 // real_products.cu): P k x m, Q k x n, out m x n, column-major.
@@ -155,11 +156,14 @@ struct Fp64RealJob {
     double *out; int64_t ldo;
     int64_t m, n, k;
     int32_t lower;                   // 1: only elements with row >= col (m == n required)
+    int32_t parts;                   // 1: the contraction summed in four parts (products that alone are few tiles)
+    int32_t edge;                    // tile edge, 32, or 16 where a launch of such products has few tiles as well
     int32_t tiles_n;                 // tile columns of this job
     int64_t tile_begin;              // first global tile index of this job
 };
-int64_t fp64_real_assign(Fp64RealJob *jobs, int num_jobs, int edge);
-cudaError_t launch_fp64_real(const Fp64RealJob *d_jobs, int num_jobs, int64_t tiles, int edge, cudaStream_t st);
+// Chooses the jobs' edges and numbers their tiles for one launch.
+int64_t fp64_real_assign(Fp64RealJob *jobs, int num_jobs);
+cudaError_t launch_fp64_real(const Fp64RealJob *d_jobs, int num_jobs, int64_t tiles, cudaStream_t st);
 
 // ---- structure-factor form (atoms sharing their type's rotation)
 // One k-point of a combine: real per-type products (lower triangles, ld ldp) into the outputs

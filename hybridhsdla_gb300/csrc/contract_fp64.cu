@@ -29,7 +29,8 @@ __device__ __forceinline__ void dmma(double (&d)[4], double a0, double a1, doubl
         : "d"(a0), "d"(a1), "d"(b0));
 }
 
-__device__ __forceinline__ void tile_of(const Fp64Job &j, int64_t x, int64_t &ti, int64_t &tj) {
+template <typename Job>
+__device__ __forceinline__ void tile_of(const Job &j, int64_t x, int64_t &ti, int64_t &tj) {
     if (j.lower) {
         ti = triangle_row(x);
         tj = x - ti * (ti + 1) / 2;
@@ -49,18 +50,11 @@ __device__ __forceinline__ void tile_of(const Fp64Job &j, int64_t x, int64_t &ti
 constexpr int kJobsU = 2;           // K steps loaded ahead
 
 template <bool kSplit>
-__global__ void __launch_bounds__(128) fp64_jobs_kernel(const Fp64Job *__restrict__ jobs, int num_jobs) {
+__device__ __forceinline__ void fp64_job_tile(const Fp64Job &j, int64_t x) {
     constexpr int kT = kSplit ? 16 : 32;
-    const int64_t gt = blockIdx.x;
-    int lo = 0, hi = num_jobs - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (jobs[mid].tile_begin <= gt) lo = mid; else hi = mid - 1;
-    }
-    const Fp64Job &j = jobs[lo];
     const int64_t m = j.m, n = j.n, K = j.k;
     int64_t ti, tj;
-    tile_of(j, gt - j.tile_begin, ti, tj);
+    tile_of(j, x, ti, tj);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gid = lane >> 2, tig = lane & 3;
     const int64_t m0 = ti * kT + (kSplit ? 0 : (warp >> 1) * 16), n0 = tj * kT + (kSplit ? 0 : (warp & 1) * 16);
     double re[2][4] = {}, im[2][4] = {};
@@ -148,8 +142,10 @@ __global__ void __launch_bounds__(128) fp64_jobs_kernel(const Fp64Job *__restric
 // one m16n8k4 MMA in ~300 cycles and SM) bounds every shape, so there is no staging: fragments come
 // straight from global memory (L1 and L2 serve the reuse, 0.3-0.5 TB/s), four K steps ahead, and what
 // counts is an even share of the MMAs per SM.  A CTA of four warps has a 32 x 32 tile (a 16 x 16
-// quarter each); where a launch has fewer than kSplitBelow of those per SM, a 16 x 16 tile with the
-// contraction split over the warps.  Whole pass, complex 64 x 64 tiles before and this now: 235 columns,
+// quarter each); products with fewer than kSplitBelow of those per SM sum their contraction in four parts, on 16 x 16
+// tiles with a part per warp, or, in a launch that others fill, one part after the other on 32 x 32 tiles (the
+// same sums: a k-point's results keep their bits whatever it runs with.  3 k-points of 700 columns, one type, 0.345 ms
+// as one sum, 0.354 in parts, 0.378 on 16 x 16 tiles).  Whole pass, complex 64 x 64 tiles before and this now: 235 columns,
 // lmax 8, two types (host call) 2.98 and 0.62 ms (20 of 152 SMs were busy); 3000 columns of four types
 // 55.7 and 18.5 ms (eight real products and three, each at the FP64 rate).
 // The multiplications by S's row weights share the pipe, at a sixth of an MMA each: done once, by the T application
@@ -158,30 +154,18 @@ __global__ void __launch_bounds__(128) fp64_jobs_kernel(const Fp64Job *__restric
 constexpr int kRealU = 4;            // K steps loaded ahead
 constexpr int kSplitBelow = 8;
 
-template <bool kSplit>
-__global__ void __launch_bounds__(128) fp64_real_kernel(const Fp64RealJob *__restrict__ jobs, int num_jobs) {
+// kParts: the contraction in the split tile's four parts, summed in its order.
+template <bool kSplit, bool kParts>
+__device__ __forceinline__ void fp64_real_tile(const Fp64RealJob &j, int64_t x) {
     constexpr int kT = kSplit ? 16 : 32;
-    const int64_t gt = blockIdx.x;
-    int lo = 0, hi = num_jobs - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (jobs[mid].tile_begin <= gt) lo = mid; else hi = mid - 1;
-    }
-    const Fp64RealJob &j = jobs[lo];
-    const int64_t m = j.m, n = j.n, K = j.k, x = gt - j.tile_begin;
+    const int64_t m = j.m, n = j.n, K = j.k;
     int64_t ti, tj;
-    if (j.lower) {
-        ti = triangle_row(x);
-        tj = x - ti * (ti + 1) / 2;
-    } else {
-        ti = x / j.tiles_n;
-        tj = x - ti * j.tiles_n;
-    }
+    tile_of(j, x, ti, tj);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gid = lane >> 2, tig = lane & 3;
     const int64_t m0 = ti * kT + (kSplit ? 0 : (warp >> 1) * 16), n0 = tj * kT + (kSplit ? 0 : (warp & 1) * 16);
-    double acc[2][4] = {};
+    double acc[2][4] = {}, sum[2][4];
     const int64_t steps = (K + 3) / 4;
-    const int64_t s0 = kSplit ? steps * warp / 4 : 0, s1 = kSplit ? steps * (warp + 1) / 4 : steps;
+    int64_t s0 = kSplit ? steps * warp / 4 : 0, s1 = kSplit ? steps * (warp + 1) / 4 : steps;
     if (m0 < m && n0 < n && !(j.lower && m0 + 15 < n0)) {
         // rows and columns past the ends repeat the last one (their results are not stored)
         const double *pa0 = j.P + j.ldp * min(m0 + gid, m - 1), *pa1 = j.P + j.ldp * min(m0 + gid + 8, m - 1);
@@ -213,12 +197,28 @@ __global__ void __launch_bounds__(128) fp64_real_kernel(const Fp64RealJob *__res
             }
         };
         static_assert(kRealU == 4, "steps by number");
-        if (s0 < s1) load(0, s0);
-        for (int64_t s = s0; s < s1; s += 2 * kRealU) {
-            if (s + kRealU < s1) load(1, s + kRealU);
-            mma(0, s1 - s);
-            if (s + 2 * kRealU < s1) load(0, s + 2 * kRealU);
-            if (s + kRealU < s1) mma(1, s1 - s - kRealU);
+#pragma unroll 1
+        for (int q = 0; q < (kParts ? 4 : 1); ++q) {
+            if constexpr (kParts) {
+                s0 = steps * q / 4;
+                s1 = steps * (q + 1) / 4;
+            }
+            if (s0 < s1) load(0, s0);
+            for (int64_t s = s0; s < s1; s += 2 * kRealU) {
+                if (s + kRealU < s1) load(1, s + kRealU);
+                mma(0, s1 - s);
+                if (s + 2 * kRealU < s1) load(0, s + 2 * kRealU);
+                if (s + kRealU < s1) mma(1, s1 - s - kRealU);
+            }
+            if constexpr (kParts) {
+#pragma unroll
+                for (int t = 0; t < 2; ++t)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        sum[t][c] = q == 0 ? acc[t][c] : sum[t][c] + acc[t][c];
+                        acc[t][c] = q == 3 ? sum[t][c] : 0.0;
+                    }
+            }
         }
     }
     if constexpr (kSplit) {
@@ -255,15 +255,38 @@ __global__ void __launch_bounds__(128) fp64_real_kernel(const Fp64RealJob *__res
         }
 }
 
+// The job of a block's tile, and the tile in that job's shape.
+template <typename Job>
+__device__ __forceinline__ const Job &job_of(const Job *jobs, int num_jobs, int64_t tile) {
+    int lo = 0, hi = num_jobs - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (jobs[mid].tile_begin <= tile) lo = mid; else hi = mid - 1;
+    }
+    return jobs[lo];
+}
+__global__ void __launch_bounds__(128) fp64_jobs_kernel(const Fp64Job *__restrict__ jobs, int num_jobs) {
+    const Fp64Job &j = job_of(jobs, num_jobs, blockIdx.x);
+    if (j.edge == 16) fp64_job_tile<true>(j, blockIdx.x - j.tile_begin);
+    else fp64_job_tile<false>(j, blockIdx.x - j.tile_begin);
+}
+__global__ void __launch_bounds__(128) fp64_real_kernel(const Fp64RealJob *__restrict__ jobs, int num_jobs) {
+    const Fp64RealJob &j = job_of(jobs, num_jobs, blockIdx.x);
+    const int64_t x = blockIdx.x - j.tile_begin;
+    if (j.edge == 16) fp64_real_tile<true, false>(j, x);
+    else if (j.parts) fp64_real_tile<false, true>(j, x);
+    else fp64_real_tile<false, false>(j, x);
+}
+
 }  // namespace
 
 namespace {
 template <typename Job>
-int64_t assign(Job *jobs, int num_jobs, int edge) {
+int64_t assign(Job *jobs, int num_jobs) {
     int64_t total = 0;
     for (int i = 0; i < num_jobs; ++i) {
         Job &j = jobs[i];
-        const int64_t tm = (j.m + edge - 1) / edge, tn = (j.n + edge - 1) / edge;
+        const int64_t edge = j.edge, tm = (j.m + edge - 1) / edge, tn = (j.n + edge - 1) / edge;
         j.tiles_n = (int32_t)tn;
         j.tile_begin = total;
         total += j.lower ? tm * (tm + 1) / 2 : tm * tn;
@@ -280,22 +303,29 @@ int fp64_edge(int64_t tiles32) {
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     return tiles32 >= (int64_t)kSplitBelow * nsm ? 32 : 16;
 }
-int64_t fp64_assign(Fp64Job *jobs, int num_jobs, int edge) { return assign(jobs, num_jobs, edge); }
-int64_t fp64_real_assign(Fp64RealJob *jobs, int num_jobs, int edge) { return assign(jobs, num_jobs, edge); }
+int64_t fp64_assign(Fp64Job *jobs, int num_jobs) { return assign(jobs, num_jobs); }
+int64_t fp64_real_assign(Fp64RealJob *jobs, int num_jobs) {
+    int64_t tiles = 0;
+    for (int i = 0; i < num_jobs; ++i) {
+        const int64_t tm = (jobs[i].m + 31) / 32, tn = (jobs[i].n + 31) / 32;
+        tiles += jobs[i].lower ? tm * (tm + 1) / 2 : tm * tn;
+    }
+    const int edge = fp64_edge(tiles);
+    for (int i = 0; i < num_jobs; ++i) jobs[i].edge = jobs[i].parts ? edge : 32;
+    return assign(jobs, num_jobs);
+}
 
-cudaError_t launch_fp64_real(const Fp64RealJob *d_jobs, int num_jobs, int64_t tiles, int edge, cudaStream_t st) {
+cudaError_t launch_fp64_real(const Fp64RealJob *d_jobs, int num_jobs, int64_t tiles, cudaStream_t st) {
     if (tiles <= 0) return cudaSuccess;
     if (tiles > 0x7fffffffLL) return cudaErrorInvalidValue;
-    if (edge == 16) fp64_real_kernel<true><<<(unsigned)tiles, 128, 0, st>>>(d_jobs, num_jobs);
-    else fp64_real_kernel<false><<<(unsigned)tiles, 128, 0, st>>>(d_jobs, num_jobs);
+    fp64_real_kernel<<<(unsigned)tiles, 128, 0, st>>>(d_jobs, num_jobs);
     return cudaGetLastError();
 }
 
-cudaError_t launch_fp64_jobs(const Fp64Job *d_jobs, int num_jobs, int64_t total_tiles, int edge, cudaStream_t st) {
+cudaError_t launch_fp64_jobs(const Fp64Job *d_jobs, int num_jobs, int64_t total_tiles, cudaStream_t st) {
     if (total_tiles <= 0) return cudaSuccess;
     if (total_tiles > 0x7fffffffLL) return cudaErrorInvalidValue;
-    if (edge == 16) fp64_jobs_kernel<true><<<(unsigned)total_tiles, 128, 0, st>>>(d_jobs, num_jobs);
-    else fp64_jobs_kernel<false><<<(unsigned)total_tiles, 128, 0, st>>>(d_jobs, num_jobs);
+    fp64_jobs_kernel<<<(unsigned)total_tiles, 128, 0, st>>>(d_jobs, num_jobs);
     return cudaGetLastError();
 }
 

@@ -104,7 +104,7 @@ struct hsdla_plan {
     std::vector<Fp64Job> h_jobs;
     OzakiPlan oz{};
     // k-point groups, prepared against the context workspace (re-prepared when it moves)
-    struct RealBatch { int first = 0, jobs = 0, edge = 0; int64_t tiles = 0; };
+    struct RealBatch { int first = 0, jobs = 0; int64_t tiles = 0; };
     struct Group {
         std::vector<int> kidx;           // plan k-point indices
         KTable ktab;                     // construct / phase tables (C, M, Z, X per k-point)
@@ -117,7 +117,6 @@ struct hsdla_plan {
         int64_t tiles_sh = 0;
         // FP64 structure-factor form: real jobs (device), the products' in one launch per combine batch
         Fp64RealJob *d_rjobs_t = nullptr, *d_rjobs_sh = nullptr;
-        int edge_t = 0, edge_sh = 0;
         std::vector<RealBatch> batches;
         void *persist = nullptr;         // prepared tables (not shared with other groups)
         int64_t persist_bytes = 0;
@@ -664,20 +663,20 @@ int autotune_slices(hsdla_plan *pl, double2 *C, cudaStream_t st) {
         pl->h_jobs.push_back(jb);
     }
     const int64_t ns32 = (ns + 31) / 32;
-    const int e1 = fp64_edge((int64_t)pl->h_jobs.size() * ((2 * (int64_t)pl->L + 31) / 32) * ns32), e2 = fp64_edge(ns32 * (ns32 + 1));
-    const int64_t t1 = fp64_assign(pl->h_jobs.data(), (int)pl->h_jobs.size(), e1);
+    for (auto &jb : pl->h_jobs) jb.edge = fp64_edge(pl->na * ((twoL + 31) / 32) * ns32);
+    const int64_t t1 = fp64_assign(pl->h_jobs.data(), (int)pl->h_jobs.size());
     const size_t nb = pl->h_jobs.size();
     Fp64Job js{};
     js.P = Cs; js.ldp = K; js.Q = Cs; js.ldq = K; js.w = pl->w; js.out = Sr; js.ldo = ns;
-    js.m = ns; js.n = ns; js.k = K; js.lower = 1;
+    js.m = ns; js.n = ns; js.k = K; js.lower = 1; js.edge = fp64_edge(ns32 * (ns32 + 1));
     Fp64Job jh = js;
     jh.Q = Xs; jh.w = nullptr; jh.out = Hr;
     pl->h_jobs.push_back(js);
     pl->h_jobs.push_back(jh);
-    const int64_t t2 = fp64_assign(pl->h_jobs.data() + nb, 2, e2);
+    const int64_t t2 = fp64_assign(pl->h_jobs.data() + nb, 2);
     if (upload_jobs(pl, st)) return fail(HSDLA_ERR_CUDA, "job upload");
-    if (launch_fp64_jobs(pl->d_jobs, (int)nb, t1, e1, st) != cudaSuccess ||
-        launch_fp64_jobs(pl->d_jobs + nb, 2, t2, e2, st) != cudaSuccess)
+    if (launch_fp64_jobs(pl->d_jobs, (int)nb, t1, st) != cudaSuccess ||
+        launch_fp64_jobs(pl->d_jobs + nb, 2, t2, st) != cudaSuccess)
         return fail(HSDLA_ERR_CUDA, "fp64 sample");
     // Ozaki at the probe slice count (overwrites Xs after the FP64 H job, in stream order)
     OzakiInputs in;
@@ -1232,6 +1231,12 @@ void choose_panels(hsdla_plan *pl, int64_t budget) {
 // Structure-factor form: the most types per combine batch (each type of a batch keeps its own
 // products, and the batch reads and writes S and H once) whose one-k-point workspace fits the
 // budget; HSDLA_TYPE_BATCH forces a count.
+//
+// The batch where memory does not bound it.  (Many sets: a batch of 16 reads and writes S and H rarely enough;
+// its products stay a fraction of the device memory.)
+int full_batch(const hsdla_plan *pl) {
+    return pl->per_atom_sets || pl->nt > kMaxTypes ? std::min(pl->nt, 16) : pl->nt;
+}
 void choose_type_batch(hsdla_plan *pl, int64_t budget) {
     pl->tbatch = 1;
     if (!pl->sf) return;
@@ -1243,9 +1248,7 @@ void choose_type_batch(hsdla_plan *pl, int64_t budget) {
         if (pl->kps[i].n_g > 0 && (big < 0 || pl->kps[i].n_g > pl->kps[big].n_g)) big = i;
     if (big < 0) return;
     const std::vector<int> one{big};
-    // (many sets: a batch of 16 reads and writes S and H rarely enough; its products stay a fraction
-    // of the device memory)
-    pl->tbatch = pl->per_atom_sets || pl->nt > kMaxTypes ? std::min(pl->nt, 16) : pl->nt;
+    pl->tbatch = full_batch(pl);
     while (pl->tbatch > 1 && group_bytes(pl, one) > budget) --pl->tbatch;
 }
 
@@ -1301,15 +1304,12 @@ void release_groups(hsdla_plan *pl) {
 int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
     hsdla_context *ctx = pl->ctx;
     const int64_t K = pl->twoLa, twoL = 2 * (int64_t)pl->L, ldm = twoL * pl->nt;
-    // FP64 tile edges by all of the plan's k-points, so that a group's results do not depend on which it holds:
-    // `jobs` products a k-point of m rows (0: lower triangles)
-    auto edge_of = [&](int64_t jobs, int64_t m) {
-        int64_t tiles = 0;
-        for (const auto &k : pl->kps) {
-            const int64_t tn = (k.n_g + 31) / 32;
-            tiles += jobs * (m > 0 ? (m + 31) / 32 * tn : tn * (tn + 1) / 2);
-        }
-        return fp64_edge(tiles);
+    // FP64 tile edges of a k-point's `jobs` products of m rows (0: lower triangles) and G columns: by that k-point
+    // alone, so that the order of its sums depends neither on the plan's other k-points nor on the memory, by which
+    // groups and batches form
+    auto edge_of = [](int64_t jobs, int64_t m, int64_t G) {
+        const int64_t tn = (G + 31) / 32;
+        return fp64_edge(jobs * (m > 0 ? (m + 31) / 32 * tn : tn * (tn + 1) / 2));
     };
     for (auto &g : pl->groups) {
         char *p = reinterpret_cast<char *>(ws);
@@ -1411,10 +1411,11 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
                         jb.w = pl->wt + twoL * t; jb.wq = kb[q].WR + twoL * t;
                         jb.out = reinterpret_cast<double *>(kb[q].ZR) + 2 * twoL * t; jb.ldo = 2 * ldm;
                         jb.m = 2 * twoL; jb.n = kb[q].G; jb.k = twoL;
+                        jb.parts = edge_of(pl->nt, 2 * twoL, kb[q].G) == 16;
                         rt.push_back(jb);
                     }
-                g.edge_t = edge_of(pl->nt, 2 * twoL);
-                g.tiles_t = fp64_real_assign(rt.data(), (int)rt.size(), g.edge_t);
+                g.tiles_t = fp64_real_assign(rt.data(), (int)rt.size());
+                const int whole = full_batch(pl);
                 for (int t0 = 0; t0 < pl->nt; t0 += pl->tbatch) {
                     const size_t first = rsh.size();
                     for (int t = t0; t < std::min(pl->nt, t0 + pl->tbatch); ++t)
@@ -1429,13 +1430,13 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
                                          (int64_t)(t - t0) * kb[q].pstride;
                                 jb.ldo = kb[q].G;
                                 jb.m = kb[q].G; jb.n = kb[q].G; jb.k = twoL; jb.lower = 1;
+                                jb.parts = edge_of(3 * std::min(whole, pl->nt - t / whole * whole), 0, kb[q].G) == 16;
                                 rsh.push_back(jb);
                             }
                     hsdla_plan::RealBatch rb;
                     rb.first = (int)first;
                     rb.jobs = (int)(rsh.size() - first);
-                    rb.edge = edge_of(3 * (std::min(pl->nt, t0 + pl->tbatch) - t0), 0);
-                    rb.tiles = fp64_real_assign(rsh.data() + first, rb.jobs, rb.edge);
+                    rb.tiles = fp64_real_assign(rsh.data() + first, rb.jobs);
                     g.batches.push_back(rb);
                 }
                 g.n_jobs_t = (int)rt.size();
@@ -1452,6 +1453,7 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
             for (int q = 0; q < kt.nk; ++q) {
                 const KEntry &e = kt.e[q];
                 const int64_t G = pl->kps[g.kidx[q]].n_g;
+                const int edge_t = edge_of(pl->hoist ? pl->nt : pl->na, twoL, G);
                 if (pl->hoist) {
                     for (int t = 0; t < pl->nt; ++t) {
                         Fp64Job jb{};
@@ -1459,6 +1461,7 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
                         jb.Q = e.M + twoL * t; jb.ldq = ldm;
                         jb.out = const_cast<double2 *>(e.Z) + twoL * t; jb.ldo = ldm;
                         jb.m = twoL; jb.n = G; jb.k = twoL;
+                        jb.edge = edge_t;
                         jt.push_back(jb);
                     }
                 } else {
@@ -1468,21 +1471,21 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
                         jb.Q = e.C + twoL * j; jb.ldq = K;
                         jb.out = e.X + twoL * j; jb.ldo = K;
                         jb.m = twoL; jb.n = G; jb.k = twoL;
+                        jb.edge = edge_t;
                         jt.push_back(jb);
                     }
                 }
                 Fp64Job js{};
                 js.P = e.C; js.ldp = K; js.Q = e.C; js.ldq = K; js.w = pl->w;
                 js.m = G; js.n = G; js.k = K; js.lower = 1;
+                js.edge = edge_of(2, 0, G);
                 Fp64Job jh = js;
                 jh.Q = e.X; jh.w = nullptr;
                 jsh.push_back(js);
                 jsh.push_back(jh);
             }
-            g.edge_t = edge_of(pl->hoist ? pl->nt : pl->na, twoL);
-            g.edge_sh = edge_of(2, 0);
-            g.tiles_t = fp64_assign(jt.data(), (int)jt.size(), g.edge_t);
-            g.tiles_sh = fp64_assign(jsh.data(), (int)jsh.size(), g.edge_sh);
+            g.tiles_t = fp64_assign(jt.data(), (int)jt.size());
+            g.tiles_sh = fp64_assign(jsh.data(), (int)jsh.size());
             g.n_jobs_t = (int)jt.size();
             g.d_jobs_t = reinterpret_cast<Fp64Job *>(keep(sizeof(Fp64Job) * jt.size()));
             g.d_jobs_sh = reinterpret_cast<Fp64Job *>(keep(sizeof(Fp64Job) * jsh.size()));
@@ -1695,14 +1698,14 @@ int run_groups(hsdla_plan *pl, cudaStream_t st, bool timed, float *ms_ab, float 
             }
         } else if (pl->sf) {
             if (timed) CUDA_TRY(ctx, cudaEventRecord(g.ev_t[0], st));
-            CUDA_TRY(ctx, launch_fp64_real(g.d_rjobs_t, g.n_jobs_t, g.tiles_t, g.edge_t, st));
+            CUDA_TRY(ctx, launch_fp64_real(g.d_rjobs_t, g.n_jobs_t, g.tiles_t, st));
             if (timed) CUDA_TRY(ctx, cudaEventRecord(g.ev_t[1], st));
             pl->launches++;
             size_t p = 0;
             for (int t0 = 0; t0 < pl->nt; t0 += pl->tbatch, ++p) {
                 const hsdla_plan::RealBatch &rb = g.batches[p];
                 CUDA_TRY(ctx, record_event(g.ev_dom[2 * p], st));
-                CUDA_TRY(ctx, launch_fp64_real(g.d_rjobs_sh + rb.first, rb.jobs, rb.tiles, rb.edge, st));
+                CUDA_TRY(ctx, launch_fp64_real(g.d_rjobs_sh + rb.first, rb.jobs, rb.tiles, st));
                 CUDA_TRY(ctx, record_event(g.ev_dom[2 * p + 1], st));
                 pl->launches++;
                 // the batch's products into S and H
@@ -1724,7 +1727,7 @@ int run_groups(hsdla_plan *pl, cudaStream_t st, bool timed, float *ms_ab, float 
             }
         } else {
             if (timed) CUDA_TRY(ctx, cudaEventRecord(g.ev_t[0], st));
-            CUDA_TRY(ctx, launch_fp64_jobs(g.d_jobs_t, g.n_jobs_t, g.tiles_t, g.edge_t, st));
+            CUDA_TRY(ctx, launch_fp64_jobs(g.d_jobs_t, g.n_jobs_t, g.tiles_t, st));
             if (timed) CUDA_TRY(ctx, cudaEventRecord(g.ev_t[1], st));
             pl->launches++;
             if (pl->hoist) {
@@ -1734,7 +1737,7 @@ int run_groups(hsdla_plan *pl, cudaStream_t st, bool timed, float *ms_ab, float 
             CUDA_TRY(ctx, cudaMemcpyAsync(g.d_jobs_sh, g.h_jobs_sh, sizeof(Fp64Job) * 2 * g.ktab.nk,
                                           cudaMemcpyHostToDevice, st));
             CUDA_TRY(ctx, record_event(g.ev_dom[0], st));
-            CUDA_TRY(ctx, launch_fp64_jobs(g.d_jobs_sh, 2 * g.ktab.nk, g.tiles_sh, g.edge_sh, st));
+            CUDA_TRY(ctx, launch_fp64_jobs(g.d_jobs_sh, 2 * g.ktab.nk, g.tiles_sh, st));
             CUDA_TRY(ctx, record_event(g.ev_dom[1], st));
             pl->launches++;
         }
@@ -2332,13 +2335,13 @@ int hsdla_zherkx_lower(hsdla_context *ctx, int32_t precision, int32_t num_slices
         j.w = dw; j.out = reinterpret_cast<double2 *>(dOut); j.ldo = ldo;
         j.m = n; j.n = n; j.k = k; j.lower = 1;
         const int64_t t32 = (n + 31) / 32;
-        const int edge = fp64_edge(t32 * (t32 + 1) / 2);
-        const int64_t tiles = fp64_assign(jobs.data(), 1, edge);
+        j.edge = fp64_edge(t32 * (t32 + 1) / 2);
+        const int64_t tiles = fp64_assign(jobs.data(), 1);
         void *dj = nullptr;
         int rc = ctx_malloc(ctx, &dj, sizeof(Fp64Job));
         if (rc) return rc;
         cudaError_t e = cudaMemcpyAsync(dj, jobs.data(), sizeof(Fp64Job), cudaMemcpyHostToDevice, st);
-        if (e == cudaSuccess) e = launch_fp64_jobs((Fp64Job *)dj, 1, tiles, edge, st);
+        if (e == cudaSuccess) e = launch_fp64_jobs((Fp64Job *)dj, 1, tiles, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         ctx_free(ctx, dj, sizeof(Fp64Job));
         if (e != cudaSuccess) return set_err(ctx, HSDLA_ERR_CUDA, "zherkx fp64: %s", cudaGetErrorString(e));
@@ -2495,11 +2498,11 @@ int plugin_contract(hsdla_context *ctx, int kind, int32_t precision, int32_t num
             j.P = P; j.ldp = ldp; j.Q = Q; j.ldq = ldq; j.w = nullptr;
             j.out = R; j.ldo = ldr; j.m = n; j.n = n; j.k = K; j.lower = 1;
             const int64_t t32 = (n + 31) / 32;
-            const int edge = fp64_edge(t32 * (t32 + 1) / 2);
-            const int64_t tiles = fp64_assign(jobs.data(), 1, edge);
+            j.edge = fp64_edge(t32 * (t32 + 1) / 2);
+            const int64_t tiles = fp64_assign(jobs.data(), 1);
             Fp64Job *dj = reinterpret_cast<Fp64Job *>(ws + oJ);
             CUDA_TRY(ctx, cudaMemcpyAsync(dj, jobs.data(), sizeof(Fp64Job), cudaMemcpyHostToDevice, st));
-            CUDA_TRY(ctx, launch_fp64_jobs(dj, 1, tiles, edge, st));
+            CUDA_TRY(ctx, launch_fp64_jobs(dj, 1, tiles, st));
         } else {
             rc = ozaki_plan_init(ctx->plugin_oz, s, 1e-13);
             if (rc) return set_err(ctx, rc, "%s: %s", nm, ozaki_last_error());
