@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "../../include/hsdla.h"
 
 namespace hsdla {
@@ -183,6 +185,7 @@ struct SfEntry {
     double2 *Sx = nullptr, *Hx = nullptr;
     int64_t ldx = 0;
 };
+constexpr int kSfItemTypes = 4;                   // types of an item, the unit of a combine's work
 struct SfTab {
     int nk = 0, type = 0, ntypes = 1;             // the batch: types [type, type + ntypes) in slots
     int slot0 = 0;                                // slot0, slot0 + 1, ...
@@ -193,16 +196,28 @@ struct SfTab {
     int dx = 0, dy = 0, dz = 0, ny = 0, nz = 0;   // box offsets (half widths) and extents
     int64_t box = 0;                              // entries
     int nt = 1;                                   // row sets of the structure-factor table
-    int sfbits = 0;                               // its fixed point (launch_sf_table), 0: FP64
+    const int32_t *bits = nullptr;                // host: its fixed points (launch_sf_table) [nt], NULL: FP64,
+    const int32_t *group = nullptr;               // and the groups that are summed in integers
+    // set by launch_sf_combine: the batch's items, each at most kSfItemTypes types of one group: its first
+    // type, bits 8-15 their number, and where the integer sums end with it bits 16-23 the fixed point, bit 24
+    // for the first such item
+    int nitems = 0;
+    uint32_t item[kMaxTypes];
+    int bits0 = 0;                                // the first type's fixed point
+    bool listed = false;                          // whether the items are other than four types each, in sums of two
     SfEntry e[kMaxGroup];
 };
 // SF_t(dG) = sum_{a of type t} e^{i 2pi dG.tau_a} over the box of G-vector differences, from
 // per-atom factors ex[a][dGx + dx] = e^{i 2pi dGx tau_a,x} (and y, z); atoms listed by type.  The table
-// holds entry dG's types together (type fastest), 16 bytes each: FP64 (re, im), or with sfbits > 0
-// each part as the limbs {f >> 28, f & (2^28 - 1)} of f = rint(part 2^sfbits), |f| < 2^55.
+// holds entry dG's types together (type fastest), 16 bytes each: FP64 (re, im), or with bits (device) each
+// part as the limbs {f >> 28, f & (2^28 - 1)} of f = rint(part 2^bits[t]), |f| < 2^59.
 cudaError_t launch_sf_table(const double2 *ex, const double2 *ey, const double2 *ez, const int32_t *order,
-                            const int32_t *type_begin, int nt, int nx, int ny, int nz, int sfbits, void *sf,
+                            const int32_t *type_begin, const int32_t *bits, int nt, int nx, int ny, int nz, void *sf,
                             cudaStream_t st);
+// The order in which row sets of atoms[q] atoms are combined, and by their place in it the groups of sets whose
+// terms are summed in integers and the groups' fixed points.
+void sf_fixed_points(const std::vector<int32_t> &atoms, std::vector<int32_t> &order, std::vector<int32_t> &bits,
+                     std::vector<int32_t> &group);
 // S (+)= sum_b SF_{type+b} (.) S_b and H (+)= sum_b SF_{type+b} (.) H_b over the lower triangles
 // of every entry, b over the batch's type slots, in columns [tab.col0, tab.col1) (multiples of 32
 // but for the end); rows below tab.xrow1 into Sx, Hx instead for entries that give them.

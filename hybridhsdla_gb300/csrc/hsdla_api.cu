@@ -88,6 +88,8 @@ struct hsdla_plan {
     int L = 0, na = 0, nt = 0, max_lmax = 0;    // nt: row sets (types, or (type, rotation) classes)
     int ntypes = 0;                  // types of the T blocks
     std::vector<int32_t> set_type;   // type of each row set
+    std::vector<int32_t> order;      // the row sets in the order in which they are combined
+    std::vector<int32_t> sf_bits, sf_group;   // digit form: their structure factors' fixed points, in that order
     int64_t twoLa = 0;
     DevSystem dsys{};
     std::vector<PlanKpoint> kps;
@@ -942,7 +944,7 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
                 for (int c = 0; c < 3; ++c) half[c] = std::max(half[c], 2 * std::abs(kpts[i].g[3 * q + c]));
         for (int c = 0; c < 3; ++c) ext[c] = 2 * half[c] + 1;
         add(sizeof(double) * 2 * L * ns);
-        add(sizeof(int32_t) * (na + ns + 1));
+        add(sizeof(int32_t) * (na + 2 * ns + 1));
     }
     const int64_t upload_bytes = bytes;
     // filled on the device: the assembled T blocks and their checks; the structure-factor form's
@@ -1040,27 +1042,28 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
                     wt[(size_t)2 * L * q + L + lm] = (l <= s->type_lmax[t]) ? pair * s->type_dE_u_norm[t * nl + l] : 0.0;
                 }
         pl->wt = (double *)put(wt.data(), sizeof(double) * wt.size());
-        // the atoms set by set
-        std::vector<int32_t> ord, tb(ns + 1, 0);
-        for (int j = 0; j < na; ++j) ++tb[sets.atom_set[j] + 1];
-        for (int q = 0; q < ns; ++q) tb[q + 1] += tb[q];
-        ord.resize(na);
-        std::vector<int32_t> at(tb.begin(), tb.end() - 1);
+        std::vector<int32_t> atoms(ns, 0);
+        for (int j = 0; j < na; ++j) ++atoms[sets.atom_set[j]];
+        if (pl->opts.precision == HSDLA_PREC_OZAKI_FP8) sf_fixed_points(atoms, pl->order, pl->sf_bits, pl->sf_group);
+        else
+            for (int q = 0; q < ns; ++q) pl->order.push_back(q);
+        // the atoms set by set, in the combine's order
+        std::vector<int32_t> ord(na), tb(ns + 1, 0), at(ns);
+        for (int p = 0; p < ns; ++p) {
+            at[pl->order[p]] = tb[p];
+            tb[p + 1] = tb[p] + atoms[pl->order[p]];
+        }
         for (int j = 0; j < na; ++j) ord[at[sets.atom_set[j]]++] = j;
         ord.insert(ord.end(), tb.begin(), tb.end());
+        ord.insert(ord.end(), pl->sf_bits.begin(), pl->sf_bits.end());
         d_order = (const int32_t *)put(ord.data(), sizeof(int32_t) * ord.size());
         SfTab &dm = pl->sf_dims;
         dm.dx = half[0]; dm.dy = half[1]; dm.dz = half[2];
         dm.ny = ext[1]; dm.nz = ext[2];
         dm.box = (int64_t)ext[0] * ext[1] * ext[2];
         dm.nt = ns;
-        if (pl->opts.precision == HSDLA_PREC_OZAKI_FP8) {
-            // |SF_t| <= atoms of the set < 2^(55 - sfbits)
-            int most = 0, b = 0;
-            for (int q = 0; q < ns; ++q) most = std::max(most, tb[q + 1] - tb[q]);
-            while ((1 << b) <= most) ++b;
-            dm.sfbits = 55 - b;
-        }
+        dm.bits = pl->sf_bits.empty() ? nullptr : pl->sf_bits.data();
+        dm.group = pl->sf_group.data();
     }
     // past the uploaded part: what the device fills
     auto dev_only = [&](int64_t b) -> void * {
@@ -1113,7 +1116,8 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     if (e == cudaSuccess && pl->sf) e = launch_sf_phases(D.atom_pos, na, half, ext, d_ex, ctx->stream);
     if (e == cudaSuccess && pl->sf)
         e = launch_sf_table(d_ex, d_ex + (size_t)na * ext[0], d_ex + (size_t)na * (ext[0] + ext[1]), d_order,
-                            d_order + na, ns, ext[0], ext[1], ext[2], pl->sf_dims.sfbits, pl->sf_tab, ctx->stream);
+                            d_order + na, pl->sf_bits.empty() ? nullptr : d_order + na + ns + 1, ns, ext[0], ext[1], ext[2],
+                            pl->sf_tab, ctx->stream);
     const bool defer = defer_tcheck && ctx->staging != nullptr;
     unsigned long long *stats_host =
         defer ? reinterpret_cast<unsigned long long *>(reinterpret_cast<char *>(ctx->staging) + stats_off) : tstats.data();
@@ -1242,7 +1246,7 @@ void choose_type_batch(hsdla_plan *pl, int64_t budget) {
     if (!pl->sf) return;
     const char *ev = getenv("HSDLA_TYPE_BATCH");
     const int64_t forced = ev ? strtoll(ev, nullptr, 10) : 0;
-    if (forced > 0) { pl->tbatch = (int)std::min<int64_t>(forced, pl->nt); return; }
+    if (forced > 0) { pl->tbatch = (int)std::min<int64_t>(forced, std::min(pl->nt, kMaxTypes)); return; }
     int big = -1;
     for (int i = 0; i < (int)pl->kps.size(); ++i)
         if (pl->kps[i].n_g > 0 && (big < 0 || pl->kps[i].n_g > pl->kps[big].n_g)) big = i;
@@ -1379,12 +1383,13 @@ int prepare_groups(hsdla_plan *pl, void *ws, cudaStream_t st) {
             const SfTab &dm = pl->sf_dims;
             ft.nk = kt.nk;
             ft.dx = dm.dx; ft.dy = dm.dy; ft.dz = dm.dz; ft.ny = dm.ny; ft.nz = dm.nz; ft.box = dm.box;
-            ft.nt = dm.nt; ft.sfbits = dm.sfbits;
+            ft.nt = dm.nt; ft.bits = dm.bits; ft.group = dm.group;
         }
         if (pl->opts.precision == HSDLA_PREC_OZAKI_FP8) {
             OzGroupDesc d;
             d.twoL = twoL; d.na = pl->na; d.nt = pl->nt; d.hoist = pl->hoist;
             d.ntypes = pl->ntypes; d.set_type = pl->set_type.data(); d.d_set_type = pl->dsys.set_type;
+            d.order = pl->order.data();
             d.w = pl->w; d.Tfull = pl->Tfull; d.atom_type = pl->atom_type.data();
             d.panels = pl->panels;
             d.split = pl->split; d.split_bytes = pl->split_bytes;

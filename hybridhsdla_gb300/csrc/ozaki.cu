@@ -2008,7 +2008,7 @@ static int group_prepare_sf(OzakiPlan &oz, const OzGroupDesc &d, const std::vect
             j.out = kb[k].ZR + 2 * d.twoL * t; j.ldo = 2 * d.twoL * d.nt;
             jt.push_back(j);
         }
-    for (int64_t t = 0; t < d.nt; ++t)
+    for (int64_t t = 0; t < d.nt; ++t)                    // (place t of the combine's order)
         for (int k = 0; k < g->nk; ++k)
             for (int which = 0; which < 3; ++which) {     // S, Re H, Im H
                 RealJob j;
@@ -2017,7 +2017,7 @@ static int group_prepare_sf(OzakiPlan &oz, const OzGroupDesc &d, const std::vect
                 j.rstep = which == 0 ? 1 : 2; j.rpart = which == 2 ? 1 : 0;
                 j.lplane = g->rows; j.rplane = g->rows;
                 j.lrow0 = g->row0[k]; j.rrow0 = g->row0[k];
-                j.lk0 = t * g->bpad; j.rk0 = t * g->bpad;
+                j.lk0 = j.rk0 = d.order[t] * g->bpad;
                 j.nkb = tkb; j.ksteps_last = ksl;
                 j.m = kb[k].G; j.n = kb[k].G;
                 j.out = (which == 0 ? kb[k].RS : which == 1 ? kb[k].RHr : kb[k].RHi) + (t % g->tbatch) * kb[k].pstride;

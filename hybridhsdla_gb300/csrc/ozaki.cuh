@@ -66,6 +66,7 @@ struct OzGroupDesc {
     int64_t ntypes = 0;                    // types of Tfull and TR (row sets: nt)
     const int32_t *set_type = nullptr;     // type of each row set: host [nt],
     const int32_t *d_set_type = nullptr;   // and device
+    const int32_t *order = nullptr;        // the sets in the order in which they are combined: host [nt]
     void *split = nullptr;                 // ozaki_split_bytes for the S/H products, or null
     int64_t split_bytes = 0;
     void *split_t = nullptr;               // ozaki_split_bytes_t for the per-atom T application, or null

@@ -8,6 +8,8 @@
 //     SF_t(dG) = sum_{a of type t} e^{i 2pi dG.tau_a}          (k cancels),
 // so the contractions run over 2L rows per type instead of 2L rows per atom (a factor of atoms
 // per type fewer products), and the structure factors enter once per element and type.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace hsdla {
@@ -28,9 +30,9 @@ __global__ void __launch_bounds__(kSfTabThreads) sf_table_kernel(const double2 *
                                                                  const double2 *__restrict__ ey,
                                                                  const double2 *__restrict__ ez,
                                                                  const int32_t *__restrict__ order,
-                                                                 const int32_t *__restrict__ type_begin, int nx,
-                                                                 int ny, int nz, int chunk, int sfbits,
-                                                                 void *__restrict__ sf) {
+                                                                 const int32_t *__restrict__ type_begin,
+                                                                 const int32_t *__restrict__ bits, int nx, int ny, int nz,
+                                                                 int chunk, void *__restrict__ sf) {
     extern __shared__ double2 pxy[];            // [chunk][ny]
     const int ix = blockIdx.x, t = blockIdx.y;
     const int64_t nyz = (int64_t)ny * nz;
@@ -58,10 +60,10 @@ __global__ void __launch_bounds__(kSfTabThreads) sf_table_kernel(const double2 *
         }
         if (e < nyz) {
             const int64_t o = ((int64_t)ix * nyz + e) * nt + t;
-            if (sfbits == 0) {
+            if (!bits) {
                 static_cast<double2 *>(sf)[o] = acc;
             } else {
-                const double s = __longlong_as_double((long long)(1023 + sfbits) << 52);
+                const double s = __longlong_as_double((long long)(1023 + bits[t]) << 52);
                 const long long re = __double2ll_rn(acc.x * s), im = __double2ll_rn(acc.y * s);
                 constexpr int kLow = (1 << 28) - 1;
                 static_cast<int4 *>(sf)[o] = make_int4((int)(re >> 28), (int)(re & kLow), (int)(im >> 28), (int)(im & kLow));
@@ -70,10 +72,10 @@ __global__ void __launch_bounds__(kSfTabThreads) sf_table_kernel(const double2 *
     }
 }
 
-// Exact sums of products p f of 64-bit fixed-point products p and 55-bit structure factors f, in four
-// 64-bit sums of the limb products: p = p1 2^32 + p0 with p0 in [-2^31, 2^31), f = f1 2^28 + f0 with f0
-// in (-2^28, 2^28).  With |p1| < 2^31 and |f1| <= 2^27, kSumTypes types of two terms each overflow none
-// of them, so a term is four multiply-adds and no carry.
+// Exact sums of products p f of 64-bit fixed-point products p and structure factors f of up to 59 bits, in four
+// 64-bit sums of the limb products: p = p1 2^32 + p0 with p0 in [-2^31, 2^31) and |p1| < 2^31, f = f1 2^28 + f0
+// with f0 in (-2^28, 2^28).  kSumTypes types of two terms each overflow no sum with f0, and a group's types
+// (sf_fixed_points) none with f1, so a term is four multiply-adds and no carry.
 constexpr int kSumTypes = 8;
 struct Limbs {
     int hi, lo;
@@ -134,7 +136,7 @@ constexpr int kSfTile = 32;
 // ms.  Bound now by the wide multiply-adds (a warp's takes four cycles; 24 an element and type) on 16 warps an
 // SM; 20 warps leave too little L1 beside the stages (1.67 and 1.44 ms).  Loads into registers, four types
 // ahead of their use on 24 warps, took 1.59 and 1.41 ms.
-constexpr int kChunk = 4, kSumItems = kSumTypes / kChunk;        // types of an item; items of a sum
+constexpr int kChunk = kSfItemTypes, kSumItems = kSumTypes / kChunk;     // types of an item; items of a full sum
 constexpr int kSfPitch = kChunk + 1;                             // 16-byte words of an element's structure factors
 constexpr int kStageSf = kSfTile * kSfPitch * 16, kStageBytesWarp = kStageSf + 3 * kChunk * kSfTile * 8;
 
@@ -177,7 +179,9 @@ struct Sums<true> {
 // 8000 columns above where this took 1.42)
 __device__ __noinline__ double2 sum2(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 
-template <bool kFixed, int kRows>
+// kItems: the items and ends of the sums as listed (SfTab::item); else four types each (the last fewer) and every second
+// item or the last, of one fixed point, SfTab::bits0 (listed, 8000 columns of 8 equal types 1.44 ms).
+template <bool kFixed, int kRows, bool kItems>
 __global__ void __launch_bounds__(kSfTile *kRows, 512 / (kSfTile * kRows)) sf_combine_kernel(const __grid_constant__ SfTab tab,
                                                                                      const int4 *__restrict__ sf, int first) {
     extern __shared__ __align__(16) unsigned char stages[];
@@ -210,28 +214,29 @@ __global__ void __launch_bounds__(kSfTile *kRows, 512 / (kSfTile * kRows)) sf_co
     int64_t from[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) from[i] = __shfl_sync(0xffffffffu, prow, lane / 4 + 8 * i) - lane % 4;
-    const int kr = kFixed ? E.el[rowc] - 8 - tab.frac - tab.sfbits : 0;
+    const int kr = kFixed ? E.el[rowc] - 8 - tab.frac - (kItems ? 0 : tab.bits0) : 0;
     const int kcs = kFixed ? E.ers[colc] : 0, kch = kFixed ? E.erh[colc] : 0;
     // the warp's columns of the tile: threadIdx.y, + kRows, ... below cend (those of the lower triangle)
     const int cend = (int)min((int64_t)kSfTile, (tr == tc ? E.n : min(E.n, tc * kSfTile + kSfTile)) - tc * kSfTile);
-    const int ntypes = tab.ntypes, nchunk = (ntypes + kChunk - 1) / kChunk;
+    const int ntypes = tab.ntypes, nitems = kItems ? tab.nitems : (ntypes + kChunk - 1) / kChunk;
     const int64_t ps = E.pstride, ldp = E.ldp, ldo = E.ldo;
     unsigned char *mem = stages + threadIdx.y * 2 * kStageBytesWarp;
     const uint32_t smem = (uint32_t)__cvta_generic_to_shared(mem);
-    // the item to be fetched next: column ic, chunk it; its column's first product
+    // the item to be fetched next: column ic, item it; its column's first product
     int ic = threadIdx.y, it = 0;
+    uint32_t next = kItems ? tab.item[0] : 0;      // (loaded an item ahead of its use)
     int64_t o = rowc + tab.slot0 * ps + ldp * (tc * kSfTile + ic);
     auto fetch = [&](uint32_t st) {
         if (ic < cend) {
-            const int n = min(kChunk, ntypes - kChunk * it);
-            const int4 *base = sf + __shfl_sync(0xffffffffu, pcol, ic) + kChunk * it;
+            const int t0 = kItems ? next & 0xff : kChunk * it, n = kItems ? (next >> 8) & 0xff : min(kChunk, ntypes - t0);
+            const int4 *base = sf + __shfl_sync(0xffffffffu, pcol, ic) + t0;
             const uint32_t ds = st + (lane / 4 * kSfPitch + lane % 4) * 16;
             if (lane % 4 < n) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) cp_async16(ds + i * (8 * kSfPitch * 16), base - from[i]);
             }
             const uint32_t dp = st + kStageSf + lane * 8;
-            int64_t x = o + kChunk * it * ps;
+            int64_t x = o + t0 * ps;
 #pragma unroll
             for (int t = 0; t < kChunk; ++t, x += ps)
                 if (t < n) {
@@ -239,15 +244,17 @@ __global__ void __launch_bounds__(kSfTile *kRows, 512 / (kSfTile * kRows)) sf_co
                     cp_async8(dp + (3 * t + 1) * (kSfTile * 8), static_cast<const int2 *>(E.RHr) + x);
                     cp_async8(dp + (3 * t + 2) * (kSfTile * 8), static_cast<const int2 *>(E.RHi) + x);
                 }
-            if (++it == nchunk) {
+            if (++it == nitems) {
                 it = 0;
                 ic += kRows;
                 o += kRows * ldp;
             }
+            if (kItems) next = tab.item[it];
         }
         cp_async_commit();
     };
     int stage = 0;
+    uint32_t item = next, item1 = next;            // the item being summed, the one fetched last
     fetch(smem);
     int64_t oo = row + ldo * (tc * kSfTile + threadIdx.y);
 #pragma unroll 1
@@ -256,11 +263,13 @@ __global__ void __launch_bounds__(kSfTile *kRows, 512 / (kSfTile * kRows)) sf_co
         Sums<kFixed> v;
         const int ks = kFixed ? kr + __shfl_sync(0xffffffffu, kcs, c) : 0, kh = kFixed ? kr + __shfl_sync(0xffffffffu, kch, c) : 0;
 #pragma unroll 1
-        for (int q = 0; q < nchunk; ++q) {
+        for (int q = 0; q < nitems; ++q) {
+            item = item1;
+            item1 = next;
             fetch(smem + (stage ^ 1) * kStageBytesWarp);
             cp_async_wait_but_one();
             __syncwarp();
-            const int n = min(kChunk, ntypes - kChunk * q);
+            const int n = kItems ? (item >> 8) & 0xff : min(kChunk, ntypes - kChunk * q);
             const int4 *w = reinterpret_cast<const int4 *>(mem + stage * kStageBytesWarp) + lane * kSfPitch;
             const int2 *p = reinterpret_cast<const int2 *>(mem + stage * kStageBytesWarp + kStageSf) + lane;
             if (n == kChunk) {
@@ -274,10 +283,12 @@ __global__ void __launch_bounds__(kSfTile *kRows, 512 / (kSfTile * kRows)) sf_co
             __syncwarp();
             stage ^= 1;
             if constexpr (kFixed) {
-                if (q % kSumItems == kSumItems - 1 || q + 1 == nchunk) {
-                    // one power of two for every type's products of an element
-                    const double2 s = make_double2(v.sr.value(ks), v.si.value(ks)), h = make_double2(v.hr.value(kh), v.hi.value(kh));
-                    if (q < kSumItems) { vs = s; vh = h; }
+                const int fb = kItems ? (item >> 16) & 0xff : 0;
+                if (kItems ? fb != 0 : q % kSumItems == kSumItems - 1 || q + 1 == nitems) {
+                    // one power of two for the products of an element and the structure factors of these types
+                    const double2 s = make_double2(v.sr.value(ks - fb), v.si.value(ks - fb));
+                    const double2 h = make_double2(v.hr.value(kh - fb), v.hi.value(kh - fb));
+                    if (kItems ? item >> 24 : q < kSumItems) { vs = s; vh = h; }
                     else { vs = sum2(vs, s); vh = sum2(vh, h); }
                     v = Sums<kFixed>();
                 }
@@ -301,27 +312,27 @@ __global__ void __launch_bounds__(kSfTile *kRows, 512 / (kSfTile * kRows)) sf_co
     }
 }
 
-template <bool kFixed>
+template <bool kFixed, bool kItems>
 cudaError_t combine_launch(const SfTab &t, const void *sf, bool first, int64_t tiles, cudaStream_t st) {
     // 4 columns of a tile at a time where there are tiles enough, 8 where not
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     const bool few = tiles < 8 * (int64_t)nsm;
-    const void *kernel = few ? (const void *)sf_combine_kernel<kFixed, 8> : (const void *)sf_combine_kernel<kFixed, 4>;
+    const void *kernel = few ? (const void *)sf_combine_kernel<kFixed, 8, kItems> : (const void *)sf_combine_kernel<kFixed, 4, kItems>;
     const int rows = few ? 8 : 4, smem = rows * 2 * kStageBytesWarp;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     const int4 *f = static_cast<const int4 *>(sf);
-    if (few) sf_combine_kernel<kFixed, 8><<<(unsigned)tiles, dim3(kSfTile, 8), smem, st>>>(t, f, first ? 1 : 0);
-    else sf_combine_kernel<kFixed, 4><<<(unsigned)tiles, dim3(kSfTile, 4), smem, st>>>(t, f, first ? 1 : 0);
+    if (few) sf_combine_kernel<kFixed, 8, kItems><<<(unsigned)tiles, dim3(kSfTile, 8), smem, st>>>(t, f, first ? 1 : 0);
+    else sf_combine_kernel<kFixed, 4, kItems><<<(unsigned)tiles, dim3(kSfTile, 4), smem, st>>>(t, f, first ? 1 : 0);
     return cudaGetLastError();
 }
 
 }  // namespace
 
 cudaError_t launch_sf_table(const double2 *ex, const double2 *ey, const double2 *ez, const int32_t *order,
-                            const int32_t *type_begin, int nt, int nx, int ny, int nz, int sfbits, void *sf,
+                            const int32_t *type_begin, const int32_t *bits, int nt, int nx, int ny, int nz, void *sf,
                             cudaStream_t st) {
     const int64_t n = (int64_t)nx * ny * nz * nt;
     if (n <= 0) return cudaSuccess;
@@ -329,9 +340,65 @@ cudaError_t launch_sf_table(const double2 *ex, const double2 *ey, const double2 
     const int chunk = std::min<int>(kSfChunk, kSfSmem / (int)sizeof(double2) / std::max(ny, 1));
     if (nx > 65535 || nt > 65535 || chunk < 1) return cudaErrorInvalidValue;
     const size_t smem = sizeof(double2) * (size_t)chunk * ny;
-    sf_table_kernel<<<dim3((unsigned)nx, (unsigned)nt), kSfTabThreads, smem, st>>>(ex, ey, ez, order, type_begin, nx,
-                                                                                 ny, nz, chunk, sfbits, sf);
+    sf_table_kernel<<<dim3((unsigned)nx, (unsigned)nt), kSfTabThreads, smem, st>>>(ex, ey, ez, order, type_begin,
+                                                                                 bits, nx, ny, nz, chunk, sf);
     return cudaGetLastError();
+}
+
+// A set of N atoms has |Re SF| + |Im SF| <= sqrt(2) N, so the sums with f1 stay below 2^63 while the group's atoms are no
+// more than 2^(59 - f), f the fixed point, and f1 fits 32 bits while N is less.  A group ends after kSumTypes types, or
+// before one of which its fixed point would keep fewer bits than an FP64 number of N's magnitude has: one atom
+// takes f = 53, 4000 leave 47.
+void sf_fixed_points(const std::vector<int32_t> &atoms, std::vector<int32_t> &order, std::vector<int32_t> &bits,
+                     std::vector<int32_t> &group) {
+    const int n = (int)atoms.size();
+    order.resize(n);
+    bits.resize(n);
+    group.resize(n);
+    for (int i = 0; i < n; ++i) order[i] = i;
+    std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return atoms[a] > atoms[b]; });
+    auto log2_up = [](int64_t x) {            // least b with x <= 2^b
+        int b = 0;
+        while (((int64_t)1 << b) < x) ++b;
+        return b;
+    };
+    for (int a = 0, g = 0; a < n; ++g) {
+        int64_t sum = 0;
+        int b = a, f = 0;
+        for (; b < n && b - a < kSumTypes; ++b) {
+            const int64_t N = atoms[order[b]];
+            const int fb = std::min(56, 59 - log2_up(std::max<int64_t>(sum + N, atoms[order[a]] + 1)));
+            if (b > a && fb < 54 - log2_up(N + 1)) break;
+            sum += N;
+            f = fb;
+        }
+        for (; a < b; ++a) {
+            bits[a] = f;
+            group[a] = g;
+        }
+    }
+}
+
+// The batch's items and the ends of its integer sums, both within the groups.
+static void sf_items(SfTab &t) {
+    t.nitems = 0;
+    t.bits0 = t.bits ? t.bits[t.type] : 0;
+    t.listed = false;
+    bool first = true;
+    for (int a = 0; a < t.ntypes; ++t.nitems) {
+        auto same = [&](int x) { return x < t.ntypes && (!t.bits || t.group[t.type + x] == t.group[t.type + a]); };
+        int b = a + 1;
+        while (b - a < kSfItemTypes && same(b)) ++b;
+        t.item[t.nitems] = (uint32_t)a | (uint32_t)(b - a) << 8;
+        if (t.bits && !same(b)) {
+            t.item[t.nitems] |= (uint32_t)t.bits[t.type + a] << 16 | (first ? 1u << 24 : 0u);
+            first = false;
+        }
+        if (t.bits && (t.bits[t.type + a] != t.bits0 || a != kSfItemTypes * t.nitems ||
+                       !same(b) != (t.nitems % kSumItems == kSumItems - 1 || b == t.ntypes)))
+            t.listed = true;
+        a = b;
+    }
 }
 
 int64_t sf_tab_tiles(SfTab &tab) {
@@ -357,8 +424,10 @@ cudaError_t launch_sf_combine(const SfTab &tab, const void *sf, bool first, cuda
         }
     const int64_t tiles = sf_tab_tiles(t);
     if (tiles <= 0) return cudaSuccess;
-    if (tiles > 0x7fffffffLL) return cudaErrorInvalidValue;
-    return t.nk > 0 && t.e[0].el ? combine_launch<true>(t, sf, first, tiles, st) : combine_launch<false>(t, sf, first, tiles, st);
+    if (tiles > 0x7fffffffLL || t.ntypes < 1 || t.ntypes > kMaxTypes) return cudaErrorInvalidValue;
+    sf_items(t);
+    if (t.nk < 1 || !t.e[0].el) return combine_launch<false, false>(t, sf, first, tiles, st);
+    return t.listed ? combine_launch<true, true>(t, sf, first, tiles, st) : combine_launch<true, false>(t, sf, first, tiles, st);
 }
 
 }  // namespace hsdla
