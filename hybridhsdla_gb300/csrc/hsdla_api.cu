@@ -144,7 +144,7 @@ struct hsdla_plan {
     // the structure factors SF_t over the box of G-vector differences
     bool sf = false;
     int classes = 0;                 // (type, rotation) classes the structure-factor form runs over (0: types)
-    bool per_atom_sets = false;      // ... more than 3/4 as many as atoms (reported as the per-atom form)
+    bool per_atom_sets = false;      // ... more than 3/4 as many as atoms
     // T-block check read after the call's own synchronisation (hsdla_create_hs): the device's
     // statistics land in the context's page-locked staging, checked once the stream is idle
     bool tcheck_pending = false;
@@ -1961,6 +1961,7 @@ int hsdla_plan_execute(hsdla_plan *pl, hsdla_cx *const *dH, hsdla_cx *const *dS,
         rep->kernel_launches = pl->launches;
         rep->num_panels = pl->opts.precision == HSDLA_PREC_OZAKI_FP8 ? pl->panels : 0;
         rep->num_row_sets = pl->sf && !pl->per_atom_sets ? pl->nt : 0;
+        rep->contracted_sets = pl->sf ? pl->nt : 0;
         rep->rotation_classes = pl->classes > 0 && !pl->per_atom_sets ? 1 : 0;
         if (!pl->groups.empty() && pl->groups[0].oz && ozaki_group_tunable(pl->groups[0].oz)) {
             int h = 0, m = 0;

@@ -128,9 +128,9 @@ typedef struct hsdla_report {
     int32_t kernel_launches;     /* kernels launched per execution */
     int32_t num_panels;          /* Ozaki: atom panels the contraction was streamed in (1 = resident) */
     int32_t outputs_in_place;    /* hsdla_create_hs: 1 = the GPU wrote the page-locked host H, S itself */
-    int32_t num_row_sets;        /* structure-factor form: the row sets contracted (types, or (type, rotation)
-                                    classes when atoms carry rotations); 0 = rows per atom (also where more than
-                                    three quarters as many classes as atoms are contracted) */
+    int32_t num_row_sets;        /* structure-factor form: the row sets that atoms share (types, or (type, rotation)
+                                    classes when atoms carry rotations); 0 = rows per atom (the per-atom form, and
+                                    row sets more than three quarters as many as the atoms: contracted_sets) */
     int32_t rotation_classes;    /* 1: the row sets are (type, rotation) classes */
     int32_t tile_halves;         /* Ozaki, structure-factor form: the S/H products' bands of digit diagonals alternate */
                                  /* between two halves of TMEM (2) or wait for each other in one (1); 0 otherwise */
@@ -138,7 +138,8 @@ typedef struct hsdla_report {
     int32_t tile_tuned;          /* 1 = those two were chosen by timing on this plan's data (or a cached result) */
     int32_t output_blocks;       /* hsdla_create_hs, outputs written in place: the column blocks they were written
                                     in while the digit products of the next block ran (0 = after all products) */
-    int32_t reserved[1];
+    int32_t contracted_sets;     /* which form ran: the row sets whose products H and S were combined from
+                                    (structure-factor form), 0 = the per-atom form */
     double ms_host_setup;        /* hsdla_create_hs: host time from the call's start to its first launch (plan
                                     creation and set-up; the device is idle meanwhile, and ms_total counts it) */
 } hsdla_report;
