@@ -499,6 +499,12 @@ __global__ void __launch_bounds__(kThreads) apply_phase_kernel(DevSystem sys, co
 // the L x L entries (r fastest): each writes the four quadrant entries at (r, c) and folds its
 // checks into the CTA's, then one atomic each.
 constexpr int kTfThreads = 256;
+// A non-finite entry is flagged by the checks and taken as zero, so that nothing downstream (the digit
+// slicing above all) meets it before the flag is read.
+__device__ __forceinline__ double2 finite_or_zero(double2 v) {
+    return (isfinite(v.x) && isfinite(v.y)) ? v : make_double2(0.0, 0.0);
+}
+// (tf NULL: the checks alone)
 __global__ void __launch_bounds__(kTfThreads) tfull_kernel(const double2 *__restrict__ aa_all,
                                                            const double2 *__restrict__ ab_all,
                                                            const double2 *__restrict__ bb_all, int L, double2 *tf,
@@ -506,7 +512,7 @@ __global__ void __launch_bounds__(kTfThreads) tfull_kernel(const double2 *__rest
     const int t = blockIdx.y;
     const int64_t LL = (int64_t)L * L, n = 2 * (int64_t)L;
     const double2 *aa = aa_all + t * LL, *ab = ab_all + t * LL, *bb = bb_all + t * LL;
-    double2 *out = tf + t * 4 * LL;
+    double2 *out = tf ? tf + t * 4 * LL : nullptr;
     unsigned int flags = 0;
     unsigned long long st[4] = {0, 0, 0, 0};
     auto bits = [](double v) { return (unsigned long long)__double_as_longlong(v); };
@@ -518,13 +524,12 @@ __global__ void __launch_bounds__(kTfThreads) tfull_kernel(const double2 *__rest
         if (!isfinite(x.x) || !isfinite(x.y)) flags |= 2u;
         if (!isfinite(b.x) || !isfinite(b.y)) flags |= 4u;
         const bool low = r >= c;
-        // a non-finite entry is flagged above and assembled as zero, so that nothing downstream
-        // (the digit slicing above all) meets it before the flag is read
-        auto fin = [](double2 v) { return (isfinite(v.x) && isfinite(v.y)) ? v : make_double2(0.0, 0.0); };
-        out[r + n * c] = fin(low ? a : make_double2(aT.x, -aT.y));
-        out[(L + r) + n * (L + c)] = fin(low ? b : make_double2(bT.x, -bT.y));
-        out[r + n * (L + c)] = fin(x);
-        out[(L + r) + n * c] = fin(make_double2(xT.x, -xT.y));
+        if (out) {
+            out[r + n * c] = finite_or_zero(low ? a : make_double2(aT.x, -aT.y));
+            out[(L + r) + n * (L + c)] = finite_or_zero(low ? b : make_double2(bT.x, -bT.y));
+            out[r + n * (L + c)] = finite_or_zero(x);
+            out[(L + r) + n * c] = finite_or_zero(make_double2(xT.x, -xT.y));
+        }
         if (low) {
             // |T|^2 of the pair and |T - T^H|^2 (the mirror element is the pair's other half)
             st[0] = max(st[0], bits(fmax(a.x * a.x + a.y * a.y, aT.x * aT.x + aT.y * aT.y)));
@@ -558,10 +563,24 @@ __global__ void __launch_bounds__(kTfThreads) tfull_kernel(const double2 *__rest
 
 // T' = V^H T V of every type: rows and columns (l, m > 0) and (l, -m) of T, whose matching rows
 // are p + i q and (-1)^m (p - i q), become those of the real rows p and q; four entries of T per
-// entry of T', added in an order that keeps T' Hermitian.
-__global__ void __launch_bounds__(kTfThreads) treal_kernel(const double2 *__restrict__ tf, int L, double *__restrict__ tr) {
+// entry of T', added in an order that keeps T' Hermitian.  T's entries are those tfull_kernel assembles, taken
+// from the blocks: the structure-factor form needs no assembled T of its own.
+__global__ void __launch_bounds__(kTfThreads) treal_kernel(const double2 *__restrict__ aa_all,
+                                                           const double2 *__restrict__ ab_all,
+                                                           const double2 *__restrict__ bb_all, int L,
+                                                           double *__restrict__ tr) {
     const int n = 2 * L, t = blockIdx.y;
-    const double2 *T = tf + (int64_t)t * n * n;
+    const int64_t LL = (int64_t)L * L;
+    const double2 *aa = aa_all + t * LL, *ab = ab_all + t * LL, *bb = bb_all + t * LL;
+    auto T = [&](int a, int b) {
+        const bool qa = a >= L, qb = b >= L;
+        const int r = qa ? a - L : a, c = qb ? b - L : b;
+        // the stored entry (r, c), or the conjugate of (c, r)
+        const bool own = qa == qb ? r >= c : !qa;
+        const double2 *blk = qa != qb ? ab : qa ? bb : aa;
+        const double2 v = blk[own ? r + (int64_t)L * c : c + (int64_t)L * r];
+        return finite_or_zero(own ? v : make_double2(v.x, -v.y));
+    };
     double *out = tr + (int64_t)t * 2 * n * n;
     // the indices of rows (l, |m|) and (l, -|m|), m's sign and parity of row x of a type
     auto split = [&](int x, int &p, int &q, int &m) {
@@ -581,7 +600,7 @@ __global__ void __launch_bounds__(kTfThreads) treal_kernel(const double2 *__rest
         split(k, cp, cq, cm);
         const double sr = (rm & 1) ? -1.0 : 1.0, sc = (cm & 1) ? -1.0 : 1.0;
         auto at = [&](int a, int b, double s) {
-            const double2 v = T[a + (int64_t)n * b];
+            const double2 v = T(a, b);
             return make_double2(s * v.x, s * v.y);
         };
         const double2 z = make_double2(0.0, 0.0);
@@ -650,11 +669,12 @@ cudaError_t launch_tfull(const double2 *aa, const double2 *ab, const double2 *bb
     return cudaGetLastError();
 }
 
-cudaError_t launch_treal(const double2 *tf, int nt, int L, double *tr, cudaStream_t st) {
+cudaError_t launch_treal(const double2 *aa, const double2 *ab, const double2 *bb, int nt, int L, double *tr,
+                         cudaStream_t st) {
     if (nt <= 0 || L <= 0) return cudaSuccess;
     const int64_t nn = 4 * (int64_t)L * L;
     const dim3 grid((unsigned)std::min<int64_t>((nn + kTfThreads - 1) / kTfThreads, 128), (unsigned)nt);
-    treal_kernel<<<grid, kTfThreads, 0, st>>>(tf, L, tr);
+    treal_kernel<<<grid, kTfThreads, 0, st>>>(aa, ab, bb, L, tr);
     return cudaGetLastError();
 }
 

@@ -117,12 +117,13 @@ cudaError_t launch_construct_ab(const DevSystem &sys, const DevKpoint &kp, doubl
 // nt x L x L, column-major per type), with the input checks per type in stats[5 t .. 5 t + 4]
 // (zeroed by the caller): bit q of [0] set when block q (0 AA, 1 AB, 2 BB) holds a non-finite
 // value; [1], [2] = max |T|^2 and max |T - T^H|^2 over T_AA's lower triangle, [3], [4] the same
-// for T_BB (doubles as bit patterns).
+// for T_BB (doubles as bit patterns).  tf NULL: the checks alone.
 cudaError_t launch_tfull(const double2 *aa, const double2 *ab, const double2 *bb, int nt, int L, double2 *tf,
                          unsigned long long *stats, cudaStream_t st);
 // The real form of the T blocks (see real_products.cu): tr holds per type 4L columns of 2L values,
-// column r the row r of Re T', column 2L + r the row r of Im T', T' = V^H T V with T from launch_tfull.
-cudaError_t launch_treal(const double2 *tf, int nt, int L, double *tr, cudaStream_t st);
+// column r the row r of Re T', column 2L + r the row r of Im T', T' = V^H T V with launch_tfull's T.
+cudaError_t launch_treal(const double2 *aa, const double2 *ab, const double2 *bb, int nt, int L, double *tr,
+                         cudaStream_t st);
 // Per-atom structure phases along each axis, ph[o] = e^{i 2pi (i - half_c) pos[3 j + c]} with o
 // running over c, then atom j, then i in [0, ext_c).
 cudaError_t launch_sf_phases(const double *pos, int na, const int *half, const int *ext, double2 *ph, cudaStream_t st);

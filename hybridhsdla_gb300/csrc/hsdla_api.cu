@@ -98,9 +98,8 @@ struct hsdla_plan {
     // device allocations owned by the plan
     void *tables = nullptr;          // system arrays, T blocks, weights, G lists
     int64_t tables_bytes = 0;
-    double2 *Tfull = nullptr;        // [nt][2L][2L]
+    double2 *Tfull = nullptr;        // [nt][2L][2L] (null in the structure-factor form but for the slice autotuner)
     double *w = nullptr;             // [2La] S row weights
-    double *wsqrt = nullptr;         // [2La] sqrt of the S row weights (Ozaki left operand)
     Fp64Job *d_jobs = nullptr;       // job table (device)
     int64_t jobs_cap = 0;
     std::vector<Fp64Job> h_jobs;
@@ -906,15 +905,15 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
             inv_w[tl] = 1. / (s->type_dE_u[tl] * s->type_u_dr[tl] - s->type_u[tl] * s->type_dE_u_dr[tl]);
         }
     std::vector<double> yn = ylm_norms(s->max_lmax);
-    std::vector<double> w(pl->twoLa), wsq(pl->twoLa);
+    std::vector<double> w(pl->twoLa);
     for (int j = 0; j < na; ++j) {
         const int t = s->atom_type[j];
         for (int l = 0; l < nl; ++l)
             for (int lm = l * l; lm < (l + 1) * (l + 1); ++lm) {
                 const int64_t rA = 2 * (int64_t)L * j + lm, rB = rA + L;
                 const double un = (l <= s->type_lmax[t]) ? s->type_dE_u_norm[t * nl + l] : 0.0;
-                w[rA] = 1.0; wsq[rA] = 1.0;
-                w[rB] = un; wsq[rB] = std::sqrt(un);
+                w[rA] = 1.0;
+                w[rB] = un;
             }
     }
     const size_t tf_elems = (size_t)nt * 4 * L * L;
@@ -931,7 +930,7 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     for (int q = 0; q < 5; ++q) add(sizeof(double) * nt * nl);
     add(sizeof(double) * L);
     for (int q = 0; q < 3; ++q) add(sizeof(double2) * LLnt);     // T_AA, T_AB, T_BB as given
-    add(sizeof(double) * pl->twoLa); add(sizeof(double) * pl->twoLa);
+    add(sizeof(double) * pl->twoLa);
     for (int i = 0; i < nk; ++i) add(sizeof(int32_t) * 3 * kpts[i].n_g);
     // structure-factor form: per-type weights, per-atom phase factors along each axis, the atoms
     // grouped by type and the table itself over the box of G-vector differences g_col - g_row
@@ -948,8 +947,9 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     }
     const int64_t upload_bytes = bytes;
     // filled on the device: the assembled T blocks and their checks; the structure-factor form's
-    // per-atom phase factors and its table
-    add(sizeof(double2) * tf_elems);
+    // per-atom phase factors, its table and its real T blocks
+    const bool want_tfull = !pl->sf || (pl->opts.precision == HSDLA_PREC_OZAKI_FP8 && pl->opts.num_slices == 0);
+    if (want_tfull) add(sizeof(double2) * tf_elems);
     add(sizeof(unsigned long long) * 5 * nt);
     if (pl->sf) {
         add(sizeof(double2) * (int64_t)na * (ext[0] + ext[1] + ext[2]));
@@ -1017,7 +1017,6 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     const double2 *d_tab = (const double2 *)put(s->type_t_ab, sizeof(double2) * LLnt);
     const double2 *d_tbb = (const double2 *)put(s->type_t_bb, sizeof(double2) * LLnt);
     pl->w = (double *)put(w.data(), sizeof(double) * pl->twoLa);
-    pl->wsqrt = (double *)put(wsq.data(), sizeof(double) * pl->twoLa);
     for (int i = 0; i < nk; ++i) {
         PlanKpoint pk;
         pk.n_g = kpts[i].n_g;
@@ -1071,7 +1070,7 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
         dp += (b + 255) & ~int64_t(255);
         return d;
     };
-    pl->Tfull = (double2 *)dev_only(sizeof(double2) * tf_elems);
+    if (want_tfull) pl->Tfull = (double2 *)dev_only(sizeof(double2) * tf_elems);
     unsigned long long *d_stats = (unsigned long long *)dev_only(sizeof(unsigned long long) * 5 * nt);
     if (pl->sf) {
         d_ex = (double2 *)dev_only(sizeof(double2) * (int64_t)na * (ext[0] + ext[1] + ext[2]));
@@ -1112,7 +1111,7 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     cudaError_t e = cudaMemcpyAsync(pl->tables, stage, upload_bytes, cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(d_stats, 0, sizeof(unsigned long long) * 5 * nt, ctx->stream);
     if (e == cudaSuccess) e = launch_tfull(d_taa, d_tab, d_tbb, nt, L, pl->Tfull, d_stats, ctx->stream);
-    if (e == cudaSuccess && pl->sf) e = launch_treal(pl->Tfull, nt, L, pl->TR, ctx->stream);
+    if (e == cudaSuccess && pl->sf) e = launch_treal(d_taa, d_tab, d_tbb, nt, L, pl->TR, ctx->stream);
     if (e == cudaSuccess && pl->sf) e = launch_sf_phases(D.atom_pos, na, half, ext, d_ex, ctx->stream);
     if (e == cudaSuccess && pl->sf)
         e = launch_sf_table(d_ex, d_ex + (size_t)na * ext[0], d_ex + (size_t)na * (ext[0] + ext[1]), d_order,
@@ -1990,7 +1989,7 @@ int hsdla_contract_ab(hsdla_context *ctx, int32_t L, int32_t a, int64_t G, const
     const int nl = max_lmax + 1;
     const int64_t twoL = 2 * (int64_t)L;
     std::vector<cx> tf_all((size_t)a * twoL * twoL, 0.0);
-    std::vector<double> w(twoL * a), wsq(twoL * a);
+    std::vector<double> w(twoL * a);
     for (int j = 0; j < a; ++j) {
         const int na_ = t_sizes[3 * j], nab = t_sizes[3 * j + 1], nb = t_sizes[3 * j + 2];
         if (na_ < 0 || nab < 0 || nb < 0 || na_ > L || nab > L || nb > L || lmaxs[j] < 0 || lmaxs[j] > max_lmax)
@@ -2017,10 +2016,9 @@ int hsdla_contract_ab(hsdla_context *ctx, int32_t L, int32_t a, int64_t G, const
         for (int l = 0; l < nl; ++l) {
             const double su = sqrt_u_norms[j * nl + l];
             for (int lm = l * l; lm < (l + 1) * (l + 1); ++lm) {
-                w[twoL * j + lm] = 1.0; wsq[twoL * j + lm] = 1.0;
+                w[twoL * j + lm] = 1.0;
                 // rows above the atom's lmax are left unset by apply_u_norm_s (:64-86) while B is 0 there
-                const double u = (l <= lmaxs[j]) ? su * su : 0.0;
-                w[twoL * j + L + lm] = u; wsq[twoL * j + L + lm] = std::sqrt(u);
+                w[twoL * j + L + lm] = (l <= lmaxs[j]) ? su * su : 0.0;
             }
         }
     }
@@ -2042,7 +2040,7 @@ int hsdla_contract_ab(hsdla_context *ctx, int32_t L, int32_t a, int64_t G, const
     pl->twoLa = twoL * a;
     pl->atom_type.resize(a);
     for (int j = 0; j < a; ++j) pl->atom_type[j] = j;
-    const int64_t bytes = ((int64_t)sizeof(double2) * tf_all.size() + 255) / 256 * 256 + 2 * 8 * pl->twoLa + 512;
+    const int64_t bytes = ((int64_t)sizeof(double2) * tf_all.size() + 255) / 256 * 256 + 8 * pl->twoLa + 512;
     int rc = ctx_malloc(ctx, &pl->tables, bytes);
     if (rc) { delete pl; return rc; }
     pl->tables_bytes = bytes;
@@ -2050,7 +2048,6 @@ int hsdla_contract_ab(hsdla_context *ctx, int32_t L, int32_t a, int64_t G, const
     char *dp = reinterpret_cast<char *>(pl->tables);
     pl->Tfull = reinterpret_cast<double2 *>(dp);
     pl->w = reinterpret_cast<double *>(dp + ((int64_t)sizeof(double2) * tf_all.size() + 255) / 256 * 256);
-    pl->wsqrt = pl->w + pl->twoLa;
     PlanKpoint pk;
     pk.n_g = G;
     pk.dk.n_g = G;
@@ -2073,7 +2070,6 @@ int hsdla_contract_ab(hsdla_context *ctx, int32_t L, int32_t a, int64_t G, const
     if (cudaMemcpyAsync(pl->Tfull, tf_all.data(), sizeof(double2) * tf_all.size(), cudaMemcpyHostToDevice, st) !=
             cudaSuccess ||
         cudaMemcpyAsync(pl->w, w.data(), 8 * pl->twoLa, cudaMemcpyHostToDevice, st) != cudaSuccess ||
-        cudaMemcpyAsync(pl->wsqrt, wsq.data(), 8 * pl->twoLa, cudaMemcpyHostToDevice, st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
         return done(set_err(ctx, HSDLA_ERR_CUDA, "table upload failed"));
     if (pl->opts.precision == HSDLA_PREC_OZAKI_FP8) {
