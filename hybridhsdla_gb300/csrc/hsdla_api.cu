@@ -217,8 +217,8 @@ void ctx_cache_release(hsdla_context *ctx) {
 }
 
 // Device allocations of the context.  Blocks up to kCacheBlockMax are served from the blocks
-// earlier plans released when one of at most twice the size is kept; the memory cap counts kept
-// blocks as used (they are released first when a request would exceed it).
+// earlier plans released when one of at most twice the size is kept (under a memory cap a sixteenth more than the
+// request); the cap counts kept blocks as used (they are released first when a request would exceed it).
 int ctx_malloc(hsdla_context *ctx, void **p, int64_t bytes) {
     *p = nullptr;
     if (bytes <= 0) return HSDLA_OK;
@@ -226,7 +226,7 @@ int ctx_malloc(hsdla_context *ctx, void **p, int64_t bytes) {
     if (ctx->mem_cap > 0 && ctx->mem_used > ctx->mem_cap) ctx_cache_release(ctx);
     if (bytes <= kCacheBlockMax && (ctx->mem_cap == 0 || ctx->mem_used <= ctx->mem_cap)) {
         auto it = ctx->cache.lower_bound(bytes);
-        if (it != ctx->cache.end() && it->first <= 2 * bytes) {
+        if (it != ctx->cache.end() && it->first <= (ctx->mem_cap > 0 ? bytes + bytes / 16 : 2 * bytes)) {
             *p = it->second;
             ctx->live[*p] = it->first;
             ctx->cached_bytes -= it->first;
@@ -408,6 +408,8 @@ int ctx_workspace_tail(hsdla_context *ctx, int64_t bytes, int64_t extra, void **
     }
     return ctx_workspace(ctx, bytes, out);
 }
+
+int64_t r1k(int64_t b) { return (b + 1023) / 1024 * 1024; }
 
 bool finite_all(const double *p, int64_t n) {
     for (int64_t i = 0; i < n; ++i)
@@ -819,39 +821,67 @@ int hsdla_prepare_tmat(int32_t lmax, int32_t lmax_nonsph, const hsdla_cx *taa, c
 
 namespace {
 int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoint *kpts, int32_t nk,
-                     const hsdla_opts *opts, hsdla_plan **out, bool defer_tcheck);
+                     const hsdla_opts *opts, hsdla_plan **out, bool defer_tcheck, bool host_outputs);
 }
 
 extern "C" {
 
 int hsdla_plan_create(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoint *kpts, int32_t nk,
                       const hsdla_opts *opts, hsdla_plan **out) {
-    return plan_create_impl(ctx, s, kpts, nk, opts, out, false);
+    return plan_create_impl(ctx, s, kpts, nk, opts, out, false, false);
 }
 
 }  // extern "C"
 
 namespace {
 int64_t workspace_budget(hsdla_context *ctx);
+int64_t sf_kpoint_bytes(bool fp64, int64_t ldm, int64_t G, int64_t tbatch);
+int64_t fp64_persist_bytes(bool sf, int64_t nk, int64_t t_jobs, int64_t sets);
 
-// Device bytes of one k-point (the largest) over `ns` row sets, with one product slot: real rows, Z',
-// digit planes of 12 slices, products, structure factors.
-int64_t sets_bytes(const hsdla_system *s, const hsdla_kpoint *kpts, int nk, int64_t ns) {
-    const int64_t L = (int64_t)(s->max_lmax + 1) * (s->max_lmax + 1);
-    int64_t G = 0, half[3] = {0, 0, 0};
+// Whether a plan over `ns` row sets, in groups of one k-point with one product slot, fits: its workspace the budget,
+// and all that it and the call hold on the device (`tables` bytes of it the plan's, `outputs` the device H and S of a
+// host call) the cap or the device's free memory.
+bool sets_fit(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoint *kpts, int nk, const hsdla_opts &o,
+              int64_t ns, int64_t tables, int64_t outputs) {
+    const int64_t twoL = 2 * (int64_t)(s->max_lmax + 1) * (s->max_lmax + 1), K = twoL * s->num_atoms;
+    const bool fp64 = o.precision == HSDLA_PREC_FP64, tuned = !fp64 && o.num_slices == 0;
+    const int slices = o.num_slices > 0 ? o.num_slices : kOzMaxSlices;
+    int64_t G = 0, ws = 0, persist = 0;
     for (int i = 0; i < nk; ++i) {
-        G = std::max(G, kpts[i].n_g);
-        for (int64_t q = 0; q < kpts[i].n_g; ++q)
-            for (int c = 0; c < 3; ++c) half[c] = std::max<int64_t>(half[c], 2 * std::abs((int64_t)kpts[i].g[3 * q + c]));
+        const int64_t n = kpts[i].n_g;
+        if (n == 0) continue;
+        G = std::max(G, n);
+        const std::vector<int64_t> one{n};
+        ws = std::max(ws, sf_kpoint_bytes(fp64, twoL * ns, n, 1) +
+                              (fp64 ? 0 : 1024 + ozaki_group_bytes(slices, twoL, s->num_atoms, ns, one, 1, true, true)));
+        persist += fp64 ? fp64_persist_bytes(true, 1, ns, ns)
+                        : ozaki_group_persist_bytes(slices, twoL, s->num_atoms, ns, one, 1, true, s->num_types);
     }
-    const int64_t box = (2 * half[0] + 1) * (2 * half[1] + 1) * (2 * half[2] + 1);
-    return 8 * 3 * 2 * L * ns * G + 4 * 12 * (G + 256) * (ns * (2 * L + 64) + 256) + 24 * G * G + 16 * ns * box;
+    if (G == 0) return true;
+    if (ws > workspace_budget(ctx)) return false;
+    const int64_t rows = 2 * (int64_t)sizeof(double2) * K * G + 4096;     // (hsdla_plan_workspace_bytes' least)
+    int64_t most = std::max(ws + 4096, rows) + persist;
+    if (tuned) {                                                          // autotune_slices' buffers
+        const int64_t n = std::min<int64_t>(G, 384);
+        most = std::max(most, rows + 2 * K * n * (int64_t)sizeof(double2) + 4 * n * n * (int64_t)sizeof(double2) +
+                                  ozaki_pipeline_workspace(8, twoL, s->num_atoms, s->num_types, n) + 1024 +
+                                  (int64_t)sizeof(Fp64Job) * (s->num_atoms + 2));
+    }
+    int64_t avail = ctx->ws_bytes + ctx->hout_bytes + ctx->cached_bytes;
+    if (ctx->mem_cap > 0) {
+        avail += ctx->mem_cap - ctx->mem_used;
+    } else {
+        size_t fr = 0, tot = 0;
+        cudaMemGetInfo(&fr, &tot);
+        avail += (int64_t)fr;
+    }
+    return tables + outputs + most <= avail;
 }
 
 // defer_tcheck: leave the T-block check to the caller (after its own synchronisation), so that the
-// device runs on while the host sets up the execution
+// device runs on while the host sets up the execution; host_outputs: the call also holds device H and S
 int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoint *kpts, int32_t nk,
-                     const hsdla_opts *opts, hsdla_plan **out, bool defer_tcheck) {
+                     const hsdla_opts *opts, hsdla_plan **out, bool defer_tcheck, bool host_outputs) {
     if (!ctx || !out) return HSDLA_ERR_ARG;
     *out = nullptr;
     CUDA_TRY(ctx, cudaSetDevice(ctx->device));
@@ -869,9 +899,57 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     RowSets sets;
     bool use_classes = s->atom_rotmat && !(sf_env0 && strtol(sf_env0, nullptr, 10) == 0) &&
                              env_flag("HSDLA_CLASSES", true) && make_classes(s, sets);
-    // many sets: only where one k-point's workspace (one product slot) fits, else the per-atom form,
-    // which can stream its contraction in atom panels
-    if (use_classes && (!sets.shared || sets.n > kMaxTypes) && sets_bytes(s, kpts, nk, sets.n) > workspace_budget(ctx))
+    hsdla_opts o{};
+    if (opts) o = *opts;
+    if (o.precision != HSDLA_PREC_FP64 && o.precision != HSDLA_PREC_OZAKI_FP8)
+        return set_err(ctx, HSDLA_ERR_ARG, "unknown precision %d", o.precision);
+    const int na = s->num_atoms, nt = s->num_types, nl = s->max_lmax + 1, L = nl * nl;
+    const size_t tf_elems = (size_t)nt * 4 * L * L;
+    const int64_t LLnt = (int64_t)nt * L * L, twoLa = 2 * (int64_t)L * na;
+    // structure-factor form: the box of G-vector differences g_col - g_row
+    int half[3] = {0, 0, 0}, ext[3] = {1, 1, 1};
+    if (!s->atom_rotmat || use_classes) {
+        for (int i = 0; i < nk; ++i)
+            for (int64_t q = 0; q < kpts[i].n_g; ++q)
+                for (int c = 0; c < 3; ++c) half[c] = std::max(half[c], 2 * std::abs(kpts[i].g[3 * q + c]));
+        for (int c = 0; c < 3; ++c) ext[c] = 2 * half[c] + 1;
+    }
+    const auto tfull_wanted = [&](bool sf) { return !sf || (o.precision == HSDLA_PREC_OZAKI_FP8 && o.num_slices == 0); };
+    // the plan's tables, one device block: the uploaded part, then what the device fills
+    const auto table_bytes = [&](const RowSets &q, bool sf, int64_t &upload) {
+        int64_t bytes = 0;
+        auto add = [&](int64_t b) { bytes += (b + 255) & ~int64_t(255); };
+        add(sizeof(int32_t) * na); add(sizeof(double) * 3 * na); add(s->atom_rotmat ? sizeof(double) * 9 * na : 0);
+        add(sizeof(int32_t) * q.n);
+        add(sizeof(double) * q.rots.size()); add(sizeof(int32_t) * q.rot_begin.size());
+        add(sizeof(double) * 2 * nl * nl);
+        add(sizeof(double) * nt); add(sizeof(int32_t) * nt);
+        for (int i = 0; i < 5; ++i) add(sizeof(double) * nt * nl);
+        add(sizeof(double) * L);
+        for (int i = 0; i < 3; ++i) add(sizeof(double2) * LLnt);     // T_AA, T_AB, T_BB as given
+        add(sizeof(double) * twoLa);
+        for (int i = 0; i < nk; ++i) add(sizeof(int32_t) * 3 * kpts[i].n_g);
+        if (sf) {                // row weights, the atoms set by set with the structure factors' fixed points
+            add(sizeof(double) * 2 * L * q.n);
+            add(sizeof(int32_t) * (na + 2 * q.n + 1));
+        }
+        upload = bytes;
+        // the assembled T blocks and their checks; the per-atom phase factors along each axis, the structure
+        // factors and the real T blocks
+        if (tfull_wanted(sf)) add(sizeof(double2) * tf_elems);
+        add(sizeof(unsigned long long) * 5 * nt);
+        if (sf) {
+            add(sizeof(double2) * (int64_t)na * (ext[0] + ext[1] + ext[2]));
+            add(sizeof(double2) * (int64_t)q.n * ext[0] * ext[1] * ext[2]);
+            add(sizeof(double) * 2 * tf_elems);
+        }
+        return bytes;
+    };
+    // many sets: only where they fit, else the per-atom form, which can stream its contraction in atom panels
+    int64_t upload_bytes = 0, outputs = 0;
+    for (int i = 0; host_outputs && i < nk; ++i) outputs += 2 * (int64_t)sizeof(double2) * kpts[i].n_g * kpts[i].n_g;
+    if (use_classes && (!sets.shared || sets.n > kMaxTypes) &&
+        !sets_fit(ctx, s, kpts, nk, o, sets.n, table_bytes(sets, true, upload_bytes), outputs))
         use_classes = false;
     if (!use_classes) {      // the types, no rotations
         sets = RowSets();
@@ -883,18 +961,13 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
     pl->ctx = ctx;
     pl->classes = use_classes ? sets.n : 0;
     pl->per_atom_sets = use_classes && !sets.shared;
-    if (opts) pl->opts = *opts;
-    if (pl->opts.precision != HSDLA_PREC_FP64 && pl->opts.precision != HSDLA_PREC_OZAKI_FP8) {
-        delete pl;
-        return set_err(ctx, HSDLA_ERR_ARG, "unknown precision %d", pl->opts.precision);
-    }
+    pl->opts = o;
     if (pl->opts.target_rel_err <= 0.0) pl->opts.target_rel_err = 1e-13;
-    const int na = s->num_atoms, nt = s->num_types, nl = s->max_lmax + 1, L = nl * nl;
     const int ns = sets.n;
     pl->L = L; pl->na = na; pl->nt = ns; pl->ntypes = nt; pl->max_lmax = s->max_lmax;
     pl->set_type = sets.set_type;
     pl->hoist = s->atom_rotmat == nullptr || use_classes;
-    pl->twoLa = 2 * (int64_t)L * na;
+    pl->twoLa = twoLa;
     pl->atom_type.assign(s->atom_type, s->atom_type + na);
 
     // ---- host tables
@@ -916,46 +989,9 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
                 w[rB] = un;
             }
     }
-    const size_t tf_elems = (size_t)nt * 4 * L * L;
-    const int64_t LLnt = (int64_t)nt * L * L;
-
-    // ---- one device block for all tables: the uploaded part, then what the device fills
-    int64_t bytes = 0;
-    auto add = [&](int64_t b) { bytes += (b + 255) & ~int64_t(255); };
-    add(sizeof(int32_t) * na); add(sizeof(double) * 3 * na); add(s->atom_rotmat ? sizeof(double) * 9 * na : 0);
-    add(sizeof(int32_t) * ns);
-    add(sizeof(double) * sets.rots.size()); add(sizeof(int32_t) * sets.rot_begin.size());
-    add(sizeof(double) * 2 * nl * nl);
-    add(sizeof(double) * nt); add(sizeof(int32_t) * nt);
-    for (int q = 0; q < 5; ++q) add(sizeof(double) * nt * nl);
-    add(sizeof(double) * L);
-    for (int q = 0; q < 3; ++q) add(sizeof(double2) * LLnt);     // T_AA, T_AB, T_BB as given
-    add(sizeof(double) * pl->twoLa);
-    for (int i = 0; i < nk; ++i) add(sizeof(int32_t) * 3 * kpts[i].n_g);
-    // structure-factor form: per-type weights, per-atom phase factors along each axis, the atoms
-    // grouped by type and the table itself over the box of G-vector differences g_col - g_row
-    const char *sf_env = getenv("HSDLA_SF");
-    pl->sf = pl->hoist && !(sf_env && strtol(sf_env, nullptr, 10) == 0);
-    int half[3] = {0, 0, 0}, ext[3] = {1, 1, 1};
-    if (pl->sf) {
-        for (int i = 0; i < nk; ++i)
-            for (int64_t q = 0; q < kpts[i].n_g; ++q)
-                for (int c = 0; c < 3; ++c) half[c] = std::max(half[c], 2 * std::abs(kpts[i].g[3 * q + c]));
-        for (int c = 0; c < 3; ++c) ext[c] = 2 * half[c] + 1;
-        add(sizeof(double) * 2 * L * ns);
-        add(sizeof(int32_t) * (na + 2 * ns + 1));
-    }
-    const int64_t upload_bytes = bytes;
-    // filled on the device: the assembled T blocks and their checks; the structure-factor form's
-    // per-atom phase factors, its table and its real T blocks
-    const bool want_tfull = !pl->sf || (pl->opts.precision == HSDLA_PREC_OZAKI_FP8 && pl->opts.num_slices == 0);
-    if (want_tfull) add(sizeof(double2) * tf_elems);
-    add(sizeof(unsigned long long) * 5 * nt);
-    if (pl->sf) {
-        add(sizeof(double2) * (int64_t)na * (ext[0] + ext[1] + ext[2]));
-        add(sizeof(double2) * (int64_t)ns * ext[0] * ext[1] * ext[2]);
-    }
-    if (pl->sf) add(sizeof(double) * 2 * tf_elems);
+    pl->sf = pl->hoist && !(sf_env0 && strtol(sf_env0, nullptr, 10) == 0);
+    const bool want_tfull = tfull_wanted(pl->sf);
+    const int64_t bytes = table_bytes(sets, pl->sf, upload_bytes);
     const double p_tables = pms();
     rc = ctx_malloc(ctx, &pl->tables, bytes);
     if (rc) { delete pl; return rc; }
@@ -1156,15 +1192,17 @@ int plan_create_impl(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoi
 
 namespace {
 
+// One k-point of a group's workspace, each buffer 1 KB aligned.  Structure-factor form: the real rows R (FP64: and
+// diag(w) R), Z' (two parts) and the three products of each type of a combine batch (no C, no X).
+int64_t sf_kpoint_bytes(bool fp64, int64_t ldm, int64_t G, int64_t tbatch) {
+    return (fp64 ? 2 : 1) * r1k(ldm * G * (int64_t)sizeof(double)) + r1k(2 * ldm * G * (int64_t)sizeof(double)) +
+           3 * r1k(tbatch * G * G * (int64_t)sizeof(double));
+}
 // FP64 buffers of one k-point inside a group workspace.
 int64_t kpoint_fp64_bytes(const hsdla_plan *pl, int64_t G) {
     const int64_t K = pl->twoLa, ldm = 2 * (int64_t)pl->L * pl->nt;
-    auto r = [](int64_t x) { return (x + 1023) / 1024 * 1024; };        // each buffer is 1 KB aligned
-    // structure-factor form: the real rows R (FP64: and diag(w) R), Z' (two parts) and the three products of each
-    // type of a combine batch (no C, no X)
-    if (pl->sf)
-        return (pl->opts.precision == HSDLA_PREC_FP64 ? 2 : 1) * r(ldm * G * (int64_t)sizeof(double)) +
-               r(2 * ldm * G * (int64_t)sizeof(double)) + 3 * r(pl->tbatch * G * G * (int64_t)sizeof(double));
+    auto r = r1k;
+    if (pl->sf) return sf_kpoint_bytes(pl->opts.precision == HSDLA_PREC_FP64, ldm, G, pl->tbatch);
     const int64_t nCX = pl->opts.precision == HSDLA_PREC_FP64 ? 2 : 1;   // FP64 keeps C and X apart
     int64_t b = nCX * r(K * G * (int64_t)sizeof(double2));
     if (pl->hoist) b += 2 * r(ldm * G * (int64_t)sizeof(double2));
@@ -1181,26 +1219,26 @@ int64_t group_bytes(const hsdla_plan *pl, const std::vector<int> &kidx) {
     return b;
 }
 
+// The FP64 group keeps two job tables, each rounded up to 1 KiB: the T applications (one per
+// type when hoisted, else one per atom, per k-point) and the S/H products (three per type in
+// the structure-factor form, else two, per k-point).
+int64_t fp64_persist_bytes(bool sf, int64_t nk, int64_t t_jobs, int64_t sets) {
+    const int64_t js = sf ? sizeof(Fp64RealJob) : sizeof(Fp64Job);
+    return r1k(js * nk * t_jobs) + r1k(js * nk * (sf ? 3 * sets : 2));
+}
+
 int64_t group_persist_bytes(const hsdla_plan *pl, const std::vector<int> &kidx) {
     std::vector<int64_t> G;
     for (int i : kidx) G.push_back(pl->kps[i].n_g);
     if (pl->opts.precision == HSDLA_PREC_OZAKI_FP8)
         return ozaki_group_persist_bytes(pl->oz.num_slices, 2 * (int64_t)pl->L, pl->na, pl->nt, G, pl->panels, pl->sf,
                                          pl->ntypes);
-    // the FP64 group keeps two job tables, each rounded up to 1 KiB: the T applications (one per
-    // type when hoisted, else one per atom, per k-point) and the S/H products (three per type in
-    // the structure-factor form, else two, per k-point)
-    const int64_t nk = (int64_t)kidx.size();
-    const int64_t n_t = nk * (pl->hoist ? pl->nt : pl->na);
-    const int64_t n_sh = nk * (pl->sf ? 3 * pl->nt : 2);
-    auto up = [](int64_t b) { return (b + 1023) / 1024 * 1024; };
-    const int64_t js = pl->sf ? sizeof(Fp64RealJob) : sizeof(Fp64Job);
-    return up(js * n_t) + up(js * n_sh);
+    return fp64_persist_bytes(pl->sf, (int64_t)kidx.size(), pl->hoist ? pl->nt : pl->na, pl->nt);
 }
 
 // Device-memory budget for one group's workspace: HSDLA_WORKSPACE_BUDGET (bytes), else 85% of
 // what is free now (plus the workspace this context already holds) less 2 GiB, reduced to fit
-// the context's memory cap.
+// the context's memory cap (which kept blocks make way for).
 int64_t workspace_budget(hsdla_context *ctx) {
     int64_t budget = 0;
     if (const char *v = getenv("HSDLA_WORKSPACE_BUDGET")) budget = strtoll(v, nullptr, 10);
@@ -1210,7 +1248,7 @@ int64_t workspace_budget(hsdla_context *ctx) {
         budget = (int64_t)(0.85 * (double)(fr + (size_t)ctx->ws_bytes)) - ((int64_t)2 << 30);
         budget = std::max<int64_t>(budget, (int64_t)1 << 30);
     }
-    if (ctx->mem_cap > 0) budget = std::min(budget, ctx->mem_cap - ctx->mem_used + ctx->ws_bytes);
+    if (ctx->mem_cap > 0) budget = std::min(budget, ctx->mem_cap - ctx->mem_used + ctx->cached_bytes + ctx->ws_bytes);
     return budget;
 }
 
@@ -1256,7 +1294,7 @@ void choose_type_batch(hsdla_plan *pl, int64_t budget) {
 }
 
 // Greedy k-point groups whose workspace fits the budget (at least one k-point per group).
-void form_groups(hsdla_plan *pl, int64_t budget) {
+void form_groups_within(hsdla_plan *pl, int64_t budget) {
     choose_panels(pl, budget);
     choose_type_batch(pl, budget);
     pl->groups.clear();
@@ -1281,6 +1319,22 @@ void form_groups(hsdla_plan *pl, int64_t budget) {
     }
     pl->group_ws_bytes = 0;
     for (auto &g : pl->groups) pl->group_ws_bytes = std::max(pl->group_ws_bytes, group_bytes(pl, g.kidx));
+}
+
+// ... and under a memory cap the groups' tables beside it: as much less for the workspace as they take, until both fit
+// (or, where nothing does, as first formed).
+void form_groups(hsdla_plan *pl, int64_t budget) {
+    form_groups_within(pl, budget);
+    int64_t b = budget;
+    for (int i = 0; i < 16 && pl->ctx->mem_cap > 0; ++i) {
+        int64_t tables = 0;
+        for (const auto &g : pl->groups) tables += r1k(group_persist_bytes(pl, g.kidx));
+        if (hsdla_plan_workspace_bytes(pl) + tables <= budget) return;
+        if (b == 1) break;
+        b = std::max<int64_t>(1, std::min(b - b / 16, budget - tables - 4096));
+        form_groups_within(pl, b);
+    }
+    if (b != budget) form_groups_within(pl, budget);
 }
 
 void release_groups(hsdla_plan *pl) {
@@ -2170,7 +2224,7 @@ int hsdla_create_hs(hsdla_context *ctx, const hsdla_system *s, const hsdla_kpoin
     cudaEventRecord(e0, ctx->stream);
     hsdla_plan *pl = nullptr;
     // the T blocks' check read after the launches (HSDLA_DEFER_TCHECK=0: before them)
-    int rc = plan_create_impl(ctx, s, kpts, nk, opts, &pl, env_flag("HSDLA_DEFER_TCHECK", true));
+    int rc = plan_create_impl(ctx, s, kpts, nk, opts, &pl, env_flag("HSDLA_DEFER_TCHECK", true), true);
     t_plan = ms_since(t_start);
     if (rc) { cudaEventDestroy(e0); cudaEventDestroy(e1); return rc; }
     // device outputs: one buffer of the largest size, reused per k-point group
@@ -2391,8 +2445,6 @@ bool host_memory(const void *p) {
     }
     return a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeUnregistered;
 }
-
-int64_t r1k(int64_t b) { return (b + 1023) / 1024 * 1024; }
 
 //   zherk : C = alpha op(A) op(A)^H + beta C                       (alpha, beta real)
 //   zher2k: C = alpha op(A) op(B)^H + conj(alpha) op(B) op(A)^H + beta C
