@@ -538,12 +538,17 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     const uint32_t rank = cluster_rank();
     const bool leader = rank == 0;
     // bounded wait that records where it expired (first failure wins)
-    auto pwait = [&](uint64_t *bar, uint32_t parity, int where, int stage_, int count) -> bool {
-        if (mbar_wait(bar, parity, &abort_flag, err, where)) return true;
+    auto expired = [&](uint32_t parity, int stage_, int count) -> bool {
         if (atomicCAS(err + 7, 0, 1) == 0) {
             err[1] = blockIdx.x; err[2] = (int)rank; err[3] = stage_; err[4] = (int)parity; err[5] = count;
         }
         return false;
+    };
+    auto pwait = [&](uint64_t *bar, uint32_t parity, int where, int stage_, int count) -> bool {
+        return mbar_wait(bar, parity, &abort_flag, err, where) || expired(parity, stage_, count);
+    };
+    auto pwait_pair = [&](uint64_t *bar, uint32_t parity, int where, int stage_, int count) -> bool {
+        return mbar_wait<true>(bar, parity, &abort_flag, err, where) || expired(parity, stage_, count);
     };
     const int64_t pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
     auto map_of = [&](int i) -> const CUtensorMap * {
@@ -654,7 +659,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
                         const int64_t ce = min(jnkb, cb + ck);
                         const int end = step + (int)(ce - cb) * (ihi - ilo + 1);
                         if (end <= part.x || step >= part.y) { step = end; continue; }
-                        if (!pwait(&bars.tempty, (uint32_t)((unit & 1) ^ 1), 2, stage, (int)unit)) { ok = false; break; }
+                        if (!pwait_pair(&bars.tempty, (uint32_t)((unit & 1) ^ 1), 2, stage, (int)unit)) { ok = false; break; }
                         tc_fence_after();
                         bool first = true;
                         for (int64_t kb = cb; ok && kb < ce; ++kb) {
@@ -801,7 +806,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
                                 if (c == kCh - 1 && hh + kLdCols >= 32) {
                                     tc_fence_before();
                                     __syncwarp();
-                                    if (lane == 0) mbar_arrive_remote(tempty_leader);
+                                    if (lane == 0) mbar_arrive_pair(tempty_leader);
                                 }
 #pragma unroll
                                 for (int g4 = 0; g4 < kLdCols; g4 += kStageCols, ++rd) {

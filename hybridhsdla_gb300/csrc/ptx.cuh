@@ -24,22 +24,33 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
 }
+// kPair: the phase is completed by arrivals of both CTAs of a pair (mbar_arrive_pair).
+template <bool kPair = false>
 __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
     uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
+    if constexpr (kPair)
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n"
+            " selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
+    else
+        asm volatile(
+            "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(ok)
+            : "r"(smem_u32(bar)), "r"(parity)
+            : "memory");
     return ok != 0;
 }
 // Bounded wait.  Returns false (and raises the CTA abort flag) when the budget expires
 // or another role already aborted.
+template <bool kPair = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag, int *err,
                                           int where, long long budget = kWaitCycles) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (mbar_try_wait<kPair>(bar, parity)) return true;
     const long long t0 = clock64();
-    while (!mbar_try_wait(bar, parity)) {
+    while (!mbar_try_wait<kPair>(bar, parity)) {
         if (*abort_flag) return false;
         if (clock64() - t0 > budget) {
             *abort_flag = 1;
@@ -139,8 +150,13 @@ __device__ __forceinline__ uint32_t mapa_rank(uint32_t saddr, uint32_t rank) {
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
 }
-__device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_addr) : "memory");
+// Arrival on a barrier of the pair's leader: hands over TMEM that this warp has read (tcgen05.wait::ld, then
+// tcgen05.fence::before_thread_sync; mbar_wait<true> and tcgen05.fence::after_thread_sync on the other side).  The
+// fences order TMEM; no ordinary memory changes hands, so the barrier's own order is relaxed, at the scope of
+// both CTAs.  (A release at that scope also waits for the warp's output stores in flight: the real products of one
+// type and 8000 columns 1.41 ms, 0.87 here.)
+__device__ __forceinline__ void mbar_arrive_pair(uint32_t cluster_addr) {
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ void tma_load_2d_pair(void *dst, const CUtensorMap *map, uint32_t bar_cluster, int x,
                                                  int y) {

@@ -156,12 +156,17 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t rank = cluster_rank();
     const bool leader = rank == 0;
     const int s = bands.s;
-    auto pwait = [&](uint64_t *bar, uint32_t parity, int where, int slot, int count) -> bool {
-        if (mbar_wait(bar, parity, &abort_flag, err, where)) return true;
+    auto expired = [&](uint32_t parity, int slot, int count) -> bool {
         if (atomicCAS(err + 7, 0, 1) == 0) {
             err[1] = blockIdx.x; err[2] = (int)rank; err[3] = slot; err[4] = (int)parity; err[5] = count;
         }
         return false;
+    };
+    auto pwait = [&](uint64_t *bar, uint32_t parity, int where, int slot, int count) -> bool {
+        return mbar_wait(bar, parity, &abort_flag, err, where) || expired(parity, slot, count);
+    };
+    auto pwait_pair = [&](uint64_t *bar, uint32_t parity, int where, int slot, int count) -> bool {
+        return mbar_wait<true>(bar, parity, &abort_flag, err, where) || expired(parity, slot, count);
     };
     const int64_t pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
     unsigned char *abuf = smem, *bbuf = smem + kNA * kABytes;
@@ -285,7 +290,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                         const bool last = b + step >= nbands, pairs = bands.w[b] == 2;
                         const uint32_t use = nbuf == 1 ? seq : seq / kBufs;
                         const int h = (int)(seq - use * nbuf);
-                        if (!pwait(&bars.tempty[h], (use & 1) ^ 1, 2, b, (int)seq)) { ok = false; break; }
+                        if (!pwait_pair(&bars.tempty[h], (use & 1) ^ 1, 2, b, (int)seq)) { ok = false; break; }
                         for (; ready <= (last ? nbatch - 1 : (T - 2) / kBatch); ++ready)
                             if (!pwait(&bars.full[(n + ready) % kRing], ((n + ready) / kRing) & 1, 3, ready, (int)seq)) { ok = false; break; }
                         if (!ok) break;
@@ -396,7 +401,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                     tmem_ld_wait();
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive_remote(tempty_leader + h * 8);
+                    if (lane == 0) mbar_arrive_pair(tempty_leader + h * 8);
                     if (kb == 0 && b == 0) {
                         // the tile before leaves only here, after this band has left its buffer: the MMAs
                         // run ahead by one more band while it is being stored
