@@ -368,7 +368,7 @@ void sf_fixed_points(const std::vector<int32_t> &atoms, std::vector<int32_t> &or
         for (; b < n && b - a < kSumTypes; ++b) {
             const int64_t N = atoms[order[b]];
             const int fb = std::min(56, 59 - log2_up(std::max<int64_t>(sum + N, atoms[order[a]] + 1)));
-            if (b > a && fb < 54 - log2_up(N + 1)) break;
+            if (b > a && N > 0 && fb < 54 - log2_up(N + 1)) break;
             sum += N;
             f = fb;
         }
