@@ -132,7 +132,7 @@ constexpr int kSfTile = 32;
 // arrive in one of two stages of shared memory by asynchronous copies while the item before is summed.
 // kFixed: fixed-point products and structure factors, summed exactly in integers.  GB300's FP64 pipe
 // (2 multiply-adds per cycle and SM) bounded this kernel at 0.95 of its rate.  8000 columns of 8 types:
-// FP64 2.60 ms, integers 1.39 ms (0.66 of the DRAM rate); 2 k-points of 6300 columns and 4 types: 1.74 and 1.13
+// FP64 2.60 ms, integers 1.39 ms (0.77 of the measured copy rate); 2 k-points of 6300 columns and 4 types: 1.74 and 1.13
 // ms.  Bound now by the wide multiply-adds (a warp's takes four cycles; 24 an element and type) on 16 warps an
 // SM; 20 warps leave too little L1 beside the stages (1.67 and 1.44 ms).  Loads into registers, four types
 // ahead of their use on 24 warps, took 1.59 and 1.41 ms.
@@ -314,11 +314,13 @@ __global__ void __launch_bounds__(kSfTile *kRows, 512 / (kSfTile * kRows)) sf_co
 
 template <bool kFixed, bool kItems>
 cudaError_t combine_launch(const SfTab &t, const void *sf, bool first, int64_t tiles, cudaStream_t st) {
-    // 4 columns of a tile at a time where there are tiles enough, 8 where not
+    // 4 columns of a tile at a time from two tiles per SM on, 8 below.  Combine and slicing, us, by 8 and by 4: 235 columns of 2
+    // types (36 tiles) 42 and 47, 501 of 2 (136) 43 and 49, 1000 of 4 (528) 70 and 67, 1500 of 4 (1128) 96 and 93, 3000 of 8
+    // (4465) 337 and 316
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const bool few = tiles < 8 * (int64_t)nsm;
+    const bool few = tiles < 2 * (int64_t)nsm;
     const void *kernel = few ? (const void *)sf_combine_kernel<kFixed, 8, kItems> : (const void *)sf_combine_kernel<kFixed, 4, kItems>;
     const int rows = few ? 8 : 4, smem = rows * 2 * kStageBytesWarp;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
