@@ -180,7 +180,8 @@ struct Sums<true> {
 __device__ __noinline__ double2 sum2(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 
 // kItems: the items and ends of the sums as listed (SfTab::item); else four types each (the last fewer) and every second
-// item or the last, of one fixed point, SfTab::bits0 (listed, 8000 columns of 8 equal types 1.44 ms).
+// item or the last, of one fixed point, SfTab::bits0 (combine and slicing of 8000 columns of 8 equal types: listed 1.84 ms,
+// 1.79 here; of 1 to 33 atoms, a group of seven types and one of one: 2.23).
 template <bool kFixed, int kRows, bool kItems>
 __global__ void __launch_bounds__(kSfTile *kRows, 512 / (kSfTile * kRows)) sf_combine_kernel(const __grid_constant__ SfTab tab,
                                                                                      const int4 *__restrict__ sf, int first) {
@@ -228,7 +229,7 @@ __global__ void __launch_bounds__(kSfTile *kRows, 512 / (kSfTile * kRows)) sf_co
     int64_t o = rowc + tab.slot0 * ps + ldp * (tc * kSfTile + ic);
     auto fetch = [&](uint32_t st) {
         if (ic < cend) {
-            const int t0 = kItems ? next & 0xff : kChunk * it, n = kItems ? (next >> 8) & 0xff : min(kChunk, ntypes - t0);
+            const int t0 = kItems ? (int)(next & 0xff) : kChunk * it, n = kItems ? (int)((next >> 8) & 0xff) : min(kChunk, ntypes - kChunk * it);
             const int4 *base = sf + __shfl_sync(0xffffffffu, pcol, ic) + t0;
             const uint32_t ds = st + (lane / 4 * kSfPitch + lane % 4) * 16;
             if (lane % 4 < n) {
@@ -269,7 +270,7 @@ __global__ void __launch_bounds__(kSfTile *kRows, 512 / (kSfTile * kRows)) sf_co
             fetch(smem + (stage ^ 1) * kStageBytesWarp);
             cp_async_wait_but_one();
             __syncwarp();
-            const int n = kItems ? (item >> 8) & 0xff : min(kChunk, ntypes - kChunk * q);
+            const int n = kItems ? (int)((item >> 8) & 0xff) : min(kChunk, ntypes - kChunk * q);
             const int4 *w = reinterpret_cast<const int4 *>(mem + stage * kStageBytesWarp) + lane * kSfPitch;
             const int2 *p = reinterpret_cast<const int2 *>(mem + stage * kStageBytesWarp + kStageSf) + lane;
             if (n == kChunk) {
