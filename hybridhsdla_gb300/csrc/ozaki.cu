@@ -1492,6 +1492,7 @@ struct OzGroup {
     int *d_progress = nullptr;
     int *d_err = nullptr;
     bool pair = false;          // S/H on CTA-pair tiles
+    bool pair_t = false;        // the T application on CTA-pair tiles
     PairSplit split, split_t;   // of the S/H products' and the T application's tiles
     bool sf = false;            // structure-factor form, on real rows:
     RealSliceTab rM, rX;        // the slicing of R (and R diag(w)) and of Z'
@@ -1622,6 +1623,33 @@ bool split_rule(int64_t N, int64_t steps, SplitRule &r) {
     if (r.R == 0 || r.P <= r.R) return false;
     r.per = (r.R * steps + r.P - 1) / r.P;
     return steps - r.per >= std::max(kSplitGain, steps / 4);
+}
+
+// Whether the T application of `jobs` runs on CTA-pair tiles (256 x 256) or on single-CTA ones (128 x 128).  Where both
+// take as many waves a tile's own time decides: ~0.14-0.16 ms a wave of pair tiles of one k-block (lmax 6 and below), 0.26 of
+// two, 0.33 and 0.40 of three and four, against 0.21, 0.25, 0.27 and 0.30 on single tiles, which at 40 columns take
+// 0.16, 0.17, 0.19 and 0.24 and at 7 0.09 to 0.20 (pair tiles 0.14 to 0.35).  Tiles cut over the idle pairs (`cut`) always
+// are pair ones: 1 atom, lmax 7, 232 columns 68 us, 184 uncut.
+bool pair_t_tiles(const std::vector<OzJob> &jobs, bool cut, int64_t steps) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[2];
+    int np = 0;
+    if (jobs.empty() || !use_pair()) return use_pair();
+    if (pair_config(cfg, at, np, nullptr) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    int64_t n1 = 0, n2 = 0, cols = 0;
+    for (const OzJob &j : jobs) {
+        n1 += job_tiles(j, kTileM);
+        n2 += job_tiles(j, kPairTile);
+        cols = std::max(cols, j.n);
+    }
+    SplitRule r;
+    if (cut && split_rule(n2, steps, r)) return true;
+    if ((n1 + 2 * np - 1) / (2 * np) > (n2 + np - 1) / np) return true;
+    const int64_t kblocks = jobs[0].nkb;
+    return cols > (kblocks < 2 ? 16 : kblocks < 3 ? 64 : INT64_MAX - 1);
 }
 
 // `mem`, `bytes`: as ozaki_split_bytes says, or none (no split).
@@ -2165,6 +2193,7 @@ int ozaki_group_prepare(OzakiPlan &oz, const OzGroupDesc &d, const std::vector<O
     // (b) T application: per type once (hoisted), or per atom of each panel
     g->pair = use_pair();
     const int64_t tile = g->pair ? kPairTile : kTileN;
+    g->pair_t = true;
     if (d.hoist) {
         std::vector<OzJob> jt;
         for (int k = 0; k < g->nk; ++k)
@@ -2182,7 +2211,8 @@ int ozaki_group_prepare(OzakiPlan &oz, const OzGroupDesc &d, const std::vector<O
                 jt.push_back(j);
             }
         g->n_jobs_t = (int)jt.size();
-        rc = upload_schedule(jt, g->d_jobs_t, g->d_list_t, g->tiles_t, tile);
+        g->pair_t = pair_t_tiles(jt, false, 0);
+        rc = upload_schedule(jt, g->d_jobs_t, g->d_list_t, g->tiles_t, g->pair_t ? kPairTile : kTileN);
         if (rc) return fail(rc);
     } else {
         int64_t joff = 0, loff = 0;
@@ -2206,8 +2236,11 @@ int ozaki_group_prepare(OzakiPlan &oz, const OzGroupDesc &d, const std::vector<O
             p.jt_off = joff;
             p.lt_off = loff;
             p.n_jobs_t = (int)jt.size();
-            rc = upload_schedule(jt, g->d_jobs_t + joff, g->d_list_t + loff, p.tiles_t, tile, &g->split_t, tkb * s * (s + 1) / 2,
-                                 g->pair && g->panels == 1 ? d.split_t : nullptr, d.split_t_bytes);
+            // (one shape for all panels, by the first and largest)
+            void *cut = g->pair && g->panels == 1 ? d.split_t : nullptr;
+            if (&p == &g->pan[0]) g->pair_t = pair_t_tiles(jt, cut != nullptr, tkb * s * (s + 1) / 2);
+            rc = upload_schedule(jt, g->d_jobs_t + joff, g->d_list_t + loff, p.tiles_t, g->pair_t ? kPairTile : kTileN, &g->split_t,
+                                 tkb * s * (s + 1) / 2, g->pair_t ? cut : nullptr, d.split_t_bytes);
             if (rc) return fail(rc);
             joff += p.n_jobs_t;
             loff += p.tiles_t;
@@ -2280,13 +2313,13 @@ void ozaki_group_set_outputs(OzGroup *g, double2 *const *S, double2 *const *H, c
     }
 }
 
-// The T application of the complex forms, on CTA-pair tiles as well: 272 us for 8 atoms, lmax 8, 1501 columns (507
-// on single-CTA tiles), 161 for 2 atoms, lmax 1, 100 columns (207), 602 for 16, lmax 10, 1500 (813).
+// The T application of the complex forms, on CTA-pair tiles or single-CTA ones (pair_t_tiles): 272 us for 8 atoms, lmax 8,
+// 1501 columns (507 on single-CTA tiles), 161 for 2 atoms, lmax 1, 100 columns (207), 602 for 16, lmax 10, 1500 (813).
 // Cut over the idle pairs (the contraction entry): 236 us of the first; 1 atom, lmax 7, 232 columns 184 -> 68, 4 atoms,
 // lmax 8, 400 columns 268 -> 91.
 static cudaError_t launch_t(const OzGroup *g, const OzJob *jobs, int n_jobs, int64_t tiles, const int4 *list, cudaStream_t st) {
-    return g->pair ? launch_pair(g->maps_t, g->s, g->d_err, jobs, n_jobs, tiles, list, nullptr, st, &g->split_t)
-                   : launch_prepared(g->maps_t, g->s, g->d_err, jobs, n_jobs, tiles, list, nullptr, st);
+    return g->pair_t ? launch_pair(g->maps_t, g->s, g->d_err, jobs, n_jobs, tiles, list, nullptr, st, &g->split_t)
+                     : launch_prepared(g->maps_t, g->s, g->d_err, jobs, n_jobs, tiles, list, nullptr, st);
 }
 
 // Events around the S/H launch; under stream capture they become external event-record nodes
