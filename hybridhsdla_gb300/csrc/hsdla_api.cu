@@ -1622,7 +1622,7 @@ void run_groups_flop_one(const hsdla_plan *pl, const hsdla_plan::Group &g, doubl
         const double G = (double)g.ktab.e[q].kp.n_g;
         const double lower = 4.0 * G * (G + 1.0) * Klen;
         // (digit products: the real form's three where the complex form has eight; FP64: the flops of
-        // the complex products that the real ones replace)
+        // the complex products, of which the real ones run 3/8)
         *dom_flop += 2.0 * lower * (g.oz ? sl * (sl + 1) / 2 * (pl->sf ? 0.375 : 1.0) : 1.0);
     }
 }

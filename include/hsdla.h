@@ -121,8 +121,10 @@ typedef struct hsdla_report {
     double ms_tapply;            /* the T-application launches (X = T C, or Z_t = T_t M_t per type), */
     double ms_contract;          /* and the rest (slicing, S/H products, combine) */
     double ms_dominant;          /* device time of the dominant launch: the S/H contraction of the last k-point */
-    double dominant_flop;        /* algorithmic flops of that launch (FP8 digit products for Ozaki, FP64 for plain) */
-    double est_rel_err;          /* Ozaki: relative error predicted by the slice autotuner (0 if not tuned) */
+    double dominant_flop;        /* algorithmic flops of that launch: FP8 digit products for Ozaki; plain FP64: those of
+                                    the complex products, of which the structure-factor form's real ones run 3/8 */
+    double est_rel_err;          /* Ozaki: relative error of the digits' truncation, predicted by the slice autotuner (0 if
+                                    not tuned; the rounding of the sums, ~1e-16, is not part of it) */
     int32_t num_slices;          /* slices used (Ozaki) */
     int32_t num_kpoints;
     int32_t kernel_launches;     /* kernels launched per execution */
@@ -154,7 +156,10 @@ void hsdla_context_destroy(hsdla_context *ctx);
 /* The context's last error message.  With ctx = NULL: the calling thread's last message of the
  * entry point that takes no context, hsdla_zherkx_lower_noalloc ("" after a call that succeeded). */
 const char *hsdla_last_error(const hsdla_context *ctx);
-/* Cap on device bytes the context may allocate (0 = no cap); exceeding it returns HSDLA_ERR_NOMEM. */
+/* Cap on device bytes the context may allocate (0 = no cap); exceeding it returns HSDLA_ERR_NOMEM.  A capped context takes
+ * no memory beyond what a call needs: the digit products of hsdla_contract_ab, hsdla_zherkx_lower and the plugin then do
+ * without the buffers that let idle SMs share a tile, and their sums can differ in the last place from an
+ * uncapped context's. */
 int hsdla_set_mem_cap(hsdla_context *ctx, int64_t bytes);
 
 /* T-matrix preparation for one type: TMat::TMat + zero_nonsph + augment_tmats
